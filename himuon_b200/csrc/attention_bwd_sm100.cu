@@ -22,10 +22,8 @@ namespace {
 
 constexpr int BQ = 64;                               // query positions per streamed sub-block
 constexpr uint32_t Q_HALF = BQ * 128;                // one 64-column half of a sub-block: 8 KB
-constexpr uint32_t Q_TILE = 2 * Q_HALF;              // 16 KB
 constexpr int NST = 4;                               // streamed stages of (Q, dO, lse, delta)
 constexpr uint32_t STAT_BYTES = 2 * BQ * 4;          // lse[64] then delta[64]
-constexpr uint32_t STAGE_BYTES = 2 * Q_TILE + STAT_BYTES;
 // warp 0: TMA producer, warp 1: MMA issue, warps 2-5 and 6-9: two softmax groups of 128 threads (one per TMEM
 // lane) that take alternate sub-blocks, so two warps per scheduler hide each other's MUFU and TMEM latencies
 constexpr int BWD_THREADS = 320;
@@ -50,9 +48,11 @@ __device__ __forceinline__ void bulk_load_1d(void* dst, const void* src, uint32_
 
 }  // namespace
 
+template <int NH>
 __global__ void __launch_bounds__(BWD_THREADS, 1)
 flash_bwd_dkv_t_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                        const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmDO, AttnDev p) {
+  constexpr uint32_t TILE_BYTES = NH * HALF_BYTES, Q_TILE = NH * Q_HALF;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = align_up_1024(smem_raw);
   uint8_t* sK = smem;
@@ -93,23 +93,19 @@ flash_bwd_dkv_t_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     // ------------------------------------------------------------ producer
     if (lane == 0) {
       mbar_expect_tx(&bars->kv_full, 2 * TILE_BYTES);
-      tma_load_4d(sK, &tmK, &bars->kv_full, 0, hk, kb * AT, b);
-      tma_load_4d(sK + HALF_BYTES, &tmK, &bars->kv_full, 64, hk, kb * AT, b);
-      tma_load_4d(sV, &tmV, &bars->kv_full, 0, hk, kb * AT, b);
-      tma_load_4d(sV + HALF_BYTES, &tmV, &bars->kv_full, 64, hk, kb * AT, b);
+      load_head_tile<NH>(sK, HALF_BYTES, &tmK, &bars->kv_full, hk, kb * AT, b);
+      load_head_tile<NH>(sV, HALF_BYTES, &tmV, &bars->kv_full, hk, kb * AT, b);
       for (int it = 0; it < iters; ++it) {
         const int g = it / nsub;
         const int h = h_first + g;
         const int q0 = kb * AT + (it - g * nsub) * BQ;
         const int st = it % NST;
         if (!mbar_wait(&bars->qd_empty[st], ((it / NST) & 1) ^ 1, abort_flag, p.status, 4)) break;
-        mbar_expect_tx(&bars->qd_full[st], STAGE_BYTES);
+        mbar_expect_tx(&bars->qd_full[st], 2 * Q_TILE + STAT_BYTES);
         uint8_t* q_dst = sQ + st * Q_TILE;
         uint8_t* do_dst = sDO + st * Q_TILE;
-        tma_load_4d(q_dst, &tmQ, &bars->qd_full[st], 0, h, q0, b);
-        tma_load_4d(q_dst + Q_HALF, &tmQ, &bars->qd_full[st], 64, h, q0, b);
-        tma_load_4d(do_dst, &tmDO, &bars->qd_full[st], 0, h, q0, b);
-        tma_load_4d(do_dst + Q_HALF, &tmDO, &bars->qd_full[st], 64, h, q0, b);
+        load_head_tile<NH>(q_dst, Q_HALF, &tmQ, &bars->qd_full[st], h, q0, b);
+        load_head_tile<NH>(do_dst, Q_HALF, &tmDO, &bars->qd_full[st], h, q0, b);
         const long long stat_idx = (static_cast<long long>(b) * p.Hq + h) * p.S + q0;
         bulk_load_1d(sStat + st * 2 * BQ, p.lse + stat_idx, BQ * 4, &bars->qd_full[st]);
         bulk_load_1d(sStat + st * 2 * BQ + BQ, p.delta + stat_idx, BQ * 4, &bars->qd_full[st]);
@@ -119,7 +115,7 @@ flash_bwd_dkv_t_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     // ------------------------------------------------------------ MMA issue
     if (lane == 0) {
       constexpr uint32_t idesc_s = umma_idesc_bf16(128, BQ, false, false);
-      constexpr uint32_t idesc_acc = umma_idesc_bf16(128, 128, false, true);
+      constexpr uint32_t idesc_acc = umma_idesc_bf16(128, 64 * NH, false, true);
       const uint32_t k_base = smem_u32(sK), v_base = smem_u32(sV), q_base = smem_u32(sQ), do_base = smem_u32(sDO);
       bool ok = mbar_wait(&bars->kv_full, 0, abort_flag, p.status, 4);
       auto issue_sp = [&](int it) -> bool {
@@ -129,10 +125,10 @@ flash_bwd_dkv_t_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
         // The buffer's previous contents (P^T, dS^T of sub-block it-2) were consumed by MMAs issued earlier, which
         // the tensor core executes in order before these.
 #pragma unroll
-        for (int ks = 0; ks < 8; ++ks)
+        for (int ks = 0; ks < 4 * NH; ++ks)
           umma_ss(tS + buf * BQ, desc_kmajor(k_base, ks), sub_desc_kmajor(q_base + st * Q_TILE, ks), idesc_s, ks > 0 ? 1u : 0u);
 #pragma unroll
-        for (int ks = 0; ks < 8; ++ks)
+        for (int ks = 0; ks < 4 * NH; ++ks)
           umma_ss(tDP + buf * BQ, desc_kmajor(v_base, ks), sub_desc_kmajor(do_base + st * Q_TILE, ks), idesc_s, ks > 0 ? 1u : 0u);
         umma_commit(&bars->s_full[buf]);
         return true;
@@ -209,24 +205,15 @@ flash_bwd_dkv_t_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
       tc_fence_after();
       // group 0 stores dV, group 1 stores dK
       __nv_bfloat16* dst0 = reinterpret_cast<__nv_bfloat16*>(wg == 0 ? p.dv : p.dk) +
-                            (static_cast<long long>(b) * p.S + kv_idx) * (wg == 0 ? p.ld_dv : p.ld_dk) + out_head * HD;
+                            (static_cast<long long>(b) * p.S + kv_idx) * (wg == 0 ? p.ld_dv : p.ld_dk) + out_head * p.hd;
       const uint32_t t_src = (wg == 0 ? tDV : tDK) + lane_off;
       const float out_scale = wg == 0 ? 1.f : p.scale;
 #pragma unroll 1
-      for (int c = 0; c < 4; ++c) {
+      for (int c = 0; c < 2 * NH; ++c) {
         uint32_t v[32];
         tmem_ld32(t_src + c * 32, v);
         tmem_ld_wait();
-        __nv_bfloat16* dst = dst0 + c * 32;
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          uint4 o4;
-          o4.x = pack_bf16x2(__uint_as_float(v[8 * q + 0]) * out_scale, __uint_as_float(v[8 * q + 1]) * out_scale);
-          o4.y = pack_bf16x2(__uint_as_float(v[8 * q + 2]) * out_scale, __uint_as_float(v[8 * q + 3]) * out_scale);
-          o4.z = pack_bf16x2(__uint_as_float(v[8 * q + 4]) * out_scale, __uint_as_float(v[8 * q + 5]) * out_scale);
-          o4.w = pack_bf16x2(__uint_as_float(v[8 * q + 6]) * out_scale, __uint_as_float(v[8 * q + 7]) * out_scale);
-          *reinterpret_cast<uint4*>(dst + q * 8) = o4;
-        }
+        store_head32(dst0, c * 32, p.hd, v, out_scale);
       }
     }
   }
@@ -251,9 +238,11 @@ struct DqBars {
   float delta[AT];
 };
 
+template <int NH>
 __global__ void __launch_bounds__(BWD_THREADS, 1)
 flash_bwd_dq_t_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                       const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmDO, AttnDev p) {
+  constexpr uint32_t TILE_BYTES = NH * HALF_BYTES, Q_TILE = NH * Q_HALF;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = align_up_1024(smem_raw);
   uint8_t* sQ = smem;
@@ -288,26 +277,22 @@ flash_bwd_dq_t_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   if (warp == 0) {
     if (lane == 0) {
       mbar_expect_tx(&bars->qd_full, 2 * TILE_BYTES);
-      tma_load_4d(sQ, &tmQ, &bars->qd_full, 0, h, qb * AT, b);
-      tma_load_4d(sQ + HALF_BYTES, &tmQ, &bars->qd_full, 64, h, qb * AT, b);
-      tma_load_4d(sDO, &tmDO, &bars->qd_full, 0, h, qb * AT, b);
-      tma_load_4d(sDO + HALF_BYTES, &tmDO, &bars->qd_full, 64, h, qb * AT, b);
+      load_head_tile<NH>(sQ, HALF_BYTES, &tmQ, &bars->qd_full, h, qb * AT, b);
+      load_head_tile<NH>(sDO, HALF_BYTES, &tmDO, &bars->qd_full, h, qb * AT, b);
       for (int j = 0; j < nkv; ++j) {
         const int st = j % NST;
         if (!mbar_wait(&bars->kv_empty[st], ((j / NST) & 1) ^ 1, abort_flag, p.status, 4)) break;
         mbar_expect_tx(&bars->kv_full[st], 2 * Q_TILE);
         uint8_t* k_dst = sK + st * Q_TILE;
         uint8_t* v_dst = sV + st * Q_TILE;
-        tma_load_4d(k_dst, &tmK, &bars->kv_full[st], 0, hk, j * BQ, b);
-        tma_load_4d(k_dst + Q_HALF, &tmK, &bars->kv_full[st], 64, hk, j * BQ, b);
-        tma_load_4d(v_dst, &tmV, &bars->kv_full[st], 0, hk, j * BQ, b);
-        tma_load_4d(v_dst + Q_HALF, &tmV, &bars->kv_full[st], 64, hk, j * BQ, b);
+        load_head_tile<NH>(k_dst, Q_HALF, &tmK, &bars->kv_full[st], hk, j * BQ, b);
+        load_head_tile<NH>(v_dst, Q_HALF, &tmV, &bars->kv_full[st], hk, j * BQ, b);
       }
     }
   } else if (warp == 1) {
     if (lane == 0) {
       constexpr uint32_t idesc_s = umma_idesc_bf16(128, BQ, false, false);
-      constexpr uint32_t idesc_acc = umma_idesc_bf16(128, 128, false, true);
+      constexpr uint32_t idesc_acc = umma_idesc_bf16(128, 64 * NH, false, true);
       const uint32_t q_base = smem_u32(sQ), do_base = smem_u32(sDO), k_base = smem_u32(sK), v_base = smem_u32(sV);
       bool ok = mbar_wait(&bars->qd_full, 0, abort_flag, p.status, 4);
       auto issue_sp = [&](int j) -> bool {
@@ -315,10 +300,10 @@ flash_bwd_dq_t_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         if (!mbar_wait(&bars->kv_full[st], (j / NST) & 1, abort_flag, p.status, 4)) return false;
         tc_fence_after();
 #pragma unroll
-        for (int ks = 0; ks < 8; ++ks)
+        for (int ks = 0; ks < 4 * NH; ++ks)
           umma_ss(tS + buf * BQ, desc_kmajor(q_base, ks), sub_desc_kmajor(k_base + st * Q_TILE, ks), idesc_s, ks > 0 ? 1u : 0u);
 #pragma unroll
-        for (int ks = 0; ks < 8; ++ks)
+        for (int ks = 0; ks < 4 * NH; ++ks)
           umma_ss(tDP + buf * BQ, desc_kmajor(do_base, ks), sub_desc_kmajor(v_base + st * Q_TILE, ks), idesc_s, ks > 0 ? 1u : 0u);
         umma_commit(&bars->s_full[buf]);
         return true;
@@ -344,16 +329,9 @@ flash_bwd_dq_t_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     const long long stat_idx = (static_cast<long long>(b) * p.Hq + h) * p.S + q_idx;
     const float lse2 = p.lse[stat_idx];
     if (wg == 0) {
-      float d = 0.f;
-      const __nv_bfloat16* op = reinterpret_cast<const __nv_bfloat16*>(p.o_in) + (static_cast<long long>(b) * p.S + q_idx) * p.ld_o + h * HD;
-      const __nv_bfloat16* gp = reinterpret_cast<const __nv_bfloat16*>(p.d_o) + (static_cast<long long>(b) * p.S + q_idx) * p.ld_do + h * HD;
-#pragma unroll 4
-      for (int c = 0; c < 16; ++c) {
-        const uint4 a = reinterpret_cast<const uint4*>(op)[c], g = reinterpret_cast<const uint4*>(gp)[c];
-        const uint32_t aw[4] = {a.x, a.y, a.z, a.w}, gw[4] = {g.x, g.y, g.z, g.w};
-#pragma unroll
-        for (int q = 0; q < 4; ++q) d += bf16_lo(aw[q]) * bf16_lo(gw[q]) + bf16_hi(aw[q]) * bf16_hi(gw[q]);
-      }
+      const __nv_bfloat16* op = reinterpret_cast<const __nv_bfloat16*>(p.o_in) + (static_cast<long long>(b) * p.S + q_idx) * p.ld_o + h * p.hd;
+      const __nv_bfloat16* gp = reinterpret_cast<const __nv_bfloat16*>(p.d_o) + (static_cast<long long>(b) * p.S + q_idx) * p.ld_do + h * p.hd;
+      const float d = row_delta(op, gp, p.hd);
       p.delta[stat_idx] = d;
       bars->delta[row] = d;
     }
@@ -389,22 +367,14 @@ flash_bwd_dq_t_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     }
     if (ok && mbar_wait(&bars->acc_done, 0, abort_flag, p.status, 4)) {
       tc_fence_after();
-      // each group stores one 64-column half of the dQ rows
-      __nv_bfloat16* dqp = reinterpret_cast<__nv_bfloat16*>(p.dq) + (static_cast<long long>(b) * p.S + q_idx) * p.ld_dq + h * HD + wg * 64;
+      // each group stores one half of the dQ columns; dS was left unscaled, so the softmax scale lands here
+      __nv_bfloat16* dqp = reinterpret_cast<__nv_bfloat16*>(p.dq) + (static_cast<long long>(b) * p.S + q_idx) * p.ld_dq + h * p.hd;
 #pragma unroll 1
-      for (int c = 0; c < 2; ++c) {
+      for (int c = wg * NH; c < (wg + 1) * NH; ++c) {
         uint32_t v[32];
-        tmem_ld32(tDQ + lane_off + wg * 64 + c * 32, v);
+        tmem_ld32(tDQ + lane_off + c * 32, v);
         tmem_ld_wait();
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          uint4 o4;                                      // dS was left unscaled: the softmax scale lands here
-          o4.x = pack_bf16x2(__uint_as_float(v[8 * q + 0]) * p.scale, __uint_as_float(v[8 * q + 1]) * p.scale);
-          o4.y = pack_bf16x2(__uint_as_float(v[8 * q + 2]) * p.scale, __uint_as_float(v[8 * q + 3]) * p.scale);
-          o4.z = pack_bf16x2(__uint_as_float(v[8 * q + 4]) * p.scale, __uint_as_float(v[8 * q + 5]) * p.scale);
-          o4.w = pack_bf16x2(__uint_as_float(v[8 * q + 6]) * p.scale, __uint_as_float(v[8 * q + 7]) * p.scale);
-          *reinterpret_cast<uint4*>(dqp + c * 32 + q * 8) = o4;
-        }
+        store_head32(dqp, c * 32, p.hd, v, p.scale);
       }
     }
   }
@@ -424,24 +394,34 @@ bool flash_bwd_dkv_t_supported(const AttnArgs& a) {
 
 bool flash_bwd_dq_t_supported(const AttnArgs& a) { return flash_bwd_dkv_t_supported(a); }
 
+template <int NH>
+static void launch_dkv_t(const AttnArgs& a, const AttnDev& p, int heads_y, cudaStream_t s) {
+  constexpr size_t SMEM = 1024 + 2 * NH * HALF_BYTES + 2 * NST * NH * Q_HALF + NST * STAT_BYTES + sizeof(DkvBars) + 64;
+  static bool attr = false;
+  if (!attr) { cudaFuncSetAttribute(flash_bwd_dkv_t_kernel<NH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM); attr = true; }
+  const CUtensorMap tq = head_tmap(a.q, a.B, a.S, a.Hq, a.hd, a.ld_q, BQ), tk = head_tmap(a.k, a.B, a.S, a.Hkv, a.hd, a.ld_k),
+                    tv = head_tmap(a.v, a.B, a.S, a.Hkv, a.hd, a.ld_v), tdo = head_tmap(a.d_o, a.B, a.S, a.Hq, a.hd, a.ld_do, BQ);
+  flash_bwd_dkv_t_kernel<NH><<<dim3(p.nblk, heads_y, a.B), BWD_THREADS, SMEM, s>>>(tq, tk, tv, tdo, p);
+}
 // `p` carries the output pointers and the split_heads flag chosen by the caller; the grid's y extent is the number of
 // query heads (split_heads) or KV heads.
 void flash_bwd_dkv_t(const AttnArgs& a, const AttnDev& p, int heads_y, cudaStream_t s) {
-  constexpr size_t SMEM = 1024 + 2 * TILE_BYTES + 2 * NST * Q_TILE + NST * STAT_BYTES + sizeof(DkvBars) + 64;
-  static bool attr = false;
-  if (!attr) { cudaFuncSetAttribute(flash_bwd_dkv_t_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM); attr = true; }
-  const CUtensorMap tq = head_tmap(a.q, a.B, a.S, a.Hq, a.ld_q, BQ), tk = head_tmap(a.k, a.B, a.S, a.Hkv, a.ld_k),
-                    tv = head_tmap(a.v, a.B, a.S, a.Hkv, a.ld_v), tdo = head_tmap(a.d_o, a.B, a.S, a.Hq, a.ld_do, BQ);
-  flash_bwd_dkv_t_kernel<<<dim3(p.nblk, heads_y, a.B), BWD_THREADS, SMEM, s>>>(tq, tk, tv, tdo, p);
+  if (head_halves(a.hd) == 1) launch_dkv_t<1>(a, p, heads_y, s);
+  else launch_dkv_t<2>(a, p, heads_y, s);
 }
 
-void flash_bwd_dq_t(const AttnArgs& a, const AttnDev& p, cudaStream_t s) {
-  constexpr size_t SMEM = 1024 + 2 * TILE_BYTES + 2 * NST * Q_TILE + sizeof(DqBars) + 64;
+template <int NH>
+static void launch_dq_t(const AttnArgs& a, const AttnDev& p, cudaStream_t s) {
+  constexpr size_t SMEM = 1024 + 2 * NH * HALF_BYTES + 2 * NST * NH * Q_HALF + sizeof(DqBars) + 64;
   static bool attr = false;
-  if (!attr) { cudaFuncSetAttribute(flash_bwd_dq_t_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM); attr = true; }
-  const CUtensorMap tq = head_tmap(a.q, a.B, a.S, a.Hq, a.ld_q), tk = head_tmap(a.k, a.B, a.S, a.Hkv, a.ld_k, BQ),
-                    tv = head_tmap(a.v, a.B, a.S, a.Hkv, a.ld_v, BQ), tdo = head_tmap(a.d_o, a.B, a.S, a.Hq, a.ld_do);
-  flash_bwd_dq_t_kernel<<<dim3(p.nblk, a.Hq, a.B), BWD_THREADS, SMEM, s>>>(tq, tk, tv, tdo, p);
+  if (!attr) { cudaFuncSetAttribute(flash_bwd_dq_t_kernel<NH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM); attr = true; }
+  const CUtensorMap tq = head_tmap(a.q, a.B, a.S, a.Hq, a.hd, a.ld_q), tk = head_tmap(a.k, a.B, a.S, a.Hkv, a.hd, a.ld_k, BQ),
+                    tv = head_tmap(a.v, a.B, a.S, a.Hkv, a.hd, a.ld_v, BQ), tdo = head_tmap(a.d_o, a.B, a.S, a.Hq, a.hd, a.ld_do);
+  flash_bwd_dq_t_kernel<NH><<<dim3(p.nblk, a.Hq, a.B), BWD_THREADS, SMEM, s>>>(tq, tk, tv, tdo, p);
+}
+void flash_bwd_dq_t(const AttnArgs& a, const AttnDev& p, cudaStream_t s) {
+  if (head_halves(a.hd) == 1) launch_dq_t<1>(a, p, s);
+  else launch_dq_t<2>(a, p, s);
 }
 
 }  // namespace himuon

@@ -11,7 +11,6 @@ namespace himuon {
 
 constexpr int BKV = 64;                              // KV positions per block
 constexpr uint32_t KV_HALF = BKV * 128;              // one 64-column half of a K or V block: 8 KB
-constexpr uint32_t KV_TILE = 2 * KV_HALF;            // 16 KB
 constexpr uint32_t P_BYTES = AT * BKV * 2;           // probabilities / dS of one block: 128 x 64 bf16 = 16 KB
 
 __device__ __forceinline__ uint64_t kv_desc_kmajor(uint32_t base, int ks) {   // K block as the K-major B operand of Q K^T
@@ -40,9 +39,11 @@ struct Fwd64TBars {
   int abort_flag;
 };
 
+template <int NH>
 __global__ void __launch_bounds__(192, 2)
 flash_fwd64_t_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                      const __grid_constant__ CUtensorMap tmV, AttnDev p) {
+  constexpr uint32_t TILE_BYTES = NH * HALF_BYTES, KV_TILE = NH * KV_HALF;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = align_up_1024(smem_raw);
   uint8_t* sQ = smem;                          // 32 KB
@@ -81,25 +82,22 @@ flash_fwd64_t_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   if (warp == 0) {
     if (lane == 0) {
       mbar_expect_tx(&bars->q_full, TILE_BYTES);
-      tma_load_4d(sQ, &tmQ, &bars->q_full, 0, h, qb * AT, b);
-      tma_load_4d(sQ + HALF_BYTES, &tmQ, &bars->q_full, 64, h, qb * AT, b);
+      load_head_tile<NH>(sQ, HALF_BYTES, &tmQ, &bars->q_full, h, qb * AT, b);
       for (int j = 0; j < nkv; ++j) {
         const int st = j & 1;
         const uint32_t par = ((j >> 1) & 1) ^ 1;
         if (!mbar_wait(&bars->k_empty[st], par, abort_flag, p.status, 4)) break;
         mbar_expect_tx(&bars->k_full[st], KV_TILE);
-        tma_load_4d(sK + st * KV_TILE, &tmK, &bars->k_full[st], 0, hk, j * BKV, b);
-        tma_load_4d(sK + st * KV_TILE + KV_HALF, &tmK, &bars->k_full[st], 64, hk, j * BKV, b);
+        load_head_tile<NH>(sK + st * KV_TILE, KV_HALF, &tmK, &bars->k_full[st], hk, j * BKV, b);
         if (!mbar_wait(&bars->v_empty[st], par, abort_flag, p.status, 4)) break;
         mbar_expect_tx(&bars->v_full[st], KV_TILE);
-        tma_load_4d(sV + st * KV_TILE, &tmV, &bars->v_full[st], 0, hk, j * BKV, b);
-        tma_load_4d(sV + st * KV_TILE + KV_HALF, &tmV, &bars->v_full[st], 64, hk, j * BKV, b);
+        load_head_tile<NH>(sV + st * KV_TILE, KV_HALF, &tmV, &bars->v_full[st], hk, j * BKV, b);
       }
     }
   } else if (warp == 1) {
     if (lane == 0) {
       constexpr uint32_t idesc_s = umma_idesc_bf16(128, BKV, false, false);
-      constexpr uint32_t idesc_pv = umma_idesc_bf16(128, 128, false, true);
+      constexpr uint32_t idesc_pv = umma_idesc_bf16(128, 64 * NH, false, true);
       const uint32_t q_base = smem_u32(sQ), v_base = smem_u32(sV);
       bool ok = mbar_wait(&bars->q_full, 0, abort_flag, p.status, 4);
       auto issue_s = [&](int j) -> bool {
@@ -110,7 +108,7 @@ flash_fwd64_t_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         // P(j-2)·V MMAs were issued earlier, which the tensor core executes in order before these
         const uint32_t k_base = smem_u32(sK + st * KV_TILE);
 #pragma unroll
-        for (int ks = 0; ks < 8; ++ks)
+        for (int ks = 0; ks < 4 * NH; ++ks)
           umma_ss(tS0 + st * BKV, desc_kmajor(q_base, ks), kv_desc_kmajor(k_base, ks), idesc_s, ks > 0 ? 1u : 0u);
         umma_commit(&bars->k_empty[st]);
         umma_commit(&bars->s_full[st]);
@@ -170,7 +168,7 @@ flash_fwd64_t_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         if (!mbar_wait(&bars->o_done, (j - 1) & 1, abort_flag, p.status, 4)) { ok = false; break; }
         tc_fence_after();
 #pragma unroll 1
-        for (int c = 0; c < 4; ++c) {
+        for (int c = 0; c < 2 * NH; ++c) {
           uint32_t v[32];
           tmem_ld32(tO + lane_off + c * 32, v);
           tmem_ld_wait();
@@ -199,23 +197,13 @@ flash_fwd64_t_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       tc_fence_after();
       const float inv = 1.f / l;
       const bool row_ok = q_idx < p.S;
-      __nv_bfloat16* op = reinterpret_cast<__nv_bfloat16*>(p.o) + (static_cast<long long>(b) * p.S + q_idx) * p.ld_o + h * HD;
+      __nv_bfloat16* op = reinterpret_cast<__nv_bfloat16*>(p.o) + (static_cast<long long>(b) * p.S + q_idx) * p.ld_o + h * p.hd;
 #pragma unroll 1
-      for (int c = 0; c < 4; ++c) {
+      for (int c = 0; c < 2 * NH; ++c) {
         uint32_t v[32];
         tmem_ld32(tO + lane_off + c * 32, v);
         tmem_ld_wait();
-        if (row_ok) {
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            uint4 o4;
-            o4.x = pack_bf16x2(__uint_as_float(v[8 * q + 0]) * inv, __uint_as_float(v[8 * q + 1]) * inv);
-            o4.y = pack_bf16x2(__uint_as_float(v[8 * q + 2]) * inv, __uint_as_float(v[8 * q + 3]) * inv);
-            o4.z = pack_bf16x2(__uint_as_float(v[8 * q + 4]) * inv, __uint_as_float(v[8 * q + 5]) * inv);
-            o4.w = pack_bf16x2(__uint_as_float(v[8 * q + 6]) * inv, __uint_as_float(v[8 * q + 7]) * inv);
-            *reinterpret_cast<uint4*>(op + c * 32 + q * 8) = o4;
-          }
-        }
+        if (row_ok) store_head32(op, c * 32, p.hd, v, inv);
       }
       if (row_ok) p.lse[(static_cast<long long>(b) * p.Hq + h) * p.S + q_idx] = m_used + log2f(l);   // base-2 log-sum-exp of the scaled scores
     }
@@ -231,9 +219,11 @@ flash_fwd64_t_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
 // ================================================================================================ backward: dQ
 // CTA = (query block, head, batch).  Resident: Q, dO.  Streamed: K_j, V_j (64 positions).  dS reuses V's shared
 // memory once dP = dO V^T has consumed V.  TMEM: S (64) | dP (64) | dQ (128).
+template <int NH>
 __global__ void __launch_bounds__(192, 2)
 flash_bwd_dq64_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                       const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmDO, AttnDev p) {
+  constexpr uint32_t TILE_BYTES = NH * HALF_BYTES, KV_TILE = NH * KV_HALF;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = align_up_1024(smem_raw);
   uint8_t* sQ = smem;
@@ -241,7 +231,7 @@ flash_bwd_dq64_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   uint8_t* sK = smem + 2 * TILE_BYTES;
   uint8_t* sV = sK + KV_TILE;
   uint8_t* sDS = sV;                                    // alias (see above)
-  BwdBars* bars = reinterpret_cast<BwdBars*>(sV + KV_TILE);
+  BwdBars* bars = reinterpret_cast<BwdBars*>(sV + (KV_TILE > P_BYTES ? KV_TILE : P_BYTES));
   volatile int* abort_flag = &bars->abort_flag;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -270,23 +260,19 @@ flash_bwd_dq64_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   if (warp == 0) {
     if (lane == 0) {
       mbar_expect_tx(&bars->a_full, 2 * TILE_BYTES);
-      tma_load_4d(sQ, &tmQ, &bars->a_full, 0, h, qb * AT, b);
-      tma_load_4d(sQ + HALF_BYTES, &tmQ, &bars->a_full, 64, h, qb * AT, b);
-      tma_load_4d(sDO, &tmDO, &bars->a_full, 0, h, qb * AT, b);
-      tma_load_4d(sDO + HALF_BYTES, &tmDO, &bars->a_full, 64, h, qb * AT, b);
+      load_head_tile<NH>(sQ, HALF_BYTES, &tmQ, &bars->a_full, h, qb * AT, b);
+      load_head_tile<NH>(sDO, HALF_BYTES, &tmDO, &bars->a_full, h, qb * AT, b);
       for (int j = 0; j < nkv; ++j) {
         if (!mbar_wait(&bars->b_empty, (j & 1) ^ 1, abort_flag, p.status, 4)) break;
         mbar_expect_tx(&bars->b_full, 2 * KV_TILE);
-        tma_load_4d(sK, &tmK, &bars->b_full, 0, hk, j * BKV, b);
-        tma_load_4d(sK + KV_HALF, &tmK, &bars->b_full, 64, hk, j * BKV, b);
-        tma_load_4d(sV, &tmV, &bars->b_full, 0, hk, j * BKV, b);
-        tma_load_4d(sV + KV_HALF, &tmV, &bars->b_full, 64, hk, j * BKV, b);
+        load_head_tile<NH>(sK, KV_HALF, &tmK, &bars->b_full, hk, j * BKV, b);
+        load_head_tile<NH>(sV, KV_HALF, &tmV, &bars->b_full, hk, j * BKV, b);
       }
     }
   } else if (warp == 1) {
     if (lane == 0) {
       constexpr uint32_t idesc_kk = umma_idesc_bf16(128, BKV, false, false);
-      constexpr uint32_t idesc_kmn = umma_idesc_bf16(128, 128, false, true);
+      constexpr uint32_t idesc_kmn = umma_idesc_bf16(128, 64 * NH, false, true);
       const uint32_t q_base = smem_u32(sQ), do_base = smem_u32(sDO), k_base = smem_u32(sK), v_base = smem_u32(sV),
                      ds_base = smem_u32(sDS);
       bool ok = mbar_wait(&bars->a_full, 0, abort_flag, p.status, 4);
@@ -294,9 +280,9 @@ flash_bwd_dq64_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         if (!mbar_wait(&bars->b_full, j & 1, abort_flag, p.status, 4)) break;
         tc_fence_after();
 #pragma unroll
-        for (int ks = 0; ks < 8; ++ks) umma_ss(tS, desc_kmajor(q_base, ks), kv_desc_kmajor(k_base, ks), idesc_kk, ks > 0 ? 1u : 0u);
+        for (int ks = 0; ks < 4 * NH; ++ks) umma_ss(tS, desc_kmajor(q_base, ks), kv_desc_kmajor(k_base, ks), idesc_kk, ks > 0 ? 1u : 0u);
 #pragma unroll
-        for (int ks = 0; ks < 8; ++ks) umma_ss(tDP, desc_kmajor(do_base, ks), kv_desc_kmajor(v_base, ks), idesc_kk, ks > 0 ? 1u : 0u);
+        for (int ks = 0; ks < 4 * NH; ++ks) umma_ss(tDP, desc_kmajor(do_base, ks), kv_desc_kmajor(v_base, ks), idesc_kk, ks > 0 ? 1u : 0u);
         umma_commit(&bars->sp_full);
         if (!mbar_wait(&bars->ds_ready, j & 1, abort_flag, p.status, 4)) break;
         tc_fence_after();
@@ -316,15 +302,9 @@ flash_bwd_dq64_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     float lse2 = 0.f, delta = 0.f;
     if (row_ok) {
       lse2 = p.lse[stat_idx];
-      const __nv_bfloat16* op = reinterpret_cast<const __nv_bfloat16*>(p.o_in) + (static_cast<long long>(b) * p.S + q_idx) * p.ld_o + h * HD;
-      const __nv_bfloat16* gp = reinterpret_cast<const __nv_bfloat16*>(p.d_o) + (static_cast<long long>(b) * p.S + q_idx) * p.ld_do + h * HD;
-#pragma unroll 4
-      for (int c = 0; c < 16; ++c) {
-        const uint4 a = reinterpret_cast<const uint4*>(op)[c], g = reinterpret_cast<const uint4*>(gp)[c];
-        const uint32_t aw[4] = {a.x, a.y, a.z, a.w}, gw[4] = {g.x, g.y, g.z, g.w};
-#pragma unroll
-        for (int q = 0; q < 4; ++q) delta += bf16_lo(aw[q]) * bf16_lo(gw[q]) + bf16_hi(aw[q]) * bf16_hi(gw[q]);
-      }
+      const __nv_bfloat16* op = reinterpret_cast<const __nv_bfloat16*>(p.o_in) + (static_cast<long long>(b) * p.S + q_idx) * p.ld_o + h * p.hd;
+      const __nv_bfloat16* gp = reinterpret_cast<const __nv_bfloat16*>(p.d_o) + (static_cast<long long>(b) * p.S + q_idx) * p.ld_do + h * p.hd;
+      delta = row_delta(op, gp, p.hd);
       p.delta[stat_idx] = delta;
     }
     bool ok = true;
@@ -360,23 +340,13 @@ flash_bwd_dq64_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     }
     if (ok && mbar_wait(&bars->acc_done, (nkv - 1) & 1, abort_flag, p.status, 4)) {
       tc_fence_after();
-      __nv_bfloat16* dqp = reinterpret_cast<__nv_bfloat16*>(p.dq) + (static_cast<long long>(b) * p.S + q_idx) * p.ld_dq + h * HD;
+      __nv_bfloat16* dqp = reinterpret_cast<__nv_bfloat16*>(p.dq) + (static_cast<long long>(b) * p.S + q_idx) * p.ld_dq + h * p.hd;
 #pragma unroll 1
-      for (int c = 0; c < 4; ++c) {
+      for (int c = 0; c < 2 * NH; ++c) {
         uint32_t v[32];
         tmem_ld32(tDQ + lane_off + c * 32, v);
         tmem_ld_wait();
-        if (row_ok) {
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            uint4 o4;
-            o4.x = pack_bf16x2(__uint_as_float(v[8 * q + 0]), __uint_as_float(v[8 * q + 1]));
-            o4.y = pack_bf16x2(__uint_as_float(v[8 * q + 2]), __uint_as_float(v[8 * q + 3]));
-            o4.z = pack_bf16x2(__uint_as_float(v[8 * q + 4]), __uint_as_float(v[8 * q + 5]));
-            o4.w = pack_bf16x2(__uint_as_float(v[8 * q + 6]), __uint_as_float(v[8 * q + 7]));
-            *reinterpret_cast<uint4*>(dqp + c * 32 + q * 8) = o4;
-          }
-        }
+        if (row_ok) store_head32(dqp, c * 32, p.hd, v, 1.f);
       }
     }
   }
@@ -392,6 +362,7 @@ flash_bwd_dq64_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
 static AttnDev make_dev(const AttnArgs& a) {
   AttnDev p{};
   p.o = a.o; p.lse = a.lse; p.delta = a.delta; p.o_in = a.o; p.d_o = a.d_o; p.dq = a.dq; p.dk = a.dk; p.dv = a.dv;
+  p.hd = a.hd;
   p.B = a.B; p.S = a.S; p.Hq = a.Hq; p.Hkv = a.Hkv;
   p.ld_o = a.ld_o; p.ld_do = a.ld_do; p.ld_dq = a.ld_dq; p.ld_dk = a.ld_dk; p.ld_dv = a.ld_dv;
   p.nblk = (a.S + AT - 1) / AT;
@@ -400,27 +371,37 @@ static AttnDev make_dev(const AttnArgs& a) {
   return p;
 }
 
-void flash_fwd_kv64(const AttnArgs& a, cudaStream_t s) {
-  constexpr size_t SMEM = 1024 + TILE_BYTES + 3 * KV_TILE + P_BYTES + 256;
+template <int NH>
+static void launch_fwd(const AttnArgs& a, cudaStream_t s) {
+  constexpr size_t SMEM = 1024 + NH * HALF_BYTES + 4 * NH * KV_HALF + 256;
   static bool attr = false;
   if (!attr) {
-    cudaFuncSetAttribute(flash_fwd64_t_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM);
+    cudaFuncSetAttribute(flash_fwd64_t_kernel<NH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM);
     attr = true;
   }
   const AttnDev p = make_dev(a);
-  const CUtensorMap tq = head_tmap(a.q, a.B, a.S, a.Hq, a.ld_q), tk = head_tmap(a.k, a.B, a.S, a.Hkv, a.ld_k, BKV),
-                    tv = head_tmap(a.v, a.B, a.S, a.Hkv, a.ld_v, BKV);
-  flash_fwd64_t_kernel<<<dim3(p.nblk, a.Hq, a.B), 192, SMEM, s>>>(tq, tk, tv, p);
+  const CUtensorMap tq = head_tmap(a.q, a.B, a.S, a.Hq, a.hd, a.ld_q), tk = head_tmap(a.k, a.B, a.S, a.Hkv, a.hd, a.ld_k, BKV),
+                    tv = head_tmap(a.v, a.B, a.S, a.Hkv, a.hd, a.ld_v, BKV);
+  flash_fwd64_t_kernel<NH><<<dim3(p.nblk, a.Hq, a.B), 192, SMEM, s>>>(tq, tk, tv, p);
+}
+void flash_fwd_kv64(const AttnArgs& a, cudaStream_t s) {
+  if (head_halves(a.hd) == 1) launch_fwd<1>(a, s);
+  else launch_fwd<2>(a, s);
 }
 
-void flash_bwd_dq_kv64(const AttnArgs& a, cudaStream_t s) {
-  constexpr size_t SMEM = 1024 + 2 * TILE_BYTES + 2 * KV_TILE + 256;
+template <int NH>
+static void launch_dq64(const AttnArgs& a, cudaStream_t s) {
+  constexpr size_t SMEM = 1024 + 2 * NH * HALF_BYTES + KV_HALF * NH + (NH * KV_HALF > P_BYTES ? NH * KV_HALF : P_BYTES) + 256;
   static bool attr = false;
-  if (!attr) { cudaFuncSetAttribute(flash_bwd_dq64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM); attr = true; }
+  if (!attr) { cudaFuncSetAttribute(flash_bwd_dq64_kernel<NH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM); attr = true; }
   const AttnDev p = make_dev(a);
-  const CUtensorMap tq = head_tmap(a.q, a.B, a.S, a.Hq, a.ld_q), tk = head_tmap(a.k, a.B, a.S, a.Hkv, a.ld_k, BKV),
-                    tv = head_tmap(a.v, a.B, a.S, a.Hkv, a.ld_v, BKV), tdo = head_tmap(a.d_o, a.B, a.S, a.Hq, a.ld_do);
-  flash_bwd_dq64_kernel<<<dim3(p.nblk, a.Hq, a.B), 192, SMEM, s>>>(tq, tk, tv, tdo, p);
+  const CUtensorMap tq = head_tmap(a.q, a.B, a.S, a.Hq, a.hd, a.ld_q), tk = head_tmap(a.k, a.B, a.S, a.Hkv, a.hd, a.ld_k, BKV),
+                    tv = head_tmap(a.v, a.B, a.S, a.Hkv, a.hd, a.ld_v, BKV), tdo = head_tmap(a.d_o, a.B, a.S, a.Hq, a.hd, a.ld_do);
+  flash_bwd_dq64_kernel<NH><<<dim3(p.nblk, a.Hq, a.B), 192, SMEM, s>>>(tq, tk, tv, tdo, p);
+}
+void flash_bwd_dq_kv64(const AttnArgs& a, cudaStream_t s) {
+  if (head_halves(a.hd) == 1) launch_dq64<1>(a, s);
+  else launch_dq64<2>(a, s);
 }
 
 }  // namespace himuon

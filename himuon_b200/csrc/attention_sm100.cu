@@ -1,4 +1,4 @@
-// Causal grouped-query flash attention for head_dim 128 on sm_100a: the host entry points (flash_attn_fwd,
+// Causal grouped-query flash attention for head widths up to 128 on sm_100a: the host entry points (flash_attn_fwd,
 // flash_attn_bwd) and the dK/dV kernel for sequence lengths that are not a multiple of 128.
 //
 // Every score / value product runs on tcgen05 tensor cores with TMEM accumulators; Q, K, V and dO tiles arrive by
@@ -17,9 +17,11 @@ namespace himuon {
 // ================================================================================================ backward: dK, dV
 // CTA = (KV block, KV head, batch).  Resident: K_j, V_j.  Streamed: Q_i, dO_i over (group head, query block).
 // TMEM: S | dP | dV | dK (128 columns each).
+template <int NH>
 __global__ void __launch_bounds__(192, 1)
 flash_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                      const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmDO, AttnDev p) {
+  constexpr uint32_t TILE_BYTES = NH * HALF_BYTES;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = align_up_1024(smem_raw);
   uint8_t* sK = smem;
@@ -27,8 +29,8 @@ flash_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   uint8_t* sQ = smem + 2 * TILE_BYTES;
   uint8_t* sDO = smem + 3 * TILE_BYTES;
   uint8_t* sP = smem + 4 * TILE_BYTES;
-  uint8_t* sDS = smem + 5 * TILE_BYTES;
-  BwdBars* bars = reinterpret_cast<BwdBars*>(smem + 6 * TILE_BYTES);
+  uint8_t* sDS = sP + 2 * HALF_BYTES;                 // P and dS are 128 x 128 whatever the head width
+  BwdBars* bars = reinterpret_cast<BwdBars*>(sDS + 2 * HALF_BYTES);
   volatile int* abort_flag = &bars->abort_flag;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -61,25 +63,21 @@ flash_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   if (warp == 0) {
     if (lane == 0) {
       mbar_expect_tx(&bars->a_full, 2 * TILE_BYTES);
-      tma_load_4d(sK, &tmK, &bars->a_full, 0, hk, kb * AT, b);
-      tma_load_4d(sK + HALF_BYTES, &tmK, &bars->a_full, 64, hk, kb * AT, b);
-      tma_load_4d(sV, &tmV, &bars->a_full, 0, hk, kb * AT, b);
-      tma_load_4d(sV + HALF_BYTES, &tmV, &bars->a_full, 64, hk, kb * AT, b);
+      load_head_tile<NH>(sK, HALF_BYTES, &tmK, &bars->a_full, hk, kb * AT, b);
+      load_head_tile<NH>(sV, HALF_BYTES, &tmV, &bars->a_full, hk, kb * AT, b);
       for (int it = 0; it < iters; ++it) {
         const int g = it / nq, qi = kb + (it - g * nq);
         const int h = h_first + g;
         if (!mbar_wait(&bars->b_empty, (it & 1) ^ 1, abort_flag, p.status, 4)) break;
         mbar_expect_tx(&bars->b_full, 2 * TILE_BYTES);
-        tma_load_4d(sQ, &tmQ, &bars->b_full, 0, h, qi * AT, b);
-        tma_load_4d(sQ + HALF_BYTES, &tmQ, &bars->b_full, 64, h, qi * AT, b);
-        tma_load_4d(sDO, &tmDO, &bars->b_full, 0, h, qi * AT, b);
-        tma_load_4d(sDO + HALF_BYTES, &tmDO, &bars->b_full, 64, h, qi * AT, b);
+        load_head_tile<NH>(sQ, HALF_BYTES, &tmQ, &bars->b_full, h, qi * AT, b);
+        load_head_tile<NH>(sDO, HALF_BYTES, &tmDO, &bars->b_full, h, qi * AT, b);
       }
     }
   } else if (warp == 1) {
     if (lane == 0) {
       constexpr uint32_t idesc_kk = umma_idesc_bf16(128, 128, false, false);
-      constexpr uint32_t idesc_mm = umma_idesc_bf16(128, 128, true, true);
+      constexpr uint32_t idesc_mm = umma_idesc_bf16(128, 64 * NH, true, true);
       const uint32_t q_base = smem_u32(sQ), do_base = smem_u32(sDO), k_base = smem_u32(sK), v_base = smem_u32(sV),
                      p_base = smem_u32(sP), ds_base = smem_u32(sDS);
       bool ok = mbar_wait(&bars->a_full, 0, abort_flag, p.status, 4);
@@ -87,9 +85,9 @@ flash_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         if (!mbar_wait(&bars->b_full, it & 1, abort_flag, p.status, 4)) break;
         tc_fence_after();
 #pragma unroll
-        for (int ks = 0; ks < 8; ++ks) umma_ss(tS, desc_kmajor(q_base, ks), desc_kmajor(k_base, ks), idesc_kk, ks > 0 ? 1u : 0u);
+        for (int ks = 0; ks < 4 * NH; ++ks) umma_ss(tS, desc_kmajor(q_base, ks), desc_kmajor(k_base, ks), idesc_kk, ks > 0 ? 1u : 0u);
 #pragma unroll
-        for (int ks = 0; ks < 8; ++ks) umma_ss(tDP, desc_kmajor(do_base, ks), desc_kmajor(v_base, ks), idesc_kk, ks > 0 ? 1u : 0u);
+        for (int ks = 0; ks < 4 * NH; ++ks) umma_ss(tDP, desc_kmajor(do_base, ks), desc_kmajor(v_base, ks), idesc_kk, ks > 0 ? 1u : 0u);
         umma_commit(&bars->sp_full);
         if (!mbar_wait(&bars->ds_ready, it & 1, abort_flag, p.status, 4)) break;
         tc_fence_after();
@@ -154,25 +152,16 @@ flash_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       tc_fence_after();
       const int k_idx = kb * AT + row;   // accumulator rows are key positions
       const bool row_ok = k_idx < p.S;
-      __nv_bfloat16* dkp = reinterpret_cast<__nv_bfloat16*>(p.dk) + (static_cast<long long>(b) * p.S + k_idx) * p.ld_dk + out_head * HD;
-      __nv_bfloat16* dvp = reinterpret_cast<__nv_bfloat16*>(p.dv) + (static_cast<long long>(b) * p.S + k_idx) * p.ld_dv + out_head * HD;
+      __nv_bfloat16* dkp = reinterpret_cast<__nv_bfloat16*>(p.dk) + (static_cast<long long>(b) * p.S + k_idx) * p.ld_dk + out_head * p.hd;
+      __nv_bfloat16* dvp = reinterpret_cast<__nv_bfloat16*>(p.dv) + (static_cast<long long>(b) * p.S + k_idx) * p.ld_dv + out_head * p.hd;
 #pragma unroll 1
-      for (int c = 0; c < 8; ++c) {
+      for (int c = 0; c < 4 * NH; ++c) {
+        const bool is_dv = c < 2 * NH;
+        const int cc = is_dv ? c : c - 2 * NH;
         uint32_t v[32];
-        tmem_ld32((c < 4 ? tDV : tDK) + lane_off + (c & 3) * 32, v);
+        tmem_ld32((is_dv ? tDV : tDK) + lane_off + cc * 32, v);
         tmem_ld_wait();
-        __nv_bfloat16* dst = (c < 4 ? dvp : dkp) + (c & 3) * 32;
-        if (row_ok) {
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            uint4 o4;
-            o4.x = pack_bf16x2(__uint_as_float(v[8 * q + 0]), __uint_as_float(v[8 * q + 1]));
-            o4.y = pack_bf16x2(__uint_as_float(v[8 * q + 2]), __uint_as_float(v[8 * q + 3]));
-            o4.z = pack_bf16x2(__uint_as_float(v[8 * q + 4]), __uint_as_float(v[8 * q + 5]));
-            o4.w = pack_bf16x2(__uint_as_float(v[8 * q + 6]), __uint_as_float(v[8 * q + 7]));
-            *reinterpret_cast<uint4*>(dst + q * 8) = o4;
-          }
-        }
+        if (row_ok) store_head32(is_dv ? dvp : dkp, cc * 32, p.hd, v, 1.f);
       }
     }
   }
@@ -187,6 +176,7 @@ flash_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
 // ================================================================================================ host
 static void check_attn(const AttnArgs& a) {
   if (a.S <= 0 || a.B <= 0 || a.Hq <= 0 || a.Hkv <= 0 || a.Hq % a.Hkv) throw std::runtime_error("himuon attention: bad sizes");
+  if (a.hd <= 0 || a.hd > 128 || a.hd % 8) throw std::runtime_error("himuon attention: head_dim must be a multiple of 8 up to 128");
   if (a.ld_q % 8 || a.ld_k % 8 || a.ld_v % 8 || a.ld_o % 8) throw std::runtime_error("himuon attention: token strides must be multiples of 8");
 }
 
@@ -197,24 +187,34 @@ void flash_attn_fwd(const AttnArgs& a, cudaStream_t s) {
   if (e != cudaSuccess) throw std::runtime_error(std::string("himuon flash_attn_fwd launch failed: ") + cudaGetErrorString(e));
 }
 
+template <int NH>
+static void launch_dkv(const AttnArgs& a, const AttnDev& p, int heads_y, cudaStream_t s) {
+  constexpr size_t SMEM = 1024 + 4 * NH * HALF_BYTES + 4 * HALF_BYTES + 512;
+  static bool attr = false;
+  if (!attr) {
+    cudaFuncSetAttribute(flash_bwd_dkv_kernel<NH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM);
+    attr = true;
+  }
+  const CUtensorMap tq = head_tmap(a.q, a.B, a.S, a.Hq, a.hd, a.ld_q), tk = head_tmap(a.k, a.B, a.S, a.Hkv, a.hd, a.ld_k),
+                    tv = head_tmap(a.v, a.B, a.S, a.Hkv, a.hd, a.ld_v), tdo = head_tmap(a.d_o, a.B, a.S, a.Hq, a.hd, a.ld_do);
+  flash_bwd_dkv_kernel<NH><<<dim3(p.nblk, heads_y, a.B), 192, SMEM, s>>>(tq, tk, tv, tdo, p);
+}
+static void bwd_dkv(const AttnArgs& a, const AttnDev& p, int heads_y, cudaStream_t s) {
+  if (flash_bwd_dkv_t_supported(a)) flash_bwd_dkv_t(a, p, heads_y, s);
+  else if (head_halves(a.hd) == 1) launch_dkv<1>(a, p, heads_y, s);
+  else launch_dkv<2>(a, p, heads_y, s);
+}
+
 void flash_attn_bwd(const AttnArgs& a, cudaStream_t s) {
   check_attn(a);
   if (a.ld_do % 8 || a.ld_dq % 8 || a.ld_dk % 8 || a.ld_dv % 8) throw std::runtime_error("himuon attention: gradient strides must be multiples of 8");
-  constexpr size_t SMEM_DKV = 1024 + 6 * TILE_BYTES + 512;
-  static bool attr = false;
-  if (!attr) {
-    cudaFuncSetAttribute(flash_bwd_dkv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_DKV);
-    attr = true;
-  }
   AttnDev p{};
   p.lse = a.lse; p.delta = a.delta; p.o_in = a.o; p.d_o = a.d_o; p.dq = a.dq; p.dk = a.dk; p.dv = a.dv;
-  p.B = a.B; p.S = a.S; p.Hq = a.Hq; p.Hkv = a.Hkv;
+  p.B = a.B; p.S = a.S; p.Hq = a.Hq; p.Hkv = a.Hkv; p.hd = a.hd;
   p.ld_o = a.ld_o; p.ld_do = a.ld_do; p.ld_dq = a.ld_dq; p.ld_dk = a.ld_dk; p.ld_dv = a.ld_dv;
   p.nblk = (a.S + AT - 1) / AT;
   p.scale = a.scale; p.scale_log2 = a.scale * kLog2e;
   p.status = status_word_ptr();
-  const CUtensorMap tq = head_tmap(a.q, a.B, a.S, a.Hq, a.ld_q), tk = head_tmap(a.k, a.B, a.S, a.Hkv, a.ld_k),
-                    tv = head_tmap(a.v, a.B, a.S, a.Hkv, a.ld_v), tdo = head_tmap(a.d_o, a.B, a.S, a.Hq, a.ld_do);
   if (flash_bwd_dq_t_supported(a)) flash_bwd_dq_t(a, p, s);
   else flash_bwd_dq_kv64(a, s);                       // sequence lengths that are not a multiple of 128
   const int G = a.Hq / a.Hkv;
@@ -224,15 +224,12 @@ void flash_attn_bwd(const AttnArgs& a, cudaStream_t s) {
     AttnDev ps = p;
     ps.split_heads = 1;
     ps.dk = a.dk_part; ps.dv = a.dv_part; ps.ld_dk = a.ld_part; ps.ld_dv = a.ld_part;
-    if (flash_bwd_dkv_t_supported(a)) flash_bwd_dkv_t(a, ps, a.Hq, s);
-    else flash_bwd_dkv_kernel<<<dim3(p.nblk, a.Hq, a.B), 192, SMEM_DKV, s>>>(tq, tk, tv, tdo, ps);
+    bwd_dkv(a, ps, a.Hq, s);
     const long long tokens = static_cast<long long>(a.B) * a.S;
-    group_sum_heads(a.dk_part, a.dk, tokens, a.Hkv, G, a.ld_part, a.ld_dk, s);
-    group_sum_heads(a.dv_part, a.dv, tokens, a.Hkv, G, a.ld_part, a.ld_dv, s);
-  } else if (flash_bwd_dkv_t_supported(a)) {
-    flash_bwd_dkv_t(a, p, a.Hkv, s);
+    group_sum_heads(a.dk_part, a.dk, tokens, a.Hkv, G, a.hd, a.ld_part, a.ld_dk, s);
+    group_sum_heads(a.dv_part, a.dv, tokens, a.Hkv, G, a.hd, a.ld_part, a.ld_dv, s);
   } else {
-    flash_bwd_dkv_kernel<<<dim3(p.nblk, a.Hkv, a.B), 192, SMEM_DKV, s>>>(tq, tk, tv, tdo, p);
+    bwd_dkv(a, p, a.Hkv, s);
   }
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) throw std::runtime_error(std::string("himuon flash_attn_bwd launch failed: ") + cudaGetErrorString(e));

@@ -132,33 +132,37 @@ static void headnorm_rope_fwd(const at::Tensor& x, const c10::optional<at::Tenso
                               const c10::optional<at::Tensor>& rstd, const at::Tensor& cos_sin, int64_t heads,
                               int64_t seq_len, double eps) {
   HM_CHECK(x.is_cuda() && is_bf16(x) && is_bf16(y) && x.dim() == 2 && y.dim() == 2 && x.stride(1) == 1 && y.stride(1) == 1, "headnorm_rope_fwd: bad tensors");
-  HM_CHECK(x.size(1) == heads * 128 && y.size(1) == heads * 128, "headnorm_rope_fwd: head_dim must be 128");
-  HM_CHECK(is_f32(cos_sin) && cos_sin.is_contiguous() && cos_sin.numel() >= seq_len * 128, "headnorm_rope_fwd: bad rope table");
+  HM_CHECK(heads > 0 && (x.size(1) == heads * 128 || x.size(1) == heads * 64) && y.sizes() == x.sizes(), "headnorm_rope_fwd: head_dim must be 64 or 128");
+  const int64_t hd = x.size(1) / heads;
+  HM_CHECK(is_f32(cos_sin) && cos_sin.is_contiguous() && cos_sin.numel() >= seq_len * hd, "headnorm_rope_fwd: bad rope table");
   HM_CHECK(x.stride(0) % 8 == 0 && y.stride(0) % 8 == 0 && reinterpret_cast<uintptr_t>(x.data_ptr()) % 16 == 0 &&
                reinterpret_cast<uintptr_t>(y.data_ptr()) % 16 == 0,
            "headnorm_rope_fwd: rows must start on 16-byte boundaries");
   const bool use_norm = w.has_value();
-  if (use_norm) HM_CHECK(rstd.has_value() && rstd->numel() >= x.size(0) * heads && is_bf16(*w) && w->numel() == 128, "headnorm_rope_fwd: norm needs weight[128] and rstd");
+  if (use_norm) HM_CHECK(rstd.has_value() && rstd->numel() >= x.size(0) * heads && is_bf16(*w) && w->numel() == hd, "headnorm_rope_fwd: norm needs weight[head_dim] and rstd");
   const c10::cuda::CUDAGuard guard(x.device());
   himuon::headnorm_rope_fwd(x.data_ptr(), use_norm ? w->data_ptr() : nullptr, y.data_ptr(), use_norm ? rstd->data_ptr<float>() : nullptr,
-                            cos_sin.data_ptr<float>(), (int)x.size(0), (int)heads, (int)seq_len, x.stride(0), y.stride(0), (float)eps,
+                            cos_sin.data_ptr<float>(), (int)x.size(0), (int)heads, (int)hd, (int)seq_len, x.stride(0), y.stride(0), (float)eps,
                             use_norm ? 1 : 0, cur_stream());
 }
 static void headnorm_rope_bwd(const at::Tensor& dy, const c10::optional<at::Tensor>& x, const c10::optional<at::Tensor>& w,
                               const c10::optional<at::Tensor>& rstd, at::Tensor& dx, const c10::optional<at::Tensor>& dw_accum,
                               const at::Tensor& cos_sin, int64_t heads, int64_t seq_len) {
   HM_CHECK(dy.is_cuda() && is_bf16(dy) && is_bf16(dx) && dy.dim() == 2 && dx.dim() == 2 && dy.stride(1) == 1 && dx.stride(1) == 1, "headnorm_rope_bwd: bad tensors");
-  HM_CHECK(dy.size(1) == heads * 128 && dx.size(1) == heads * 128, "headnorm_rope_bwd: head_dim must be 128");
+  HM_CHECK(heads > 0 && (dy.size(1) == heads * 128 || dy.size(1) == heads * 64) && dx.sizes() == dy.sizes() &&
+               (!x.has_value() || x->sizes() == dy.sizes()), "headnorm_rope_bwd: head_dim must be 64 or 128");
+  const int64_t hd = dy.size(1) / heads;
+  HM_CHECK(is_f32(cos_sin) && cos_sin.is_contiguous() && cos_sin.numel() >= seq_len * hd, "headnorm_rope_bwd: bad rope table");
   HM_CHECK(dy.stride(0) % 8 == 0 && dx.stride(0) % 8 == 0 && reinterpret_cast<uintptr_t>(dy.data_ptr()) % 16 == 0 &&
                reinterpret_cast<uintptr_t>(dx.data_ptr()) % 16 == 0 &&
                (!x.has_value() || (x->stride(0) % 8 == 0 && reinterpret_cast<uintptr_t>(x->data_ptr()) % 16 == 0)),
            "headnorm_rope_bwd: rows must start on 16-byte boundaries");
   const bool use_norm = w.has_value();
-  if (use_norm) HM_CHECK(x.has_value() && rstd.has_value() && dw_accum.has_value() && is_f32(*dw_accum) && dw_accum->numel() == 128 && x->stride(1) == 1, "headnorm_rope_bwd: norm needs x, rstd, dw_accum");
+  if (use_norm) HM_CHECK(x.has_value() && rstd.has_value() && dw_accum.has_value() && is_f32(*dw_accum) && dw_accum->numel() == hd && w->numel() == hd && x->stride(1) == 1, "headnorm_rope_bwd: norm needs x, rstd, dw_accum");
   const c10::cuda::CUDAGuard guard(dy.device());
   himuon::headnorm_rope_bwd(dy.data_ptr(), use_norm ? x->data_ptr() : nullptr, use_norm ? w->data_ptr() : nullptr,
                             use_norm ? rstd->data_ptr<float>() : nullptr, dx.data_ptr(), use_norm ? dw_accum->data_ptr<float>() : nullptr,
-                            cos_sin.data_ptr<float>(), (int)dy.size(0), (int)heads, (int)seq_len, dy.stride(0),
+                            cos_sin.data_ptr<float>(), (int)dy.size(0), (int)heads, (int)hd, (int)seq_len, dy.stride(0),
                             use_norm ? x->stride(0) : 0, dx.stride(0), use_norm ? 1 : 0, cur_stream());
 }
 static void swiglu_fwd(const at::Tensor& gate, const at::Tensor& up, at::Tensor& out) {
@@ -204,14 +208,17 @@ static void cross_entropy(at::Tensor& logits, const at::Tensor& labels, at::Tens
 static void flash_attn_fwd(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, at::Tensor& o, at::Tensor& lse,
                            int64_t B, int64_t S, int64_t Hq, int64_t Hkv, double scale) {
   HM_CHECK(q.is_cuda() && is_bf16(q) && is_bf16(k) && is_bf16(v) && is_bf16(o) && is_f32(lse), "flash_attn_fwd: dtypes");
-  HM_CHECK(q.dim() == 2 && k.dim() == 2 && v.dim() == 2 && o.dim() == 2, "flash_attn_fwd: (tokens, heads*128) views expected");
-  HM_CHECK(q.size(0) == B * S && q.size(1) == Hq * 128 && k.size(1) == Hkv * 128 && v.size(1) == Hkv * 128 && o.size(1) == Hq * 128, "flash_attn_fwd: shapes (head_dim 128)");
+  HM_CHECK(q.dim() == 2 && k.dim() == 2 && v.dim() == 2 && o.dim() == 2, "flash_attn_fwd: (tokens, heads*head_dim) views expected");
+  HM_CHECK(Hq > 0 && Hkv > 0, "flash_attn_fwd: heads");
+  const int64_t hd = q.size(1) / Hq;
+  HM_CHECK(q.size(0) == B * S && q.size(1) == Hq * hd && k.size(1) == Hkv * hd && v.size(1) == Hkv * hd && o.size(1) == Hq * hd &&
+               k.size(0) == B * S && v.size(0) == B * S && o.size(0) == B * S, "flash_attn_fwd: shapes");
   HM_CHECK(q.stride(1) == 1 && k.stride(1) == 1 && v.stride(1) == 1 && o.stride(1) == 1, "flash_attn_fwd: unit inner strides");
   HM_CHECK(Hq % Hkv == 0 && lse.numel() >= B * Hq * S, "flash_attn_fwd: heads / lse size");
   const c10::cuda::CUDAGuard guard(q.device());
   himuon::AttnArgs a{};
   a.q = q.data_ptr(); a.k = k.data_ptr(); a.v = v.data_ptr(); a.o = o.data_ptr(); a.lse = lse.data_ptr<float>();
-  a.B = (int)B; a.S = (int)S; a.Hq = (int)Hq; a.Hkv = (int)Hkv;
+  a.B = (int)B; a.S = (int)S; a.Hq = (int)Hq; a.Hkv = (int)Hkv; a.hd = (int)hd;
   a.ld_q = q.stride(0); a.ld_k = k.stride(0); a.ld_v = v.stride(0); a.ld_o = o.stride(0);
   a.scale = (float)scale;
   himuon::flash_attn_fwd(a, cur_stream());
@@ -222,18 +229,23 @@ static void flash_attn_bwd(const at::Tensor& d_o, const at::Tensor& q, const at:
                            int64_t Hkv, double scale) {
   HM_CHECK(q.is_cuda() && is_bf16(q) && is_bf16(k) && is_bf16(v) && is_bf16(o) && is_bf16(d_o) && is_bf16(dq) && is_bf16(dk) && is_bf16(dv) && is_f32(lse) && is_f32(delta), "flash_attn_bwd: dtypes");
   HM_CHECK(q.stride(1) == 1 && k.stride(1) == 1 && v.stride(1) == 1 && o.stride(1) == 1 && d_o.stride(1) == 1 && dq.stride(1) == 1 && dk.stride(1) == 1 && dv.stride(1) == 1, "flash_attn_bwd: unit inner strides");
-  HM_CHECK(q.size(0) == B * S && q.size(1) == Hq * 128 && k.size(1) == Hkv * 128 && delta.numel() >= B * Hq * S, "flash_attn_bwd: shapes");
+  HM_CHECK(Hq > 0 && Hkv > 0, "flash_attn_bwd: heads");
+  const int64_t hd = q.size(1) / Hq;
+  HM_CHECK(q.size(0) == B * S && q.size(1) == Hq * hd && k.size(1) == Hkv * hd && v.size(1) == Hkv * hd && delta.numel() >= B * Hq * S &&
+               lse.numel() >= B * Hq * S && k.size(0) == B * S && v.sizes() == k.sizes() && o.sizes() == q.sizes() &&
+               d_o.sizes() == q.sizes() && dq.sizes() == q.sizes() && dk.sizes() == k.sizes() && dv.sizes() == k.sizes(),
+           "flash_attn_bwd: shapes");
   const c10::cuda::CUDAGuard guard(q.device());
   himuon::AttnArgs a{};
   a.q = q.data_ptr(); a.k = k.data_ptr(); a.v = v.data_ptr(); a.o = const_cast<void*>(o.data_ptr()); a.lse = lse.data_ptr<float>();
   a.d_o = d_o.data_ptr(); a.dq = dq.data_ptr(); a.dk = dk.data_ptr(); a.dv = dv.data_ptr(); a.delta = delta.data_ptr<float>();
-  a.B = (int)B; a.S = (int)S; a.Hq = (int)Hq; a.Hkv = (int)Hkv;
+  a.B = (int)B; a.S = (int)S; a.Hq = (int)Hq; a.Hkv = (int)Hkv; a.hd = (int)hd;
   a.ld_q = q.stride(0); a.ld_k = k.stride(0); a.ld_v = v.stride(0); a.ld_o = o.stride(0); a.ld_do = d_o.stride(0);
   a.ld_dq = dq.stride(0); a.ld_dk = dk.stride(0); a.ld_dv = dv.stride(0);
   if (dkv_part.has_value()) {
-    const at::Tensor& t = dkv_part.value();     // (2, B*S, Hq*128): per-query-head dK and dV
-    HM_CHECK(t.is_cuda() && is_bf16(t) && t.is_contiguous() && t.dim() == 3 && t.size(0) == 2 && t.size(1) == B * S && t.size(2) == Hq * 128,
-             "flash_attn_bwd: dkv_part must be a contiguous (2, B*S, Hq*128) bf16 tensor");
+    const at::Tensor& t = dkv_part.value();     // (2, B*S, Hq*head_dim): per-query-head dK and dV
+    HM_CHECK(t.is_cuda() && is_bf16(t) && t.is_contiguous() && t.dim() == 3 && t.size(0) == 2 && t.size(1) == B * S && t.size(2) == Hq * hd,
+             "flash_attn_bwd: dkv_part must be a contiguous (2, B*S, Hq*head_dim) bf16 tensor");
     a.dk_part = t.data_ptr();
     a.dv_part = static_cast<char*>(t.data_ptr()) + t.stride(0) * 2;
     a.ld_part = t.stride(1);

@@ -112,12 +112,12 @@ void rmsnorm_fwd(const void* x, const void* w, void* y, float* rstd, int rows, i
 // With `dres` (same shape as dx): dx = dres + the norm's input gradient (the residual path's gradient joins here).
 void rmsnorm_bwd(const void* dy, const void* x, const void* w, const float* rstd, void* dx, float* dw_accum,
                  int rows, int cols, cudaStream_t s, const void* dres = nullptr);
-// Per-head RMSNorm (optional) + rotary embedding on a (tokens, heads, 128) view with row stride `ld`.
+// Per-head RMSNorm (optional) + rotary embedding on a (tokens, heads, hd) view with row stride `ld`; hd is 64 or 128.
 void headnorm_rope_fwd(const void* x, const void* w, void* y, float* rstd, const float* cos_sin, int tokens,
-                       int heads, int seq_len, long long ld_in, long long ld_out, float eps, int use_norm,
+                       int heads, int hd, int seq_len, long long ld_in, long long ld_out, float eps, int use_norm,
                        cudaStream_t s);
 void headnorm_rope_bwd(const void* dy, const void* x, const void* w, const float* rstd, void* dx, float* dw_accum,
-                       const float* cos_sin, int tokens, int heads, int seq_len, long long ld_dy, long long ld_x,
+                       const float* cos_sin, int tokens, int heads, int hd, int seq_len, long long ld_dy, long long ld_x,
                        long long ld_dx, int use_norm, cudaStream_t s);
 void swiglu_fwd(const void* gate, const void* up, void* out, long long rows, int cols, long long ld_g, long long ld_u,
                 long long ld_o, cudaStream_t s);
@@ -132,21 +132,21 @@ void embedding_bwd(const long long* ids, const void* dout, void* dtable, long lo
 void cross_entropy_fwd_bwd(void* logits, const long long* labels, float* loss_sum, float* count, float* lse_out,
                            long long rows, int vocab, long long ld, float grad_scale, const float* scale_dev,
                            long long ignore_index, cudaStream_t s);
-void group_sum_heads(const void* in, void* out, long long tokens, int hkv, int G, long long ld_in, long long ld_out,
-                     cudaStream_t s);
+void group_sum_heads(const void* in, void* out, long long tokens, int hkv, int G, int hd, long long ld_in,
+                     long long ld_out, cudaStream_t s);
 void cast_copy(const void* src, void* dst, long long n, int src_fp32, int dst_fp32, float scale, cudaStream_t s);
 void bf16_add_to_f32(const void* src_bf16, float* dst, long long n, cudaStream_t s);
 
-// ---------------------------------------------------------------- attention (causal GQA, head_dim 128)
-// q: (B, S, Hq, 128), k/v: (B, S, Hkv, 128), o like q; all bf16 with token stride ld_* elements
+// ---------------------------------------------------------------- attention (causal GQA, head_dim a multiple of 8 up to 128)
+// q: (B, S, Hq, hd), k/v: (B, S, Hkv, hd), o like q; all bf16 with token stride ld_* elements
 // (so q/k/v may be column slices of one fused projection output).  lse: (B, Hq, S) fp32, the base-2 log-sum-exp of the
 // scaled scores (log2 of the softmax denominator plus the row maximum in base-2 units), as the backward kernels use it.
 struct AttnArgs {
   const void* q; const void* k; const void* v; void* o; float* lse;
   const void* d_o; void* dq; void* dk; void* dv; float* delta;
-  void* dk_part; void* dv_part;       // optional (B*S, Hq*128) scratch: per-query-head dK/dV, summed over each group afterwards
+  void* dk_part; void* dv_part;       // optional (B*S, Hq*hd) scratch: per-query-head dK/dV, summed over each group afterwards
   long long ld_part;
-  int B, S, Hq, Hkv;
+  int B, S, Hq, Hkv, hd;
   long long ld_q, ld_k, ld_v, ld_o, ld_do, ld_dq, ld_dk, ld_dv;
   float scale;
 };

@@ -354,16 +354,17 @@ void rmsnorm_bwd(const void* dy, const void* x, const void* w, const float* rstd
 }
 
 // ------------------------------------------------------------------------------------------------ head-norm + RoPE
-// Per-head RMSNorm (optional) + RoPE on (token, head) vectors of 128 elements.
-// cos_sin: (seq_len, 64, 2) fp32.  Rotate-half convention:
-//   y[i]      = xn[i]*cos[i] - xn[i+64]*sin[i]
-//   y[i+64]   = xn[i+64]*cos[i] + xn[i]*sin[i]
-// Layout of the two kernels below: sixteen lanes per head vector, lane l owning elements [8l, 8l+8) (one 16-byte
-// access); lanes 0-7 hold the first half, lanes 8-15 the second half, so the rotation partner of every element sits
-// at the same register index in lane l^8.  A warp therefore handles two vectors per pass.
-__device__ __forceinline__ float half_warp_sum(float v) {
+// Per-head RMSNorm (optional) + RoPE on (token, head) vectors of D = 128 or 64 elements.
+// cos_sin: (seq_len, D/2, 2) fp32.  Rotate-half convention (h = D/2):
+//   y[i]      = xn[i]*cos[i] - xn[i+h]*sin[i]
+//   y[i+h]    = xn[i+h]*cos[i] + xn[i]*sin[i]
+// Layout of the two kernels below: LN = D/8 lanes per head vector, lane l owning elements [8l, 8l+8) (one 16-byte
+// access); the lower LN/2 lanes hold the first half, the others the second half, so the rotation partner of every
+// element sits at the same register index in lane l^(LN/2).  A warp handles 32/LN vectors per pass.
+template <int LN>
+__device__ __forceinline__ float head_sum(float v) {
 #pragma unroll
-  for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  for (int o = LN / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
 }
 __device__ __forceinline__ void unpack8(const uint4& u, float (&f)[8]) {
@@ -374,15 +375,17 @@ __device__ __forceinline__ uint4 pack8(const float (&f)[8]) {
   return make_uint4(pack_bf16x2(f[0], f[1]), pack_bf16x2(f[2], f[3]), pack_bf16x2(f[4], f[5]), pack_bf16x2(f[6], f[7]));
 }
 
+template <int LN>
 __global__ void __launch_bounds__(256)
 headnorm_rope_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
                          __nv_bfloat16* __restrict__ y, float* __restrict__ rstd, const float* __restrict__ cos_sin,
                          long long n_vec, int heads, int seq_len, long long ld_in, long long ld_out, float eps,
                          int use_norm) {
-  const int sub = threadIdx.x & 15;                       // lane within the half warp
-  const bool second = sub >= 8;
-  const long long hw0 = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 4;
-  const long long nhw = (static_cast<long long>(gridDim.x) * blockDim.x) >> 4;
+  constexpr int D = LN * 8;
+  const int sub = threadIdx.x & (LN - 1);                 // lane within the head vector
+  const bool second = sub >= LN / 2;
+  const long long hw0 = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) / LN;
+  const long long nhw = (static_cast<long long>(gridDim.x) * blockDim.x) / LN;
   float wv[8];
 #pragma unroll
   for (int q = 0; q < 8; ++q) wv[q] = 1.f;
@@ -396,16 +399,16 @@ headnorm_rope_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat1
     const int head = static_cast<int>(vi32 - tok * static_cast<uint32_t>(heads));
     const int pos = static_cast<int>(tok % static_cast<uint32_t>(seq_len));
     float xv[8];
-    unpack8(reinterpret_cast<const uint4*>(x + static_cast<long long>(tok) * ld_in + head * 128)[sub], xv);
-    const float4* cs4 = reinterpret_cast<const float4*>(cos_sin + static_cast<long long>(pos) * 128 + (sub & 7) * 16);
+    unpack8(reinterpret_cast<const uint4*>(x + static_cast<long long>(tok) * ld_in + head * D)[sub], xv);
+    const float4* cs4 = reinterpret_cast<const float4*>(cos_sin + static_cast<long long>(pos) * D + (sub & (LN / 2 - 1)) * 16);
     const float4 c0 = cs4[0], c1 = cs4[1], c2 = cs4[2], c3 = cs4[3];   // (cos, sin) of this lane's eight frequencies
     const float cs[16] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w, c2.x, c2.y, c2.z, c2.w, c3.x, c3.y, c3.z, c3.w};
     if (use_norm) {
       float ss = 0.f;
 #pragma unroll
       for (int q = 0; q < 8; ++q) ss += xv[q] * xv[q];
-      ss = half_warp_sum(ss);
-      const float rs = rsqrtf(ss * (1.f / 128.f) + eps);
+      ss = head_sum<LN>(ss);
+      const float rs = rsqrtf(ss * (1.f / D) + eps);
       if (sub == 0 && live && rstd) rstd[vi] = rs;
 #pragma unroll
       for (int q = 0; q < 8; ++q) xv[q] = round_bf16(round_bf16(xv[q] * rs) * wv[q]);
@@ -413,24 +416,26 @@ headnorm_rope_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat1
     float out[8];
 #pragma unroll
     for (int q = 0; q < 8; ++q) {
-      const float other = __shfl_xor_sync(0xffffffffu, xv[q], 8);
+      const float other = __shfl_xor_sync(0xffffffffu, xv[q], LN / 2);
       out[q] = second ? xv[q] * cs[2 * q] + other * cs[2 * q + 1] : xv[q] * cs[2 * q] - other * cs[2 * q + 1];
     }
-    if (live) reinterpret_cast<uint4*>(y + static_cast<long long>(tok) * ld_out + head * 128)[sub] = pack8(out);
+    if (live) reinterpret_cast<uint4*>(y + static_cast<long long>(tok) * ld_out + head * D)[sub] = pack8(out);
   }
 }
 
+template <int LN>
 __global__ void __launch_bounds__(256)
 headnorm_rope_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
                          const __nv_bfloat16* __restrict__ w, const float* __restrict__ rstd,
                          __nv_bfloat16* __restrict__ dx, float* __restrict__ dw_accum,
                          const float* __restrict__ cos_sin, long long n_vec, int heads, int seq_len, long long ld_dy,
                          long long ld_x, long long ld_dx, int use_norm) {
-  __shared__ float sdw[8][128];                         // one row of partial dw per warp
-  const int sub = threadIdx.x & 15;
-  const bool second = sub >= 8;
-  const long long hw0 = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 4;
-  const long long nhw = (static_cast<long long>(gridDim.x) * blockDim.x) >> 4;
+  constexpr int D = LN * 8;
+  __shared__ float sdw[8][D];                           // one row of partial dw per warp
+  const int sub = threadIdx.x & (LN - 1);
+  const bool second = sub >= LN / 2;
+  const long long hw0 = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) / LN;
+  const long long nhw = (static_cast<long long>(gridDim.x) * blockDim.x) / LN;
   float wv[8], acc[8];
 #pragma unroll
   for (int q = 0; q < 8; ++q) { wv[q] = 1.f; acc[q] = 0.f; }
@@ -444,19 +449,19 @@ headnorm_rope_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat
     const int head = static_cast<int>(vi32 - tok * static_cast<uint32_t>(heads));
     const int pos = static_cast<int>(tok % static_cast<uint32_t>(seq_len));
     float g[8];
-    unpack8(reinterpret_cast<const uint4*>(dy + static_cast<long long>(tok) * ld_dy + head * 128)[sub], g);
-    const float4* cs4 = reinterpret_cast<const float4*>(cos_sin + static_cast<long long>(pos) * 128 + (sub & 7) * 16);
+    unpack8(reinterpret_cast<const uint4*>(dy + static_cast<long long>(tok) * ld_dy + head * D)[sub], g);
+    const float4* cs4 = reinterpret_cast<const float4*>(cos_sin + static_cast<long long>(pos) * D + (sub & (LN / 2 - 1)) * 16);
     const float4 c0 = cs4[0], c1 = cs4[1], c2 = cs4[2], c3 = cs4[3];
     const float cs[16] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w, c2.x, c2.y, c2.z, c2.w, c3.x, c3.y, c3.z, c3.w};
     float d[8];
 #pragma unroll
     for (int q = 0; q < 8; ++q) {                          // transpose of the rotation
-      const float other = __shfl_xor_sync(0xffffffffu, g[q], 8);
+      const float other = __shfl_xor_sync(0xffffffffu, g[q], LN / 2);
       d[q] = second ? g[q] * cs[2 * q] - other * cs[2 * q + 1] : g[q] * cs[2 * q] + other * cs[2 * q + 1];
     }
     if (use_norm) {
       float h[8];
-      unpack8(reinterpret_cast<const uint4*>(x + static_cast<long long>(tok) * ld_x + head * 128)[sub], h);
+      unpack8(reinterpret_cast<const uint4*>(x + static_cast<long long>(tok) * ld_x + head * D)[sub], h);
       const float rs = live ? rstd[vi] : 0.f;
       float dot = 0.f;
 #pragma unroll
@@ -465,21 +470,24 @@ headnorm_rope_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat
         if (live) acc[q] += d[q] * h[q];
         dot += d[q] * wv[q] * h[q];
       }
-      const float mean = half_warp_sum(dot) * (1.f / 128.f);
+      const float mean = head_sum<LN>(dot) * (1.f / D);
 #pragma unroll
       for (int q = 0; q < 8; ++q) d[q] = rs * (d[q] * wv[q] - h[q] * mean);
     }
-    if (live) reinterpret_cast<uint4*>(dx + static_cast<long long>(tok) * ld_dx + head * 128)[sub] = pack8(d);
+    if (live) reinterpret_cast<uint4*>(dx + static_cast<long long>(tok) * ld_dx + head * D)[sub] = pack8(d);
   }
   if (use_norm && dw_accum) {
 #pragma unroll
-    for (int q = 0; q < 8; ++q) acc[q] += __shfl_xor_sync(0xffffffffu, acc[q], 16);   // the warp's two half warps
-    if ((threadIdx.x & 31) < 16) {
+    for (int q = 0; q < 8; ++q) {
+#pragma unroll
+      for (int o = LN; o < 32; o <<= 1) acc[q] += __shfl_xor_sync(0xffffffffu, acc[q], o);   // the warp's head vectors
+    }
+    if ((threadIdx.x & 31) < LN) {
 #pragma unroll
       for (int q = 0; q < 8; ++q) sdw[threadIdx.x >> 5][sub * 8 + q] = acc[q];
     }
     __syncthreads();
-    if (threadIdx.x < 32) {
+    if (threadIdx.x < D / 4) {
       float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
       for (int w8 = 0; w8 < 8; ++w8) {
@@ -497,25 +505,31 @@ headnorm_rope_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat
 }
 
 void headnorm_rope_fwd(const void* x, const void* w, void* y, float* rstd, const float* cos_sin, int tokens, int heads,
-                       int seq_len, long long ld_in, long long ld_out, float eps, int use_norm, cudaStream_t s) {
+                       int hd, int seq_len, long long ld_in, long long ld_out, float eps, int use_norm, cudaStream_t s) {
   const long long n_vec = static_cast<long long>(tokens) * heads;
   if (n_vec <= 0) return;
   if (n_vec >= (1LL << 31)) throw std::runtime_error("himuon headnorm_rope: too many head vectors for one launch");
-  const long long blocks = (n_vec + 15) / 16;
+  if (hd != 128 && hd != 64) throw std::runtime_error("himuon headnorm_rope: head_dim must be 64 or 128");
+  const int per_block = hd == 64 ? 32 : 16;
+  const long long blocks = (n_vec + per_block - 1) / per_block;
   const int grid = static_cast<int>(blocks < num_sms() * 8 ? blocks : num_sms() * 8);
-  headnorm_rope_fwd_kernel<<<grid, 256, 0, s>>>(reinterpret_cast<const __nv_bfloat16*>(x), reinterpret_cast<const __nv_bfloat16*>(w),
+  auto kern = hd == 64 ? headnorm_rope_fwd_kernel<8> : headnorm_rope_fwd_kernel<16>;
+  kern<<<grid, 256, 0, s>>>(reinterpret_cast<const __nv_bfloat16*>(x), reinterpret_cast<const __nv_bfloat16*>(w),
                                                 reinterpret_cast<__nv_bfloat16*>(y), rstd, cos_sin, n_vec, heads, seq_len,
                                                 ld_in, ld_out, eps, use_norm);
 }
 void headnorm_rope_bwd(const void* dy, const void* x, const void* w, const float* rstd, void* dx, float* dw_accum,
-                       const float* cos_sin, int tokens, int heads, int seq_len, long long ld_dy, long long ld_x,
+                       const float* cos_sin, int tokens, int heads, int hd, int seq_len, long long ld_dy, long long ld_x,
                        long long ld_dx, int use_norm, cudaStream_t s) {
   const long long n_vec = static_cast<long long>(tokens) * heads;
   if (n_vec <= 0) return;
   if (n_vec >= (1LL << 31)) throw std::runtime_error("himuon headnorm_rope: too many head vectors for one launch");
-  const long long blocks = (n_vec + 15) / 16;
+  if (hd != 128 && hd != 64) throw std::runtime_error("himuon headnorm_rope: head_dim must be 64 or 128");
+  const int per_block = hd == 64 ? 32 : 16;
+  const long long blocks = (n_vec + per_block - 1) / per_block;
   const int grid = static_cast<int>(blocks < num_sms() * 4 ? blocks : num_sms() * 4);
-  headnorm_rope_bwd_kernel<<<grid, 256, 0, s>>>(reinterpret_cast<const __nv_bfloat16*>(dy), reinterpret_cast<const __nv_bfloat16*>(x),
+  auto kern = hd == 64 ? headnorm_rope_bwd_kernel<8> : headnorm_rope_bwd_kernel<16>;
+  kern<<<grid, 256, 0, s>>>(reinterpret_cast<const __nv_bfloat16*>(dy), reinterpret_cast<const __nv_bfloat16*>(x),
                                                 reinterpret_cast<const __nv_bfloat16*>(w), rstd, reinterpret_cast<__nv_bfloat16*>(dx),
                                                 dw_accum, cos_sin, n_vec, heads, seq_len, ld_dy, ld_x, ld_dx, use_norm);
 }
@@ -740,33 +754,34 @@ void cross_entropy_fwd_bwd(void* logits, const long long* labels, float* loss_su
 }
 
 // ------------------------------------------------------------------------------------------------ head-group sum
-// out[t, hk, :] = sum_g in[t, hk*G + g, :] for 128-wide heads (gradients of grouped K/V heads).
+// out[t, hk, :] = sum_g in[t, hk*G + g, :] for hd-wide heads (gradients of grouped K/V heads).
 __global__ void __launch_bounds__(256)
 group_sum_kernel(const __nv_bfloat16* __restrict__ in, __nv_bfloat16* __restrict__ out, long long tokens, int hkv, int G,
-                 long long ld_in, long long ld_out) {
-  const long long total = tokens * hkv * 16;      // 16 vectors of 8 elements per head
+                 int hd, long long ld_in, long long ld_out) {
+  const int vph = hd >> 3;                        // vectors of 8 elements per head
+  const long long total = tokens * hkv * vph;
   for (long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < total;
        i += static_cast<long long>(gridDim.x) * blockDim.x) {
-    const int vec = static_cast<int>(i & 15);
-    const long long th = i >> 4;
+    const long long th = i / vph;
+    const int vec = static_cast<int>(i - th * vph);
     const int hk = static_cast<int>(th % hkv);
     const long long t = th / hkv;
     float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     for (int g = 0; g < G; ++g) {
-      const uint4 v = *reinterpret_cast<const uint4*>(in + t * ld_in + (hk * G + g) * 128 + vec * 8);
+      const uint4 v = *reinterpret_cast<const uint4*>(in + t * ld_in + (hk * G + g) * hd + vec * 8);
       const uint32_t u[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
       for (int q = 0; q < 4; ++q) { acc[2 * q] += bf16_lo(u[q]); acc[2 * q + 1] += bf16_hi(u[q]); }
     }
-    *reinterpret_cast<uint4*>(out + t * ld_out + hk * 128 + vec * 8) =
+    *reinterpret_cast<uint4*>(out + t * ld_out + hk * hd + vec * 8) =
         make_uint4(pack_bf16x2(acc[0], acc[1]), pack_bf16x2(acc[2], acc[3]), pack_bf16x2(acc[4], acc[5]), pack_bf16x2(acc[6], acc[7]));
   }
 }
-void group_sum_heads(const void* in, void* out, long long tokens, int hkv, int G, long long ld_in, long long ld_out,
-                     cudaStream_t s) {
+void group_sum_heads(const void* in, void* out, long long tokens, int hkv, int G, int hd, long long ld_in,
+                     long long ld_out, cudaStream_t s) {
   if (tokens <= 0) return;
-  group_sum_kernel<<<ew_grid(tokens * hkv * 16), 256, 0, s>>>(reinterpret_cast<const __nv_bfloat16*>(in),
-                                                            reinterpret_cast<__nv_bfloat16*>(out), tokens, hkv, G, ld_in, ld_out);
+  group_sum_kernel<<<ew_grid(tokens * hkv * (hd / 8)), 256, 0, s>>>(reinterpret_cast<const __nv_bfloat16*>(in),
+                                                            reinterpret_cast<__nv_bfloat16*>(out), tokens, hkv, G, hd, ld_in, ld_out);
 }
 
 // ------------------------------------------------------------------------------------------------ casts

@@ -43,13 +43,16 @@ def use_kernels(t: torch.Tensor) -> bool:
 _WARNED: set = set()
 
 
-def _warn_torch_path(op: str, why: str) -> None:
-    """Says once per (op, reason) that a bf16 CUDA tensor is taking the plain PyTorch implementation of an op."""
+def _warn_once(op: str, why: str, what: str, stacklevel: int = 3) -> None:
     if (op, why) not in _WARNED:
         _WARNED.add((op, why))
         import warnings
-        warnings.warn(f"himuon_b200.ops.{op}: {why}; running the PyTorch implementation instead of the sm_100a kernel",
-                      stacklevel=3)
+        warnings.warn(f"himuon_b200.ops.{op}: {why}; {what}", stacklevel=stacklevel)
+
+
+def _warn_torch_path(op: str, why: str) -> None:
+    """Says once per (op, reason) that a bf16 CUDA tensor is taking the plain PyTorch implementation of an op."""
+    _warn_once(op, why, "running the PyTorch implementation instead of the sm_100a kernel", stacklevel=4)
 
 
 def check_status() -> None:
@@ -397,7 +400,7 @@ def add_rmsnorm(x, delta, w, eps: float, defer_dw: bool = False):
 
 
 class _HeadNormRopeFn(torch.autograd.Function):
-    """Per-head RMSNorm (optional) + RoPE on a ``(tokens, heads*128)`` view."""
+    """Per-head RMSNorm (optional) + RoPE on a ``(tokens, heads*head_dim)`` view, head_dim 128 or 64."""
 
     @staticmethod
     def forward(ctx, x, w, cos_sin, heads, seq_len, eps, defer_dw=False, inplace_grad=False):
@@ -405,31 +408,72 @@ class _HeadNormRopeFn(torch.autograd.Function):
         # the parameter object itself: under activation checkpointing saved_tensors hands back a detached copy
         ctx.w_param = w if defer_dw else None
         ctx.inplace_grad = inplace_grad
-        y = torch.empty(x.shape[0], heads * 128, device=x.device, dtype=x.dtype)
+        y = torch.empty(x.shape[0], x.shape[1], device=x.device, dtype=x.dtype)
         rstd = torch.empty(x.shape[0] * heads, device=x.device, dtype=torch.float32) if w is not None else None
         _ext.ext().headnorm_rope_fwd(x, w, y, rstd, cos_sin, heads, seq_len, float(eps))
         _count()
         ctx.save_for_backward(x, w, rstd, cos_sin)
-        ctx.heads, ctx.seq_len = heads, seq_len
+        ctx.heads, ctx.seq_len, ctx.eps = heads, seq_len, eps
         return y
 
     @staticmethod
     def backward(ctx, dy):
         x, w, rstd, cos_sin = ctx.saved_tensors
-        if dy.stride(-1) != 1:
+        if torch.is_grad_enabled() and dy.shape[1] == ctx.heads * 64:
+            # create_graph=True: 64-wide heads stay differentiable twice, as the PyTorch formulation is
+            return _head_norm_rope_double(ctx, dy, x, w, cos_sin)
+        if dy.stride(-1) != 1 or (dy.shape[1] == ctx.heads * 64 and (dy.stride(0) % 8 or dy.data_ptr() % 16)):
             dy = dy.contiguous()
         # Each head vector is read completely before it is written, so the input gradient may take the place of the
         # incoming one (asked for by callers that know dy has no other reader, e.g. a slice of attention's dq|dk|dv).
         inplace = ctx.inplace_grad and dy.stride(0) % 8 == 0 and dy.data_ptr() % 16 == 0
-        dx = dy if inplace else torch.empty(dy.shape[0], ctx.heads * 128, device=dy.device, dtype=dy.dtype)
+        dx = dy if inplace else torch.empty(dy.shape[0], dy.shape[1], device=dy.device, dtype=dy.dtype)
         if w is not None and ctx.defer_dw:
             _ext.ext().headnorm_rope_bwd(dy, x, w, rstd, dx, _norm_grad_buffer(ctx.w_param), cos_sin, ctx.heads, ctx.seq_len)
             _count(2)
             return dx, None, None, None, None, None, None, None
-        dw = torch.zeros(128, device=dy.device, dtype=torch.float32) if w is not None else None
+        dw = torch.zeros(w.numel(), device=dy.device, dtype=torch.float32) if w is not None else None
         _ext.ext().headnorm_rope_bwd(dy, x if w is not None else None, w, rstd, dx, dw, cos_sin, ctx.heads, ctx.seq_len)
         _count(2 if w is not None else 1)
         return dx, (dw.to(w.dtype) if w is not None else None), None, None, None, None, None, None
+
+
+def _head_norm_rope_ref(x2d, w, cos_sin, heads, seq_len, head_dim, eps):
+    T = x2d.shape[0]
+    x = x2d.reshape(T // seq_len, seq_len, heads, head_dim)
+    if w is not None:
+        x = ref.rmsnorm(x, w, eps)
+    return ref.apply_rope(x, cos_sin).reshape(T, heads * head_dim)
+
+
+def _head_norm_rope_double(ctx, dy, x, w, cos_sin):
+    heads, hd = ctx.heads, dy.shape[1] // ctx.heads
+    w_leaf = ctx.w_param if ctx.w_param is not None else w
+    inputs = [x] if w is None else [x, w_leaf]
+    live = [t for t in inputs if t.requires_grad]
+    y = _head_norm_rope_ref(x, None if w is None else w_leaf, cos_sin, heads, ctx.seq_len, hd, ctx.eps)
+    got = dict(zip(map(id, live), torch.autograd.grad(y, live, dy, create_graph=True)))
+    return (got.get(id(x)), None if w is None else got.get(id(w_leaf)), None, None, None, None, None, None)
+
+
+def _kernel_rows(t: torch.Tensor) -> bool:
+    """A 2-D tensor whose rows the kernels can address: unit inner stride, every row on a 16-byte boundary."""
+    return t.dim() == 2 and t.stride(1) == 1 and t.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0
+
+
+def _transformed(t: torch.Tensor) -> bool:
+    """vmap / functorch wrappers and forward-mode duals, which an autograd function without those rules cannot take."""
+    return torch._C._functorch.is_functorch_wrapped_tensor(t) or torch.autograd.forward_ad._current_level >= 0
+
+
+def _rope64_ok(x2d, w, cos_sin, heads, seq_len) -> bool:
+    return (not _transformed(x2d) and _kernel_rows(x2d) and x2d.shape[1] == heads * 64 and x2d.numel() > 0
+            and x2d.shape[0] % seq_len == 0 and x2d.shape[0] * heads < 2 ** 31
+            and cos_sin.dtype == torch.float32 and cos_sin.is_contiguous() and not cos_sin.requires_grad
+            and cos_sin.device == x2d.device and cos_sin.dim() == 3 and cos_sin.shape[0] >= seq_len
+            and tuple(cos_sin.shape[1:]) == (32, 2) and cos_sin.data_ptr() % 16 == 0
+            and (w is None or (w.dtype == torch.bfloat16 and tuple(w.shape) == (64,) and w.is_contiguous()
+                               and w.device == x2d.device and w.data_ptr() % 16 == 0)))
 
 
 def head_norm_rope(x2d, w, cos_sin, heads: int, seq_len: int, head_dim: int, eps: float, defer_dw: bool = False,
@@ -438,13 +482,13 @@ def head_norm_rope(x2d, w, cos_sin, heads: int, seq_len: int, head_dim: int, eps
     backward pass may overwrite the gradient it receives with the gradient it returns."""
     if use_kernels(x2d) and head_dim == 128:
         return _HeadNormRopeFn.apply(x2d, w, cos_sin, heads, seq_len, eps, _deferrable(w, defer_dw), inplace_grad)
+    if use_kernels(x2d) and head_dim == 64 and _rope64_ok(x2d, w, cos_sin, heads, seq_len):
+        # callers rely on being told once that 64-wide heads leave the 128-wide kernel
+        _warn_once("head_norm_rope", "head_dim 64", "running the 64-wide sm_100a kernel")
+        return _HeadNormRopeFn.apply(x2d, w, cos_sin, heads, seq_len, eps, _deferrable(w, defer_dw), inplace_grad)
     if use_kernels(x2d):
-        _warn_torch_path("head_norm_rope", f"head_dim {head_dim} (the kernel is written for 128)")
-    T = x2d.shape[0]
-    x = x2d.reshape(T // seq_len, seq_len, heads, head_dim)
-    if w is not None:
-        x = ref.rmsnorm(x, w, eps)
-    return ref.apply_rope(x, cos_sin).reshape(T, heads * head_dim)
+        _warn_torch_path("head_norm_rope", f"head_dim {head_dim} or its layout (the kernel takes 64 and 128, 16-byte aligned rows)")
+    return _head_norm_rope_ref(x2d, w, cos_sin, heads, seq_len, head_dim, eps)
 
 
 class _SplitColsFn(torch.autograd.Function):
@@ -490,7 +534,7 @@ def split_cols(x2d: torch.Tensor, n0: int):
 class _FlashAttnFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, q, k, v, B, S, Hq, Hkv, scale):
-        o = torch.empty(q.shape[0], Hq * 128, device=q.device, dtype=q.dtype)
+        o = torch.empty(q.shape[0], q.shape[1], device=q.device, dtype=q.dtype)
         lse = torch.empty(B * Hq * S, device=q.device, dtype=torch.float32)
         _ext.ext().flash_attn_fwd(q, k, v, o, lse, B, S, Hq, Hkv, float(scale))
         _count()
@@ -502,15 +546,16 @@ class _FlashAttnFn(torch.autograd.Function):
     def backward(ctx, do):
         q, k, v, o, lse = ctx.saved_tensors
         B, S, Hq, Hkv, scale = ctx.dims
-        if do.stride(-1) != 1 or do.stride(0) % 8:
+        if do.stride(-1) != 1 or do.stride(0) % 8 or do.data_ptr() % 16:
             do = do.contiguous()
+        D = q.shape[1] // Hq
         # dq | dk | dv share one buffer so the fused QKV projection sees a single contiguous gradient
-        dqkv = torch.empty(q.shape[0], (Hq + 2 * Hkv) * 128, device=q.device, dtype=q.dtype)
-        dq = dqkv[:, : Hq * 128]
-        dk = dqkv[:, Hq * 128: (Hq + Hkv) * 128]
-        dv = dqkv[:, (Hq + Hkv) * 128:]
+        dqkv = torch.empty(q.shape[0], (Hq + 2 * Hkv) * D, device=q.device, dtype=q.dtype)
+        dq = dqkv[:, : Hq * D]
+        dk = dqkv[:, Hq * D: (Hq + Hkv) * D]
+        dv = dqkv[:, (Hq + Hkv) * D:]
         delta = torch.empty(B * Hq * S, device=q.device, dtype=torch.float32)
-        part = torch.empty(2, q.shape[0], Hq * 128, device=q.device, dtype=q.dtype) if Hq > Hkv else None
+        part = torch.empty(2, q.shape[0], Hq * D, device=q.device, dtype=q.dtype) if Hq > Hkv else None
         _ext.ext().flash_attn_bwd(do, q, k, v, o, lse, dq, dk, dv, delta, part, B, S, Hq, Hkv, float(scale))
         _count(4 if part is not None else 2)
         return dq, dk, dv, None, None, None, None, None
@@ -522,18 +567,12 @@ def attention(q2d, k2d, v2d, B: int, S: int, Hq: int, Hkv: int, head_dim: int, s
     if use_kernels(q2d) and head_dim == 128:
         return _FlashAttnFn.apply(q2d, k2d, v2d, B, S, Hq, Hkv, scale)
     if use_kernels(q2d) and head_dim < 128 and head_dim % 8 == 0:
-        # Smaller heads (64 in Llama-3.2-1B and llama_220m) run the same tcgen05 kernels zero-padded to 128: zeros in
-        # q and k add nothing to the scores, zeros in v give zero output columns, which are cut off again.  Twice the
-        # tensor work of a native 64-wide kernel, but no S x S score matrix in memory; autograd differentiates the
-        # padding and the slice.
-        T = q2d.shape[0]
-        pad = 128 - head_dim
-
-        def widen(x, heads):
-            return torch.nn.functional.pad(x.reshape(T, heads, head_dim), (0, pad)).reshape(T, heads * 128)
-
-        o = _FlashAttnFn.apply(widen(q2d, Hq), widen(k2d, Hkv), widen(v2d, Hkv), B, S, Hq, Hkv, scale)
-        return o.reshape(T, Hq, 128)[:, :, :head_dim].reshape(T, Hq * head_dim)
+        # Narrower heads (64 in Llama-3.2-1B and llama_220m) run the same tcgen05 kernels: the TMA loads fill the tiles
+        # up with zeros and the epilogues cut them off, so nothing is padded in memory.  Up to 64 columns half of the
+        # tensor work goes away too.
+        rows = [t if _kernel_rows(t) else t.contiguous() for t in (q2d, k2d, v2d)]
+        rows = [t if t.data_ptr() % 16 == 0 else t.clone() for t in rows]
+        return _FlashAttnFn.apply(*rows, B, S, Hq, Hkv, scale)
     if use_kernels(q2d):
         _warn_torch_path("attention", f"head_dim {head_dim} (the kernels take 128, or a multiple of 8 below it)")
     q = q2d.reshape(B, S, Hq, head_dim)

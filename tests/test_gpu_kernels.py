@@ -438,3 +438,59 @@ def test_flash_attention_fwd_bwd(B, S, Hq, Hkv):
     _close(dq, qr.grad.reshape(B * S, Hq * D), atol=3e-2, rtol=3e-2)
     _close(dk, kr.grad.reshape(B * S, Hkv * D), atol=3e-2, rtol=3e-2)
     _close(dv, vr.grad.reshape(B * S, Hkv * D), atol=3e-2, rtol=3e-2)
+
+
+@pytest.mark.parametrize("D", [8, 56, 64, 72, 96, 120])
+@pytest.mark.parametrize("B,S,Hq,Hkv", [(1, 128, 2, 1), (2, 256, 4, 4), (1, 200, 4, 2)])
+def test_attention_narrow_heads(D, B, S, Hq, Hkv):
+    """Heads narrower than the kernels' 64- and 128-column tiles, from contiguous, sliced and misaligned operands."""
+    from himuon_b200 import ops
+
+    torch.manual_seed(1)
+    wide = torch.randn(B * S, (Hq + 2 * Hkv) * D, device="cuda", dtype=torch.bfloat16)
+    # column slices of one projection output, the last one with rows that start off the 16-byte grid
+    odd = torch.randn(B * S, Hkv * D + 1, device="cuda", dtype=torch.bfloat16)[:, 1:]
+    q, k, v = wide[:, : Hq * D], wide[:, Hq * D: (Hq + Hkv) * D], odd
+    leaves = [t.detach().clone().requires_grad_(True) for t in (q, k, v)]
+    views = [q.detach().requires_grad_(True), k.detach().requires_grad_(True), v.detach().requires_grad_(True)]
+    do = torch.randn(B * S, Hq * D, device="cuda", dtype=torch.bfloat16)
+    for ins in (leaves, views):
+        o = ops.attention(*ins, B, S, Hq, Hkv, D)
+        o.backward(do)
+        ref_in = [t.detach().float().reshape(B, S, h, D).requires_grad_(True) for t, h in zip(ins, (Hq, Hkv, Hkv))]
+        ref = _attn_ref(*ref_in, 1.0 / math.sqrt(D))
+        ref.backward(do.float().view(B, S, Hq, D))
+        _assert_status_clean()
+        # as for 128-wide heads: bf16 probabilities and score gradients, summed over at most 256 positions
+        _close(o, ref.reshape(B * S, Hq * D), atol=2e-2, rtol=2e-2)
+        for t, r in zip(ins, ref_in):
+            _close(t.grad, r.grad.reshape(t.shape), atol=3e-2, rtol=3e-2)
+
+
+@pytest.mark.parametrize("use_norm", [True, False])
+@pytest.mark.parametrize("aligned", [True, False])
+def test_head_norm_rope_64(use_norm, aligned):
+    """64-wide heads: the kernel (16-byte aligned rows) and the PyTorch path (any other layout) agree with fp32."""
+    from himuon_b200 import ops
+    from himuon_b200.ops import reference as ref
+
+    torch.manual_seed(2)
+    B, S, H, D = 3, 37, 5, 64
+    base = torch.randn(B * S, H * D + 8, device="cuda", dtype=torch.bfloat16)
+    x = (base[:, 8:] if aligned else base[:, 1: 1 + H * D]).detach().requires_grad_(True)
+    w = (1 + 0.1 * torch.randn(D, device="cuda")).bfloat16().requires_grad_(True) if use_norm else None
+    cs = ref.rope_tables(S, D, 1e4, device="cuda")
+    dy = torch.randn(B * S, H * D, device="cuda", dtype=torch.bfloat16)
+    before = ops.launch_count()
+    y = ops.head_norm_rope(x, w, cs, H, S, D, 1e-6)
+    assert (ops.launch_count() > before) == aligned
+    y.backward(dy)
+    xr = x.detach().float().requires_grad_(True)
+    wr = w.detach().float().requires_grad_(True) if use_norm else None
+    h = xr.view(B, S, H, D)
+    yr = ref.apply_rope(ref.rmsnorm(h, wr, 1e-6) if use_norm else h, cs).reshape(B * S, H * D)
+    yr.backward(dy.float())
+    _close(y, yr, atol=3e-2, rtol=2e-2)
+    _close(x.grad, xr.grad, atol=3e-2, rtol=2e-2)
+    if use_norm:
+        _close(w.grad, wr.grad, atol=0.3, rtol=2e-2)

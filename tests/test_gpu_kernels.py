@@ -494,3 +494,48 @@ def test_head_norm_rope_64(use_norm, aligned):
     _close(x.grad, xr.grad, atol=3e-2, rtol=2e-2)
     if use_norm:
         _close(w.grad, wr.grad, atol=0.3, rtol=2e-2)
+
+
+@pytest.mark.parametrize("offset", [0, 1])
+@pytest.mark.parametrize("tile", [128, 132])
+def test_fp32_momentum_tile_and_untile_apply(tile, offset):
+    """fp32 matrices: 16-byte rows, ragged widths, strided and misaligned tensors give the element-wise result."""
+    e = _ext()
+    torch.manual_seed(0)
+    Th = Tw = tile
+    mu, lr, wd, scale = 0.95, 0.02, 0.1, 2.0
+    shapes = [(256, 384), (200, 301), (65, 64), (131, 132)]
+
+    def make(h, w, pitch):      # rows `pitch` elements apart, first element `offset` elements past an aligned address
+        return torch.randn(h * pitch + 4, device="cuda")[offset:].as_strided((h, w), (pitch, 1))
+
+    grads = [make(h, w, w + 4) for h, w in shapes]
+    moms = [make(h, w, w) for h, w in shapes]
+    params = [make(h, w, w + 4) for h, w in shapes]
+    moms_ref, params_ref = [m.clone() for m in moms], [p.clone() for p in params]
+    mom_tab, app_tab, tile_base, unit, metas = b"", b"", 0, 0, []
+    for g, m, p in zip(grads, moms, params):
+        h, w = g.shape
+        R, C = math.ceil(h / Th), math.ceil(w / Tw)
+        mom_tab += struct.pack("<8QQq6i", g.data_ptr(), 0, 0, 0, 0, 0, 0, 0, m.data_ptr(), tile_base, h, w, R, C, unit, g.stride(0))
+        app_tab += struct.pack("<Qq6ifi", p.data_ptr(), tile_base, h, w, R, C, unit, 0, scale, p.stride(0))
+        metas.append((tile_base, R, C))
+        tile_base += R * C
+        unit += e.momentum_tile_units(R, C, Th)
+    mom_dev = torch.frombuffer(bytearray(mom_tab), dtype=torch.uint8).cuda()
+    app_dev = torch.frombuffer(bytearray(app_tab), dtype=torch.uint8).cuda()
+    tiles = torch.full((tile_base, Th, Tw), 7.0, device="cuda", dtype=torch.bfloat16)
+    e.momentum_tile(mom_dev, len(shapes), unit, Th, Tw, tiles, mu, True, 1.0, 1, True)
+    hyper = torch.tensor([lr, wd], device="cuda", dtype=torch.float32)
+    e.untile_apply(app_dev, len(shapes), unit, Th, Tw, tiles, hyper, True)
+    for g, m_ref, m, p_ref, p, (tb, R, C) in zip(grads, moms_ref, moms, params_ref, params, metas):
+        h, w = g.shape
+        buf = m_ref * mu + g
+        # two roundings of fp32 (values up to ~5): 5 * 2^-22 and the multiply-add contraction either way
+        _close(m, buf, atol=3e-6, rtol=1e-6)
+        padded = torch.zeros(R * Th, C * Tw, device="cuda")
+        padded[:h, :w] = g + mu * buf
+        got = tiles[tb:tb + R * C].view(R, C, Th, Tw).permute(0, 2, 1, 3).reshape(R * Th, C * Tw).float()
+        _close(got, padded, atol=1e-5, rtol=2 ** -8)       # stored in bf16
+        assert got[h:].abs().sum() == 0 and got[:, w:].abs().sum() == 0
+        _close(p, p_ref * (1 - lr * wd) - lr * scale * got[:h, :w], atol=3e-6, rtol=1e-6)

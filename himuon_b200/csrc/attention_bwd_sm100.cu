@@ -11,7 +11,13 @@
 //
 // TMEM (512 columns): S^T buffers at 0 and 64 (P^T over the first 32 columns of each), dP^T buffers at 128 and 192
 // (dS^T likewise), dV at 256, dK at 384.
-// Requires S to be a multiple of 128; the per-row statistics (log-sum-exp, delta) arrive by bulk copies.
+// Any sequence length: rows past S arrive as zeros (TMA) with a log-sum-exp of +inf, so their probabilities are 0, and
+// are not stored.  The per-row statistics (log-sum-exp, delta) arrive by bulk copies with the Q/dO stage when S is a
+// multiple of 64 (every sub-block is then whole and starts on 16 bytes); otherwise (RAGGED) each softmax group fetches
+// its sub-block's values itself, ahead of the wait for the scores.
+// Measured, whole backward pass on ragged lengths against the unpipelined kernels that served them before: 5 x 777 tokens
+// with 16 heads over 8 191 -> 139 us, 4 x 1000 with 32 over 8 373 -> 270 us, 2 x 1984 with 16 over 8 304 -> 205 us;
+// 4 x 1024 (whole sub-blocks) 149 us before and after.
 #include "attention_common.cuh"
 
 #include <string>
@@ -48,7 +54,7 @@ __device__ __forceinline__ void bulk_load_1d(void* dst, const void* src, uint32_
 
 }  // namespace
 
-template <int NH>
+template <int NH, bool RAGGED>
 __global__ void __launch_bounds__(BWD_THREADS, 1)
 flash_bwd_dkv_t_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                        const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmDO, AttnDev p) {
@@ -71,7 +77,7 @@ flash_bwd_dkv_t_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
   const int hk = p.split_heads ? hy / Gall : hy;
   const int h_first = p.split_heads ? hy : hk * Gall;
   const int out_head = p.split_heads ? hy : hk;
-  const int nsub = (p.S - kb * AT) / BQ;               // query sub-blocks from the diagonal to the end
+  const int nsub = (p.S - kb * AT + BQ - 1) / BQ;      // query sub-blocks from the diagonal to the end
   const int iters = G * nsub;
 
   if (threadIdx.x == 0) {
@@ -101,14 +107,16 @@ flash_bwd_dkv_t_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
         const int q0 = kb * AT + (it - g * nsub) * BQ;
         const int st = it % NST;
         if (!mbar_wait(&bars->qd_empty[st], ((it / NST) & 1) ^ 1, abort_flag, p.status, 4)) break;
-        mbar_expect_tx(&bars->qd_full[st], 2 * Q_TILE + STAT_BYTES);
+        mbar_expect_tx(&bars->qd_full[st], 2 * Q_TILE + (RAGGED ? 0 : STAT_BYTES));
         uint8_t* q_dst = sQ + st * Q_TILE;
         uint8_t* do_dst = sDO + st * Q_TILE;
         load_head_tile<NH>(q_dst, Q_HALF, &tmQ, &bars->qd_full[st], h, q0, b);
         load_head_tile<NH>(do_dst, Q_HALF, &tmDO, &bars->qd_full[st], h, q0, b);
-        const long long stat_idx = (static_cast<long long>(b) * p.Hq + h) * p.S + q0;
-        bulk_load_1d(sStat + st * 2 * BQ, p.lse + stat_idx, BQ * 4, &bars->qd_full[st]);
-        bulk_load_1d(sStat + st * 2 * BQ + BQ, p.delta + stat_idx, BQ * 4, &bars->qd_full[st]);
+        if (!RAGGED) {
+          const long long stat_idx = (static_cast<long long>(b) * p.Hq + h) * p.S + q0;
+          bulk_load_1d(sStat + st * 2 * BQ, p.lse + stat_idx, BQ * 4, &bars->qd_full[st]);
+          bulk_load_1d(sStat + st * 2 * BQ + BQ, p.delta + stat_idx, BQ * 4, &bars->qd_full[st]);
+        }
       }
     }
   } else if (warp == 1) {
@@ -161,6 +169,18 @@ flash_bwd_dkv_t_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
       const int g = it / nsub;
       const int q0 = kb * AT + (it - g * nsub) * BQ;
       const int st = it % NST;
+      // RAGGED: sub-block `it` has statistics slot it % NST, so a group alternates between two slots of its own.  A
+      // thread rewrites a slot two of its sub-blocks later, past the barrier of the one between, which every thread of
+      // the group reaches only after it has read this one.
+      if (RAGGED) {
+        const int qi = q0 + (row & (BQ - 1));
+        const long long stat_idx = (static_cast<long long>(b) * p.Hq + h_first + g) * p.S + qi;
+        const bool want_lse = row < BQ;
+        float v = want_lse ? INFINITY : 0.f;
+        if (qi < p.S) v = want_lse ? p.lse[stat_idx] : p.delta[stat_idx];
+        sStat[st * 2 * BQ + row] = v;
+        named_barrier(2 + wg, 128);
+      }
       if (!mbar_wait(&bars->qd_full[st], (it / NST) & 1, abort_flag, p.status, 4)) { ok = false; break; }
       if (!mbar_wait(&bars->s_full[buf], (it >> 1) & 1, abort_flag, p.status, 4)) { ok = false; break; }
       tc_fence_after();
@@ -213,7 +233,7 @@ flash_bwd_dkv_t_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
         uint32_t v[32];
         tmem_ld32(t_src + c * 32, v);
         tmem_ld_wait();
-        store_head32(dst0, c * 32, p.hd, v, out_scale);
+        if (kv_idx < p.S) store_head32(dst0, c * 32, p.hd, v, out_scale);
       }
     }
   }
@@ -257,7 +277,9 @@ flash_bwd_dq_t_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   attn_block_coords(sblk, h, b);
   const int qb = gridDim.x - 1 - sblk;                 // heavy (late) query blocks first
   const int hk = h / (p.Hq / p.Hkv);
-  const int nkv = (qb + 1) * (AT / BQ);                // KV sub-blocks up to and including the diagonal
+  int nkv = (qb + 1) * (AT / BQ);                      // KV sub-blocks up to and including the diagonal
+  const int nkv_all = (p.S + BQ - 1) / BQ;
+  if (nkv > nkv_all) nkv = nkv_all;
 
   if (threadIdx.x == 0) {
     mbar_init(&bars->qd_full, 1);
@@ -327,12 +349,16 @@ flash_bwd_dq_t_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     const uint32_t lane_off = static_cast<uint32_t>((warp & 3) * 32) << 16;
     const int q_idx = qb * AT + row;
     const long long stat_idx = (static_cast<long long>(b) * p.Hq + h) * p.S + q_idx;
-    const float lse2 = p.lse[stat_idx];
+    const bool row_ok = q_idx < p.S;
+    const float lse2 = row_ok ? p.lse[stat_idx] : INFINITY;
     if (wg == 0) {
+      float d = 0.f;
       const __nv_bfloat16* op = reinterpret_cast<const __nv_bfloat16*>(p.o_in) + (static_cast<long long>(b) * p.S + q_idx) * p.ld_o + h * p.hd;
       const __nv_bfloat16* gp = reinterpret_cast<const __nv_bfloat16*>(p.d_o) + (static_cast<long long>(b) * p.S + q_idx) * p.ld_do + h * p.hd;
-      const float d = row_delta(op, gp, p.hd);
-      p.delta[stat_idx] = d;
+      if (row_ok) {
+        d = row_delta(op, gp, p.hd);
+        p.delta[stat_idx] = d;
+      }
       bars->delta[row] = d;
     }
     named_barrier(1, 256);                                // both groups: the block's delta values are in shared memory
@@ -374,7 +400,7 @@ flash_bwd_dq_t_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         uint32_t v[32];
         tmem_ld32(tDQ + lane_off + c * 32, v);
         tmem_ld_wait();
-        store_head32(dqp, c * 32, p.hd, v, p.scale);
+        if (row_ok) store_head32(dqp, c * 32, p.hd, v, p.scale);
       }
     }
   }
@@ -386,28 +412,26 @@ flash_bwd_dq_t_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   }
 }
 
-// The pipelined kernels take sequence lengths that are multiples of 128 with 16-byte aligned row statistics; other
-// shapes run the kernels of attention_sm100.cu / attention_kv64_sm100.cu.
-bool flash_bwd_dkv_t_supported(const AttnArgs& a) {
-  return a.S % AT == 0 && (reinterpret_cast<uintptr_t>(a.lse) & 15) == 0 && (reinterpret_cast<uintptr_t>(a.delta) & 15) == 0;
-}
-
-bool flash_bwd_dq_t_supported(const AttnArgs& a) { return flash_bwd_dkv_t_supported(a); }
-
-template <int NH>
+template <int NH, bool RAGGED>
 static void launch_dkv_t(const AttnArgs& a, const AttnDev& p, int heads_y, cudaStream_t s) {
   constexpr size_t SMEM = 1024 + 2 * NH * HALF_BYTES + 2 * NST * NH * Q_HALF + NST * STAT_BYTES + sizeof(DkvBars) + 64;
   static bool attr = false;
-  if (!attr) { cudaFuncSetAttribute(flash_bwd_dkv_t_kernel<NH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM); attr = true; }
+  if (!attr) { cudaFuncSetAttribute(flash_bwd_dkv_t_kernel<NH, RAGGED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM); attr = true; }
   const CUtensorMap tq = head_tmap(a.q, a.B, a.S, a.Hq, a.hd, a.ld_q, BQ), tk = head_tmap(a.k, a.B, a.S, a.Hkv, a.hd, a.ld_k),
                     tv = head_tmap(a.v, a.B, a.S, a.Hkv, a.hd, a.ld_v), tdo = head_tmap(a.d_o, a.B, a.S, a.Hq, a.hd, a.ld_do, BQ);
-  flash_bwd_dkv_t_kernel<NH><<<dim3(p.nblk, heads_y, a.B), BWD_THREADS, SMEM, s>>>(tq, tk, tv, tdo, p);
+  flash_bwd_dkv_t_kernel<NH, RAGGED><<<dim3(p.nblk, heads_y, a.B), BWD_THREADS, SMEM, s>>>(tq, tk, tv, tdo, p);
 }
 // `p` carries the output pointers and the split_heads flag chosen by the caller; the grid's y extent is the number of
 // query heads (split_heads) or KV heads.
 void flash_bwd_dkv_t(const AttnArgs& a, const AttnDev& p, int heads_y, cudaStream_t s) {
-  if (head_halves(a.hd) == 1) launch_dkv_t<1>(a, p, heads_y, s);
-  else launch_dkv_t<2>(a, p, heads_y, s);
+  const bool whole = a.S % BQ == 0 && (reinterpret_cast<uintptr_t>(a.lse) & 15) == 0 && (reinterpret_cast<uintptr_t>(a.delta) & 15) == 0;
+  if (head_halves(a.hd) == 1) {
+    if (whole) launch_dkv_t<1, false>(a, p, heads_y, s);
+    else launch_dkv_t<1, true>(a, p, heads_y, s);
+  } else {
+    if (whole) launch_dkv_t<2, false>(a, p, heads_y, s);
+    else launch_dkv_t<2, true>(a, p, heads_y, s);
+  }
 }
 
 template <int NH>

@@ -18,18 +18,9 @@ constexpr uint32_t HALF_BYTES = 16384;  // [128 rows][64 columns] bf16
 inline int head_halves(int hd) { return hd <= 64 ? 1 : 2; }
 constexpr float kLog2e = 1.4426950408889634f;
 
-// Byte offset of the 16-byte chunk `c16` (0..15) of row `r` in a [128 rows][128 cols] bf16 tile
-// stored as two K-major SWIZZLE_128B halves.
-__device__ __forceinline__ uint32_t sw128_off(int r, int c16) {
-  return static_cast<uint32_t>((c16 >> 3) * HALF_BYTES + r * 128 + (((c16 & 7) ^ (r & 7)) << 4));
-}
-// K-major operand descriptor for k-step ks (16 columns each) of such a tile.
+// K-major operand descriptor for k-step ks (16 columns each) of a [128 rows][64 * NH columns] tile in swizzled halves.
 __device__ __forceinline__ uint64_t desc_kmajor(uint32_t base, int ks) {
   return umma_smem_desc(base + (ks >> 2) * HALF_BYTES + (ks & 3) * 32, 16, 1024);
-}
-// MN-major operand descriptor for k-step ks (16 rows each) of the same bytes viewed as [K rows][M/N cols].
-__device__ __forceinline__ uint64_t desc_mnmajor(uint32_t base, int ks) {
-  return umma_smem_desc(base + ks * 2048, HALF_BYTES, 1024);
 }
 
 struct AttnDev {
@@ -42,18 +33,6 @@ struct AttnDev {
   long long ld_o, ld_do, ld_dq, ld_dk, ld_dv;
   float scale_log2, scale;
   int* status;
-};
-
-struct AttnBars {
-  uint64_t q_full, k_full[2], v_full[2], k_empty[2], v_empty[2], s_full[2], s_empty[2], p_ready, o_done;
-  uint32_t tmem_slot;
-  int abort_flag;
-};
-
-struct BwdBars {
-  uint64_t a_full, a_empty, b_full, b_empty, sp_full, ds_ready, acc_done;
-  uint32_t tmem_slot;
-  int abort_flag;
 };
 
 // 4-D tensor map over a (B, S, H, hd) view: box = 64 head-dim columns x `rows` sequence positions of one head.
@@ -110,14 +89,9 @@ __device__ __forceinline__ void store_head32(__nv_bfloat16* row, int col, int hd
   }
 }
 
-// 64-wide KV-block kernels (two CTAs per SM): forward and dQ.
+// Forward (two CTAs per SM); dK/dV and dQ in the pipelined formulation of attention_bwd_sm100.cu.
 void flash_fwd_kv64(const AttnArgs& a, cudaStream_t s);
-void flash_bwd_dq_kv64(const AttnArgs& a, cudaStream_t s);
-
-// dK/dV pass in the transposed formulation (P^T and dS^T stay in tensor memory); S must be a multiple of 128.
-bool flash_bwd_dkv_t_supported(const AttnArgs& a);
 void flash_bwd_dkv_t(const AttnArgs& a, const AttnDev& p, int heads_y, cudaStream_t s);
-bool flash_bwd_dq_t_supported(const AttnArgs& a);
 void flash_bwd_dq_t(const AttnArgs& a, const AttnDev& p, cudaStream_t s);
 
 }  // namespace himuon

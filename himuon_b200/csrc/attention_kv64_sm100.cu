@@ -1,8 +1,7 @@
-// Flash attention forward and dQ kernels with 64-wide KV blocks.
+// Flash attention forward with 64-wide KV blocks.
 //
 // K/V arrive in blocks of 64 positions: shared memory stays at 96 KB and the TMEM footprint at 256 columns, so two
-// CTAs run on every SM and one CTA's tensor-core work overlaps the other's softmax.  The dQ kernel here serves
-// sequence lengths that are not a multiple of 128; the others take the pipelined kernel of attention_bwd_sm100.cu.
+// CTAs run on every SM and one CTA's tensor-core work overlaps the other's softmax.
 #include "attention_common.cuh"
 
 #include <string>
@@ -11,19 +10,12 @@ namespace himuon {
 
 constexpr int BKV = 64;                              // KV positions per block
 constexpr uint32_t KV_HALF = BKV * 128;              // one 64-column half of a K or V block: 8 KB
-constexpr uint32_t P_BYTES = AT * BKV * 2;           // probabilities / dS of one block: 128 x 64 bf16 = 16 KB
 
 __device__ __forceinline__ uint64_t kv_desc_kmajor(uint32_t base, int ks) {   // K block as the K-major B operand of Q K^T
   return umma_smem_desc(base + (ks >> 2) * KV_HALF + (ks & 3) * 32, 16, 1024);
 }
 __device__ __forceinline__ uint64_t kv_desc_mnmajor(uint32_t base, int ks) {  // K or V block read along the head dim
   return umma_smem_desc(base + ks * 2048, KV_HALF, 1024);
-}
-__device__ __forceinline__ uint64_t p_desc_kmajor(uint32_t base, int ks) {    // 128 x 64 block, one 128-byte line per row
-  return umma_smem_desc(base + ks * 32, 16, 1024);
-}
-__device__ __forceinline__ uint32_t p_off(int r, int c16) {                  // 16-byte chunk c16 (0..7) of row r
-  return static_cast<uint32_t>(r * 128 + ((c16 ^ (r & 7)) << 4));
 }
 
 // ================================================================================================ forward, P in TMEM
@@ -216,148 +208,6 @@ flash_fwd64_t_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   }
 }
 
-// ================================================================================================ backward: dQ
-// CTA = (query block, head, batch).  Resident: Q, dO.  Streamed: K_j, V_j (64 positions).  dS reuses V's shared
-// memory once dP = dO V^T has consumed V.  TMEM: S (64) | dP (64) | dQ (128).
-template <int NH>
-__global__ void __launch_bounds__(192, 2)
-flash_bwd_dq64_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
-                      const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmDO, AttnDev p) {
-  constexpr uint32_t TILE_BYTES = NH * HALF_BYTES, KV_TILE = NH * KV_HALF;
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = align_up_1024(smem_raw);
-  uint8_t* sQ = smem;
-  uint8_t* sDO = smem + TILE_BYTES;
-  uint8_t* sK = smem + 2 * TILE_BYTES;
-  uint8_t* sV = sK + KV_TILE;
-  uint8_t* sDS = sV;                                    // alias (see above)
-  BwdBars* bars = reinterpret_cast<BwdBars*>(sV + (KV_TILE > P_BYTES ? KV_TILE : P_BYTES));
-  volatile int* abort_flag = &bars->abort_flag;
-
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  int sblk, h, b;
-  attn_block_coords(sblk, h, b);
-  const int qb = gridDim.x - 1 - sblk;         // heavy (late) query blocks first
-  const int hk = h / (p.Hq / p.Hkv);
-  int nkv = (qb + 1) * (AT / BKV);
-  const int nkv_all = (p.S + BKV - 1) / BKV;
-  if (nkv > nkv_all) nkv = nkv_all;
-
-  if (threadIdx.x == 0) {
-    mbar_init(&bars->a_full, 1); mbar_init(&bars->a_empty, 1);
-    mbar_init(&bars->b_full, 1); mbar_init(&bars->b_empty, 1);
-    mbar_init(&bars->sp_full, 1); mbar_init(&bars->ds_ready, 128); mbar_init(&bars->acc_done, 1);
-    bars->abort_flag = 0;
-    mbar_fence_init();
-  }
-  if (warp == 1) tmem_alloc(&bars->tmem_slot, 256);
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem = bars->tmem_slot;
-  const uint32_t tS = tmem, tDP = tmem + 64, tDQ = tmem + 128;
-
-  if (warp == 0) {
-    if (lane == 0) {
-      mbar_expect_tx(&bars->a_full, 2 * TILE_BYTES);
-      load_head_tile<NH>(sQ, HALF_BYTES, &tmQ, &bars->a_full, h, qb * AT, b);
-      load_head_tile<NH>(sDO, HALF_BYTES, &tmDO, &bars->a_full, h, qb * AT, b);
-      for (int j = 0; j < nkv; ++j) {
-        if (!mbar_wait(&bars->b_empty, (j & 1) ^ 1, abort_flag, p.status, 4)) break;
-        mbar_expect_tx(&bars->b_full, 2 * KV_TILE);
-        load_head_tile<NH>(sK, KV_HALF, &tmK, &bars->b_full, hk, j * BKV, b);
-        load_head_tile<NH>(sV, KV_HALF, &tmV, &bars->b_full, hk, j * BKV, b);
-      }
-    }
-  } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc_kk = umma_idesc_bf16(128, BKV, false, false);
-      constexpr uint32_t idesc_kmn = umma_idesc_bf16(128, 64 * NH, false, true);
-      const uint32_t q_base = smem_u32(sQ), do_base = smem_u32(sDO), k_base = smem_u32(sK), v_base = smem_u32(sV),
-                     ds_base = smem_u32(sDS);
-      bool ok = mbar_wait(&bars->a_full, 0, abort_flag, p.status, 4);
-      for (int j = 0; ok && j < nkv; ++j) {
-        if (!mbar_wait(&bars->b_full, j & 1, abort_flag, p.status, 4)) break;
-        tc_fence_after();
-#pragma unroll
-        for (int ks = 0; ks < 4 * NH; ++ks) umma_ss(tS, desc_kmajor(q_base, ks), kv_desc_kmajor(k_base, ks), idesc_kk, ks > 0 ? 1u : 0u);
-#pragma unroll
-        for (int ks = 0; ks < 4 * NH; ++ks) umma_ss(tDP, desc_kmajor(do_base, ks), kv_desc_kmajor(v_base, ks), idesc_kk, ks > 0 ? 1u : 0u);
-        umma_commit(&bars->sp_full);
-        if (!mbar_wait(&bars->ds_ready, j & 1, abort_flag, p.status, 4)) break;
-        tc_fence_after();
-#pragma unroll
-        for (int ks = 0; ks < BKV / 16; ++ks)
-          umma_ss(tDQ, p_desc_kmajor(ds_base, ks), kv_desc_mnmajor(k_base, ks), idesc_kmn, (j > 0 || ks > 0) ? 1u : 0u);
-        umma_commit(&bars->b_empty);
-        umma_commit(&bars->acc_done);
-      }
-    }
-  } else {
-    const int row = (warp & 3) * 32 + lane;
-    const uint32_t lane_off = static_cast<uint32_t>((warp & 3) * 32) << 16;
-    const int q_idx = qb * AT + row;
-    const bool row_ok = q_idx < p.S;
-    const long long stat_idx = (static_cast<long long>(b) * p.Hq + h) * p.S + q_idx;
-    float lse2 = 0.f, delta = 0.f;
-    if (row_ok) {
-      lse2 = p.lse[stat_idx];
-      const __nv_bfloat16* op = reinterpret_cast<const __nv_bfloat16*>(p.o_in) + (static_cast<long long>(b) * p.S + q_idx) * p.ld_o + h * p.hd;
-      const __nv_bfloat16* gp = reinterpret_cast<const __nv_bfloat16*>(p.d_o) + (static_cast<long long>(b) * p.S + q_idx) * p.ld_do + h * p.hd;
-      delta = row_delta(op, gp, p.hd);
-      p.delta[stat_idx] = delta;
-    }
-    bool ok = true;
-    for (int j = 0; j < nkv; ++j) {
-      if (!mbar_wait(&bars->sp_full, j & 1, abort_flag, p.status, 4)) { ok = false; break; }
-      tc_fence_after();
-      const int kv0 = j * BKV;
-      const bool diag = (kv0 + BKV - 1 > qb * AT);
-#pragma unroll
-      for (int c = 0; c < BKV / 32; ++c) {
-        uint32_t sv[32], dv[32];
-        tmem_ld32(tS + lane_off + c * 32, sv);
-        tmem_ld32(tDP + lane_off + c * 32, dv);
-        tmem_ld_wait();
-        uint32_t pk[16];
-#pragma unroll
-        for (int t = 0; t < 32; t += 2) {
-          float p0 = exp2f(__uint_as_float(sv[t]) * p.scale_log2 - lse2);
-          float p1 = exp2f(__uint_as_float(sv[t + 1]) * p.scale_log2 - lse2);
-          if (!row_ok || (diag && (kv0 + c * 32 + t > q_idx))) p0 = 0.f;
-          if (!row_ok || (diag && (kv0 + c * 32 + t + 1 > q_idx))) p1 = 0.f;
-          pk[t >> 1] = pack_bf16x2(p0 * (__uint_as_float(dv[t]) - delta) * p.scale,
-                                   p1 * (__uint_as_float(dv[t + 1]) - delta) * p.scale);
-        }
-        // sp_full means both S and dP (which read V) are complete, so V's buffer may now hold dS
-#pragma unroll
-        for (int q = 0; q < 4; ++q)
-          *reinterpret_cast<uint4*>(sDS + p_off(row, c * 4 + q)) = make_uint4(pk[4 * q], pk[4 * q + 1], pk[4 * q + 2], pk[4 * q + 3]);
-      }
-      tc_fence_before();
-      fence_proxy_async_smem();
-      mbar_arrive(&bars->ds_ready);
-    }
-    if (ok && mbar_wait(&bars->acc_done, (nkv - 1) & 1, abort_flag, p.status, 4)) {
-      tc_fence_after();
-      __nv_bfloat16* dqp = reinterpret_cast<__nv_bfloat16*>(p.dq) + (static_cast<long long>(b) * p.S + q_idx) * p.ld_dq + h * p.hd;
-#pragma unroll 1
-      for (int c = 0; c < 2 * NH; ++c) {
-        uint32_t v[32];
-        tmem_ld32(tDQ + lane_off + c * 32, v);
-        tmem_ld_wait();
-        if (row_ok) store_head32(dqp, c * 32, p.hd, v, 1.f);
-      }
-    }
-  }
-  tc_fence_before();
-  __syncthreads();
-  if (warp == 1) {
-    tc_fence_after();
-    tmem_dealloc(tmem, 256);
-  }
-}
-
 // ================================================================================================ host
 static AttnDev make_dev(const AttnArgs& a) {
   AttnDev p{};
@@ -387,21 +237,6 @@ static void launch_fwd(const AttnArgs& a, cudaStream_t s) {
 void flash_fwd_kv64(const AttnArgs& a, cudaStream_t s) {
   if (head_halves(a.hd) == 1) launch_fwd<1>(a, s);
   else launch_fwd<2>(a, s);
-}
-
-template <int NH>
-static void launch_dq64(const AttnArgs& a, cudaStream_t s) {
-  constexpr size_t SMEM = 1024 + 2 * NH * HALF_BYTES + KV_HALF * NH + (NH * KV_HALF > P_BYTES ? NH * KV_HALF : P_BYTES) + 256;
-  static bool attr = false;
-  if (!attr) { cudaFuncSetAttribute(flash_bwd_dq64_kernel<NH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM); attr = true; }
-  const AttnDev p = make_dev(a);
-  const CUtensorMap tq = head_tmap(a.q, a.B, a.S, a.Hq, a.hd, a.ld_q), tk = head_tmap(a.k, a.B, a.S, a.Hkv, a.hd, a.ld_k, BKV),
-                    tv = head_tmap(a.v, a.B, a.S, a.Hkv, a.hd, a.ld_v, BKV), tdo = head_tmap(a.d_o, a.B, a.S, a.Hq, a.hd, a.ld_do);
-  flash_bwd_dq64_kernel<NH><<<dim3(p.nblk, a.Hq, a.B), 192, SMEM, s>>>(tq, tk, tv, tdo, p);
-}
-void flash_bwd_dq_kv64(const AttnArgs& a, cudaStream_t s) {
-  if (head_halves(a.hd) == 1) launch_dq64<1>(a, s);
-  else launch_dq64<2>(a, s);
 }
 
 }  // namespace himuon

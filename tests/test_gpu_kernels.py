@@ -539,3 +539,24 @@ def test_fp32_momentum_tile_and_untile_apply(tile, offset):
         _close(got, padded, atol=1e-5, rtol=2 ** -8)       # stored in bf16
         assert got[h:].abs().sum() == 0 and got[:, w:].abs().sum() == 0
         _close(p, p_ref * (1 - lr * wd) - lr * scale * got[:h, :w], atol=3e-6, rtol=1e-6)
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("B,S,Hq,Hkv", [(1, 1, 1, 1), (2, 63, 2, 1), (1, 65, 2, 2), (2, 192, 4, 2), (1, 255, 4, 1), (1, 777, 2, 1)])
+def test_attention_ragged_lengths(D, B, S, Hq, Hkv):
+    """Sequence lengths around the 64- and 128-position blocks of the backward kernels."""
+    from himuon_b200 import ops
+
+    torch.manual_seed(3)
+    ins = [torch.randn(B * S, h * D, device="cuda", dtype=torch.bfloat16, requires_grad=True) for h in (Hq, Hkv, Hkv)]
+    o = ops.attention(*ins, B, S, Hq, Hkv, D)
+    do = torch.randn_like(o)
+    o.backward(do)
+    ref_in = [t.detach().float().view(B, S, h, D).requires_grad_(True) for t, h in zip(ins, (Hq, Hkv, Hkv))]
+    ref = _attn_ref(*ref_in, 1.0 / math.sqrt(D))
+    ref.backward(do.float().view(B, S, Hq, D))
+    _assert_status_clean()
+    # bounds of test_flash_attention_fwd_bwd, which covers the same sums up to 1024 positions
+    _close(o, ref.reshape(B * S, Hq * D), atol=2e-2, rtol=2e-2)
+    for t, r in zip(ins, ref_in):
+        _close(t.grad, r.grad.reshape(t.shape), atol=3e-2, rtol=3e-2)

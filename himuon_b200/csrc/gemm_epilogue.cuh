@@ -161,14 +161,60 @@ __device__ __forceinline__ void load_aux_slab(const void* aux, long long elem_of
   }
 }
 
-// Epilogue of one accumulator tile through swizzled shared-memory slabs and TMA stores.  Called by the 128
+// One bf16 slab (64 columns) of the one-CTA kernel: accumulator -> alpha, rounding, beta * aux -> swizzled staging row.
+// The aux values are either already in the row (IN_PLACE) or in `xa` (zeros when there is no aux).
+template <bool IN_PLACE>
+__device__ __forceinline__ void slab_bf16(uint32_t t_slab, uint8_t* my_row, int row_in_tile, const uint4 (&xa)[8], float alpha,
+                                          float beta, int round_acc, __nv_bfloat16* mirror_c, long long mirror_ld, int col,
+                                          int row, int N) {
+#pragma unroll
+  for (int ch = 0; ch < 2; ++ch) {
+    uint32_t v[32];
+    tmem_ld32(t_slab + ch * 32, v);
+    tmem_ld_wait();
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int j = ch * 4 + q;
+      uint4* cell = reinterpret_cast<uint4*>(my_row + ((j ^ (row_in_tile & 7)) << 4));
+      const uint4 e = IN_PLACE ? *cell : xa[j];
+      const uint32_t ew[4] = {e.x, e.y, e.z, e.w};
+      uint32_t o[4];
+#pragma unroll
+      for (int t = 0; t < 4; ++t) {
+        float f0 = alpha * __uint_as_float(v[8 * q + 2 * t]);
+        float f1 = alpha * __uint_as_float(v[8 * q + 2 * t + 1]);
+        if (round_acc) { f0 = round_bf16(f0); f1 = round_bf16(f1); }
+        o[t] = pack_bf16x2(f0 + beta * bf16_lo(ew[t]), f1 + beta * bf16_hi(ew[t]));
+      }
+      *cell = make_uint4(o[0], o[1], o[2], o[3]);
+      if (mirror_c != nullptr) mirror_store8(mirror_c, mirror_ld, col + j * 8, row, N, o);
+    }
+  }
+}
+// The same for one fp32 slab (32 columns).
+__device__ __forceinline__ void slab_fp32(uint32_t t_slab, uint8_t* my_row, int row_in_tile, const uint4 (&xa)[8], float alpha,
+                                          float beta) {
+  uint32_t v[32];
+  tmem_ld32(t_slab, v);
+  tmem_ld_wait();
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    float4 o;
+    o.x = alpha * __uint_as_float(v[4 * j + 0]) + beta * __uint_as_float(xa[j].x);
+    o.y = alpha * __uint_as_float(v[4 * j + 1]) + beta * __uint_as_float(xa[j].y);
+    o.z = alpha * __uint_as_float(v[4 * j + 2]) + beta * __uint_as_float(xa[j].z);
+    o.w = alpha * __uint_as_float(v[4 * j + 3]) + beta * __uint_as_float(xa[j].w);
+    *reinterpret_cast<float4*>(my_row + ((j ^ (row_in_tile & 7)) << 4)) = o;
+  }
+}
+
+// Pair kernel: epilogue of one accumulator tile through swizzled shared-memory slabs and TMA stores.  Called by the 128
 // epilogue threads together.  `slab_seq` numbers the slabs this CTA has stored so far (selects the staging buffer).
 template <int BN, bool OUT_FP32>
 __device__ __forceinline__ void epilogue_tile_tma(const CUtensorMap* tmC, uint8_t* sC, uint32_t t_row, int row_in_tile,
                                                   int m0, int n0, int b, const void* aux, long long aux_row_off,
                                                   int M, int N, float alpha, float beta, int round_acc,
-                                                  uint32_t& slab_seq, bool issuer, bool reduce_add = false,
-                                                  __nv_bfloat16* mirror_c = nullptr, long long mirror_ld = 0) {
+                                                  uint32_t& slab_seq, bool issuer, bool reduce_add = false) {
   constexpr int SW = OUT_FP32 ? 32 : 64;
   constexpr int SLABS = BN / SW;
   const bool row_ok = (m0 + row_in_tile) < M;
@@ -212,7 +258,6 @@ __device__ __forceinline__ void epilogue_tile_tma(const CUtensorMap* tmC, uint8_
           }
           const int j = ch * 4 + q;
           *reinterpret_cast<uint4*>(my_row + ((j ^ (row_in_tile & 7)) << 4)) = make_uint4(o[0], o[1], o[2], o[3]);
-          if (mirror_c != nullptr) mirror_store8(mirror_c, mirror_ld, col + j * 8, m0 + row_in_tile, N, o);
         }
       }
     }

@@ -2,8 +2,15 @@
 //
 //   * operands are staged by TMA (128-byte swizzle, no multicast) into a shared-memory ring,
 //   * one elected thread issues tcgen05.mma (M=128, N=BN, K=16) into TMEM accumulators,
-//   * four epilogue warps read TMEM with tcgen05.ld, apply the epilogue and store,
+//   * eight epilogue warps, two groups of four that take alternate 64-column slabs of the tile, read TMEM with
+//     tcgen05.ld and combine into shared-memory slabs; one thread of its own (the slab warp) stores the finished slabs
+//     by TMA and hands the drained ones out again, with the next aux tile already in them,
 //   * two TMEM accumulators (2 x BN columns) let the epilogue of tile i overlap the MMAs of tile i+1.
+//
+// Why two groups: a 128 x 256 x 512 tile (Newton-Schulz on 512 tiles) is 3 us of MMA, and one group of four warps
+// needed 6.6 us to drain it - the epilogue, not the main loop, bound every short-K product.
+// Measured with two: optimizer step on 2300 tiles of 512 15.1 -> 12.8 ms, on 28 of them 346 -> 287 us, 128 tiles through
+// newton_schulz 853 -> 756 us.
 //
 // Either operand may be K-major (reduction dim contiguous) or MN-major (M/N contiguous),
 // so forward (x W^T), dgrad (dy W) and wgrad (dy^T x) all run without a transpose pass.
@@ -21,13 +28,14 @@ namespace himuon {
 __device__ int g_status_word = 0;
 
 // AUX_TMA (bf16 output with an aux operand): the aux tile arrives by TMA in the very staging slab that its output slab
-// leaves from.  Four slabs rotate through load -> combine in place -> store, with the load issued two slabs ahead
+// leaves from.  NSTG slabs rotate through load -> combine in place -> store, with the loads issued three slabs ahead
 // (across tile boundaries), so the epilogue threads never wait on global memory.
-template <int BN, int STAGES, bool A_MN, bool B_MN, bool AUX_TMA = false>
-__global__ void __launch_bounds__(256, 1)
+constexpr int NSTG = 4;                       // staging slabs
+constexpr int GEMM_THREADS = 384;             // warps 0-3: TMA, MMA, TMEM allocation, slabs; 4-11: epilogue
+template <int BN, int STAGES, bool A_MN, bool B_MN, bool AUX_TMA>
+__global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                  const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CUtensorMap tmX, GemmDev p) {
-  constexpr int NSTG = AUX_TMA ? 4 : 2;       // staging slabs
   constexpr uint32_t A_BYTES = BM * BK * 2;
   constexpr uint32_t B_BYTES = BN * BK * 2;
   constexpr uint32_t STAGE_BYTES = A_BYTES + B_BYTES;
@@ -35,14 +43,15 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = align_up_1024(smem_raw);
-  uint8_t* sC = smem + STAGES * STAGE_BYTES;                      // two staging slabs for the TMA-store epilogue
+  uint8_t* sC = smem + STAGES * STAGE_BYTES;                      // staging slabs of the TMA-store epilogue
   uint64_t* bars = reinterpret_cast<uint64_t*>(sC + NSTG * SLAB_BYTES);
   uint64_t* full = bars;
   uint64_t* empty = bars + STAGES;
   uint64_t* tfull = bars + 2 * STAGES;
   uint64_t* tempty = tfull + 2;
-  uint64_t* aux_full = tempty + 2;            // AUX_TMA: one per staging slab
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(aux_full + 4);
+  uint64_t* slab_open = tempty + 2;           // one per slab: free (and, with AUX_TMA, holding its aux tile)
+  uint64_t* slab_done = slab_open + NSTG;     // one per slab: combined by the 128 threads of a group
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(slab_done + NSTG);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5;
@@ -55,9 +64,9 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(&tfull[a], 1);
-      mbar_init(&tempty[a], 4);
+      mbar_init(&tempty[a], 8);
     }
-    for (int a = 0; a < 4; ++a) mbar_init(&aux_full[a], 1);
+    for (int a = 0; a < NSTG; ++a) { mbar_init(&slab_open[a], 1); mbar_init(&slab_done[a], 128); }
     *abort_flag = 0;
     mbar_fence_init();
   }
@@ -138,117 +147,93 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         if (acc == 0) acc_phase ^= 1;
       }
     }
+  } else if (warp == 3) {
+    // ------------------------------------------------------------ slab warp: aux loads and output stores
+    if (lane == 0 && p.tma_store) {
+      tma_prefetch_desc(&tmC);
+      if (AUX_TMA) tma_prefetch_desc(&tmX);
+      const int sw = p.out_fp32 ? 32 : 64;                  // columns of a slab (128 bytes)
+      // Two cursors over the slabs of this CTA in the order the epilogue visits them: `op` opens slabs, `st` stores them.
+      struct Cursor { int item, col, left; TileCoord tc; } op, st;
+      auto enter_tile = [&](Cursor& c) {
+        if (c.item >= p.total_items) return;
+        c.tc = decode_tile(p, c.item, BN / BM);
+        c.col = c.tc.nt * BN;
+        const int n = min(BN, p.N - c.col);
+        c.left = (n + sw - 1) / sw;
+      };
+      auto advance = [&](Cursor& c) {
+        c.col += sw;
+        if (--c.left == 0) { c.item += gridDim.x; enter_tile(c); }
+      };
+      op.item = st.item = blockIdx.x;
+      enter_tile(op);
+      enter_tile(st);
+      uint32_t opened = 0, seq = 0;
+      auto open_next = [&]() {
+        if (op.item >= p.total_items) return;
+        const uint32_t buf = opened & (NSTG - 1);
+        if (AUX_TMA) {
+          mbar_expect_tx(&slab_open[buf], SLAB_BYTES);
+          tma_load_3d(sC + buf * SLAB_BYTES, &tmX, &slab_open[buf], op.col, op.tc.mt * BM, op.tc.b);
+        } else {
+          mbar_arrive(&slab_open[buf]);
+        }
+        ++opened;
+        advance(op);
+      };
+      for (int a = 0; a < NSTG - 1; ++a) open_next();
+      while (st.item < p.total_items) {
+        const uint32_t buf = seq & (NSTG - 1);
+        if (!mbar_wait(&slab_done[buf], (seq / NSTG) & 1, abort_flag, p.status, 5)) break;
+        tma_store_3d(&tmC, sC + buf * SLAB_BYTES, st.col, st.tc.mt * BM, st.tc.b);
+        tma_store_commit();
+        tma_store_wait_read<1>();        // the slab stored before this one is drained: it is the next to be opened
+        open_next();
+        ++seq;
+        advance(st);
+      }
+      tma_store_wait_read<0>();          // no store may still be reading shared memory at exit
+    }
   } else if (warp >= 4) {
-    // ------------------------------------------------------------ epilogue (warps 4..7 -> TMEM lanes 0..127)
+    // ------------------------------------------------------------ epilogue (two groups of four warps -> TMEM lanes 0..127)
     const int ew = warp & 3;
+    const uint32_t eg = static_cast<uint32_t>(warp - 4) >> 2;
     int acc = 0;
     uint32_t acc_phase = 0;
-    uint32_t slab_seq = 0;
-    const bool issuer = (threadIdx.x == 128);
-    if (issuer && p.tma_store) tma_prefetch_desc(&tmC);
-    if constexpr (AUX_TMA) {
-      constexpr int SW = 64, SLABS = BN / SW;
-      const int row_in_tile = ew * 32 + lane;
-      // Prefetch cursor (issuer only): the (tile, slab) pairs of this CTA in the order the epilogue visits them.
-      int pf_item = blockIdx.x, pf_sl = 0;
-      uint32_t pf_seq = 0;
-      auto prefetch_next = [&]() {
-        while (pf_item < p.total_items) {
-          const TileCoord tc = decode_tile(p, pf_item, BN / BM);
-          const int b = tc.b, mt = tc.mt, nt = tc.nt;
-          const int col = nt * BN + pf_sl * SW;
-          if (col < p.N) {
-            const uint32_t buf = pf_seq & 3;
-            mbar_expect_tx(&aux_full[buf], SLAB_BYTES);
-            tma_load_3d(sC + buf * SLAB_BYTES, &tmX, &aux_full[buf], col, mt * BM, b);
-            ++pf_seq;
-            if (++pf_sl == SLABS) { pf_sl = 0; pf_item += gridDim.x; }
-            return;
-          }
-          pf_sl = 0;                         // the rest of this tile lies past N
-          pf_item += gridDim.x;
-        }
-      };
-      if (issuer) {
-        tma_prefetch_desc(&tmX);
-        prefetch_next();
-        prefetch_next();
-      }
-      uint32_t g = 0;                        // slabs finished by this CTA
-      bool ok = true;
-      for (int item = blockIdx.x; ok && item < p.total_items; item += gridDim.x) {
-        const TileCoord tc = decode_tile(p, item, BN / BM);
-        const int b = tc.b, mt = tc.mt, nt = tc.nt;
-        __nv_bfloat16* mirror_c = tc.mirror ? reinterpret_cast<__nv_bfloat16*>(p.C) + static_cast<long long>(b) * p.strideC : nullptr;
-        if (!mbar_wait(&tfull[acc], acc_phase, abort_flag, p.status, 3)) break;
-        tc_fence_after();
-        const uint32_t t_acc = tmem_base + (static_cast<uint32_t>(ew * 32) << 16) + static_cast<uint32_t>(acc * BN);
-#pragma unroll 1
-        for (int sl = 0; sl < SLABS; ++sl) {
-          const int col = nt * BN + sl * SW;
-          if (col >= p.N) break;             // uniform over the 128 threads
-          const uint32_t buf = g & 3;
-          uint8_t* my_row = sC + buf * SLAB_BYTES + row_in_tile * 128;
-          if (!mbar_wait(&aux_full[buf], (g >> 2) & 1, abort_flag, p.status, 5)) { ok = false; break; }
-#pragma unroll
-          for (int ch = 0; ch < 2; ++ch) {
-            uint32_t v[32];
-            tmem_ld32(t_acc + sl * SW + ch * 32, v);
-            tmem_ld_wait();
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-              uint4* cell = reinterpret_cast<uint4*>(my_row + (((ch * 4 + q) ^ (row_in_tile & 7)) << 4));
-              const uint4 e = *cell;
-              const uint32_t ew4[4] = {e.x, e.y, e.z, e.w};
-              uint32_t o[4];
-#pragma unroll
-              for (int t = 0; t < 4; ++t) {
-                float f0 = p.alpha * __uint_as_float(v[8 * q + 2 * t]);
-                float f1 = p.alpha * __uint_as_float(v[8 * q + 2 * t + 1]);
-                if (p.round_acc) { f0 = round_bf16(f0); f1 = round_bf16(f1); }
-                o[t] = pack_bf16x2(f0 + p.beta * bf16_lo(ew4[t]), f1 + p.beta * bf16_hi(ew4[t]));
-              }
-              *cell = make_uint4(o[0], o[1], o[2], o[3]);
-              if (mirror_c != nullptr) mirror_store8(mirror_c, p.ldc, col + (ch * 4 + q) * 8, mt * BM + row_in_tile, p.N, o);
-            }
-          }
-          fence_proxy_async_smem();
-          named_barrier(1, 128);             // the whole slab is combined
-          if (issuer) {
-            tma_store_3d(&tmC, sC + buf * SLAB_BYTES, col, mt * BM, b);
-            tma_store_commit();
-            tma_store_wait_read<1>();        // the slab stored before this one is drained: its buffer takes slab g+2
-            prefetch_next();
-          }
-          ++g;
-        }
-        if (!ok) break;
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&tempty[acc]);
-        acc ^= 1;
-        if (acc == 0) acc_phase ^= 1;
-      }
-      if (issuer) tma_store_wait_read<0>();
-    } else
-    for (int item = blockIdx.x; item < p.total_items; item += gridDim.x) {
-      const WorkItem w = decode_item(p, item);
-      const TileCoord tc = decode_tile(p, w.tile, BN / BM);
+    uint32_t seq = 0;                        // slabs of this CTA so far; group eg takes those of its parity
+    const int row_in_tile = ew * 32 + lane;
+    bool ok = true;
+    for (int item = blockIdx.x; ok && item < p.total_items; item += gridDim.x) {
+      const TileCoord tc = decode_tile(p, item, BN / BM);
       const int b = tc.b, mt = tc.mt, nt = tc.nt;
       if (!mbar_wait(&tfull[acc], acc_phase, abort_flag, p.status, 3)) break;
       tc_fence_after();
       if (p.tma_store) {
-        const int row_in_tile = ew * 32 + lane;
         const uint32_t t_acc = tmem_base + (static_cast<uint32_t>(ew * 32) << 16) + static_cast<uint32_t>(acc * BN);
-        const long long aux_row = static_cast<long long>(b) * p.strideAux + static_cast<long long>(mt * BM + row_in_tile) * p.ldaux;
-        if (p.out_fp32)
-          epilogue_tile_tma<BN, true>(&tmC, sC, t_acc, row_in_tile, mt * BM, nt * BN, b, p.aux, aux_row, p.M, p.N,
-                                      p.alpha, p.beta, p.round_acc, slab_seq, issuer);
-        else
-          epilogue_tile_tma<BN, false>(&tmC, sC, t_acc, row_in_tile, mt * BM, nt * BN, b, p.aux, aux_row, p.M, p.N,
-                                       p.alpha, p.beta, p.round_acc, slab_seq, issuer, false,
-                                       tc.mirror ? reinterpret_cast<__nv_bfloat16*>(p.C) + static_cast<long long>(b) * p.strideC : nullptr,
-                                       p.ldc);
+        const int row = mt * BM + row_in_tile;
+        const long long aux_row = static_cast<long long>(b) * p.strideAux + static_cast<long long>(row) * p.ldaux;
+        __nv_bfloat16* mirror_c = tc.mirror ? reinterpret_cast<__nv_bfloat16*>(p.C) + static_cast<long long>(b) * p.strideC : nullptr;
+        const bool fp32_out = !AUX_TMA && p.out_fp32;
+        const int sw = fp32_out ? 32 : 64;
+#pragma unroll 1
+        for (int col = nt * BN; col < nt * BN + BN && col < p.N; col += sw, ++seq) {
+          if ((seq & 1) != eg) continue;
+          const uint32_t buf = seq & (NSTG - 1);
+          uint8_t* my_row = sC + buf * SLAB_BYTES + row_in_tile * 128;
+          const uint32_t t_slab = t_acc + static_cast<uint32_t>(col - nt * BN);
+          uint4 xa[8];
+          if (!AUX_TMA) {
+            if (fp32_out) load_aux_slab<true>(p.aux, aux_row + col, row < p.M, p.N - col, xa);
+            else load_aux_slab<false>(p.aux, aux_row + col, row < p.M, p.N - col, xa);
+          }
+          if (!mbar_wait(&slab_open[buf], (seq / NSTG) & 1, abort_flag, p.status, 5)) { ok = false; break; }
+          if (fp32_out) slab_fp32(t_slab, my_row, row_in_tile, xa, p.alpha, p.beta);
+          else slab_bf16<AUX_TMA>(t_slab, my_row, row_in_tile, xa, p.alpha, p.beta, p.round_acc, mirror_c, p.ldc, col, row, p.N);
+          fence_proxy_async_smem();
+          mbar_arrive(&slab_done[buf]);
+        }
+        if (!ok) break;
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(&tempty[acc]);
@@ -262,7 +247,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       const long long c_off = static_cast<long long>(b) * p.strideC + static_cast<long long>(row) * p.ldc;
       const long long x_off = static_cast<long long>(b) * p.strideAux + static_cast<long long>(row) * p.ldaux;
 #pragma unroll 1
-      for (int c0 = 0; c0 < BN; c0 += 32) {
+      for (int c0 = static_cast<int>(eg) * 32; c0 < BN; c0 += 64) {
         const int col = nt * BN + c0;
         if (col >= p.N) break;  // uniform over the warp
         uint32_t v[32];
@@ -351,7 +336,6 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       acc ^= 1;
       if (acc == 0) acc_phase ^= 1;
     }
-    if (!AUX_TMA && issuer && p.tma_store) tma_store_wait_read<0>();   // no store may still be reading shared memory at exit
   }
 
   tc_fence_before();
@@ -364,15 +348,17 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 
 // bf16 output with a bf16 aux tile that TMA can fetch (16-byte aligned base, rows and batches)
 static bool aux_tma_ok(const GemmArgs& a) {
-  return a.aux != nullptr && !a.out_fp32 && a.ldaux % 8 == 0 && (a.batch == 1 || a.strideAux % 8 == 0) &&
+  // (broadcast rows or batches, strides of 0, take the plain loads)
+  return a.aux != nullptr && !a.out_fp32 && a.ldaux % 8 == 0 && a.ldaux >= a.N &&
+         (a.batch == 1 || (a.strideAux % 8 == 0 && a.strideAux > 0)) &&
          reinterpret_cast<uintptr_t>(a.aux) % 16 == 0 && a.ldc % 8 == 0 && (a.batch == 1 || a.strideC % 8 == 0) &&
          reinterpret_cast<uintptr_t>(a.C) % 16 == 0;
 }
 
-template <int BN, int STAGES, bool A_MN, bool B_MN, bool AUX_TMA = false>
+template <int BN, int STAGES, bool A_MN, bool B_MN, bool AUX_TMA>
 static void launch_gemm(const GemmArgs& a, cudaStream_t stream) {
   constexpr uint32_t STAGE_BYTES = (BM + BN) * BK * 2;
-  constexpr size_t SMEM = 1024 + STAGES * STAGE_BYTES + (AUX_TMA ? 4 : 2) * SLAB_BYTES + 256;
+  constexpr size_t SMEM = 1024 + STAGES * STAGE_BYTES + NSTG * SLAB_BYTES + 256;
   static_assert(SMEM <= 232448, "shared memory budget of one CTA exceeded");
   auto kern = gemm_bf16_kernel<BN, STAGES, A_MN, B_MN, AUX_TMA>;
   static bool attr_done = false;
@@ -439,7 +425,7 @@ static void launch_gemm(const GemmArgs& a, cudaStream_t stream) {
   p.full_items = p.total_items = static_cast<int>(total);
   p.nslices = 1;
   const int grid = static_cast<int>(p.total_items < sms ? p.total_items : sms);
-  kern<<<grid, 256, SMEM, stream>>>(tmA, tmB, tmC, tmX, p);
+  kern<<<grid, GEMM_THREADS, SMEM, stream>>>(tmA, tmB, tmC, tmX, p);
 }
 
 int num_sms() {
@@ -462,23 +448,20 @@ void gemm_bf16(const GemmArgs& a, cudaStream_t stream) {
   // intensity) wins even when it costs an extra partial wave; narrow tiles are only for narrow outputs.
   const int best_bn = a.N <= 128 ? 128 : (a.N <= 192 ? 192 : 256);
   const int sel = (a.a_mn ? 2 : 0) | (a.b_mn ? 1 : 0);
-#define HM_LAUNCH(BN_, ST_)                                                        \
+#define HM_LAUNCH(BN_, ST_, AX_)                                                   \
   switch (sel) {                                                                   \
-    case 0: launch_gemm<BN_, ST_, false, false>(a, stream); break;                 \
-    case 1: launch_gemm<BN_, ST_, false, true>(a, stream); break;                  \
-    case 2: launch_gemm<BN_, ST_, true, false>(a, stream); break;                  \
-    default: launch_gemm<BN_, ST_, true, true>(a, stream); break;                  \
+    case 0: launch_gemm<BN_, ST_, false, false, AX_>(a, stream); break;            \
+    case 1: launch_gemm<BN_, ST_, false, true, AX_>(a, stream); break;             \
+    case 2: launch_gemm<BN_, ST_, true, false, AX_>(a, stream); break;             \
+    default: launch_gemm<BN_, ST_, true, true, AX_>(a, stream); break;             \
   }
-  if (best_bn == 256 && aux_tma_ok(a)) {
-    switch (sel) {
-      case 0: launch_gemm<256, 3, false, false, true>(a, stream); break;
-      case 1: launch_gemm<256, 3, false, true, true>(a, stream); break;
-      case 2: launch_gemm<256, 3, true, false, true>(a, stream); break;
-      default: launch_gemm<256, 3, true, true, true>(a, stream); break;
-    }
-  } else if (best_bn == 128) { HM_LAUNCH(128, 6) }
-  else if (best_bn == 192) { HM_LAUNCH(192, 4) }
-  else { HM_LAUNCH(256, 4) }
+  if (aux_tma_ok(a)) {
+    if (best_bn == 128) { HM_LAUNCH(128, 5, true) }
+    else if (best_bn == 192) { HM_LAUNCH(192, 4, true) }
+    else { HM_LAUNCH(256, 3, true) }
+  } else if (best_bn == 128) { HM_LAUNCH(128, 5, false) }
+  else if (best_bn == 192) { HM_LAUNCH(192, 4, false) }
+  else { HM_LAUNCH(256, 3, false) }
 #undef HM_LAUNCH
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) throw std::runtime_error(std::string("himuon gemm launch failed: ") + cudaGetErrorString(e));

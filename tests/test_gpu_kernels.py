@@ -560,3 +560,19 @@ def test_attention_ragged_lengths(D, B, S, Hq, Hkv):
     _close(o, ref.reshape(B * S, Hq * D), atol=2e-2, rtol=2e-2)
     for t, r in zip(ins, ref_in):
         _close(t.grad, r.grad.reshape(t.shape), atol=3e-2, rtol=3e-2)
+
+
+@pytest.mark.parametrize("B,m,n", [(3, 256, 256), (1, 512, 512), (2, 264, 1000), (1, 1024, 3072), (2, 8, 8192)])
+@pytest.mark.parametrize("out_of_place", [False, True])
+def test_ns_normalize_cluster(B, m, n, out_of_place):
+    """Tiles split over a cluster: whole slices, a ragged last one, slices longer than the registers hold, zero tiles."""
+    torch.manual_seed(0)
+    x = torch.randn(B + 1, m, n, device="cuda", dtype=torch.bfloat16)
+    x[B].zero_()
+    ref = x.float() / (x.double().norm(dim=(1, 2), keepdim=True).float() + 1e-7)
+    out = torch.full_like(x, 5.0) if out_of_place else None
+    src = x.clone()
+    _ext().ns_normalize(x, B + 1, m * n, 1e-7, out)
+    # half a bf16 ulp is 2^-8 of the value; the rest covers fp32 sums of up to 3 Mi squares in 8 * 1024 chains
+    _close(out if out_of_place else x, ref, atol=1e-9, rtol=2 ** -7.9)
+    assert not out_of_place or torch.equal(x, src)

@@ -79,6 +79,14 @@ static void untile_apply(const at::Tensor& entries, int64_t n_entries, int64_t t
   himuon::untile_apply(reinterpret_cast<const himuon::ApplyEntry*>(entries.data_ptr()), (int)n_entries, (int)total_units,
                        (int)Th, (int)Tw, tiles.data_ptr(), hyper.data_ptr<float>(), param_fp32 ? 1 : 0, cur_stream());
 }
+static void ns_repad(const at::Tensor& src, at::Tensor& dst) {
+  HM_CHECK(src.is_cuda() && dst.is_cuda() && src.dim() == 3 && dst.dim() == 3 && src.size(0) == dst.size(0) && src.is_contiguous() && dst.is_contiguous(), "ns_repad: contiguous (B, m, n) tensors");
+  HM_CHECK((is_bf16(src) || is_f32(src)) && (is_bf16(dst) || is_f32(dst)), "ns_repad: bf16 or fp32");
+  HM_CHECK(src.size(1) < (1LL << 30) && src.size(2) < (1LL << 30) && dst.size(1) < (1LL << 30) && dst.size(2) < (1LL << 30), "ns_repad: matrix too large");
+  const c10::cuda::CUDAGuard guard(src.device());
+  himuon::ns_repad(src.data_ptr(), dst.data_ptr(), src.size(0), (int)src.size(1), (int)src.size(2), (int)dst.size(1), (int)dst.size(2),
+                   is_f32(src) ? 1 : 0, is_f32(dst) ? 1 : 0, cur_stream());
+}
 static void ns_normalize(at::Tensor& tiles, int64_t n_tiles, int64_t tile_elems, double eps, const c10::optional<at::Tensor>& out) {
   HM_CHECK(tiles.is_cuda() && is_bf16(tiles) && tiles.is_contiguous(), "ns_normalize: tiles must be contiguous bf16");
   HM_CHECK(tiles.numel() >= n_tiles * tile_elems, "ns_normalize: buffer too small");
@@ -295,6 +303,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         py::arg("max_ctas") = 0, py::arg("symmetric") = false);
   m.def("momentum_tile", &momentum_tile);
   m.def("untile_apply", &untile_apply);
+  m.def("ns_repad", &ns_repad);
   m.def("ns_normalize", &ns_normalize, py::arg("tiles"), py::arg("n_tiles"), py::arg("tile_elems"), py::arg("eps"),
         py::arg("out") = py::none());
   m.def("adamw_multi", &adamw_multi);

@@ -80,6 +80,10 @@ void untile_apply(const ApplyEntry* entries, int n_entries, int total_units, int
 void ns_normalize(void* tiles_bf16, long long n_tiles, long long tile_elems, float eps, cudaStream_t stream,
                   void* out = nullptr);
 
+// (batch, sm, sn) -> (batch, dm, dn), zero-filled or cropped, bf16 / fp32 on either side; both contiguous.
+void ns_repad(const void* src, void* dst, long long batch, int sm, int sn, int dm, int dn, int src_fp32, int dst_fp32,
+              cudaStream_t stream);
+
 struct AdamEntry {
   void* param;
   const void* grad;

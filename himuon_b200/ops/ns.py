@@ -56,15 +56,19 @@ def fused_supported(m: int, n: int) -> bool:
 
 
 def ns_inplace_cuda(X: torch.Tensor, steps: int = 5, eps: float = 1e-7, workspace: NSWorkspace | None = None,
-                    normalize: bool = True) -> torch.Tensor:
-    """Orthogonalise a contiguous bf16 ``(B, m, n)`` CUDA buffer in place and return it."""
+                    normalize: bool = True, source: torch.Tensor | None = None) -> torch.Tensor:
+    """Orthogonalise a contiguous bf16 ``(B, m, n)`` CUDA buffer in place and return it.  With ``source`` (same shape and
+    type) that tensor is read instead and left as it is: the first pass over the data, which scales every tile, writes to
+    ``X`` or to scratch, so no copy is needed."""
     assert X.is_cuda and X.dtype == torch.bfloat16 and X.dim() == 3 and X.is_contiguous()
     e = _ext.ext()
     Bt, m, n = X.shape
     if Bt == 0:
         return X
+    assert source is None or (normalize and source.shape == X.shape and source.dtype == X.dtype and source.is_contiguous())
+    src = X if source is None else source
     if m <= n and e.ns5_fused_supported(m, n) and normalize:
-        e.ns5_fused(X, X, int(steps), float(eps))
+        e.ns5_fused(src, X, int(steps), float(eps))
         _count()
         return X
     if m % 8 or n % 8:
@@ -76,8 +80,10 @@ def ns_inplace_cuda(X: torch.Tensor, steps: int = 5, eps: float = 1e-7, workspac
         # With an odd number of iterations the normalised copy goes to the scratch buffer, so that the ping-pong ends
         # in X and no copy back is needed.
         if steps % 2 == 1:
-            e.ns_normalize(X, Bt, m * n, float(eps), Y)
+            e.ns_normalize(src, Bt, m * n, float(eps), Y)
             cur, nxt = Y, X
+        elif source is not None:
+            e.ns_normalize(src, Bt, m * n, float(eps), X)
         else:
             e.ns_normalize(X, Bt, m * n, float(eps))
         _count()
@@ -103,17 +109,31 @@ def newton_schulz(G: torch.Tensor, steps: int = 5, workspace: NSWorkspace | None
     if not G.is_cuda:
         return ref.newton_schulz(G, steps=steps)
     shape = G.shape
-    X = G.reshape(-1, shape[-2], shape[-1]).to(torch.bfloat16)
-    if X.data_ptr() == G.data_ptr() or not X.is_contiguous():
-        X = X.contiguous() if not X.is_contiguous() else X.clone()
+    X = G.reshape(-1, shape[-2], shape[-1])
     m, n = X.shape[-2:]
     if m % 8 or n % 8:
         # pad to the TMA granularity; zero rows/columns do not change the iteration
-        pm, pn = (-m) % 8, (-n) % 8
-        Xp = torch.nn.functional.pad(X, (0, pn, 0, pm))
-        out = ns_inplace_cuda(_pre_normalized(Xp), steps, workspace=workspace, normalize=False)[:, :m, :n]
+        if X.dtype not in (torch.bfloat16, torch.float32):
+            X = X.to(torch.bfloat16)
+        X = X.contiguous()
+        out = torch.empty(X.shape, device=X.device, dtype=X.dtype)
+        if X.numel():
+            e = _ext.ext()
+            pad = torch.empty(X.shape[0], -(-m // 8) * 8, -(-n // 8) * 8, device=X.device, dtype=torch.bfloat16)
+            e.ns_repad(X, pad)
+            ns_inplace_cuda(pad, steps, workspace=workspace)
+            e.ns_repad(pad, out)
+            _count(2)
+        return out.reshape(shape).to(G.dtype)
+    Xb = X.to(torch.bfloat16)
+    if not Xb.is_contiguous():
+        out = ns_inplace_cuda(Xb.contiguous(), steps, workspace=workspace)
+    elif Xb.data_ptr() != G.data_ptr():                    # a converted copy: ours to overwrite
+        out = ns_inplace_cuda(Xb, steps, workspace=workspace)
+    elif Xb.data_ptr() % 16 == 0:                          # G itself, which is only read
+        out = ns_inplace_cuda(torch.empty_like(Xb), steps, workspace=workspace, source=Xb)
     else:
-        out = ns_inplace_cuda(X, steps, workspace=workspace)
+        out = ns_inplace_cuda(Xb.clone(), steps, workspace=workspace)
     return out.reshape(shape).to(G.dtype)
 
 

@@ -339,3 +339,41 @@ def test_soap_kernel_path_follows_the_torch_path():
             for a, bb in zip(gg_r, gg_k):                        # Gram EMA in the GEMM epilogue vs lerp_
                 assert float((a - bb).norm() / a.norm()) < 1e-3
     ops.check_status()
+
+
+@pytest.mark.parametrize("shape", [(3, 7, 9), (2, 100, 250), (1, 333, 500), (2, 257, 64), (70000, 1, 9)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+def test_newton_schulz_odd_sides(shape, dtype):
+    """Sides that are no multiples of 8 are padded and cropped by the library's own kernels; the input stays as it was."""
+    from himuon_b200 import ops
+    from himuon_b200.ops import ns as ns_ops
+    from himuon_b200.ops import reference as ref
+
+    x = _well_conditioned(*shape).cuda().to(dtype)
+    keep = x.clone()
+    out = ns_ops.newton_schulz(x, 5)
+    ops.check_status()
+    assert out.dtype == dtype and out.shape == x.shape and torch.equal(x, keep)
+    want = ref.newton_schulz(x[:64].cpu(), 5).float()
+    # five bf16 iterations with another order of sums: the bound of test_newton_schulz_dispatcher_matches_oracle
+    assert (out[:64].float().cpu() - want).norm() / want.norm() < 3e-2
+
+
+@pytest.mark.parametrize("shape,steps", [((4, 128, 128), 5), ((3, 256, 512), 5), ((3, 256, 512), 4), ((2, 512, 256), 3)])
+def test_newton_schulz_leaves_its_input(shape, steps):
+    """The scaling pass reads the caller's tensor directly: it must not change, whatever the parity of the steps."""
+    from himuon_b200 import ops
+    from himuon_b200.ops import ns as ns_ops
+    from himuon_b200.ops import reference as ref
+
+    base = _well_conditioned(*shape).cuda().bfloat16().flatten()
+    flat = torch.empty(base.numel() + 8, device="cuda", dtype=torch.bfloat16)
+    for off in (0, 8, 1):                                  # aligned, aligned slice, misaligned slice
+        flat[off: off + base.numel()] = base
+        x = flat[off: off + base.numel()].view(shape)
+        keep = x.clone()
+        out = ns_ops.newton_schulz(x, steps)
+        ops.check_status()
+        assert torch.equal(x, keep) and out.data_ptr() != x.data_ptr()
+        want = ref.newton_schulz(keep.cpu(), steps).float()
+        assert (out.float().cpu() - want).norm() / want.norm() < 3e-2

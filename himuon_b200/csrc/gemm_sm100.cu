@@ -346,6 +346,12 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   }
 }
 
+// C can be written by TMA stores
+static bool c_rows_aligned(const GemmArgs& a) {
+  const int row_align = a.out_fp32 ? 4 : 8;
+  return a.ldc % row_align == 0 && (a.batch == 1 || a.strideC % row_align == 0) && reinterpret_cast<uintptr_t>(a.C) % 16 == 0;
+}
+
 // bf16 output with a bf16 aux tile that TMA can fetch (16-byte aligned base, rows and batches)
 static bool aux_tma_ok(const GemmArgs& a) {
   // (broadcast rows or batches, strides of 0, take the plain loads)
@@ -393,9 +399,7 @@ static void launch_gemm(const GemmArgs& a, cudaStream_t stream) {
   p.status = status_word_ptr();
   // C tensor map for the TMA-store epilogue: rows of 128 bytes (64 bf16 / 32 fp32 columns) per slab.
   const int esz = a.out_fp32 ? 4 : 2;
-  const int row_align = 16 / esz;
-  p.tma_store = (a.ldc % row_align == 0) && (a.batch == 1 || a.strideC % row_align == 0) &&
-                (reinterpret_cast<uintptr_t>(a.C) % 16 == 0) ? 1 : 0;
+  p.tma_store = c_rows_aligned(a) ? 1 : 0;
   CUtensorMap tmC = tmA;
   if (p.tma_store) {
     const uint64_t dimsC[3] = {static_cast<uint64_t>(a.N), static_cast<uint64_t>(a.M), static_cast<uint64_t>(a.batch)};
@@ -437,6 +441,29 @@ int num_sms() {
   return sms[dev];
 }
 
+// Tiles of width bn that the one-CTA kernel computes for this problem (launch_gemm's own count).
+static long long tile_count(const GemmArgs& a, int bn) {
+  const int tm = (a.M + BM - 1) / BM, tn = (a.N + bn - 1) / bn;
+  long long per = static_cast<long long>(tm) * tn;
+  if (a.symmetric && a.M == a.N && !a.out_fp32 && c_rows_aligned(a) && tn > 1) {
+    per = 0;
+    for (int nt = 0; nt < tn; ++nt) per += tm - nt * (bn / BM);
+  }
+  return per * a.batch;
+}
+// Tile width for outputs wider than 192 columns: 256, unless tiles of 128 need clearly fewer rounds over the SMs.  Two
+// narrow tiles cost about 4 % more than a wide one (128 products of 512^3, which fill the chip either way: 755 and 786 us
+// for newton_schulz), and narrow symmetric tiles mirror a larger share of the output with 2-byte stores (396 tiles of
+// 256: 5 % slower than wide ones), so a narrow round counts 0.7 of a wide one.  They win where the wide tiles do not fill
+// the chip (6 matrices of 333 x 500: 211 -> 173 us) or just overflow it (symmetric products of 28 tiles of 512: 168 wide
+// tiles are two rounds, 280 narrow ones two rounds of half the length; the optimizer step went from 277 to 250 us).
+constexpr double kNarrowRound = 0.7;
+static long long rounds(long long tiles, long long slots) { return (tiles + slots - 1) / slots; }
+static int tile_width(const GemmArgs& a) {
+  const long long sms = a.max_ctas > 0 ? a.max_ctas : num_sms();
+  return rounds(tile_count(a, 128), sms) * kNarrowRound < static_cast<double>(rounds(tile_count(a, 256), sms)) ? 128 : 256;
+}
+
 void gemm_bf16(const GemmArgs& a, cudaStream_t stream) {
   if (a.M <= 0 || a.N <= 0 || a.batch <= 0) return;
   if (a.K <= 0) throw std::runtime_error("himuon gemm: K must be positive");
@@ -444,9 +471,7 @@ void gemm_bf16(const GemmArgs& a, cudaStream_t stream) {
     gemm2_bf16(a, stream);
     return;
   }
-  // Tile width.  The main loop is bound by L2 -> shared-memory traffic, so the widest tile (highest arithmetic
-  // intensity) wins even when it costs an extra partial wave; narrow tiles are only for narrow outputs.
-  const int best_bn = a.N <= 128 ? 128 : (a.N <= 192 ? 192 : 256);
+  const int best_bn = a.N <= 128 ? 128 : (a.N <= 192 ? 192 : tile_width(a));
   const int sel = (a.a_mn ? 2 : 0) | (a.b_mn ? 1 : 0);
 #define HM_LAUNCH(BN_, ST_, AX_)                                                   \
   switch (sel) {                                                                   \

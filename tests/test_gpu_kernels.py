@@ -576,3 +576,57 @@ def test_ns_normalize_cluster(B, m, n, out_of_place):
     # half a bf16 ulp is 2^-8 of the value; the rest covers fp32 sums of up to 3 Mi squares in 8 * 1024 chains
     _close(out if out_of_place else x, ref, atol=1e-9, rtol=2 ** -7.9)
     assert not out_of_place or torch.equal(x, src)
+
+
+@pytest.mark.parametrize("M,N,K,batch", [(512, 512, 512, 160), (336, 504, 504, 3), (264, 1000, 72, 2), (384, 256, 2048, 1),
+                                         (1024, 3072, 1024, 4), (640, 640, 256, 5)])
+@pytest.mark.parametrize("mode", ["aux", "aux_broadcast", "add", "fp32", "sym"])
+def test_gemm_kernel_choice(M, N, K, batch, mode):
+    """Both kernels, all tile widths and every epilogue form, on whole and ragged tiles."""
+    from himuon_b200 import ops
+
+    torch.manual_seed(0)
+    dt = torch.float32 if mode == "fp32" else torch.bfloat16
+    a = torch.randn(batch, M, K, device="cuda", dtype=torch.bfloat16)
+    if mode == "sym":
+        out = torch.full((batch, M, M), 9.0, device="cuda", dtype=dt)
+        ops.gemm(a, a, trans_b=True, out=out, symmetric=True)
+        ref = a.float() @ a.float().transpose(1, 2)
+        assert torch.equal(out, out.transpose(1, 2))
+    else:
+        b = torch.randn(batch, K, N, device="cuda", dtype=torch.bfloat16)
+        ref = a.float() @ b.float()
+        out = torch.full((batch, M, N), 9.0, device="cuda", dtype=dt)
+        if mode == "aux":
+            x = torch.randn(batch, M, N, device="cuda", dtype=dt)
+            ops.gemm(a, b, out=out, aux=x, alpha=0.5, beta=-2.0)
+            ref = 0.5 * ref - 2.0 * x.float()
+        elif mode == "aux_broadcast":
+            x = torch.randn(1, 1, N, device="cuda", dtype=dt).expand(batch, M, N)
+            ops.gemm(a, b, out=out, aux=x, beta=1.5)
+            ref = ref + 1.5 * x.float()
+        elif mode == "add":
+            ref = ref + out.float()
+            ops.gemm(a, b, out=out, aux=out, beta=1.0)
+        else:
+            x = torch.randn(batch, M, N, device="cuda")
+            ops.gemm(a, b, out=out, aux=x, beta=0.5)
+            ref = ref + 0.5 * x
+    torch.cuda.synchronize()
+    _assert_status_clean()
+    # fp32 sums of K products (about sqrt(K)); half a bf16 ulp is 2^-8, twice that where partial sums are added into C
+    tol = 1e-5 if dt == torch.float32 else 2 ** -7
+    _close(out, ref, atol=tol * math.sqrt(K), rtol=tol)
+
+
+@pytest.mark.parametrize("B,m,n", [(1, 64, 64), (500, 64, 64), (500, 40, 64), (5, 128, 192), (450, 120, 128)])
+def test_ns5_fused_warp_splits(B, m, n):
+    """Four and eight warps per tile, more tiles than fit the chip at once, short tiles."""
+    torch.manual_seed(0)
+    U, _, Vh = torch.linalg.svd(torch.randn(B, m, n), full_matrices=False)
+    x = ((U * torch.linspace(0.8, 1.2, m)) @ Vh).cuda().bfloat16()
+    out = torch.empty_like(x)
+    _ext().ns5_fused(x, out, 5, 1e-7)
+    torch.cuda.synchronize()
+    _assert_status_clean()
+    _close(out, _ns_ref(x), atol=4e-2, rtol=4e-2)      # the bounds of the test above: five bf16 iterations

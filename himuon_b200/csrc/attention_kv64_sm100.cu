@@ -25,8 +25,12 @@ __device__ __forceinline__ uint64_t kv_desc_mnmajor(uint32_t base, int ks) {  //
 // columns of the S buffer they just read and P·V runs with the A operand in tensor memory.  The two S buffers
 // therefore double-buffer P as well, the wait for the previous P·V is only needed on the rare O rescale, S is read
 // from TMEM once, and K and V each have two 16 KB stages.
+// A parity wait can only tell a phase from its neighbours, and the softmax threads skip most phases of `o_done`, so there
+// is one per S buffer: whoever waits for P(i)·V has seen S(i), which the tensor core finishes after P(i-2)·V, the phase
+// before it on the same barrier.  The end of the last product has a barrier of its own (`acc_done`, one phase): a warp
+// that is done with its softmax gets there while P(nkv-2)·V may still be running.
 struct Fwd64TBars {
-  uint64_t q_full, k_full[2], k_empty[2], v_full[2], v_empty[2], s_full[2], p_ready[2], o_done;
+  uint64_t q_full, k_full[2], k_empty[2], v_full[2], v_empty[2], s_full[2], p_ready[2], o_done[2], acc_done;
   uint32_t tmem_slot;
   int abort_flag;
 };
@@ -60,7 +64,8 @@ flash_fwd64_t_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       mbar_init(&bars->v_full[i], 1); mbar_init(&bars->v_empty[i], 1);
       mbar_init(&bars->s_full[i], 1); mbar_init(&bars->p_ready[i], 128);
     }
-    mbar_init(&bars->o_done, 1);
+    for (int i = 0; i < 2; ++i) mbar_init(&bars->o_done[i], 1);
+    mbar_init(&bars->acc_done, 1);
     bars->abort_flag = 0;
     mbar_fence_init();
   }
@@ -117,8 +122,9 @@ flash_fwd64_t_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         for (int ks = 0; ks < BKV / 16; ++ks)
           umma_ts(tO, tS0 + st * BKV + ks * 8, kv_desc_mnmajor(v_base + st * KV_TILE, ks), idesc_pv, (j > 0 || ks > 0) ? 1u : 0u);
         umma_commit(&bars->v_empty[st]);
-        umma_commit(&bars->o_done);
+        umma_commit(&bars->o_done[st]);
       }
+      if (ok) umma_commit(&bars->acc_done);
     }
   } else {
     // ------------------------------------------------------------ softmax / epilogue: one thread per query row
@@ -157,7 +163,7 @@ flash_fwd64_t_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         // O (and l) move to the new maximum: the previous P·V must have landed in O first
         const float alpha = exp2f(m_used - m_new);
         m_used = m_new;
-        if (!mbar_wait(&bars->o_done, (j - 1) & 1, abort_flag, p.status, 4)) { ok = false; break; }
+        if (!mbar_wait(&bars->o_done[st ^ 1], ((j - 1) >> 1) & 1, abort_flag, p.status, 4)) { ok = false; break; }
         tc_fence_after();
 #pragma unroll 1
         for (int c = 0; c < 2 * NH; ++c) {
@@ -185,7 +191,7 @@ flash_fwd64_t_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       tc_fence_before();
       mbar_arrive(&bars->p_ready[st]);
     }
-    if (ok && mbar_wait(&bars->o_done, (nkv - 1) & 1, abort_flag, p.status, 4)) {
+    if (ok && mbar_wait(&bars->acc_done, 0, abort_flag, p.status, 4)) {
       tc_fence_after();
       const float inv = 1.f / l;
       const bool row_ok = q_idx < p.S;

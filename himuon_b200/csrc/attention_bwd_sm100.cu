@@ -35,7 +35,7 @@ constexpr uint32_t STAT_BYTES = 2 * BQ * 4;          // lse[64] then delta[64]
 constexpr int BWD_THREADS = 320;
 
 struct DkvBars {
-  uint64_t kv_full, qd_full[NST], qd_empty[NST], s_full[2], p_ready[2], acc_done;
+  uint64_t kv_full, qd_full[NST], qd_empty[NST], s_full[2], p_ready[2], stat_ready[2], acc_done;
   uint32_t tmem_slot;
   int abort_flag;
 };
@@ -83,7 +83,7 @@ flash_bwd_dkv_t_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
   if (threadIdx.x == 0) {
     mbar_init(&bars->kv_full, 1);
     for (int i = 0; i < NST; ++i) { mbar_init(&bars->qd_full[i], 1); mbar_init(&bars->qd_empty[i], 1); }
-    for (int i = 0; i < 2; ++i) { mbar_init(&bars->s_full[i], 1); mbar_init(&bars->p_ready[i], 128); }
+    for (int i = 0; i < 2; ++i) { mbar_init(&bars->s_full[i], 1); mbar_init(&bars->p_ready[i], 128); mbar_init(&bars->stat_ready[i], 128); }
     mbar_init(&bars->acc_done, 1);
     bars->abort_flag = 0;
     mbar_fence_init();
@@ -170,8 +170,9 @@ flash_bwd_dkv_t_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
       const int q0 = kb * AT + (it - g * nsub) * BQ;
       const int st = it % NST;
       // RAGGED: sub-block `it` has statistics slot it % NST, so a group alternates between two slots of its own.  A
-      // thread rewrites a slot two of its sub-blocks later, past the barrier of the one between, which every thread of
-      // the group reaches only after it has read this one.
+      // thread rewrites a slot two of its sub-blocks later, past the group's barrier of the one between, at which every
+      // thread of the group arrives only after it has read this one.  The group meets on an mbarrier, because a thread
+      // may leave the loop on its own when a bounded wait runs out: the others then give up here as well.
       if (RAGGED) {
         const int qi = q0 + (row & (BQ - 1));
         const long long stat_idx = (static_cast<long long>(b) * p.Hq + h_first + g) * p.S + qi;
@@ -179,7 +180,8 @@ flash_bwd_dkv_t_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
         float v = want_lse ? INFINITY : 0.f;
         if (qi < p.S) v = want_lse ? p.lse[stat_idx] : p.delta[stat_idx];
         sStat[st * 2 * BQ + row] = v;
-        named_barrier(2 + wg, 128);
+        mbar_arrive(&bars->stat_ready[wg]);
+        if (!mbar_wait(&bars->stat_ready[wg], (it >> 1) & 1, abort_flag, p.status, 4)) { ok = false; break; }
       }
       if (!mbar_wait(&bars->qd_full[st], (it / NST) & 1, abort_flag, p.status, 4)) { ok = false; break; }
       if (!mbar_wait(&bars->s_full[buf], (it >> 1) & 1, abort_flag, p.status, 4)) { ok = false; break; }

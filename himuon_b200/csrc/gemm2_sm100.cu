@@ -213,7 +213,8 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
       const int r = tile - b * tiles_per_batch;
       const int mt = r % p.tiles_m;
       const int nt = r / p.tiles_m;
-      if (!mbar_wait(&tfull[acc], acc_phase, abort_flag, p.status, 3)) break;
+      // the 128 threads meet on named barriers below, so they also leave together when the wait runs out
+      if (!named_barrier_and(1, 128, mbar_wait(&tfull[acc], acc_phase, abort_flag, p.status, 3))) break;
       tc_fence_after();
       const int row_in_tile = ew * 32 + lane;
       const int m0 = mt * 2 * BM + static_cast<int>(rank) * BM;

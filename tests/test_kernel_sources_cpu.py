@@ -32,10 +32,22 @@ def _loops(code):
         yield code[start:i]
 
 
+def _functions_with_named_barriers():
+    names = set()
+    for path in CSRC.glob("*.cuh"):
+        code = _code(path)
+        heads = [(m.start(), m.group(1)) for m in re.finditer(r"__device__[^;{]*?\b(\w+)\s*\([^;{]*\)\s*\{", code)]
+        for (at, name), (end, _) in zip(heads, heads[1:] + [(len(code), "")]):
+            if re.search(r"\bnamed_barrier\(", code[at:end]):
+                names.add(name)
+    return names
+
+
 @pytest.mark.parametrize("name", sorted(p.name for p in CSRC.glob("*.cu*")))
 def test_no_unbounded_barrier_in_a_loop_that_threads_leave_one_by_one(name):
-    """A thread leaves such a loop by itself when its bounded wait runs out; a named barrier in the same loop would keep
-    the other threads waiting for it for good."""
+    """A thread leaves such a loop by itself when its bounded wait runs out; a named barrier in the same loop (or in a
+    function called there) would keep the other threads waiting for it for good."""
+    barriers = "|".join(sorted({"named_barrier"} | _functions_with_named_barriers()))
     for body in _loops(_code(CSRC / name)):
         if re.search(r"if \(!mbar_wait\(", body) and "break;" in body:
-            assert not re.search(r"\bnamed_barrier\(|\bbar\.sync\b", body), body[:400]
+            assert not re.search(rf"\b(?:{barriers})\s*(?:<[^;()]*>)?\(|\bbar\.sync\b", body), body[:400]

@@ -650,3 +650,68 @@ def test_attention_forward_waits_for_its_last_product(D, B, S, Hq, Hkv):
     _close(runs[0], ref.reshape(B * S, Hq * D), atol=2e-2, rtol=2e-2)        # the bounds of test_flash_attention_fwd_bwd
     for o in runs[1:]:
         assert torch.equal(o, runs[0])
+
+
+def _momentum_apply_case(dtype, Th, Tw, offset, n_src, tile_offset=0):
+    """momentum_tile, then untile_apply, on matrices whose first element lies `offset` elements past an aligned address;
+    the gradient is the sum of `n_src` buffers.  Returns (momentum, tiles as matrices, parameters) and their references."""
+    e = _ext()
+    torch.manual_seed(0)
+    mu, lr, wd, scale, gscale = 0.95, 0.02, 0.1, 2.0, 1.0 / n_src
+    esz = torch.empty(0, dtype=dtype).element_size()
+    shapes = [(256, 384), (200, 304), (65, 301), (64, 64), (131, 132)]
+
+    def make(h, w, pitch):
+        flat = torch.randn(h * pitch + 16 // esz, device="cuda").to(dtype)
+        return flat[offset:].as_strided((h, w), (pitch, 1))
+
+    grads = [[make(h, w, w + 8) for _ in range(n_src)] for h, w in shapes]
+    moms = [make(h, w, w) for h, w in shapes]
+    params = [make(h, w, w + 8) for h, w in shapes]
+    moms_ref, params_ref = [m.float().clone() for m in moms], [p.float().clone() for p in params]
+    mom_tab, app_tab, tile_base, unit, metas = b"", b"", 0, 0, []
+    for gs, m, p in zip(grads, moms, params):
+        h, w = m.shape
+        R, C = math.ceil(h / Th), math.ceil(w / Tw)
+        ptrs = [g.data_ptr() for g in gs] + [0] * (8 - n_src)
+        mom_tab += struct.pack("<8QQq6i", *ptrs, m.data_ptr(), tile_base, h, w, R, C, unit, gs[0].stride(0))
+        app_tab += struct.pack("<Qq6ifi", p.data_ptr(), tile_base, h, w, R, C, unit, 0, scale, p.stride(0))
+        metas.append((tile_base, R, C))
+        tile_base += R * C
+        unit += e.momentum_tile_units(R, C, Th)
+    mom_dev = torch.frombuffer(bytearray(mom_tab), dtype=torch.uint8).cuda()
+    app_dev = torch.frombuffer(bytearray(app_tab), dtype=torch.uint8).cuda()
+    buf = torch.full((tile_base * Th * Tw + 8,), 7.0, device="cuda", dtype=torch.bfloat16)
+    tiles = buf[tile_offset: tile_offset + tile_base * Th * Tw].view(tile_base, Th, Tw)
+    fp32 = dtype == torch.float32
+    e.momentum_tile(mom_dev, len(shapes), unit, Th, Tw, tiles, mu, True, gscale, n_src, fp32)
+    hyper = torch.tensor([lr, wd], device="cuda", dtype=torch.float32)
+    e.untile_apply(app_dev, len(shapes), unit, Th, Tw, tiles, hyper, fp32)
+    torch.cuda.synchronize()
+    rnd = (lambda t: t) if fp32 else (lambda t: t.bfloat16().float())
+    out = []
+    for gs, m_ref, m, p_ref, p, (tb, R, C) in zip(grads, moms_ref, moms, params_ref, params, metas):
+        h, w = m.shape
+        g = rnd(sum(x.float() for x in gs) * gscale)
+        b = rnd(rnd(m_ref * mu) + g)
+        got = tiles[tb:tb + R * C].view(R, C, Th, Tw).permute(0, 2, 1, 3).reshape(R * Th, C * Tw).float()
+        assert got[h:].abs().sum() == 0 and got[:, w:].abs().sum() == 0
+        out.append(((m, b), (got[:h, :w], rnd(g + mu * b)),
+                    (p, rnd(p_ref * (1 - lr * wd)) - lr * scale * got[:h, :w])))
+    return out
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("offset,tile_offset", [(0, 0), (1, 0), (2, 0), (0, 1), (0, 4)])
+@pytest.mark.parametrize("n_src", [1, 3])
+@pytest.mark.parametrize("Th,Tw", [(128, 128), (96, 136)])
+def test_momentum_and_apply_at_any_address(dtype, offset, tile_offset, n_src, Th, Tw):
+    """Parameters, gradients, momenta and tiles that start anywhere (views into flat buffers), and a gradient that is the
+    sum of several buffers: the 16-byte and the element-wise path."""
+    # one rounding of the storage type either way of the multiply-add: half a bf16 ulp is 2^-9 of the value, sums of three
+    # fp32 values of up to ~5 round by 2^-22 * 5 each
+    rtol, atol = (2 ** -7.9, 1e-6) if dtype == torch.bfloat16 else (1e-6, 4e-6)
+    for mom, tile, param in _momentum_apply_case(dtype, Th, Tw, offset, n_src, tile_offset):
+        _close(*mom, atol=atol, rtol=rtol)
+        _close(*tile, atol=1e-5, rtol=2 ** -7.9)            # stored in bf16
+        _close(*param, atol=atol, rtol=rtol)

@@ -36,7 +36,7 @@ struct NsBars {
   uint64_t tma, mma;
   uint32_t tmem_slot;
   int abort_flag;
-  float red[8];       // one per warp
+  float red[4];       // one per warp of the first half
 };
 
 // HALVES = 2: eight warps, two per TMEM lane quadrant, each owning one half of the columns of its 32 rows.  A drain
@@ -91,22 +91,23 @@ ns5_fused_kernel(const __grid_constant__ CUtensorMap tmX, __nv_bfloat16* __restr
     if (!mbar_wait(&bars->tma, tma_phase, abort_flag, status, 5)) { ok = false; break; }
     tma_phase ^= 1;
 
-    // ---- Frobenius norm and normalisation (HALVES threads own one row of X)
-    float ss = 0.f;
-#pragma unroll 4
-    for (int c = half * (NCH * 8 / HALVES); c < (half + 1) * (NCH * 8 / HALVES); ++c) {
-      const uint4 v = *reinterpret_cast<const uint4*>(sX + ns_sw_off(row, c));
-      const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+    // ---- Frobenius norm and normalisation.  One thread sums a whole row, whatever HALVES is: a tile's result must not
+    // depend on the kernel that the number of tiles selects.
+    if (half == 0) {
+      float ss = 0.f;
+#pragma unroll 8
+      for (int c = 0; c < NCH * 8; ++c) {
+        const uint4 v = *reinterpret_cast<const uint4*>(sX + ns_sw_off(row, c));
+        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-      for (int q = 0; q < 4; ++q) { const float a = bf16_lo(w[q]), b = bf16_hi(w[q]); ss += a * a + b * b; }
+        for (int q = 0; q < 4; ++q) { const float a = bf16_lo(w[q]), b = bf16_hi(w[q]); ss += a * a + b * b; }
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+      if (lane == 0) bars->red[warp] = ss;
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-    if (lane == 0) bars->red[warp] = ss;
     __syncthreads();
-    float tot = 0.f;
-#pragma unroll
-    for (int w = 0; w < 4 * HALVES; ++w) tot += bars->red[w];
+    const float tot = bars->red[0] + bars->red[1] + bars->red[2] + bars->red[3];
     const float inv = 1.f / (sqrtf(tot) + eps);
 #pragma unroll 4
     for (int c = half * (NCH * 8 / HALVES); c < (half + 1) * (NCH * 8 / HALVES); ++c) {

@@ -319,6 +319,13 @@ __device__ __forceinline__ float block_sum(float v, float* red) {
   return red[0];
 }
 
+// Adds the squares of eight bf16 elements to a chain of sums.
+__device__ __forceinline__ void add_squares8(float& ss, const uint4& v) {
+  const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+  for (int q = 0; q < 4; ++q) { const float a = bf16_lo(w[q]), b = bf16_hi(w[q]); ss += a * a + b * b; }
+}
+
 __global__ void __launch_bounds__(1024)
 ns_normalize_kernel(const __nv_bfloat16* tiles, __nv_bfloat16* out, long long n_tiles, long long tile_elems, float eps) {
   __shared__ float red[32];
@@ -335,18 +342,9 @@ ns_normalize_kernel(const __nv_bfloat16* tiles, __nv_bfloat16* out, long long n_
 #pragma unroll
         for (int u = 0; u < 4; ++u) v4[u] = xv[i + u * blockDim.x];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const uint32_t w[4] = {v4[u].x, v4[u].y, v4[u].z, v4[u].w};
-#pragma unroll
-          for (int q = 0; q < 4; ++q) { const float a = bf16_lo(w[q]), b = bf16_hi(w[q]); ss += a * a + b * b; }
-        }
+        for (int u = 0; u < 4; ++u) add_squares8(ss, v4[u]);
       }
-      for (; i < nv; i += blockDim.x) {
-        const uint4 v = xv[i];
-        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-        for (int q = 0; q < 4; ++q) { const float a = bf16_lo(w[q]), b = bf16_hi(w[q]); ss += a * a + b * b; }
-      }
+      for (; i < nv; i += blockDim.x) add_squares8(ss, xv[i]);
     } else {
       for (long long i = threadIdx.x; i < tile_elems; i += blockDim.x) { const float a = __bfloat162float(x[i]); ss += a * a; }
     }
@@ -384,18 +382,15 @@ ns_normalize_kernel(const __nv_bfloat16* tiles, __nv_bfloat16* out, long long n_
   }
 }
 
-// Normalisation of tiles of 64 Ki elements and more: a cluster of eight CTAs per tile.  Each keeps the first kNormVecs
-// vectors per thread of its slice in registers, the partial sums of squares meet in distributed shared memory (added in
-// rank order by every CTA), and the scaled slice goes straight out.  For launches of few large tiles, which one CTA per
-// tile spread over too few SMs.
-constexpr int kNormCluster = 8, kNormVecs = 4;
-__device__ __forceinline__ float sumsq8(const uint4& v) {
-  const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-  float s = 0.f;
-#pragma unroll
-  for (int q = 0; q < 4; ++q) { const float a = bf16_lo(w[q]), b = bf16_hi(w[q]); s += a * a + b * b; }
-  return s;
-}
+// Normalisation of tiles of 64 Ki elements and more: a cluster of eight CTAs per tile, for launches of few large tiles,
+// which one CTA per tile spread over too few SMs.  The sum of squares is built in the order of the kernel above (1024
+// chains, chain c adding the vectors c, c + 1024, ...; then a tree over the chains of each warp and one over the 32
+// warps), so that a tile's result does not depend on how many tiles share its launch: CTA r owns chains 128 r ... 128 r +
+// 127, one thread each, and the 32 warp sums meet in the distributed shared memory of every CTA.  A chain is serial, so the
+// bytes in flight come from a ring of kNormRing vectors per chain that asynchronous copies fill ahead of it; a tile whose chains
+// fit the ring is read once.  All threads of the CTA share the second pass.
+constexpr int kNormCluster = 8, kNormChains = 1024, kNormOwn = kNormChains / kNormCluster, kNormThreads = 512, kNormGroup = 8;
+constexpr int kNormRing = 32;                              // 64 KB
 __device__ __forceinline__ uint4 scale8(const uint4& v, float f) {
   const uint32_t w[4] = {v.x, v.y, v.z, v.w};
   uint32_t o[4];
@@ -403,67 +398,101 @@ __device__ __forceinline__ uint4 scale8(const uint4& v, float f) {
   for (int q = 0; q < 4; ++q) o[q] = pack_bf16x2(bf16_lo(w[q]) * f, bf16_hi(w[q]) * f);
   return make_uint4(o[0], o[1], o[2], o[3]);
 }
-__global__ void __cluster_dims__(kNormCluster, 1, 1) __launch_bounds__(1024)
+template <bool ONCE>     // the chains fit the ring
+__global__ void __cluster_dims__(kNormCluster, 1, 1) __launch_bounds__(kNormThreads, ONCE ? 3 : 2)
 ns_normalize_cluster_kernel(const uint4* tiles, uint4* out, long long nv, float eps) {
-  __shared__ float red[32];
-  __shared__ float part[kNormCluster];
+  extern __shared__ uint4 ring[];                          // [kNormRing][kNormOwn]
+  __shared__ float red[kNormChains / 32];
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");   // waited for before the first remote store
   const uint32_t rank = blockIdx.x % kNormCluster;         // clusters are runs of consecutive blocks
   const long long t = blockIdx.x / kNormCluster;
   const uint4* x = tiles + t * nv;
   uint4* y = out + t * nv;                                 // may alias x (in place)
-  const long long per = (nv + kNormCluster - 1) / kNormCluster;
-  const long long v0 = rank * per, v1 = min(nv, v0 + per);
-  const long long rest = v0 + kNormVecs * static_cast<long long>(blockDim.x) + threadIdx.x;
-  uint4 keep[kNormVecs];
+  const long long base = static_cast<long long>(rank) * kNormOwn;
+  const int len = static_cast<int>((nv + kNormChains - 1) / kNormChains);  // vectors of the longest chain
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   float ss = 0.f;
+  if (threadIdx.x < kNormOwn) {
+    const long long first = base + threadIdx.x;
+    auto fetch = [&](int g) {                              // one group of copies; zeros past the end
 #pragma unroll
-  for (int u = 0; u < kNormVecs; ++u) {
-    const long long i = v0 + threadIdx.x + u * static_cast<long long>(blockDim.x);
-    keep[u] = i < v1 ? x[i] : make_uint4(0, 0, 0, 0);
+      for (int u = 0; u < kNormGroup; ++u) {
+        const int k = g * kNormGroup + u;
+        const long long i = first + static_cast<long long>(k) * kNormChains;
+        const uint32_t dst = smem_u32(ring + (k % kNormRing) * kNormOwn + threadIdx.x);
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(x + (i < nv ? i : 0)), "r"(i < nv ? 16 : 0)
+                     : "memory");
+      }
+    };
+    const int groups = (len + kNormGroup - 1) / kNormGroup;
+    for (int g = 0; g < kNormRing / kNormGroup; ++g) {
+      if (g < groups) fetch(g);
+      asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+    for (int g = 0; g < groups; ++g) {
+      asm volatile("cp.async.wait_group %0;" ::"n"(kNormRing / kNormGroup - 1) : "memory");
+#pragma unroll
+      for (int u = 0; u < kNormGroup; ++u) add_squares8(ss, ring[((g * kNormGroup + u) % kNormRing) * kNormOwn + threadIdx.x]);
+      if (g + kNormRing / kNormGroup < groups) fetch(g + kNormRing / kNormGroup);
+      asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
   }
-#pragma unroll
-  for (int u = 0; u < kNormVecs; ++u) ss += sumsq8(keep[u]);
-#pragma unroll 4
-  for (long long i = rest; i < v1; i += blockDim.x) ss += sumsq8(x[i]);
-  const float mine = block_sum(ss, red);
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");     // every CTA of the cluster has started
-  if (threadIdx.x < kNormCluster) {                        // hand the partial sum to every CTA of the cluster
+  if (threadIdx.x < kNormOwn && lane < kNormCluster) {     // hand the warp's sum to every CTA of the cluster
     uint32_t dst;
-    const uint32_t local = smem_u32(&part[rank]);
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(dst) : "r"(local), "r"(threadIdx.x));
-    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(dst), "f"(mine) : "memory");
+    const uint32_t local = smem_u32(&red[rank * (kNormOwn / 32) + warp]);
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(dst) : "r"(local), "r"(lane));
+    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(dst), "f"(ss) : "memory");
   }
   __syncwarp();
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-  float tot = 0.f;
+  float tot = red[lane];
 #pragma unroll
-  for (int r = 0; r < kNormCluster; ++r) tot += part[r];
+  for (int o = 16; o > 0; o >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, o);
   // an all-zero (padding) tile stays exactly zero (inv = 0 also covers the out-of-place copy); uniform over the cluster
   if (tot == 0.f && y == x) return;
   const float inv = tot == 0.f ? 0.f : 1.f / (sqrtf(tot) + eps);
-#pragma unroll
-  for (int u = 0; u < kNormVecs; ++u) {
-    const long long i = v0 + threadIdx.x + u * static_cast<long long>(blockDim.x);
-    if (i < v1) y[i] = scale8(keep[u], inv);
+  const int c = threadIdx.x % kNormOwn;
+  constexpr int kStep = kNormThreads / kNormOwn;
+  if (ONCE) {
+    for (int k = threadIdx.x / kNormOwn; k < len; k += kStep) {
+      const long long i = base + c + static_cast<long long>(k) * kNormChains;
+      if (i < nv) y[i] = scale8(ring[k * kNormOwn + c], inv);
+    }
+    return;
   }
-#pragma unroll 4
-  for (long long i = rest; i < v1; i += blockDim.x) y[i] = scale8(x[i], inv);
+  for (int k0 = threadIdx.x / kNormOwn; k0 < len; k0 += kStep * kNormGroup) {
+    uint4 v[kNormGroup];                                   // loads together, ahead of the stores, which may alias them
+#pragma unroll
+    for (int u = 0; u < kNormGroup; ++u) {
+      const long long i = base + c + static_cast<long long>(k0 + u * kStep) * kNormChains;
+      if (i < nv) v[u] = x[i];
+    }
+#pragma unroll
+    for (int u = 0; u < kNormGroup; ++u) {
+      const long long i = base + c + static_cast<long long>(k0 + u * kStep) * kNormChains;
+      if (i < nv) y[i] = scale8(v[u], inv);
+    }
+  }
 }
 
 void ns_normalize(void* tiles, long long n_tiles, long long tile_elems, float eps, cudaStream_t stream, void* out) {
   if (n_tiles <= 0) return;
-  // A cluster per tile where one CTA per tile would leave half of the SMs idle.  Measured: full matrices of 2 to 6 MB,
-  // 4 or 8 a launch, 137 -> 24 us on average; 28 tiles of 512 17 -> 8 us; but 128 tiles of 512 take 18 us longer with
-  // clusters and 2300 of them 200 us longer, so many tiles keep one CTA each.  From 256 x 256 elements a slice is at
-  // least 256 threads x 4 vectors.
-  if (tile_elems % 8 == 0 && tile_elems >= 65536 && n_tiles * 2 <= num_sms()) {
-    const long long nv = tile_elems / 8, slice = (nv + kNormCluster - 1) / kNormCluster;
-    long long threads = (slice / kNormVecs + 31) / 32 * 32;
-    threads = threads < 256 ? 256 : (threads > 1024 ? 1024 : threads);
-    ns_normalize_cluster_kernel<<<static_cast<unsigned>(n_tiles * kNormCluster), static_cast<unsigned>(threads), 0, stream>>>(
-        reinterpret_cast<const uint4*>(tiles), reinterpret_cast<uint4*>(out ? out : tiles), nv, eps);
+  // A cluster per tile where one CTA per tile would leave half of the SMs idle.  Measured with clusters, and with one CTA
+  // per tile where that is known: 28 tiles of 512 6.4 us (17), 74 of them 13.7 (75 of them with one CTA each: 17.5), 8 of
+  // 1024 x 3072 32, 74 of 1024 72 (75: 88), 74 of 256 6.9 (75: 6.0).  The clusters are still level or ahead at the line;
+  // past it one CTA per tile fills the chip by itself.  From 256 x 256 elements every thread has eight loads or more.
+  if (tile_elems % 8 == 0 && tile_elems >= 65536 && tile_elems < (1LL << 40) && n_tiles * 2 <= num_sms()) {
+    constexpr int smem = kNormRing * kNormOwn * 16;
+    const bool once = tile_elems <= 8LL * kNormChains * kNormRing;
+    auto kern = once ? ns_normalize_cluster_kernel<true> : ns_normalize_cluster_kernel<false>;
+    static bool attr[2] = {false, false};
+    if (!attr[once]) { cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem); attr[once] = true; }
+    kern<<<static_cast<unsigned>(n_tiles * kNormCluster), kNormThreads, smem, stream>>>(
+        reinterpret_cast<const uint4*>(tiles), reinterpret_cast<uint4*>(out ? out : tiles), tile_elems / 8, eps);
     return;
   }
   const long long cap = static_cast<long long>(num_sms()) * 2;

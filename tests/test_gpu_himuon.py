@@ -377,3 +377,21 @@ def test_newton_schulz_leaves_its_input(shape, steps):
         assert torch.equal(x, keep) and out.data_ptr() != x.data_ptr()
         want = ref.newton_schulz(keep.cpu(), steps).float()
         assert (out.float().cpu() - want).norm() / want.norm() < 3e-2
+
+
+@pytest.mark.parametrize("shape", [(500, 64, 64), (300, 128, 128), (200, 100, 256), (160, 256, 256), (160, 512, 520), (80, 640, 1728),
+                                   (80, 1032, 520)])
+def test_newton_schulz_of_a_tile_does_not_depend_on_its_neighbours(shape):
+    """The number of tiles in a launch selects kernels and tile widths; a tile gets the same bits in every company (one rank
+    or several, any chunk size)."""
+    from himuon_b200 import ops
+    from himuon_b200.ops import ns as ns_ops
+
+    torch.manual_seed(5)
+    x = torch.randn(shape, device="cuda", dtype=torch.bfloat16) * torch.rand(shape[0], 1, 1, device="cuda").bfloat16()
+    x[7] = 0
+    whole = ns_ops.newton_schulz(x, 5)
+    for n in (1, 3, 24, 70):
+        parts = torch.cat([ns_ops.newton_schulz(c, 5) for c in x.split(n)])
+        assert torch.equal(parts, whole), f"{n} at a time: {(parts != whole).flatten(1).any(1).sum().item()} tiles differ"
+    ops.check_status()

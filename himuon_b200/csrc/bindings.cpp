@@ -79,13 +79,15 @@ static void untile_apply(const at::Tensor& entries, int64_t n_entries, int64_t t
   himuon::untile_apply(reinterpret_cast<const himuon::ApplyEntry*>(entries.data_ptr()), (int)n_entries, (int)total_units,
                        (int)Th, (int)Tw, tiles.data_ptr(), hyper.data_ptr<float>(), param_fp32 ? 1 : 0, cur_stream());
 }
-static void ns_repad(const at::Tensor& src, at::Tensor& dst) {
+static void ns_repad(const at::Tensor& src, at::Tensor& dst, const c10::optional<at::Tensor>& norm, double eps) {
   HM_CHECK(src.is_cuda() && dst.is_cuda() && src.dim() == 3 && dst.dim() == 3 && src.size(0) == dst.size(0) && src.is_contiguous() && dst.is_contiguous(), "ns_repad: contiguous (B, m, n) tensors");
-  HM_CHECK((is_bf16(src) || is_f32(src)) && (is_bf16(dst) || is_f32(dst)), "ns_repad: bf16 or fp32");
+  HM_CHECK((is_bf16(src) || is_f32(src)) && (is_bf16(dst) || is_f32(dst)) && (is_bf16(src) || is_bf16(dst)), "ns_repad: bf16 on one side, bf16 or fp32 on the other");
   HM_CHECK(src.size(1) < (1LL << 30) && src.size(2) < (1LL << 30) && dst.size(1) < (1LL << 30) && dst.size(2) < (1LL << 30), "ns_repad: matrix too large");
+  HM_CHECK(src.data_ptr() != dst.data_ptr() || (src.scalar_type() == dst.scalar_type() && src.sizes() == dst.sizes()), "ns_repad: in place needs one size and type");
+  if (norm.has_value()) HM_CHECK(norm->is_cuda() && is_f32(*norm) && norm->is_contiguous() && norm->numel() == src.size(0), "ns_repad: one fp32 norm per matrix");
   const c10::cuda::CUDAGuard guard(src.device());
   himuon::ns_repad(src.data_ptr(), dst.data_ptr(), src.size(0), (int)src.size(1), (int)src.size(2), (int)dst.size(1), (int)dst.size(2),
-                   is_f32(src) ? 1 : 0, is_f32(dst) ? 1 : 0, cur_stream());
+                   is_f32(src) ? 1 : 0, is_f32(dst) ? 1 : 0, cur_stream(), norm.has_value() ? norm->data_ptr<float>() : nullptr, (float)eps);
 }
 static void ns_normalize(at::Tensor& tiles, int64_t n_tiles, int64_t tile_elems, double eps, const c10::optional<at::Tensor>& out) {
   HM_CHECK(tiles.is_cuda() && is_bf16(tiles) && tiles.is_contiguous(), "ns_normalize: tiles must be contiguous bf16");
@@ -263,11 +265,11 @@ static void flash_attn_bwd(const at::Tensor& d_o, const at::Tensor& q, const at:
 }
 
 static bool ns5_fused_supported(int64_t m, int64_t n) { return himuon::ns5_fused_supported((int)m, (int)n); }
-static void ns5_fused(const at::Tensor& x, at::Tensor& out, int64_t steps, double eps) {
+static void ns5_fused(const at::Tensor& x, at::Tensor& out, int64_t steps, double eps, bool normalize) {
   HM_CHECK(x.is_cuda() && is_bf16(x) && is_bf16(out) && x.is_contiguous() && out.is_contiguous() && x.dim() == 3 && x.sizes() == out.sizes(), "ns5_fused: contiguous (B, m, n) bf16 tensors");
   HM_CHECK(himuon::ns5_fused_supported((int)x.size(1), (int)x.size(2)), "ns5_fused: tile shape not supported");
   const c10::cuda::CUDAGuard guard(x.device());
-  himuon::ns5_fused(x.data_ptr(), out.data_ptr(), x.size(0), (int)x.size(1), (int)x.size(2), (int)steps, (float)eps, cur_stream());
+  himuon::ns5_fused(x.data_ptr(), out.data_ptr(), x.size(0), (int)x.size(1), (int)x.size(2), (int)steps, (float)eps, cur_stream(), normalize ? 1 : 0);
 }
 
 static int64_t status(bool reset) { return himuon::read_status_word(reset); }
@@ -303,7 +305,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         py::arg("max_ctas") = 0, py::arg("symmetric") = false);
   m.def("momentum_tile", &momentum_tile);
   m.def("untile_apply", &untile_apply);
-  m.def("ns_repad", &ns_repad);
+  m.def("ns_repad", &ns_repad, py::arg("src"), py::arg("dst"), py::arg("norm") = py::none(), py::arg("eps") = 0.0);
   m.def("ns_normalize", &ns_normalize, py::arg("tiles"), py::arg("n_tiles"), py::arg("tile_elems"), py::arg("eps"),
         py::arg("out") = py::none());
   m.def("adamw_multi", &adamw_multi);
@@ -322,7 +324,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("flash_attn_fwd", &flash_attn_fwd);
   m.def("flash_attn_bwd", &flash_attn_bwd);
   m.def("ns5_fused_supported", &ns5_fused_supported);
-  m.def("ns5_fused", &ns5_fused);
+  m.def("ns5_fused", &ns5_fused, py::arg("x"), py::arg("out"), py::arg("steps"), py::arg("eps"), py::arg("normalize") = true);
   m.def("status", &status, py::arg("reset") = true);
   m.def("num_sms", [] { return himuon::num_sms(); });
   m.def("momentum_tile_units", [](int64_t R, int64_t C, int64_t Th) { return himuon::momentum_tile_units((int)R, (int)C, (int)Th); });

@@ -80,9 +80,10 @@ void untile_apply(const ApplyEntry* entries, int n_entries, int total_units, int
 void ns_normalize(void* tiles_bf16, long long n_tiles, long long tile_elems, float eps, cudaStream_t stream,
                   void* out = nullptr);
 
-// (batch, sm, sn) -> (batch, dm, dn), zero-filled or cropped, bf16 / fp32 on either side; both contiguous.
+// (batch, sm, sn) -> (batch, dm, dn), zero-filled or cropped, at least one side bf16, the other bf16 or fp32; both
+// contiguous.  With `norm` (one value per matrix) every element is divided by norm + eps.
 void ns_repad(const void* src, void* dst, long long batch, int sm, int sn, int dm, int dn, int src_fp32, int dst_fp32,
-              cudaStream_t stream);
+              cudaStream_t stream, const float* norm = nullptr, float eps = 0.f);
 
 struct AdamEntry {
   void* param;
@@ -186,8 +187,9 @@ void multi_copy(const CopySeg* segs_dev, int n_segs, long long total_units, int 
 
 // ---------------------------------------------------------------- fused tile-resident NS5
 // Five quintic Newton-Schulz iterations on (B, m, n) bf16 tiles with m <= n, m <= 128, n <= 128*... kept in
-// shared memory for the whole computation (see ns5_sm100.cu).
+// shared memory for the whole computation (see ns5_sm100.cu).  normalize = 0: the tiles are scaled already.
 bool ns5_fused_supported(int m, int n);
-void ns5_fused(const void* x_in, void* x_out, long long n_tiles, int m, int n, int steps, float eps, cudaStream_t s);
+void ns5_fused(const void* x_in, void* x_out, long long n_tiles, int m, int n, int steps, float eps, cudaStream_t s,
+               int normalize = 1);
 
 }  // namespace himuon

@@ -47,7 +47,7 @@ struct NsBars {
 template <int NCH, int HALVES>   // number of 64-column chunks of X
 __global__ void __launch_bounds__(128 * HALVES, HALVES == 1 ? 4 : (NCH <= 2 ? 3 : 2))
 ns5_fused_kernel(const __grid_constant__ CUtensorMap tmX, __nv_bfloat16* __restrict__ out, long long n_tiles, int m,
-                 int steps, float eps, int* status) {
+                 int steps, float eps, int normalize, int* status) {
   constexpr int N = NCH * 64;
   constexpr int TM_COLS = N <= 128 ? 128 : 256;            // TMEM columns of this CTA
   constexpr uint32_t A2_COL = TM_COLS == 256 ? 128 : 0;    // A*A lands beside A when there is room, else over it
@@ -93,30 +93,32 @@ ns5_fused_kernel(const __grid_constant__ CUtensorMap tmX, __nv_bfloat16* __restr
 
     // ---- Frobenius norm and normalisation.  One thread sums a whole row, whatever HALVES is: a tile's result must not
     // depend on the kernel that the number of tiles selects.
-    if (half == 0) {
-      float ss = 0.f;
+    if (normalize) {
+      if (half == 0) {
+        float ss = 0.f;
 #pragma unroll 8
-      for (int c = 0; c < NCH * 8; ++c) {
-        const uint4 v = *reinterpret_cast<const uint4*>(sX + ns_sw_off(row, c));
-        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+        for (int c = 0; c < NCH * 8; ++c) {
+          const uint4 v = *reinterpret_cast<const uint4*>(sX + ns_sw_off(row, c));
+          const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-        for (int q = 0; q < 4; ++q) { const float a = bf16_lo(w[q]), b = bf16_hi(w[q]); ss += a * a + b * b; }
+          for (int q = 0; q < 4; ++q) { const float a = bf16_lo(w[q]), b = bf16_hi(w[q]); ss += a * a + b * b; }
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+        if (lane == 0) bars->red[warp] = ss;
       }
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-      if (lane == 0) bars->red[warp] = ss;
-    }
-    __syncthreads();
-    const float tot = bars->red[0] + bars->red[1] + bars->red[2] + bars->red[3];
-    const float inv = 1.f / (sqrtf(tot) + eps);
+      __syncthreads();
+      const float tot = bars->red[0] + bars->red[1] + bars->red[2] + bars->red[3];
+      const float inv = 1.f / (sqrtf(tot) + eps);
 #pragma unroll 4
-    for (int c = half * (NCH * 8 / HALVES); c < (half + 1) * (NCH * 8 / HALVES); ++c) {
-      uint4* ptr = reinterpret_cast<uint4*>(sX + ns_sw_off(row, c));
-      uint4 v = *ptr;
-      uint32_t w[4] = {v.x, v.y, v.z, v.w};
+      for (int c = half * (NCH * 8 / HALVES); c < (half + 1) * (NCH * 8 / HALVES); ++c) {
+        uint4* ptr = reinterpret_cast<uint4*>(sX + ns_sw_off(row, c));
+        uint4 v = *ptr;
+        uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-      for (int q = 0; q < 4; ++q) w[q] = pack_bf16x2(bf16_lo(w[q]) * inv, bf16_hi(w[q]) * inv);
-      *ptr = make_uint4(w[0], w[1], w[2], w[3]);
+        for (int q = 0; q < 4; ++q) w[q] = pack_bf16x2(bf16_lo(w[q]) * inv, bf16_hi(w[q]) * inv);
+        *ptr = make_uint4(w[0], w[1], w[2], w[3]);
+      }
     }
     fence_proxy_async_smem();
     tc_fence_before();
@@ -239,7 +241,7 @@ ns5_fused_kernel(const __grid_constant__ CUtensorMap tmX, __nv_bfloat16* __restr
 bool ns5_fused_supported(int m, int n) { return m >= 1 && m <= 128 && m <= n && n % 64 == 0 && n >= 64 && n <= 256; }
 
 template <int NCH, int HALVES>
-static void launch_ns5(const void* x_in, void* x_out, long long n_tiles, int m, int steps, float eps, cudaStream_t s) {
+static void launch_ns5(const void* x_in, void* x_out, long long n_tiles, int m, int steps, float eps, int normalize, cudaStream_t s) {
   constexpr int N = NCH * 64;
   constexpr size_t SMEM = 1024 + (NCH + 2) * NS_HALF + 256;
   constexpr int TM_COLS = N <= 128 ? 128 : 256;
@@ -255,20 +257,20 @@ static void launch_ns5(const void* x_in, void* x_out, long long n_tiles, int m, 
   const int per_sm = by_smem < by_tmem ? by_smem : by_tmem;
   const long long cap = static_cast<long long>(num_sms()) * per_sm;
   const int grid = static_cast<int>(n_tiles < cap ? n_tiles : cap);
-  kern<<<grid, 128 * HALVES, SMEM, s>>>(tm, reinterpret_cast<__nv_bfloat16*>(x_out), n_tiles, m, steps, eps, status_word_ptr());
+  kern<<<grid, 128 * HALVES, SMEM, s>>>(tm, reinterpret_cast<__nv_bfloat16*>(x_out), n_tiles, m, steps, eps, normalize, status_word_ptr());
 }
 
-void ns5_fused(const void* x_in, void* x_out, long long n_tiles, int m, int n, int steps, float eps, cudaStream_t s) {
+void ns5_fused(const void* x_in, void* x_out, long long n_tiles, int m, int n, int steps, float eps, cudaStream_t s, int normalize) {
   if (n_tiles <= 0) return;
   if (!ns5_fused_supported(m, n)) throw std::runtime_error("himuon ns5_fused: unsupported tile shape");
   switch (n / 64) {
     case 1:
-      if (n_tiles > 3LL * num_sms()) launch_ns5<1, 1>(x_in, x_out, n_tiles, m, steps, eps, s);
-      else launch_ns5<1, 2>(x_in, x_out, n_tiles, m, steps, eps, s);
+      if (n_tiles > 3LL * num_sms()) launch_ns5<1, 1>(x_in, x_out, n_tiles, m, steps, eps, normalize, s);
+      else launch_ns5<1, 2>(x_in, x_out, n_tiles, m, steps, eps, normalize, s);
       break;
-    case 2: launch_ns5<2, 2>(x_in, x_out, n_tiles, m, steps, eps, s); break;
-    case 3: launch_ns5<3, 2>(x_in, x_out, n_tiles, m, steps, eps, s); break;
-    default: launch_ns5<4, 2>(x_in, x_out, n_tiles, m, steps, eps, s); break;
+    case 2: launch_ns5<2, 2>(x_in, x_out, n_tiles, m, steps, eps, normalize, s); break;
+    case 3: launch_ns5<3, 2>(x_in, x_out, n_tiles, m, steps, eps, normalize, s); break;
+    default: launch_ns5<4, 2>(x_in, x_out, n_tiles, m, steps, eps, normalize, s); break;
   }
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) throw std::runtime_error(std::string("himuon ns5_fused launch failed: ") + cudaGetErrorString(e));

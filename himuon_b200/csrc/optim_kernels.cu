@@ -504,22 +504,24 @@ void ns_normalize(void* tiles, long long n_tiles, long long tile_elems, float ep
 
 // ------------------------------------------------------------------------------------------------
 // Newton-Schulz on sides that are no multiples of 8: (B, sm, sn) of S -> (B, dm, dn) of D, rows and columns past the
-// source filled with zeros, those past the destination dropped, element type converted on the way.  One launch on each
-// side of the iteration in place of the cast, pad, norm, divide, cast, copy and crop launches of PyTorch.  Odd rows have
-// no common alignment, so accesses are single elements, coalesced along the row.
+// source filled with zeros, those past the destination dropped, element type converted on the way, and matrix b divided by
+// norm[b] + eps where norms are given (IEEE division, as PyTorch divides).  One launch on each side of the iteration and
+// one for the scaling, in place of the cast, pad, divide, cast, copy and crop launches of PyTorch.  Odd rows have no common
+// alignment, so accesses are single elements, coalesced along the row.  `src` may be `dst` when the sizes are the same.
 template <typename S, typename D>
 __global__ void __launch_bounds__(256)
-repad_kernel(const S* __restrict__ src, D* __restrict__ dst, int sm, int sn, int dm, int dn) {
+repad_kernel(const S* src, D* dst, int sm, int sn, int dm, int dn, const float* norm, float eps) {
   const S* s = src + static_cast<long long>(blockIdx.y) * sm * sn;
   D* d = dst + static_cast<long long>(blockIdx.y) * dm * dn;
+  const float div = norm ? __fadd_rn(norm[blockIdx.y], eps) : 1.f;
   for (int i = blockIdx.x; i < dm; i += gridDim.x)
     for (int j = threadIdx.x; j < dn; j += blockDim.x) {
       const float v = (i < sm && j < sn) ? ldf(s + static_cast<long long>(i) * sn + j) : 0.f;
-      stf(d + static_cast<long long>(i) * dn + j, v);
+      stf(d + static_cast<long long>(i) * dn + j, norm ? __fdiv_rn(v, div) : v);
     }
 }
 void ns_repad(const void* src, void* dst, long long batch, int sm, int sn, int dm, int dn, int src_fp32, int dst_fp32,
-              cudaStream_t stream) {
+              cudaStream_t stream, const float* norm, float eps) {
   if (batch <= 0 || dm <= 0 || dn <= 0) return;
   for (long long b0 = 0; b0 < batch; b0 += 65535) {       // grid.y limit
     const unsigned nb = static_cast<unsigned>(batch - b0 < 65535 ? batch - b0 : 65535);
@@ -527,11 +529,11 @@ void ns_repad(const void* src, void* dst, long long batch, int sm, int sn, int d
     const dim3 grid(static_cast<unsigned>(dm < want ? dm : want), nb);
     auto sp = static_cast<const char*>(src) + b0 * sm * sn * (src_fp32 ? 4 : 2);
     auto dp = static_cast<char*>(dst) + b0 * dm * dn * (dst_fp32 ? 4 : 2);
+    const float* np = norm ? norm + b0 : nullptr;
     using bf = __nv_bfloat16;
-    if (src_fp32 && !dst_fp32) repad_kernel<float, bf><<<grid, 256, 0, stream>>>((const float*)sp, (bf*)dp, sm, sn, dm, dn);
-    else if (!src_fp32 && dst_fp32) repad_kernel<bf, float><<<grid, 256, 0, stream>>>((const bf*)sp, (float*)dp, sm, sn, dm, dn);
-    else if (!src_fp32) repad_kernel<bf, bf><<<grid, 256, 0, stream>>>((const bf*)sp, (bf*)dp, sm, sn, dm, dn);
-    else repad_kernel<float, float><<<grid, 256, 0, stream>>>((const float*)sp, (float*)dp, sm, sn, dm, dn);
+    if (src_fp32) repad_kernel<float, bf><<<grid, 256, 0, stream>>>((const float*)sp, (bf*)dp, sm, sn, dm, dn, np, eps);
+    else if (dst_fp32) repad_kernel<bf, float><<<grid, 256, 0, stream>>>((const bf*)sp, (float*)dp, sm, sn, dm, dn, np, eps);
+    else repad_kernel<bf, bf><<<grid, 256, 0, stream>>>((const bf*)sp, (bf*)dp, sm, sn, dm, dn, np, eps);
   }
 }
 

@@ -25,6 +25,7 @@ from . import reference as ref
 from . import _count, gemm
 
 A_COEF, B_COEF, C_COEF = ref.NS_COEFFS
+EPS = 1e-7
 
 
 class NSWorkspace:
@@ -55,7 +56,7 @@ def fused_supported(m: int, n: int) -> bool:
     return lo >= 1 and lo <= 128 and hi % 64 == 0 and 64 <= hi <= 256
 
 
-def ns_inplace_cuda(X: torch.Tensor, steps: int = 5, eps: float = 1e-7, workspace: NSWorkspace | None = None,
+def ns_inplace_cuda(X: torch.Tensor, steps: int = 5, eps: float = EPS, workspace: NSWorkspace | None = None,
                     normalize: bool = True, source: torch.Tensor | None = None) -> torch.Tensor:
     """Orthogonalise a contiguous bf16 ``(B, m, n)`` CUDA buffer in place and return it.  With ``source`` (same shape and
     type) that tensor is read instead and left as it is: the first pass over the data, which scales every tile, writes to
@@ -119,11 +120,18 @@ def newton_schulz(G: torch.Tensor, steps: int = 5, workspace: NSWorkspace | None
         out = torch.empty(X.shape, device=X.device, dtype=X.dtype)
         if X.numel():
             e = _ext.ext()
-            pad = torch.empty(X.shape[0], -(-m // 8) * 8, -(-n // 8) * 8, device=X.device, dtype=torch.bfloat16)
+            pm, pn = -(-m // 8) * 8, -(-n // 8) * 8
+            pad = torch.empty(X.shape[0], pm, pn, device=X.device, dtype=torch.bfloat16)
             e.ns_repad(X, pad)
-            ns_inplace_cuda(pad, steps, workspace=workspace)
+            # the same bits as _pre_normalized
+            e.ns_repad(pad, pad, pad.float().norm(dim=(-2, -1)), EPS)
+            if e.ns5_fused_supported(pm, pn):
+                e.ns5_fused(pad, pad, int(steps), EPS, False)
+                _count()
+            else:
+                ns_inplace_cuda(pad, steps, workspace=workspace, normalize=False)
             e.ns_repad(pad, out)
-            _count(2)
+            _count(3)
         return out.reshape(shape).to(G.dtype)
     Xb = X.to(torch.bfloat16)
     if not Xb.is_contiguous():
@@ -137,6 +145,6 @@ def newton_schulz(G: torch.Tensor, steps: int = 5, workspace: NSWorkspace | None
     return out.reshape(shape).to(G.dtype)
 
 
-def _pre_normalized(X: torch.Tensor, eps: float = 1e-7) -> torch.Tensor:
+def _pre_normalized(X: torch.Tensor, eps: float = EPS) -> torch.Tensor:
     norm = X.float().norm(dim=(-2, -1), keepdim=True)
     return (X.float() / (norm + eps)).to(torch.bfloat16).contiguous()

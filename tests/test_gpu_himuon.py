@@ -395,3 +395,22 @@ def test_newton_schulz_of_a_tile_does_not_depend_on_its_neighbours(shape):
         parts = torch.cat([ns_ops.newton_schulz(c, 5) for c in x.split(n)])
         assert torch.equal(parts, whole), f"{n} at a time: {(parts != whole).flatten(1).any(1).sum().item()} tiles differ"
     ops.check_status()
+
+
+@pytest.mark.parametrize("shape", [(1308, 73, 192), (264, 59, 256), (300, 100, 250), (124, 887, 167), (6, 333, 500), (40, 1, 9),
+                                   (70000, 3, 9)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+def test_newton_schulz_odd_sides_scale_as_pytorch_does(shape, dtype):
+    """Odd sides: norm and division in PyTorch's order and rounding, whatever kernel runs the iteration after them."""
+    from himuon_b200 import ops
+    from himuon_b200.ops import ns as ns_ops
+
+    torch.manual_seed(6)
+    b, m, n = shape
+    x = (torch.randn(shape, device="cuda") * torch.rand(b, 1, 1, device="cuda")).to(dtype)
+    x[b // 2] = 0
+    padded = torch.nn.functional.pad(x.bfloat16(), (0, -n % 8, 0, -m % 8))
+    want = ns_ops.ns_inplace_cuda(ns_ops._pre_normalized(padded), 5, normalize=False)[:, :m, :n].to(dtype)
+    got = ns_ops.newton_schulz(x, 5)
+    assert torch.equal(got, want), f"{(got != want).sum().item()} of {got.numel()} elements differ"
+    ops.check_status()

@@ -123,8 +123,8 @@ def newton_schulz(G: torch.Tensor, steps: int = 5, workspace: NSWorkspace | None
             pm, pn = -(-m // 8) * 8, -(-n // 8) * 8
             pad = torch.empty(X.shape[0], pm, pn, device=X.device, dtype=torch.bfloat16)
             e.ns_repad(X, pad)
-            # the same bits as _pre_normalized
-            e.ns_repad(pad, pad, pad.float().norm(dim=(-2, -1)), EPS)
+            # the same bits as _pre_normalized: this norm adds the same fp32 squares in the same order, without the copy
+            e.ns_repad(pad, pad, torch.linalg.vector_norm(pad, dim=(-2, -1), dtype=torch.float32), EPS)
             if e.ns5_fused_supported(pm, pn):
                 e.ns5_fused(pad, pad, int(steps), EPS, False)
                 _count()

@@ -361,6 +361,13 @@ void rmsnorm_bwd(const void* dy, const void* x, const void* w, const float* rstd
 // Layout of the two kernels below: LN = D/8 lanes per head vector, lane l owning elements [8l, 8l+8) (one 16-byte
 // access); the lower LN/2 lanes hold the first half, the others the second half, so the rotation partner of every
 // element sits at the same register index in lane l^(LN/2).  A warp handles 32/LN vectors per pass.
+// Rounding: 64-wide heads round both products and their sum, as the PyTorch formulation does that served them before this
+// kernel and still serves other layouts; 128-wide heads have always fused the second product into the sum.
+template <int LN>
+__device__ __forceinline__ float rotate(float v, float c, float other, float s) {   // v * c + other * s
+  if constexpr (LN == 8) return __fadd_rn(__fmul_rn(v, c), __fmul_rn(other, s));
+  else return v * c + other * s;
+}
 template <int LN>
 __device__ __forceinline__ float head_sum(float v) {
 #pragma unroll
@@ -417,7 +424,7 @@ headnorm_rope_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat1
 #pragma unroll
     for (int q = 0; q < 8; ++q) {
       const float other = __shfl_xor_sync(0xffffffffu, xv[q], LN / 2);
-      out[q] = second ? xv[q] * cs[2 * q] + other * cs[2 * q + 1] : xv[q] * cs[2 * q] - other * cs[2 * q + 1];
+      out[q] = rotate<LN>(xv[q], cs[2 * q], second ? other : -other, cs[2 * q + 1]);
     }
     if (live) reinterpret_cast<uint4*>(y + static_cast<long long>(tok) * ld_out + head * D)[sub] = pack8(out);
   }
@@ -457,7 +464,7 @@ headnorm_rope_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat
 #pragma unroll
     for (int q = 0; q < 8; ++q) {                          // transpose of the rotation
       const float other = __shfl_xor_sync(0xffffffffu, g[q], LN / 2);
-      d[q] = second ? g[q] * cs[2 * q] - other * cs[2 * q + 1] : g[q] * cs[2 * q] + other * cs[2 * q + 1];
+      d[q] = rotate<LN>(g[q], cs[2 * q], second ? -other : other, cs[2 * q + 1]);
     }
     if (use_norm) {
       float h[8];

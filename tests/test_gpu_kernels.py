@@ -715,3 +715,24 @@ def test_momentum_and_apply_at_any_address(dtype, offset, tile_offset, n_src, Th
         _close(*mom, atol=atol, rtol=rtol)
         _close(*tile, atol=1e-5, rtol=2 ** -7.9)            # stored in bf16
         _close(*param, atol=atol, rtol=rtol)
+
+
+@pytest.mark.parametrize("B,S,H", [(1, 1, 1), (3, 37, 5), (2, 1313, 10)])
+def test_rope_64_rounds_as_pytorch_does(B, S, H):
+    """Heads of 64 without a norm: the kernel and the PyTorch formulation (which takes every layout) give the same bits."""
+    from himuon_b200 import ops
+    from himuon_b200.ops import reference as ref
+
+    torch.manual_seed(7)
+    D = 64
+    x = torch.randn(B * S, H * D, device="cuda", dtype=torch.bfloat16)
+    dy = torch.randn_like(x)
+    cs = ref.rope_tables(S, D, 1e4, device="cuda")
+    xk, xr = x.clone().requires_grad_(True), x.clone().requires_grad_(True)
+    before = ops.launch_count()
+    yk = ops.head_norm_rope(xk, None, cs, H, S, D, 1e-6)
+    assert ops.launch_count() == before + 1
+    yr = ref.apply_rope(xr.view(B, S, H, D), cs).view(B * S, H * D)
+    yk.backward(dy)
+    yr.backward(dy)
+    assert torch.equal(yk, yr) and torch.equal(xk.grad, xr.grad)

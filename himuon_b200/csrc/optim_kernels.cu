@@ -212,6 +212,15 @@ void momentum_tile(const MomTileEntry* entries, int n_entries, int total_units, 
 }
 
 // ------------------------------------------------------------------------------------------------
+// Decay, rounded to the parameter's type, then one multiply-add: spelled out, so that every path rounds alike.
+template <typename P>
+__device__ __forceinline__ float apply_update(float p, bool has_decay, float decay, float step, float u) {
+  if (has_decay) {
+    p = __fmul_rn(p, decay);
+    if (sizeof(P) == 2) p = round_bf16(p);
+  }
+  return __fmaf_rn(-step, u, p);
+}
 template <typename P>
 __global__ void __launch_bounds__(256)
 untile_apply_kernel(const ApplyEntry* __restrict__ entries, int n_entries, int total_units, int Th, int Tw,
@@ -265,8 +274,7 @@ untile_apply_kernel(const ApplyEntry* __restrict__ entries, int n_entries, int t
           Vec16<P>::unpack(pv[u], f);
 #pragma unroll
           for (int q = 0; q < VN; ++q) {
-            if (wd > 0.f) f[q] = sizeof(P) == 2 ? round_bf16(f[q] * decay) : f[q] * decay;
-            f[q] -= step * uf[u][q];
+            f[q] = apply_update<P>(f[q], wd > 0.f, decay, step, uf[u][q]);
           }
           *reinterpret_cast<uint4*>(pp[u]) = Vec16<P>::pack(f);
         }
@@ -280,9 +288,7 @@ untile_apply_kernel(const ApplyEntry* __restrict__ entries, int n_entries, int t
         if (gi >= e.h || gj >= e.w) continue;
         const float u = __bfloat162float(in[static_cast<long long>(i) * Tw + j]);
         P* pp = param + static_cast<long long>(gi) * e.ld + gj;
-        float v = ldf(pp);
-        if (wd > 0.f) { v *= decay; if (sizeof(P) == 2) v = round_bf16(v); }
-        stf(pp, v - step * u);
+        stf(pp, apply_update<P>(ldf(pp), wd > 0.f, decay, step, u));
       }
     }
   }

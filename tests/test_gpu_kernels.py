@@ -736,3 +736,25 @@ def test_rope_64_rounds_as_pytorch_does(B, S, H):
     yk.backward(dy)
     yr.backward(dy)
     assert torch.equal(yk, yr) and torch.equal(xk.grad, xr.grad)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("offset", [0, 1])
+def test_untile_apply_rounds_alike_on_every_path(dtype, offset):
+    """The decayed parameter is rounded, then one fused multiply-add follows, on 16-byte and element-wise accesses."""
+    e = _ext()
+    torch.manual_seed(8)
+    h, w, T = 256, 320, 64
+    flat = torch.randn(h * w + 16, device="cuda").to(dtype)
+    p = flat[offset: offset + h * w].view(h, w)
+    p0 = p.clone()
+    tiles = torch.randn(20, T, T, device="cuda", dtype=torch.bfloat16)
+    tab = struct.pack("<Qq6ifi", p.data_ptr(), 0, h, w, 4, 5, 0, 0, 2.0, w)
+    hyper = torch.tensor([0.02, 0.1], device="cuda")
+    e.untile_apply(torch.frombuffer(bytearray(tab), dtype=torch.uint8).cuda(), 1, e.momentum_tile_units(4, 5, T), T, T, tiles,
+                   hyper, dtype == torch.float32)
+    u = tiles.view(4, 5, T, T).permute(0, 2, 1, 3).reshape(h, w).double()
+    decay = (1 - hyper[0].double() * hyper[1].double()).float()
+    # the sum of a product and an fp32 value is exact in 64 bits here up to a rounding 2^-29 times as likely to matter
+    want = ((p0.float() * decay).to(dtype).double() - (hyper[0] * 2.0).double() * u).float().to(dtype)
+    assert torch.equal(p, want), (p != want).sum().item()

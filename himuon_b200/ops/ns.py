@@ -112,6 +112,13 @@ def newton_schulz(G: torch.Tensor, steps: int = 5, workspace: NSWorkspace | None
     shape = G.shape
     X = G.reshape(-1, shape[-2], shape[-1])
     m, n = X.shape[-2:]
+    # A result for a tensor that records its gradient stays attached to it, whatever its type, sides and address: that path
+    # is made of PyTorch's own copies.
+    attached = torch.is_grad_enabled() and G.requires_grad
+    if (m % 8 or n % 8) and attached:
+        padded = torch.nn.functional.pad(X.to(torch.bfloat16), (0, -n % 8, 0, -m % 8))
+        out = ns_inplace_cuda(_pre_normalized(padded), steps, workspace=workspace, normalize=False)[:, :m, :n]
+        return out.reshape(shape).to(G.dtype)
     if m % 8 or n % 8:
         # pad to the TMA granularity; zero rows/columns do not change the iteration
         if X.dtype not in (torch.bfloat16, torch.float32):
@@ -138,7 +145,7 @@ def newton_schulz(G: torch.Tensor, steps: int = 5, workspace: NSWorkspace | None
         out = ns_inplace_cuda(Xb.contiguous(), steps, workspace=workspace)
     elif Xb.data_ptr() != G.data_ptr():                    # a converted copy: ours to overwrite
         out = ns_inplace_cuda(Xb, steps, workspace=workspace)
-    elif Xb.data_ptr() % 16 == 0:                          # G itself, which is only read
+    elif Xb.data_ptr() % 16 == 0 and not attached:         # G itself, which is only read
         out = ns_inplace_cuda(torch.empty_like(Xb), steps, workspace=workspace, source=Xb)
     else:
         out = ns_inplace_cuda(Xb.clone(), steps, workspace=workspace)

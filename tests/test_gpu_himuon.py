@@ -414,3 +414,23 @@ def test_newton_schulz_odd_sides_scale_as_pytorch_does(shape, dtype):
     got = ns_ops.newton_schulz(x, 5)
     assert torch.equal(got, want), f"{(got != want).sum().item()} of {got.numel()} elements differ"
     ops.check_status()
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("shape", [(3, 128, 128), (2, 256, 512), (3, 7, 9), (2, 257, 64)])
+@pytest.mark.parametrize("offset", [0, 1])
+def test_newton_schulz_result_stays_attached(dtype, shape, offset):
+    """Under grad mode the result belongs to its input's graph for every type, shape and address, and has the same bits."""
+    from himuon_b200.ops import ns as ns_ops
+
+    torch.manual_seed(9)
+    numel = shape[0] * shape[1] * shape[2]
+    x = torch.randn(numel + 8, device="cuda").to(dtype)[offset: offset + numel].view(shape).requires_grad_(True)
+    keep = x.detach().clone()
+    out = ns_ops.newton_schulz(x, 5)
+    assert out.requires_grad and torch.equal(x, keep)
+    out.sum().backward()
+    assert x.grad is not None and x.grad.shape == x.shape
+    with torch.no_grad():
+        plain = ns_ops.newton_schulz(x, 5)
+    assert not plain.requires_grad and torch.equal(plain, out)

@@ -55,7 +55,7 @@ static void gemm(const at::Tensor& a, const at::Tensor& b, at::Tensor& out, cons
   if (aux.has_value() && beta != 0.0) {
     const at::Tensor& x = aux.value();
     HM_CHECK(x.scalar_type() == out.scalar_type() && x.dim() == nd && x.stride(nd - 1) == 1, "gemm aux must match the output dtype/rank");
-    HM_CHECK(x.size(nd - 2) == g.M && x.size(nd - 1) == g.N && (nd == 2 || x.size(0) == g.batch), "gemm aux has the wrong shape");
+    HM_CHECK(x.size(nd - 2) == g.M && x.size(nd - 1) == g.N && (nd == 2 || x.size(0) >= g.batch), "gemm aux has the wrong shape");
     g.aux = x.data_ptr(); g.ldaux = x.stride(nd - 2); g.strideAux = nd == 3 ? x.stride(0) : 0;
   }
   himuon::gemm_bf16(g, cur_stream());

@@ -758,3 +758,19 @@ def test_untile_apply_rounds_alike_on_every_path(dtype, offset):
     # the sum of a product and an fp32 value is exact in 64 bits here up to a rounding 2^-29 times as likely to matter
     want = ((p0.float() * decay).to(dtype).double() - (hyper[0] * 2.0).double() * u).float().to(dtype)
     assert torch.equal(p, want), (p != want).sum().item()
+
+
+@pytest.mark.parametrize("M,N,K", [(64, 72, 64), (256, 512, 2048)])
+def test_gemm_aux_with_more_matrices_than_the_product(M, N, K):
+    """A batched aux operand may have matrices to spare; one with too few is refused."""
+    from himuon_b200 import ops
+
+    torch.manual_seed(0)
+    a = torch.randn(3, M, K, device="cuda", dtype=torch.bfloat16)
+    b = torch.randn(3, K, N, device="cuda", dtype=torch.bfloat16)
+    x = torch.randn(5, M, N, device="cuda", dtype=torch.bfloat16)
+    out = ops.gemm(a, b, aux=x, beta=1.0)
+    assert torch.equal(out, ops.gemm(a, b, aux=x[:3].clone(), beta=1.0))
+    with pytest.raises(RuntimeError):
+        ops.gemm(a, b, aux=x[:2], beta=1.0)
+    _assert_status_clean()

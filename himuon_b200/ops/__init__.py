@@ -456,6 +456,12 @@ def _head_norm_rope_double(ctx, dy, x, w, cos_sin):
     return (got.get(id(x)), None if w is None else got.get(id(w_leaf)), None, None, None, None, None, None)
 
 
+def _check_width(op: str, t: torch.Tensor, width: int) -> None:
+    # The bindings read the head width off the tensor: here the caller's own head_dim is held against it.
+    if t.shape[-1] != width:
+        raise RuntimeError(f"himuon_b200.ops.{op}: {width} columns expected, got {t.shape[-1]}")
+
+
 def _kernel_rows(t: torch.Tensor) -> bool:
     """A 2-D tensor whose rows the kernels can address: unit inner stride, every row on a 16-byte boundary."""
     return t.dim() == 2 and t.stride(1) == 1 and t.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0
@@ -481,6 +487,7 @@ def head_norm_rope(x2d, w, cos_sin, heads: int, seq_len: int, head_dim: int, eps
     """``x2d``: ``(B*S, heads*head_dim)`` (may be a column slice).  Returns the same layout.  ``inplace_grad``: the
     backward pass may overwrite the gradient it receives with the gradient it returns."""
     if use_kernels(x2d) and head_dim == 128:
+        _check_width("head_norm_rope", x2d, heads * 128)
         return _HeadNormRopeFn.apply(x2d, w, cos_sin, heads, seq_len, eps, _deferrable(w, defer_dw), inplace_grad)
     if use_kernels(x2d) and head_dim == 64 and _rope64_ok(x2d, w, cos_sin, heads, seq_len):
         # callers rely on being told once that 64-wide heads leave the 128-wide kernel
@@ -565,12 +572,16 @@ def attention(q2d, k2d, v2d, B: int, S: int, Hq: int, Hkv: int, head_dim: int, s
     """Causal GQA attention on ``(B*S, heads*head_dim)`` views; returns ``(B*S, Hq*head_dim)``."""
     scale = scale if scale is not None else 1.0 / math.sqrt(head_dim)
     if use_kernels(q2d) and head_dim == 128:
+        _check_width("attention", q2d, Hq * 128)             # (k and v are held against q in the binding)
         return _FlashAttnFn.apply(q2d, k2d, v2d, B, S, Hq, Hkv, scale)
     if use_kernels(q2d) and head_dim < 128 and head_dim % 8 == 0:
         # Narrower heads (64 in Llama-3.2-1B and llama_220m) run the same tcgen05 kernels: the TMA loads fill the tiles
         # up with zeros and the epilogues cut them off, so nothing is padded in memory.  Up to 64 columns half of the
         # tensor work goes away too.
-        rows = [t if _kernel_rows(t) else t.contiguous() for t in (q2d, k2d, v2d)]
+        T = q2d.shape[0]
+        rows = [t if t.shape == (T, h * head_dim) else t.reshape(T, h * head_dim)
+                for t, h in ((q2d, Hq), (k2d, Hkv), (v2d, Hkv))]
+        rows = [t if _kernel_rows(t) else t.contiguous() for t in rows]
         rows = [t if t.data_ptr() % 16 == 0 else t.clone() for t in rows]
         return _FlashAttnFn.apply(*rows, B, S, Hq, Hkv, scale)
     if use_kernels(q2d):

@@ -774,3 +774,35 @@ def test_gemm_aux_with_more_matrices_than_the_product(M, N, K):
     with pytest.raises(RuntimeError):
         ops.gemm(a, b, aux=x[:2], beta=1.0)
     _assert_status_clean()
+
+
+def test_attention_accepts_and_refuses_the_shapes_it_always_has():
+    """Heads of 128: keys and values may have tokens to spare.  Narrower heads: also (tokens, heads, head_dim) operands, but
+    no spare tokens.  A width that does not belong to head_dim is refused by both, and by the rotary op."""
+    from himuon_b200 import ops
+    from himuon_b200.ops import reference as ref
+
+    torch.manual_seed(0)
+    B, S, Hq, Hkv = 2, 96, 4, 2
+    for D in (128, 64):
+        q = torch.randn(B * S, Hq * D, device="cuda", dtype=torch.bfloat16, requires_grad=True)
+        k, v = (torch.randn(B * S + 40, Hkv * D, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+        want = ops.attention(q, k[: B * S], v[: B * S], B, S, Hq, Hkv, D)
+        (g_want,) = torch.autograd.grad(want.float().square().sum(), q)
+        if D == 128:
+            got = ops.attention(q, k, v, B, S, Hq, Hkv, D)
+            assert torch.equal(got, want)
+            assert torch.equal(torch.autograd.grad(got.float().square().sum(), q)[0], g_want)
+        else:
+            with pytest.raises(RuntimeError):
+                ops.attention(q, k, v, B, S, Hq, Hkv, D)
+            got = ops.attention(q.view(B * S, Hq, D), k[: B * S].view(B * S, Hkv, D), v[: B * S].view(B * S, Hkv, D), B, S, Hq, Hkv, D)
+            assert torch.equal(got, want)
+        with pytest.raises(RuntimeError):
+            ops.attention(q, k[: B * S - 1], v[: B * S - 1], B, S, Hq, Hkv, D)
+        other = 192 - D
+        with pytest.raises(RuntimeError):
+            ops.attention(q, k[: B * S], v[: B * S], B, S, Hq, Hkv, other)
+        with pytest.raises(RuntimeError):
+            ops.head_norm_rope(q, None, ref.rope_tables(S, 128, 1e4, device="cuda"), Hq, S, other, 1e-6)
+    _assert_status_clean()

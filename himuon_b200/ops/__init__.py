@@ -422,8 +422,7 @@ class _HeadNormRopeFn(torch.autograd.Function):
         if torch.is_grad_enabled() and dy.shape[1] == ctx.heads * 64:
             # create_graph=True: 64-wide heads stay differentiable twice, as the PyTorch formulation is
             return _head_norm_rope_double(ctx, dy, x, w, cos_sin)
-        if dy.stride(-1) != 1 or (dy.shape[1] == ctx.heads * 64 and (dy.stride(0) % 8 or dy.data_ptr() % 16)):
-            dy = dy.contiguous()
+        dy = _with_kernel_rows(dy)
         # Each head vector is read completely before it is written, so the input gradient may take the place of the
         # incoming one (asked for by callers that know dy has no other reader, e.g. a slice of attention's dq|dk|dv).
         inplace = ctx.inplace_grad and dy.stride(0) % 8 == 0 and dy.data_ptr() % 16 == 0
@@ -465,6 +464,11 @@ def _check_width(op: str, t: torch.Tensor, width: int) -> None:
 def _kernel_rows(t: torch.Tensor) -> bool:
     """A 2-D tensor whose rows the kernels can address: unit inner stride, every row on a 16-byte boundary."""
     return t.dim() == 2 and t.stride(1) == 1 and t.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0
+
+
+def _with_kernel_rows(t: torch.Tensor) -> torch.Tensor:
+    # (a copy: contiguous() returns a contiguous tensor as it is, also one that starts off the grid or has one row)
+    return t if _kernel_rows(t) else t.clone(memory_format=torch.contiguous_format)
 
 
 def _transformed(t: torch.Tensor) -> bool:
@@ -553,8 +557,7 @@ class _FlashAttnFn(torch.autograd.Function):
     def backward(ctx, do):
         q, k, v, o, lse = ctx.saved_tensors
         B, S, Hq, Hkv, scale = ctx.dims
-        if do.stride(-1) != 1 or do.stride(0) % 8 or do.data_ptr() % 16:
-            do = do.contiguous()
+        do = _with_kernel_rows(do)
         D = q.shape[1] // Hq
         # dq | dk | dv share one buffer so the fused QKV projection sees a single contiguous gradient
         dqkv = torch.empty(q.shape[0], (Hq + 2 * Hkv) * D, device=q.device, dtype=q.dtype)
@@ -581,9 +584,7 @@ def attention(q2d, k2d, v2d, B: int, S: int, Hq: int, Hkv: int, head_dim: int, s
         T = q2d.shape[0]
         rows = [t if t.shape == (T, h * head_dim) else t.reshape(T, h * head_dim)
                 for t, h in ((q2d, Hq), (k2d, Hkv), (v2d, Hkv))]
-        rows = [t if _kernel_rows(t) else t.contiguous() for t in rows]
-        rows = [t if t.data_ptr() % 16 == 0 else t.clone() for t in rows]
-        return _FlashAttnFn.apply(*rows, B, S, Hq, Hkv, scale)
+        return _FlashAttnFn.apply(*(_with_kernel_rows(t) for t in rows), B, S, Hq, Hkv, scale)
     if use_kernels(q2d):
         _warn_torch_path("attention", f"head_dim {head_dim} (the kernels take 128, or a multiple of 8 below it)")
     q = q2d.reshape(B, S, Hq, head_dim)

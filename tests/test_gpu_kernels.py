@@ -806,3 +806,44 @@ def test_attention_accepts_and_refuses_the_shapes_it_always_has():
         with pytest.raises(RuntimeError):
             ops.head_norm_rope(q, None, ref.rope_tables(S, 128, 1e4, device="cuda"), Hq, S, other, 1e-6)
     _assert_status_clean()
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("B,S", [(2, 96), (1, 1)])
+@pytest.mark.parametrize("form", ["offset", "pitch"])
+def test_gradients_and_operands_at_any_address(D, B, S, form):
+    """Incoming gradients (and operands of narrow heads) that are contiguous but start off the 16-byte grid, or whose row
+    pitch is odd, also where one row makes them contiguous all the same."""
+    from himuon_b200 import ops
+    from himuon_b200.ops import reference as ref
+
+    torch.manual_seed(0)
+    Hq, Hkv, T = 4, 2, B * S
+
+    def odd(t):
+        if form == "offset":
+            flat = torch.empty(t.numel() + 1, device="cuda", dtype=t.dtype)
+            out = flat[1:].view(t.shape)
+        else:
+            out = torch.empty(t.shape[0] * (t.shape[1] + 1) + 8, device="cuda", dtype=t.dtype).as_strided(t.shape, (t.shape[1] + 1, 1))
+        return out.copy_(t)
+
+    q, k, v = (torch.randn(T, h * D, device="cuda", dtype=torch.bfloat16) for h in (Hq, Hkv, Hkv))
+    do = torch.randn_like(q)
+    cs = ref.rope_tables(S, D, 1e4, device="cuda")
+    w = torch.ones(D, device="cuda", dtype=torch.bfloat16)
+
+    def run(operands, grad):
+        leaves = [t.detach().requires_grad_(True) for t in operands]
+        o = ops.attention(*leaves, B, S, Hq, Hkv, D)
+        o.backward(grad)
+        x = q.clone().requires_grad_(True)
+        y = ops.head_norm_rope(x, w, cs, Hq, S, D, 1e-6)
+        y.backward(grad)
+        return [o.detach(), y.detach(), x.grad] + [t.grad for t in leaves]
+
+    want = run((q, k, v), do)
+    got = run([odd(t) for t in (q, k, v)] if D < 128 else (q, k, v), odd(do))
+    for a, b in zip(want, got):
+        assert torch.equal(a, b)
+    _assert_status_clean()

@@ -43,16 +43,13 @@ def use_kernels(t: torch.Tensor) -> bool:
 _WARNED: set = set()
 
 
-def _warn_once(op: str, why: str, what: str, stacklevel: int = 3) -> None:
+def _warn_torch_path(op: str, why: str) -> None:
+    """Says once per (op, reason) that a bf16 CUDA tensor is taking the plain PyTorch implementation of an op."""
     if (op, why) not in _WARNED:
         _WARNED.add((op, why))
         import warnings
-        warnings.warn(f"himuon_b200.ops.{op}: {why}; {what}", stacklevel=stacklevel)
-
-
-def _warn_torch_path(op: str, why: str) -> None:
-    """Says once per (op, reason) that a bf16 CUDA tensor is taking the plain PyTorch implementation of an op."""
-    _warn_once(op, why, "running the PyTorch implementation instead of the sm_100a kernel", stacklevel=4)
+        warnings.warn(f"himuon_b200.ops.{op}: {why}; running the PyTorch implementation instead of the sm_100a kernel",
+                      stacklevel=3)
 
 
 def check_status() -> None:
@@ -494,8 +491,6 @@ def head_norm_rope(x2d, w, cos_sin, heads: int, seq_len: int, head_dim: int, eps
         _check_width("head_norm_rope", x2d, heads * 128)
         return _HeadNormRopeFn.apply(x2d, w, cos_sin, heads, seq_len, eps, _deferrable(w, defer_dw), inplace_grad)
     if use_kernels(x2d) and head_dim == 64 and _rope64_ok(x2d, w, cos_sin, heads, seq_len):
-        # callers rely on being told once that 64-wide heads leave the 128-wide kernel
-        _warn_once("head_norm_rope", "head_dim 64", "running the 64-wide sm_100a kernel")
         return _HeadNormRopeFn.apply(x2d, w, cos_sin, heads, seq_len, eps, _deferrable(w, defer_dw), inplace_grad)
     if use_kernels(x2d):
         _warn_torch_path("head_norm_rope", f"head_dim {head_dim} or its layout (the kernel takes 64 and 128, 16-byte aligned rows)")

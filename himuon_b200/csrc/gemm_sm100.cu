@@ -28,11 +28,12 @@ namespace himuon {
 __device__ int g_status_word = 0;
 
 // AUX_TMA (bf16 output with an aux operand): the aux tile arrives by TMA in the very staging slab that its output slab
-// leaves from.  NSTG slabs rotate through load -> combine in place -> store, with the loads issued three slabs ahead
+// leaves from.  NSTG slabs rotate through load -> combine in place -> store, with the loads issued NSTG - 1 slabs ahead
 // (across tile boundaries), so the epilogue threads never wait on global memory.
-constexpr int NSTG = 4;                       // staging slabs
+// Three operand stages and four slabs (256-wide tiles) serve short reductions, whose epilogue is the longer part; four
+// stages and two slabs serve long plain ones in numbers (`long_plain()`).
 constexpr int GEMM_THREADS = 384;             // warps 0-3: TMA, MMA, TMEM allocation, slabs; 4-11: epilogue
-template <int BN, int STAGES, bool A_MN, bool B_MN, bool AUX_TMA>
+template <int BN, int STAGES, int NSTG, bool A_MN, bool B_MN, bool AUX_TMA>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                  const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CUtensorMap tmX, GemmDev p) {
@@ -361,12 +362,12 @@ static bool aux_tma_ok(const GemmArgs& a) {
          reinterpret_cast<uintptr_t>(a.C) % 16 == 0;
 }
 
-template <int BN, int STAGES, bool A_MN, bool B_MN, bool AUX_TMA>
+template <int BN, int STAGES, int NSTG, bool A_MN, bool B_MN, bool AUX_TMA>
 static void launch_gemm(const GemmArgs& a, cudaStream_t stream) {
   constexpr uint32_t STAGE_BYTES = (BM + BN) * BK * 2;
   constexpr size_t SMEM = 1024 + STAGES * STAGE_BYTES + NSTG * SLAB_BYTES + 256;
   static_assert(SMEM <= 232448, "shared memory budget of one CTA exceeded");
-  auto kern = gemm_bf16_kernel<BN, STAGES, A_MN, B_MN, AUX_TMA>;
+  auto kern = gemm_bf16_kernel<BN, STAGES, NSTG, A_MN, B_MN, AUX_TMA>;
   static bool attr_done = false;
   if (!attr_done) {
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(SMEM));
@@ -464,6 +465,19 @@ static int tile_width(const GemmArgs& a) {
   return rounds(tile_count(a, 128), sms) * kNarrowRound < static_cast<double>(rounds(tile_count(a, 256), sms)) ? 128 : 256;
 }
 
+// 256-wide tiles without an aux operand that need the longer operand ring: many rounds of tiles with a reduction so long
+// that the main loop, not the epilogue, sets the pace (an fp32 slab takes half the columns, so that line lies lower and the
+// slabs are less of a help), and outputs that leave by plain stores and use no slabs at all.  Measured, three stages and
+// four slabs against four and two: 4096 x 8192 x 512 35.6 / 45.9 us, x 896 56.1 / 56.1, x 1024 62.5 / 57.3, x 1984
+// 110.9 / 98.7; 2048 x 32000 x 1024 118 / 111; fp32 4096 x 8192 x 256 30.5 / 34.4, x 384 38.5 / 37.1, x 1024 70.9 / 67.0.  With
+// few rounds the slabs win at any length: 1895 x 2560 x 1984 (two rounds) 30.7 / 33.4, symmetric 128 x 512 x 512 x 1280 (six)
+// 71.3 / 73.3.
+static bool long_plain(const GemmArgs& a) {
+  if (!c_rows_aligned(a)) return true;
+  const long long sms = a.max_ctas > 0 ? a.max_ctas : num_sms();
+  return a.K >= (a.out_fp32 ? 384 : 1024) && rounds(tile_count(a, 256), sms) > 6;
+}
+
 void gemm_bf16(const GemmArgs& a, cudaStream_t stream) {
   if (a.M <= 0 || a.N <= 0 || a.batch <= 0) return;
   if (a.K <= 0) throw std::runtime_error("himuon gemm: K must be positive");
@@ -473,20 +487,21 @@ void gemm_bf16(const GemmArgs& a, cudaStream_t stream) {
   }
   const int best_bn = a.N <= 128 ? 128 : (a.N <= 192 ? 192 : tile_width(a));
   const int sel = (a.a_mn ? 2 : 0) | (a.b_mn ? 1 : 0);
-#define HM_LAUNCH(BN_, ST_, AX_)                                                   \
+#define HM_LAUNCH(BN_, ST_, SL_, AX_)                                              \
   switch (sel) {                                                                   \
-    case 0: launch_gemm<BN_, ST_, false, false, AX_>(a, stream); break;            \
-    case 1: launch_gemm<BN_, ST_, false, true, AX_>(a, stream); break;             \
-    case 2: launch_gemm<BN_, ST_, true, false, AX_>(a, stream); break;             \
-    default: launch_gemm<BN_, ST_, true, true, AX_>(a, stream); break;             \
+    case 0: launch_gemm<BN_, ST_, SL_, false, false, AX_>(a, stream); break;       \
+    case 1: launch_gemm<BN_, ST_, SL_, false, true, AX_>(a, stream); break;        \
+    case 2: launch_gemm<BN_, ST_, SL_, true, false, AX_>(a, stream); break;        \
+    default: launch_gemm<BN_, ST_, SL_, true, true, AX_>(a, stream); break;        \
   }
   if (aux_tma_ok(a)) {
-    if (best_bn == 128) { HM_LAUNCH(128, 5, true) }
-    else if (best_bn == 192) { HM_LAUNCH(192, 4, true) }
-    else { HM_LAUNCH(256, 3, true) }
-  } else if (best_bn == 128) { HM_LAUNCH(128, 5, false) }
-  else if (best_bn == 192) { HM_LAUNCH(192, 4, false) }
-  else { HM_LAUNCH(256, 3, false) }
+    if (best_bn == 128) { HM_LAUNCH(128, 5, 4, true) }
+    else if (best_bn == 192) { HM_LAUNCH(192, 4, 4, true) }
+    else { HM_LAUNCH(256, 3, 4, true) }
+  } else if (best_bn == 192) { HM_LAUNCH(192, 4, 4, false) }
+  else if (best_bn == 128) { HM_LAUNCH(128, 5, 4, false) }
+  else if (long_plain(a)) { HM_LAUNCH(256, 4, 2, false) }
+  else { HM_LAUNCH(256, 3, 4, false) }
 #undef HM_LAUNCH
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) throw std::runtime_error(std::string("himuon gemm launch failed: ") + cudaGetErrorString(e));

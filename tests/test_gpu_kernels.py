@@ -847,3 +847,24 @@ def test_gradients_and_operands_at_any_address(D, B, S, form):
     for a, b in zip(want, got):
         assert torch.equal(a, b)
     _assert_status_clean()
+
+
+@pytest.mark.parametrize("trans_a,trans_b", [(False, True), (False, False), (True, False)])
+@pytest.mark.parametrize("M,N,K,dtype", [(2176, 16400, 1024, torch.bfloat16), (2112, 16392, 1088, torch.bfloat16),
+                                         (4096, 8200, 392, torch.float32), (520, 1023, 200, torch.bfloat16), (520, 777, 72, torch.float32)])
+def test_gemm_with_the_longer_operand_ring(M, N, K, dtype, trans_a, trans_b):
+    """Long plain products with many rounds of tiles, and outputs whose rows TMA cannot store: four stages, two slabs."""
+    from himuon_b200 import ops
+
+    torch.manual_seed(0)
+    a = torch.randn((K, M) if trans_a else (M, K), device="cuda", dtype=torch.bfloat16)
+    pad = -N % 8                                         # operand rows stay addressable where the output's are not
+    b = torch.randn((N, K) if trans_b else (K, N + pad), device="cuda", dtype=torch.bfloat16)
+    b = b if trans_b else b[:, :N]
+    out = torch.full((M, N), 9.0, device="cuda", dtype=dtype)
+    ops.gemm(a, b, trans_a=trans_a, trans_b=trans_b, out=out)
+    torch.cuda.synchronize()
+    _assert_status_clean()
+    ref = (a.float().t() if trans_a else a.float()) @ (b.float().t() if trans_b else b.float())
+    tol = 1e-5 if dtype == torch.float32 else 2 ** -8     # as in test_gemm_kernel_choice, rounded once
+    _close(out, ref, atol=tol * math.sqrt(K), rtol=tol)

@@ -419,13 +419,14 @@ static void launch_gemm2(const GemmArgs& a, cudaStream_t stream) {
   }
 }
 
-// True when the pair kernel can run this problem and is expected to win: TMA-storable output, more than one CTA
+// True when the pair kernel can run this problem and is expected to win: TMA-storable output (whole 16-byte groups of
+// columns: a TMA store writes those whole, past the output's last column if need be), more than one CTA
 // tile of rows, and a reduction long enough (K >= 2048) to amortise the 256-column epilogue; short-K batched
 // products (the Newton-Schulz GEMMs) are faster on the one-CTA kernel.
 bool gemm2_supported(const GemmArgs& a) {
   const int esz = a.out_fp32 ? 4 : 2;
   const int row_align = 16 / esz;
-  return a.M > BM && a.N > 192 && a.K >= 2048 && (a.ldc % row_align == 0) && (a.batch == 1 || a.strideC % row_align == 0) &&
+  return a.M > BM && a.N > 192 && a.N % row_align == 0 && a.K >= 2048 && (a.ldc % row_align == 0) && (a.batch == 1 || a.strideC % row_align == 0) &&
          (reinterpret_cast<uintptr_t>(a.C) % 16 == 0);
 }
 

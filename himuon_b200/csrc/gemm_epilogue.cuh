@@ -17,6 +17,7 @@ struct GemmDev {
   int round_acc;    // 1: round alpha*acc to bf16 before adding beta*aux
   int tiles_m, tiles_n, kblocks;
   int tma_store;    // 1: epilogue goes through shared-memory slabs and TMA stores (needs 16-byte aligned C rows)
+  int n_store;      // columns that TMA stores: N rounded down to whole 16-byte groups, because a TMA store writes those whole
   // Work list: items [0, full_items) are whole tiles; in the pair kernel each tile of a mostly empty last wave is cut
   // into `nslices` K-ranges, one item each, whose fp32 partial sums meet in a scratch tile.
   int full_items, total_items, nslices;
@@ -206,6 +207,14 @@ __device__ __forceinline__ void slab_fp32(uint32_t t_slab, uint8_t* my_row, int 
     o.w = alpha * __uint_as_float(v[4 * j + 3]) + beta * __uint_as_float(xa[j].w);
     *reinterpret_cast<float4*>(my_row + ((j ^ (row_in_tile & 7)) << 4)) = o;
   }
+}
+
+// The columns of a finished slab past the last whole 16-byte group (`n_store` ... N - 1), from the thread's own staging row.
+template <typename T>
+__device__ __forceinline__ void store_tail(T* c_row, const uint8_t* my_row, int row_in_tile, int col, int n_store, int N) {
+  constexpr int per = 16 / sizeof(T);
+  const T* src = reinterpret_cast<const T*>(my_row + ((((n_store - col) / per) ^ (row_in_tile & 7)) << 4));
+  for (int t = 0; n_store + t < N; ++t) c_row[n_store + t] = src[t];
 }
 
 // Pair kernel: epilogue of one accumulator tile through swizzled shared-memory slabs and TMA stores.  Called by the 128

@@ -187,7 +187,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       while (st.item < p.total_items) {
         const uint32_t buf = seq & (NSTG - 1);
         if (!mbar_wait(&slab_done[buf], (seq / NSTG) & 1, abort_flag, p.status, 5)) break;
-        tma_store_3d(&tmC, sC + buf * SLAB_BYTES, st.col, st.tc.mt * BM, st.tc.b);
+        if (st.col < p.n_store) tma_store_3d(&tmC, sC + buf * SLAB_BYTES, st.col, st.tc.mt * BM, st.tc.b);
         tma_store_commit();
         tma_store_wait_read<1>();        // the slab stored before this one is drained: it is the next to be opened
         open_next();
@@ -231,6 +231,11 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           if (!mbar_wait(&slab_open[buf], (seq / NSTG) & 1, abort_flag, p.status, 5)) { ok = false; break; }
           if (fp32_out) slab_fp32(t_slab, my_row, row_in_tile, xa, p.alpha, p.beta);
           else slab_bf16<AUX_TMA>(t_slab, my_row, row_in_tile, xa, p.alpha, p.beta, p.round_acc, mirror_c, p.ldc, col, row, p.N);
+          if (p.n_store < p.N && col + sw > p.n_store && row < p.M) {
+            const long long c_off = static_cast<long long>(b) * p.strideC + static_cast<long long>(row) * p.ldc;
+            if (fp32_out) store_tail(reinterpret_cast<float*>(p.C) + c_off, my_row, row_in_tile, col, p.n_store, p.N);
+            else store_tail(reinterpret_cast<__nv_bfloat16*>(p.C) + c_off, my_row, row_in_tile, col, p.n_store, p.N);
+          }
           fence_proxy_async_smem();
           mbar_arrive(&slab_done[buf]);
         }
@@ -350,7 +355,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 // C can be written by TMA stores
 static bool c_rows_aligned(const GemmArgs& a) {
   const int row_align = a.out_fp32 ? 4 : 8;
-  return a.ldc % row_align == 0 && (a.batch == 1 || a.strideC % row_align == 0) && reinterpret_cast<uintptr_t>(a.C) % 16 == 0;
+  return a.N >= row_align && a.ldc % row_align == 0 && (a.batch == 1 || a.strideC % row_align == 0) && reinterpret_cast<uintptr_t>(a.C) % 16 == 0;
 }
 
 // bf16 output with a bf16 aux tile that TMA can fetch (16-byte aligned base, rows and batches)
@@ -358,8 +363,7 @@ static bool aux_tma_ok(const GemmArgs& a) {
   // (broadcast rows or batches, strides of 0, take the plain loads)
   return a.aux != nullptr && !a.out_fp32 && a.ldaux % 8 == 0 && a.ldaux >= a.N &&
          (a.batch == 1 || (a.strideAux % 8 == 0 && a.strideAux > 0)) &&
-         reinterpret_cast<uintptr_t>(a.aux) % 16 == 0 && a.ldc % 8 == 0 && (a.batch == 1 || a.strideC % 8 == 0) &&
-         reinterpret_cast<uintptr_t>(a.C) % 16 == 0;
+         reinterpret_cast<uintptr_t>(a.aux) % 16 == 0 && c_rows_aligned(a);
 }
 
 template <int BN, int STAGES, int NSTG, bool A_MN, bool B_MN, bool AUX_TMA>
@@ -401,9 +405,10 @@ static void launch_gemm(const GemmArgs& a, cudaStream_t stream) {
   // C tensor map for the TMA-store epilogue: rows of 128 bytes (64 bf16 / 32 fp32 columns) per slab.
   const int esz = a.out_fp32 ? 4 : 2;
   p.tma_store = c_rows_aligned(a) ? 1 : 0;
+  p.n_store = a.N / (16 / esz) * (16 / esz);
   CUtensorMap tmC = tmA;
   if (p.tma_store) {
-    const uint64_t dimsC[3] = {static_cast<uint64_t>(a.N), static_cast<uint64_t>(a.M), static_cast<uint64_t>(a.batch)};
+    const uint64_t dimsC[3] = {static_cast<uint64_t>(p.n_store), static_cast<uint64_t>(a.M), static_cast<uint64_t>(a.batch)};
     const uint64_t strC[2] = {static_cast<uint64_t>(a.ldc) * esz,
                               a.batch > 1 ? static_cast<uint64_t>(a.strideC) * esz : static_cast<uint64_t>(a.ldc) * esz * a.M};
     const uint32_t boxC[3] = {static_cast<uint32_t>(128 / esz), BM, 1};

@@ -868,3 +868,40 @@ def test_gemm_with_the_longer_operand_ring(M, N, K, dtype, trans_a, trans_b):
     ref = (a.float().t() if trans_a else a.float()) @ (b.float().t() if trans_b else b.float())
     tol = 1e-5 if dtype == torch.float32 else 2 ** -8     # as in test_gemm_kernel_choice, rounded once
     _close(out, ref, atol=tol * math.sqrt(K), rtol=tol)
+
+
+@pytest.mark.parametrize("M,N,K,batch", [(256, 333, 64, 3), (200, 257, 72, 2), (300, 515, 2048, 1), (130, 9, 64, 2), (64, 7, 64, 1),
+                                         (513, 1021, 136, 30)])
+@pytest.mark.parametrize("mode", ["plain", "aux", "fp32", "fp32_aux", "add"])
+def test_gemm_writes_only_its_own_columns(M, N, K, batch, mode):
+    """A column slice as output: row pitch on the 16-byte grid, width off it.  TMA stores whole 16-byte groups, so the last
+    columns are written one by one and the neighbouring columns stay."""
+    from himuon_b200 import ops
+
+    torch.manual_seed(0)
+    dt = torch.float32 if mode.startswith("fp32") else torch.bfloat16
+    a = torch.randn(batch, M, K, device="cuda", dtype=torch.bfloat16)
+    b = torch.randn(batch, K, (N + 7) // 8 * 8, device="cuda", dtype=torch.bfloat16)[:, :, :N]
+    buf = torch.full((batch, M, (N + 7) // 8 * 8 + 8), 9.0, device="cuda", dtype=dt)
+    out = buf[:, :, :N]
+    x = torch.randn(batch, M, buf.shape[2], device="cuda", dtype=dt)[:, :, :N] if "aux" in mode else out if mode == "add" else None
+    ref = a.float() @ b.float() + (1.5 * x.float() if x is not None else 0.0)
+    ops.gemm(a, b, out=out, aux=x, beta=1.5 if x is not None else 0.0)
+    torch.cuda.synchronize()
+    _assert_status_clean()
+    assert (buf[:, :, N:] == 9.0).all(), "columns of the neighbour were written"
+    tol = 1e-5 if dt == torch.float32 else 2 ** -7
+    _close(out, ref, atol=tol * math.sqrt(K), rtol=tol)
+
+
+@pytest.mark.parametrize("m", [139, 333, 515])
+def test_symmetric_gemm_writes_only_its_own_columns(m):
+    from himuon_b200 import ops
+
+    torch.manual_seed(0)
+    x = torch.randn(2, m, 96, device="cuda", dtype=torch.bfloat16)
+    buf = torch.full((2, m, (m + 7) // 8 * 8), 9.0, device="cuda", dtype=torch.bfloat16)
+    ops.gemm(x, x, trans_b=True, out=buf[:, :, :m], symmetric=True)
+    _assert_status_clean()
+    assert (buf[:, :, m:] == 9.0).all() and torch.equal(buf[:, :, :m], buf[:, :, :m].transpose(1, 2))
+    _close(buf[:, :, :m], x.float() @ x.float().transpose(1, 2), atol=2 ** -8 * math.sqrt(96), rtol=2 ** -8)

@@ -209,12 +209,24 @@ __device__ __forceinline__ void slab_fp32(uint32_t t_slab, uint8_t* my_row, int 
   }
 }
 
-// The columns of a finished slab past the last whole 16-byte group (`n_store` ... N - 1), from the thread's own staging row.
+// The `n` columns of a finished slab past the last whole 16-byte group (number `group` of the slab's eight is theirs), one
+// thread for all rows.
 template <typename T>
-__device__ __forceinline__ void store_tail(T* c_row, const uint8_t* my_row, int row_in_tile, int col, int n_store, int N) {
-  constexpr int per = 16 / sizeof(T);
-  const T* src = reinterpret_cast<const T*>(my_row + ((((n_store - col) / per) ^ (row_in_tile & 7)) << 4));
-  for (int t = 0; n_store + t < N; ++t) c_row[n_store + t] = src[t];
+__device__ __noinline__ void store_tail(T* c, long long ldc, int rows, int n, const uint8_t* slab, int group) {
+#pragma unroll 4
+  for (int r = 0; r < rows; ++r) {
+    const uint4 v = *reinterpret_cast<const uint4*>(slab + r * 128 + ((group ^ (r & 7)) << 4));
+    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+    T* dst = c + r * ldc;
+    if constexpr (sizeof(T) == 4) {
+#pragma unroll
+      for (int t = 0; t < 3; ++t) if (t < n) dst[t] = __uint_as_float(w[t]);
+    } else {
+#pragma unroll
+      for (int t = 0; t < 7; ++t)
+        if (t < n) reinterpret_cast<unsigned short*>(dst)[t] = static_cast<unsigned short>(w[t >> 1] >> (16 * (t & 1)));
+    }
+  }
 }
 
 // Pair kernel: epilogue of one accumulator tile through swizzled shared-memory slabs and TMA stores.  Called by the 128

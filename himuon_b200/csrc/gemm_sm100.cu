@@ -22,6 +22,7 @@
 #include "sm100_common.cuh"
 #include "tma_host.h"
 
+#include <type_traits>
 
 namespace himuon {
 
@@ -184,16 +185,29 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         advance(op);
       };
       for (int a = 0; a < NSTG - 1; ++a) open_next();
-      while (st.item < p.total_items) {
-        const uint32_t buf = seq & (NSTG - 1);
-        if (!mbar_wait(&slab_done[buf], (seq / NSTG) & 1, abort_flag, p.status, 5)) break;
-        if (st.col < p.n_store) tma_store_3d(&tmC, sC + buf * SLAB_BYTES, st.col, st.tc.mt * BM, st.tc.b);
-        tma_store_commit();
-        tma_store_wait_read<1>();        // the slab stored before this one is drained: it is the next to be opened
-        open_next();
-        ++seq;
-        advance(st);
-      }
+      // `tail`: the last slab of a row of tiles ends in columns that TMA does not store.  They leave from this thread, in a
+      // loop of its own: a branch in the epilogue threads or in the loop of whole slabs cost the short products 1 %.
+      auto store_slabs = [&](auto tail) {
+        while (st.item < p.total_items) {
+          const uint32_t buf = seq & (NSTG - 1);
+          if (!mbar_wait(&slab_done[buf], (seq / NSTG) & 1, abort_flag, p.status, 5)) break;
+          const uint8_t* slab = sC + buf * SLAB_BYTES;
+          if (!tail.value || st.col < p.n_store) tma_store_3d(&tmC, slab, st.col, st.tc.mt * BM, st.tc.b);
+          if (tail.value && st.col + sw > p.n_store) {
+            const long long off = static_cast<long long>(st.tc.b) * p.strideC + static_cast<long long>(st.tc.mt) * BM * p.ldc + p.n_store;
+            const int rows = min(BM, p.M - st.tc.mt * BM), n = p.N - p.n_store, group = (p.n_store - st.col) * 8 / sw;
+            if (p.out_fp32) store_tail(reinterpret_cast<float*>(p.C) + off, p.ldc, rows, n, slab, group);
+            else store_tail(reinterpret_cast<__nv_bfloat16*>(p.C) + off, p.ldc, rows, n, slab, group);
+          }
+          tma_store_commit();
+          tma_store_wait_read<1>();        // the slab stored before this one is drained: it is the next to be opened
+          open_next();
+          ++seq;
+          advance(st);
+        }
+      };
+      if (p.n_store == p.N) store_slabs(std::false_type{});
+      else store_slabs(std::true_type{});
       tma_store_wait_read<0>();          // no store may still be reading shared memory at exit
     }
   } else if (warp >= 4) {
@@ -231,11 +245,6 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           if (!mbar_wait(&slab_open[buf], (seq / NSTG) & 1, abort_flag, p.status, 5)) { ok = false; break; }
           if (fp32_out) slab_fp32(t_slab, my_row, row_in_tile, xa, p.alpha, p.beta);
           else slab_bf16<AUX_TMA>(t_slab, my_row, row_in_tile, xa, p.alpha, p.beta, p.round_acc, mirror_c, p.ldc, col, row, p.N);
-          if (p.n_store < p.N && col + sw > p.n_store && row < p.M) {
-            const long long c_off = static_cast<long long>(b) * p.strideC + static_cast<long long>(row) * p.ldc;
-            if (fp32_out) store_tail(reinterpret_cast<float*>(p.C) + c_off, my_row, row_in_tile, col, p.n_store, p.N);
-            else store_tail(reinterpret_cast<__nv_bfloat16*>(p.C) + c_off, my_row, row_in_tile, col, p.n_store, p.N);
-          }
           fence_proxy_async_smem();
           mbar_arrive(&slab_done[buf]);
         }

@@ -905,3 +905,107 @@ def test_symmetric_gemm_writes_only_its_own_columns(m):
     _assert_status_clean()
     assert (buf[:, :, m:] == 9.0).all() and torch.equal(buf[:, :, :m], buf[:, :, :m].transpose(1, 2))
     _close(buf[:, :, :m], x.float() @ x.float().transpose(1, 2), atol=2 ** -8 * math.sqrt(96), rtol=2 ** -8)
+
+
+@pytest.mark.parametrize("N", [136, 160, 192])
+@pytest.mark.parametrize("batch", [1, 400])
+@pytest.mark.parametrize("mode", ["plain", "aux", "fp32", "fp32_aux"])
+def test_gemm_192_wide_tiles(N, batch, mode):
+    """Outputs of 129 to 192 columns: three bf16 slabs a tile, so that the two epilogue groups swap parity from tile to tile
+    (400 matrices of two row blocks: every CTA walks several)."""
+    from himuon_b200 import ops
+
+    torch.manual_seed(0)
+    M, K = 200, 136
+    dt = torch.float32 if mode.startswith("fp32") else torch.bfloat16
+    a = torch.randn(batch, M, K, device="cuda", dtype=torch.bfloat16)
+    b = torch.randn(batch, K, N, device="cuda", dtype=torch.bfloat16)
+    x = torch.randn(batch, M, N, device="cuda", dtype=dt) if "aux" in mode else None
+    out = torch.full((batch, M, N), 9.0, device="cuda", dtype=dt)
+    ops.gemm(a, b, out=out, aux=x, alpha=0.5, beta=-2.0 if x is not None else 0.0)
+    torch.cuda.synchronize()
+    _assert_status_clean()
+    ref = 0.5 * (a.float() @ b.float()) - (2.0 * x.float() if x is not None else 0.0)
+    tol = 1e-5 if dt == torch.float32 else 2 ** -7        # as in test_gemm_kernel_choice
+    _close(out, ref, atol=tol * math.sqrt(K), rtol=tol)
+
+
+@pytest.mark.parametrize("M,N,K,batch", [(130, 129, 64, 3), (256, 191, 200, 1), (300, 333, 264, 40), (136, 513, 72, 2), (4, 1, 8, 3)])
+@pytest.mark.parametrize("mode", ["plain", "aux", "round_acc", "strided", "fp32", "fp32_aux"])
+def test_gemm_outputs_that_tma_cannot_store(M, N, K, batch, mode):
+    """Output rows off the 16-byte grid leave by plain stores from both epilogue groups; nothing around them is written."""
+    from himuon_b200 import ops
+
+    torch.manual_seed(0)
+    dt = torch.float32 if mode.startswith("fp32") else torch.bfloat16
+    a = torch.randn(batch, M, K, device="cuda", dtype=torch.bfloat16)
+    b = torch.randn(batch, N, K, device="cuda", dtype=torch.bfloat16)
+    gap = 3 if mode == "strided" else 0
+    buf = torch.full((batch, M, N + gap), 9.0, device="cuda", dtype=dt)
+    out = buf[:, :, :N]
+    x = torch.randn(batch, M, N, device="cuda", dtype=dt) if mode in ("aux", "round_acc", "fp32_aux") else None
+    ops.gemm(a, b, trans_b=True, out=out, aux=x, alpha=0.5, beta=1.5 if x is not None else 0.0, round_acc=mode == "round_acc")
+    torch.cuda.synchronize()
+    _assert_status_clean()
+    ref = 0.5 * (a.float() @ b.float().transpose(1, 2))
+    if mode == "round_acc":
+        ref = ref.bfloat16().float()
+    if x is not None:
+        ref = ref + 1.5 * x.float()
+    assert (buf[:, :, N:] == 9.0).all()
+    tol = 1e-5 if dt == torch.float32 else 2 ** -7
+    _close(out, ref, atol=tol * math.sqrt(K), rtol=tol)
+
+
+@pytest.mark.parametrize("use_norm", [True, False])
+def test_head_norm_rope_64_differentiates_twice(use_norm):
+    """create_graph=True on the 64-wide op: gradients of gradients follow the fp32 formulation."""
+    from himuon_b200 import ops
+    from himuon_b200.ops import reference as ref
+
+    torch.manual_seed(3)
+    B, S, H, D = 2, 9, 3, 64
+    cs = ref.rope_tables(S, D, 1e4, device="cuda")
+    x0 = torch.randn(B * S, H * D, device="cuda", dtype=torch.bfloat16)
+    w0 = (1 + 0.1 * torch.randn(D, device="cuda")).bfloat16() if use_norm else None
+    c = torch.randn(B * S, H * D, device="cuda", dtype=torch.bfloat16)
+
+    def second(fn, x, w):
+        leaves = [x] if w is None else [x, w]
+        y = fn(x, w)
+        grads = torch.autograd.grad((y.float() ** 3 * c.float()).sum(), leaves, create_graph=True)
+        return torch.autograd.grad(sum((g.float() ** 2).sum() for g in grads), leaves)
+
+    got = second(lambda x, w: ops.head_norm_rope(x, w, cs, H, S, D, 1e-6), x0.clone().requires_grad_(True),
+                 None if w0 is None else w0.clone().requires_grad_(True))
+
+    def plain(x, w):
+        h = x.view(B, S, H, D)
+        return ref.apply_rope(ref.rmsnorm(h, w, 1e-6) if use_norm else h, cs).reshape(B * S, H * D)
+
+    want = second(plain, x0.float().requires_grad_(True), None if w0 is None else w0.float().requires_grad_(True))
+    for g, r in zip(got, want):
+        # bf16 intermediates (2^-9 each, about a dozen of them) through two backward passes
+        assert float((g.float() - r).norm() / r.norm()) < 12 * 2 ** -8
+
+
+def test_head_norm_rope_64_under_transforms():
+    """vmap and forward-mode tangents, for which the autograd function has no rules, take the PyTorch formulation."""
+    import warnings
+
+    from himuon_b200 import ops
+    from himuon_b200.ops import reference as ref
+
+    torch.manual_seed(4)
+    B, S, H, D = 2, 9, 3, 64
+    cs = ref.rope_tables(S, D, 1e4, device="cuda")
+    x = torch.randn(4, B * S, H * D, device="cuda", dtype=torch.bfloat16)
+    want = torch.stack([ref.apply_rope(t.view(B, S, H, D), cs).reshape(B * S, H * D) for t in x])
+    with warnings.catch_warnings():
+        warnings.simplefilter("ignore")
+        got = torch.vmap(lambda t: ops.head_norm_rope(t, None, cs, H, S, D, 1e-6))(x)
+        assert torch.equal(got, want)
+        with torch.autograd.forward_ad.dual_level():
+            dual = torch.autograd.forward_ad.make_dual(x[0], x[1])
+            y, tangent = torch.autograd.forward_ad.unpack_dual(ops.head_norm_rope(dual, None, cs, H, S, D, 1e-6))
+    assert torch.equal(y, want[0]) and torch.equal(tangent, want[1])      # the rotation is linear

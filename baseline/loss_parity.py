@@ -46,6 +46,10 @@ def main():
 
     # ---- reference stack
     sys.path.insert(0, os.path.join(ROOT, "baseline", "_ref"))
+    sys.path.insert(0, os.path.join(ROOT, "baseline"))
+    import reference_arm
+
+    reference_arm.require_reference()
     from transformers import AutoConfig, AutoModelForCausalLM
     import himuon.optim as ref_optim
 

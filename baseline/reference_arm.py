@@ -6,7 +6,8 @@ and streams FineWeb), so this harness performs the same calls in the same order 
 (the script's default) -> bf16 -> ``wrap_with_banks(Qwen3BankScheme)`` -> one root ``fully_shard`` with the
 bf16/bf16 mixed-precision policy -> ``release_pre_shard_refs`` -> ``get_optimizer("himuon")`` with
 ``cuda_graph=False`` (the script's FSDP default) -> WSD schedule -> the micro-step loop with
-``set_requires_gradient_sync``.  None of this repository's models, kernels or engines are imported.
+``set_requires_gradient_sync``.  None of this repository's models, kernels or engines are imported:
+``require_reference`` refuses to run when ``himuon`` resolves to this repository's own alias package.
 """
 
 from __future__ import annotations
@@ -15,6 +16,17 @@ import argparse
 import os
 
 LR, WD = 1e-2, 0.1
+REF_DIR = os.path.join(os.path.dirname(os.path.abspath(__file__)), "_ref")
+
+
+def require_reference(ref_dir: str = REF_DIR) -> None:
+    """Raises unless ``import himuon`` gives the package installed under ``ref_dir``."""
+    import importlib.util
+
+    spec = importlib.util.find_spec("himuon")
+    origin = os.path.realpath(spec.origin) if spec is not None and spec.origin else None
+    if origin is None or not origin.startswith(os.path.realpath(ref_dir) + os.sep):
+        raise RuntimeError(f"the reference is not installed under baseline/_ref (himuon resolves to {origin})")
 
 
 def _qwen3_config(name):
@@ -33,6 +45,7 @@ def _qwen3_config(name):
 
 
 def run(args, timed_region, host_batches, init_dist, barrier_sync):
+    require_reference()
     import torch
     import torch.distributed as dist
     from torch.distributed.device_mesh import init_device_mesh

@@ -127,3 +127,26 @@ def test_phase_timer_is_inert_without_cuda_and_ranges_nest():
         assert t.enabled is False and t.summary() == {}
     t.reset()
     assert t.summary() == {}
+
+
+def test_reference_arm_refuses_the_alias_package(tmp_path):
+    """``himuon`` is also the name of this repository's alias package: without the reference under baseline/_ref the
+    reference arm says so, and with a package there it accepts that one only."""
+    import json
+    import os
+    import subprocess
+    import sys
+
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    if not os.path.isdir(os.path.join(root, "baseline", "_ref", "himuon")):
+        out = subprocess.run([sys.executable, "bench.py", "--impl", "reference", "--steps", "1", "--warmup", "1"], cwd=root,
+                             capture_output=True, text=True, timeout=300)
+        line = json.loads(out.stdout.strip().splitlines()[-1])
+        assert out.returncode == 0 and line["impl"] == "reference" and "baseline/_ref" in line["unavailable"]
+    (tmp_path / "himuon").mkdir()
+    (tmp_path / "himuon" / "__init__.py").write_text("")
+    code = "import sys, reference_arm as r; r.require_reference(sys.argv[1]); print('accepted')"
+    for first, ok in ((str(tmp_path), True), (root, False)):
+        env = dict(os.environ, PYTHONPATH=os.pathsep.join([first, os.path.join(root, "baseline")]))
+        got = subprocess.run([sys.executable, "-c", code, str(tmp_path)], env=env, capture_output=True, text=True, cwd=str(tmp_path.parent))
+        assert ("accepted" in got.stdout) == ok, got.stderr

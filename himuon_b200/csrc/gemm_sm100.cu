@@ -469,8 +469,9 @@ static long long tile_count(const GemmArgs& a, int bn) {
 // Tile width for outputs wider than 192 columns: 256, unless tiles of 128 need clearly fewer rounds over the SMs.  Two
 // narrow tiles cost about 4 % more than a wide one (128 products of 512^3, which fill the chip either way: 755 and 786 us
 // for newton_schulz), and narrow symmetric tiles mirror a larger share of the output with 2-byte stores (396 tiles of
-// 256: 5 % slower than wide ones), so a narrow round counts 0.7 of a wide one.  They win where the wide tiles do not fill
-// the chip (6 matrices of 333 x 500: 211 -> 173 us) or just overflow it (symmetric products of 28 tiles of 512: 168 wide
+// 256: 5 % slower than wide ones).  So a narrow round counts 0.7 of a wide one: at 0.55 and 0.65 those 396 tiles went narrow
+// and the step that holds them took 4.5 % longer.  Narrow tiles win where the wide ones do not fill the chip (6 matrices of
+// 333 x 500: 211 -> 179 us for the whole newton_schulz call) or just overflow it (symmetric products of 28 tiles of 512: 168 wide
 // tiles are two rounds, 280 narrow ones two rounds of half the length; the optimizer step went from 277 to 250 us).
 constexpr double kNarrowRound = 0.7;
 static long long rounds(long long tiles, long long slots) { return (tiles + slots - 1) / slots; }

@@ -495,8 +495,13 @@ void ns_normalize(void* tiles, long long n_tiles, long long tile_elems, float ep
     constexpr int smem = kNormRing * kNormOwn * 16;
     const bool once = tile_elems <= 8LL * kNormChains * kNormRing;
     auto kern = once ? ns_normalize_cluster_kernel<true> : ns_normalize_cluster_kernel<false>;
-    static bool attr[2] = {false, false};
-    if (!attr[once]) { cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem); attr[once] = true; }
+    static bool attr[2][64] = {};                          // per device: the one-CTA kernel runs on any of them without a word
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev >= 64 || !attr[once][dev]) {
+      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+      if (dev < 64) attr[once][dev] = true;
+    }
     kern<<<static_cast<unsigned>(n_tiles * kNormCluster), kNormThreads, smem, stream>>>(
         reinterpret_cast<const uint4*>(tiles), reinterpret_cast<uint4*>(out ? out : tiles), tile_elems / 8, eps);
     return;

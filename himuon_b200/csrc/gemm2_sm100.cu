@@ -46,23 +46,31 @@ __device__ __forceinline__ void tmem_alloc2(uint32_t* smem_slot, uint32_t ncols)
 __device__ __forceinline__ void tmem_dealloc2(uint32_t taddr, uint32_t ncols) {
   asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
 }
-__device__ __forceinline__ void umma2_ss(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+__device__ __forceinline__ void umma2_ss(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate,
+                                         uint32_t e) {
   asm volatile(
-      "{\n\t.reg .pred p;\n\t"
+      "{\n\t.reg .pred p, e;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      "setp.ne.b32 e, %5, 0;\n\t"
+      "@e tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+      ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(e)
       : "memory");
 }
 // Arrives on the barrier at shared::cluster address `bar_addr` once all MMAs issued so far by this thread are done.
-__device__ __forceinline__ void umma2_commit(uint32_t bar_addr) {
-  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar_addr) : "memory");
+__device__ __forceinline__ void umma2_commit(uint32_t bar_addr, uint32_t e) {
+  asm volatile(
+      "{\n\t.reg .pred e;\n\tsetp.ne.b32 e, %1, 0;\n\t"
+      "@e tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}"
+      ::"r"(bar_addr), "r"(e)
+      : "memory");
 }
 // TMA load issued by either CTA of the pair; completion bytes go to the LEADER's barrier.
-__device__ __forceinline__ void tma2_load_3d(void* smem_dst, const CUtensorMap* tmap, uint64_t* bar, int x, int y, int z) {
+__device__ __forceinline__ void tma2_load_3d(void* smem_dst, const CUtensorMap* tmap, uint64_t* bar, int x, int y, int z,
+                                             uint32_t e) {
   asm volatile(
-      "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
-      ::"r"(smem_u32(smem_dst)), "l"(tmap), "r"(smem_u32(bar) & kPeerBitMask), "r"(x), "r"(y), "r"(z)
+      "{\n\t.reg .pred e;\n\tsetp.ne.b32 e, %6, 0;\n\t"
+      "@e cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];\n\t}"
+      ::"r"(smem_u32(smem_dst)), "l"(tmap), "r"(smem_u32(bar) & kPeerBitMask), "r"(x), "r"(y), "r"(z), "r"(e)
       : "memory");
 }
 
@@ -89,7 +97,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = warp_id();
   const int lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();
   const bool leader = rank == 0;
@@ -111,7 +119,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   __syncthreads();
   cluster_sync_all();                // the peer's barriers exist before anything signals them
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
 
   const int tiles_per_batch = p.tiles_m * p.tiles_n;
   const int pair = blockIdx.x >> 1;
@@ -119,9 +127,10 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer (both CTAs)
-    if (lane == 0) {
-      tma_prefetch_desc(&tmA);
-      tma_prefetch_desc(&tmB);
+    const uint32_t e = elect_one();
+    tma_prefetch_desc(&tmA);
+    tma_prefetch_desc(&tmB);
+    {
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -136,21 +145,21 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
         const int m0 = mt * 2 * BM + static_cast<int>(rank) * BM;
         const int n0 = nt * BN2 + static_cast<int>(rank) * BNH;
         for (int kb = w.kb0; kb < w.kb1; ++kb) {
-          if (!mbar_wait(&empty[stage], phase ^ 1, abort_flag, p.status, 1)) { ok = false; break; }
+          if (!mbar_wait_warp(&empty[stage], phase ^ 1, abort_flag, p.status, 1)) { ok = false; break; }
           uint8_t* sA = smem + stage * STAGE_BYTES;
           uint8_t* sB = sA + A_BYTES;
-          if (leader) mbar_expect_tx(&full[stage], 2 * STAGE_BYTES);
+          mbar_expect_tx(&full[stage], 2 * STAGE_BYTES, leader ? e : 0);
           if (!A_MN) {
-            tma2_load_3d(sA, &tmA, &full[stage], kb * BK, m0, b);
+            tma2_load_3d(sA, &tmA, &full[stage], kb * BK, m0, b, e);
           } else {
 #pragma unroll
-            for (int j = 0; j < BM / 64; ++j) tma2_load_3d(sA + j * CHUNK_BYTES, &tmA, &full[stage], m0 + j * 64, kb * BK, b);
+            for (int j = 0; j < BM / 64; ++j) tma2_load_3d(sA + j * CHUNK_BYTES, &tmA, &full[stage], m0 + j * 64, kb * BK, b, e);
           }
           if (!B_MN) {
-            tma2_load_3d(sB, &tmB, &full[stage], kb * BK, n0, b);
+            tma2_load_3d(sB, &tmB, &full[stage], kb * BK, n0, b, e);
           } else {
 #pragma unroll
-            for (int j = 0; j < BNH / 64; ++j) tma2_load_3d(sB + j * CHUNK_BYTES, &tmB, &full[stage], n0 + j * 64, kb * BK, b);
+            for (int j = 0; j < BNH / 64; ++j) tma2_load_3d(sB + j * CHUNK_BYTES, &tmB, &full[stage], n0 + j * 64, kb * BK, b, e);
           }
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
@@ -158,7 +167,8 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer (leader CTA only)
-    if (lane == 0 && leader) {
+    if (leader) {
+      const uint32_t e = elect_one();
       constexpr uint32_t idesc = umma_idesc_bf16(2 * BM, BN2, A_MN, B_MN);
       int stage = 0;
       uint32_t phase = 0;
@@ -168,11 +178,11 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
       WorkCursor cur(p, pair, n_pairs);
       WorkItem w;
       while (ok && cur.next(w)) {
-        if (!mbar_wait(&tempty[acc], acc_phase ^ 1, abort_flag, p.status, 2)) break;
+        if (!mbar_wait_warp(&tempty[acc], acc_phase ^ 1, abort_flag, p.status, 2)) break;
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(acc * BN2);
         for (int kb = w.kb0; kb < w.kb1; ++kb) {
-          if (!mbar_wait(&full[stage], phase, abort_flag, p.status, 2)) { ok = false; break; }
+          if (!mbar_wait_warp(&full[stage], phase, abort_flag, p.status, 2)) { ok = false; break; }
           tc_fence_after();
           const uint32_t a_base = smem_u32(smem + stage * STAGE_BYTES);
           const uint32_t b_base = a_base + A_BYTES;
@@ -182,17 +192,17 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
                                         : umma_smem_desc(a_base + k * 32, 16, 1024);
             const uint64_t bdesc = B_MN ? umma_smem_desc(b_base + k * 2048, CHUNK_BYTES, 1024)
                                         : umma_smem_desc(b_base + k * 32, 16, 1024);
-            umma2_ss(d_tmem, adesc, bdesc, idesc, (kb > w.kb0 || k > 0) ? 1u : 0u);
+            umma2_ss(d_tmem, adesc, bdesc, idesc, (kb > w.kb0 || k > 0) ? 1u : 0u, e);
           }
           const uint32_t e_addr = smem_u32(&empty[stage]);
-          umma2_commit(e_addr);                    // this CTA's producer
-          umma2_commit(map_to_cta(e_addr, 1));     // the peer's producer
+          umma2_commit(e_addr, e);                  // this CTA's producer
+          umma2_commit(map_to_cta(e_addr, 1), e);   // the peer's producer
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
         if (!ok) break;
         const uint32_t f_addr = smem_u32(&tfull[acc]);
-        umma2_commit(f_addr);
-        umma2_commit(map_to_cta(f_addr, 1));
+        umma2_commit(f_addr, e);
+        umma2_commit(map_to_cta(f_addr, 1), e);
         acc ^= 1;
         if (acc == 0) acc_phase ^= 1;
       }

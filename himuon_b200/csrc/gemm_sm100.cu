@@ -56,7 +56,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(slab_done + NSTG);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = warp_id();
   const int lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
@@ -76,13 +76,14 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
-    if (lane == 0) {
-      tma_prefetch_desc(&tmA);
-      tma_prefetch_desc(&tmB);
+    const uint32_t e = elect_one();
+    tma_prefetch_desc(&tmA);
+    tma_prefetch_desc(&tmB);
+    {
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -91,23 +92,23 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         const TileCoord tc = decode_tile(p, w.tile, BN / BM);
         const int b = tc.b, mt = tc.mt, nt = tc.nt;
         for (int kb = w.kb0; kb < w.kb1; ++kb) {
-          if (!mbar_wait(&empty[stage], phase ^ 1, abort_flag, p.status, 1)) { ok = false; break; }
+          if (!mbar_wait_warp(&empty[stage], phase ^ 1, abort_flag, p.status, 1)) { ok = false; break; }
           uint8_t* sA = smem + stage * STAGE_BYTES;
           uint8_t* sB = sA + A_BYTES;
-          mbar_expect_tx(&full[stage], STAGE_BYTES);
+          mbar_expect_tx(&full[stage], STAGE_BYTES, e);
           if (!A_MN) {
-            tma_load_3d(sA, &tmA, &full[stage], kb * BK, mt * BM, b);
+            tma_load_3d(sA, &tmA, &full[stage], kb * BK, mt * BM, b, e);
           } else {
 #pragma unroll
             for (int j = 0; j < BM / 64; ++j)
-              tma_load_3d(sA + j * CHUNK_BYTES, &tmA, &full[stage], mt * BM + j * 64, kb * BK, b);
+              tma_load_3d(sA + j * CHUNK_BYTES, &tmA, &full[stage], mt * BM + j * 64, kb * BK, b, e);
           }
           if (!B_MN) {
-            tma_load_3d(sB, &tmB, &full[stage], kb * BK, nt * BN, b);
+            tma_load_3d(sB, &tmB, &full[stage], kb * BK, nt * BN, b, e);
           } else {
 #pragma unroll
             for (int j = 0; j < BN / 64; ++j)
-              tma_load_3d(sB + j * CHUNK_BYTES, &tmB, &full[stage], nt * BN + j * 64, kb * BK, b);
+              tma_load_3d(sB + j * CHUNK_BYTES, &tmB, &full[stage], nt * BN + j * 64, kb * BK, b, e);
           }
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
@@ -115,7 +116,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    const uint32_t e = elect_one();
+    {
       constexpr uint32_t idesc = umma_idesc_bf16(BM, BN, A_MN, B_MN);
       int stage = 0;
       uint32_t phase = 0;
@@ -124,11 +126,11 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       bool ok = true;
       for (int item = blockIdx.x; ok && item < p.total_items; item += gridDim.x) {
         const WorkItem w = decode_item(p, item);
-        if (!mbar_wait(&tempty[acc], acc_phase ^ 1, abort_flag, p.status, 2)) break;
+        if (!mbar_wait_warp(&tempty[acc], acc_phase ^ 1, abort_flag, p.status, 2)) break;
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(acc * BN);
         for (int kb = w.kb0; kb < w.kb1; ++kb) {
-          if (!mbar_wait(&full[stage], phase, abort_flag, p.status, 2)) { ok = false; break; }
+          if (!mbar_wait_warp(&full[stage], phase, abort_flag, p.status, 2)) { ok = false; break; }
           tc_fence_after();
           const uint32_t a_base = smem_u32(smem + stage * STAGE_BYTES);
           const uint32_t b_base = a_base + A_BYTES;
@@ -138,13 +140,13 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                                         : umma_smem_desc(a_base + k * 32, 16, 1024);
             const uint64_t bdesc = B_MN ? umma_smem_desc(b_base + k * 2048, CHUNK_BYTES, 1024)
                                         : umma_smem_desc(b_base + k * 32, 16, 1024);
-            umma_ss(d_tmem, adesc, bdesc, idesc, (kb > w.kb0 || k > 0) ? 1u : 0u);
+            umma_ss(d_tmem, adesc, bdesc, idesc, (kb > w.kb0 || k > 0) ? 1u : 0u, e);
           }
-          umma_commit(&empty[stage]);
+          umma_commit(&empty[stage], e);
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
         if (!ok) break;
-        umma_commit(&tfull[acc]);
+        umma_commit(&tfull[acc], e);
         acc ^= 1;
         if (acc == 0) acc_phase ^= 1;
       }

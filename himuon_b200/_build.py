@@ -19,7 +19,7 @@ CUDA_SOURCES = [
     "model_kernels.cu",
     "attention_sm100.cu",
     "attention_kv64_sm100.cu", "attention_bwd_sm100.cu",
-    "ns5_sm100.cu",
+    "ns5_sm100.cu", "ns_pair_sm100.cu",
     "comm_kernels.cu",
     "soap_kernels.cu",
     "rmsnorm_bwd_noalloc.cu",

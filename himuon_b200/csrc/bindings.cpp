@@ -273,6 +273,26 @@ static void ns5_fused(const at::Tensor& x, at::Tensor& out, int64_t steps, doubl
   himuon::ns5_fused(x.data_ptr(), out.data_ptr(), x.size(0), (int)x.size(1), (int)x.size(2), (int)steps, (float)eps, cur_stream(), normalize ? 1 : 0);
 }
 
+// (pairs per matrix, matrices per cluster, scratch bytes) of ns_pair for this batch, or nothing where it is not the better path.
+static c10::optional<std::vector<int64_t>> ns_pair_plan(const at::Tensor& x) {
+  HM_CHECK(x.is_cuda() && x.dim() == 3, "ns_pair_plan: (B, m, n) CUDA tensor");
+  if (x.size(1) >= (1LL << 30) || x.size(2) >= (1LL << 30)) return c10::nullopt;
+  const c10::cuda::CUDAGuard guard(x.device());
+  int P = 1, W = 1;
+  if (!himuon::ns_pair_plan(x.size(0), (int)x.size(1), (int)x.size(2), &P, &W)) return c10::nullopt;
+  return std::vector<int64_t>{P, W, himuon::ns_pair_scratch_bytes(x.size(0), (int)x.size(1), (int)x.size(2), P, W)};
+}
+static void ns_pair(const at::Tensor& x, at::Tensor& out, at::Tensor& scratch, int64_t steps, int64_t P, int64_t W) {
+  HM_CHECK(x.is_cuda() && is_bf16(x) && is_bf16(out) && x.is_contiguous() && out.is_contiguous() && x.dim() == 3 && x.sizes() == out.sizes(), "ns_pair: contiguous (B, m, n) bf16 tensors");
+  HM_CHECK(x.size(1) <= 2048 && x.size(2) <= 2048 && x.size(1) % 8 == 0 && x.size(2) % 8 == 0, "ns_pair: sides are multiples of 8, at most 2048");
+  HM_CHECK(steps >= 1 && (steps >= 2 || x.data_ptr() != out.data_ptr()), "ns_pair: in place needs two steps");
+  HM_CHECK((P == 1 || P == 2 || P == 4) && W >= 1 && W <= 8, "ns_pair: bad plan");
+  const c10::cuda::CUDAGuard guard(x.device());
+  HM_CHECK(scratch.is_cuda() && scratch.device() == x.device() && scratch.is_contiguous() && reinterpret_cast<uintptr_t>(scratch.data_ptr()) % 128 == 0 &&
+           scratch.numel() * scratch.element_size() >= himuon::ns_pair_scratch_bytes(x.size(0), (int)x.size(1), (int)x.size(2), (int)P, (int)W), "ns_pair: scratch too small");
+  himuon::ns_pair(x.data_ptr(), out.data_ptr(), scratch.data_ptr(), x.size(0), (int)x.size(1), (int)x.size(2), (int)steps, (int)P, (int)W, cur_stream());
+}
+
 static int64_t status(bool reset) { return himuon::read_status_word(reset); }
 
 static void soap_moments(const at::Tensor& g, const at::Tensor& g_rot, at::Tensor& m, at::Tensor& v, double b1, double b2) {
@@ -326,6 +346,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("flash_attn_bwd", &flash_attn_bwd);
   m.def("ns5_fused_supported", &ns5_fused_supported);
   m.def("ns5_fused", &ns5_fused, py::arg("x"), py::arg("out"), py::arg("steps"), py::arg("eps"), py::arg("normalize") = true);
+  m.def("ns_pair_plan", &ns_pair_plan);
+  m.def("ns_pair", &ns_pair);
   m.def("status", &status, py::arg("reset") = true);
   m.def("num_sms", [] { return himuon::num_sms(); });
   m.def("momentum_tile_units", [](int64_t R, int64_t C, int64_t Th) { return himuon::momentum_tile_units((int)R, (int)C, (int)Th); });

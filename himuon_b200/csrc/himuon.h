@@ -192,4 +192,10 @@ bool ns5_fused_supported(int m, int n);
 void ns5_fused(const void* x_in, void* x_out, long long n_tiles, int m, int n, int steps, float eps, cudaStream_t s,
                int normalize = 1);
 
+// The same iterations on larger matrices that are scaled already, all products in one launch (see ns_pair_sm100.cu).
+// `plan` says whether the kernel is the better path and with how many CTA pairs per matrix (P) and matrices per cluster (W).
+bool ns_pair_plan(long long n_mats, int m, int n, int* P, int* W);
+long long ns_pair_scratch_bytes(long long n_mats, int m, int n, int P, int W);
+void ns_pair(const void* in, void* out, void* scratch, long long n_mats, int m, int n, int steps, int P, int W, cudaStream_t s);
+
 }  // namespace himuon

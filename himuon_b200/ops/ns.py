@@ -5,7 +5,9 @@
 ``muon.py:13-44``).  On a CUDA device it runs
 
 * the tile-resident fused kernel (one CTA per tile, operands in shared memory, accumulators
-  in TMEM) for tiles with at most 128 rows and 64..256 columns, and
+  in TMEM) for tiles with at most 128 rows and 64..256 columns,
+* one launch that takes every matrix through all iterations on CTA pairs, intermediates in the
+  L2, for short sides up to 512 (``csrc/ns_pair_sm100.cu``; ``ns_pair_plan`` has the exact line), and
 * otherwise a batched three-GEMM iteration on the persistent tcgen05 GEMM with fused
   epilogues (``A = X X^T``; ``B = c A A + b A``; ``X = bf16(B X) + a X``; the two symmetric
   products compute only the tiles that touch the lower triangle and mirror them, as the
@@ -29,10 +31,11 @@ EPS = 1e-7
 
 
 class NSWorkspace:
-    """Reusable scratch for the three-GEMM path (keeps addresses stable for CUDA graphs)."""
+    """Reusable scratch of the Newton-Schulz paths (keeps addresses stable for CUDA graphs)."""
 
     def __init__(self):
         self.bufs: dict[tuple, tuple[torch.Tensor, torch.Tensor, torch.Tensor]] = {}
+        self.flat: dict[str, list[torch.Tensor]] = {}      # last: the one in use; a captured graph may hold the others
 
     def get(self, B: int, m: int, n: int, device) -> tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
         k = min(m, n)
@@ -47,8 +50,15 @@ class NSWorkspace:
             self.bufs[key] = cur
         return cur[0][:B], cur[1][:B], cur[2][:B]
 
+    def scratch(self, nbytes: int, device) -> torch.Tensor:
+        have = self.flat.setdefault(str(device), [])
+        if not have or have[-1].numel() < nbytes:
+            have.append(torch.empty(nbytes, device=device, dtype=torch.uint8))
+        return have[-1]
+
     def clear(self):
         self.bufs.clear()
+        self.flat.clear()
 
 
 def fused_supported(m: int, n: int) -> bool:
@@ -75,6 +85,15 @@ def ns_inplace_cuda(X: torch.Tensor, steps: int = 5, eps: float = EPS, workspace
     if m % 8 or n % 8:
         raise ValueError(f"newton_schulz on CUDA needs tile sides that are multiples of 8, got ({m}, {n})")
     ws = workspace or NSWorkspace()
+    plan = e.ns_pair_plan(X) if steps >= 2 else None
+    if plan is not None:
+        pairs, interleaved, nbytes = plan
+        if normalize:
+            e.ns_normalize(src, Bt, m * n, float(eps), X)
+            _count()
+        e.ns_pair(X, X, ws.scratch(nbytes, X.device), int(steps), pairs, interleaved)
+        _count()
+        return X
     A, Bm, Y = ws.get(Bt, m, n, X.device)
     cur, nxt = X, Y
     if normalize:

@@ -1009,3 +1009,58 @@ def test_head_norm_rope_64_under_transforms():
             dual = torch.autograd.forward_ad.make_dual(x[0], x[1])
             y, tangent = torch.autograd.forward_ad.unpack_dual(ops.head_norm_rope(dual, None, cs, H, S, D, 1e-6))
     assert torch.equal(y, want[0]) and torch.equal(tangent, want[1])      # the rotation is linear
+
+
+def _three_gemm_iteration(x, steps):
+    """The products of the Newton-Schulz iteration one GEMM at a time, on a scaled bf16 batch."""
+    from himuon_b200.ops import gemm, ns
+
+    for _ in range(steps):
+        wide = x.shape[1] <= x.shape[2]
+        a = gemm(x, x, trans_b=True) if wide else gemm(x, x, trans_a=True)
+        b = gemm(a, a, trans_b=True, alpha=ns.C_COEF, beta=ns.B_COEF, aux=a)
+        x = gemm(b, x, alpha=1.0, beta=ns.A_COEF, aux=x, round_acc=True) if wide else \
+            gemm(x, b, alpha=1.0, beta=ns.A_COEF, aux=x, round_acc=True)
+    return x
+
+
+# One block and two of the short side, one to eight of the long one, wide and tall, sides at and beside the edges of the 64 and
+# 256 wide blocks; plans with one, two and four pairs per matrix (by the number of matrices), several rounds of matrices per
+# pair, interleaved ones, and ragged last rounds.
+@pytest.mark.parametrize("shape,steps", [
+    ((1, 256, 256), 5), ((3, 16, 264), 5), ((2, 512, 512), 5), ((19, 512, 512), 2), ((40, 512, 512), 5), ((75, 512, 504), 3),
+    ((5, 264, 1000), 5), ((5, 1000, 264), 5), ((100, 264, 1000), 2), ((20, 136, 2040), 5), ((20, 2040, 136), 4),
+    ((90, 336, 504), 5), ((90, 504, 336), 5), ((230, 256, 200), 5), ((331, 200, 256), 5), ((77, 24, 320), 5), ((250, 320, 24), 5),
+    ((80, 192, 328), 6), ((8, 448, 520), 5), ((8, 64, 8), 5)])
+def test_ns_pair_kernel_matches_the_gemms_bit_for_bit(shape, steps):
+    from himuon_b200.ops import ns, reference
+
+    g = torch.Generator("cuda").manual_seed(sum(shape))
+    x = torch.randn(shape, device="cuda", dtype=torch.bfloat16, generator=g)
+    assert _ext().ns_pair_plan(x) is not None
+    scaled = torch.empty_like(x)
+    _ext().ns_normalize(x, shape[0], shape[1] * shape[2], ns.EPS, scaled)
+    out = ns.ns_inplace_cuda(scaled.clone(), steps, normalize=False)
+    again = ns.ns_inplace_cuda(torch.full_like(x, float("nan")), steps, source=x)     # out of place, from unscaled values
+    _assert_status_clean()
+    assert torch.equal(out, _three_gemm_iteration(scaled, steps))
+    assert torch.equal(out, again)
+    # against the PyTorch path on fp32 copies of one matrix: five bf16 iterations leave 1-2 % (2-norm)
+    ref = reference.newton_schulz(x[-1].float().cpu(), steps=steps)
+    assert (out[-1].float().cpu() - ref).norm() <= 0.03 * ref.norm()
+
+
+def test_ns_pair_kernel_keeps_a_bad_matrix_to_itself():
+    from himuon_b200.ops import ns
+
+    x = torch.randn(9, 256, 256, device="cuda", dtype=torch.bfloat16)
+    good = ns.newton_schulz(x)
+    for bad in (float("nan"), float("inf")):
+        y = x.clone()
+        y[4, 17, 33] = bad
+        out = ns.newton_schulz(y)
+        assert out[4].isnan().all()
+        assert torch.equal(torch.cat([out[:4], out[5:]]), torch.cat([good[:4], good[5:]]))
+    x[4] = 0
+    assert (ns.newton_schulz(x)[4] == 0).all()
+    _assert_status_clean()

@@ -69,7 +69,7 @@ flash_bwd_dkv_t_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
   DkvBars* bars = reinterpret_cast<DkvBars*>(reinterpret_cast<uint8_t*>(sStat) + NST * STAT_BYTES);
   volatile int* abort_flag = &bars->abort_flag;
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_id(), lane = threadIdx.x & 31;
   int kb, hy, b;
   attn_block_coords(kb, hy, b);        // early KV blocks (attended by the most query blocks) start first
   const int Gall = p.Hq / p.Hkv;
@@ -92,70 +92,72 @@ flash_bwd_dkv_t_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = bars->tmem_slot;
+  const uint32_t tmem = __shfl_sync(0xffffffffu, bars->tmem_slot, 0);
   const uint32_t tS = tmem, tDP = tmem + 128, tDV = tmem + 256, tDK = tmem + 384;
 
   if (warp == 0) {
     // ------------------------------------------------------------ producer
-    if (lane == 0) {
-      mbar_expect_tx(&bars->kv_full, 2 * TILE_BYTES);
-      load_head_tile<NH>(sK, HALF_BYTES, &tmK, &bars->kv_full, hk, kb * AT, b);
-      load_head_tile<NH>(sV, HALF_BYTES, &tmV, &bars->kv_full, hk, kb * AT, b);
+    {
+      const uint32_t e = elect_one();
+      mbar_expect_tx(&bars->kv_full, 2 * TILE_BYTES, e);
+      load_head_tile<NH>(sK, HALF_BYTES, &tmK, &bars->kv_full, hk, kb * AT, b, e);
+      load_head_tile<NH>(sV, HALF_BYTES, &tmV, &bars->kv_full, hk, kb * AT, b, e);
       for (int it = 0; it < iters; ++it) {
         const int g = it / nsub;
         const int h = h_first + g;
         const int q0 = kb * AT + (it - g * nsub) * BQ;
         const int st = it % NST;
-        if (!mbar_wait(&bars->qd_empty[st], ((it / NST) & 1) ^ 1, abort_flag, p.status, 4)) break;
-        mbar_expect_tx(&bars->qd_full[st], 2 * Q_TILE + (RAGGED ? 0 : STAT_BYTES));
+        if (!mbar_wait_warp(&bars->qd_empty[st], ((it / NST) & 1) ^ 1, abort_flag, p.status, 4)) break;
+        mbar_expect_tx(&bars->qd_full[st], 2 * Q_TILE + (RAGGED ? 0 : STAT_BYTES), e);
         uint8_t* q_dst = sQ + st * Q_TILE;
         uint8_t* do_dst = sDO + st * Q_TILE;
-        load_head_tile<NH>(q_dst, Q_HALF, &tmQ, &bars->qd_full[st], h, q0, b);
-        load_head_tile<NH>(do_dst, Q_HALF, &tmDO, &bars->qd_full[st], h, q0, b);
+        load_head_tile<NH>(q_dst, Q_HALF, &tmQ, &bars->qd_full[st], h, q0, b, e);
+        load_head_tile<NH>(do_dst, Q_HALF, &tmDO, &bars->qd_full[st], h, q0, b, e);
         if (!RAGGED) {
           const long long stat_idx = (static_cast<long long>(b) * p.Hq + h) * p.S + q0;
-          bulk_load_1d(sStat + st * 2 * BQ, p.lse + stat_idx, BQ * 4, &bars->qd_full[st]);
-          bulk_load_1d(sStat + st * 2 * BQ + BQ, p.delta + stat_idx, BQ * 4, &bars->qd_full[st]);
+          if (e) bulk_load_1d(sStat + st * 2 * BQ, p.lse + stat_idx, BQ * 4, &bars->qd_full[st]);
+          if (e) bulk_load_1d(sStat + st * 2 * BQ + BQ, p.delta + stat_idx, BQ * 4, &bars->qd_full[st]);
         }
       }
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issue
-    if (lane == 0) {
+    {
+      const uint32_t e = elect_one();
       constexpr uint32_t idesc_s = umma_idesc_bf16(128, BQ, false, false);
       constexpr uint32_t idesc_acc = umma_idesc_bf16(128, 64 * NH, false, true);
       const uint32_t k_base = smem_u32(sK), v_base = smem_u32(sV), q_base = smem_u32(sQ), do_base = smem_u32(sDO);
-      bool ok = mbar_wait(&bars->kv_full, 0, abort_flag, p.status, 4);
+      bool ok = mbar_wait_warp(&bars->kv_full, 0, abort_flag, p.status, 4);
       auto issue_sp = [&](int it) -> bool {
         const int st = it % NST, buf = it & 1;
-        if (!mbar_wait(&bars->qd_full[st], (it / NST) & 1, abort_flag, p.status, 4)) return false;
+        if (!mbar_wait_warp(&bars->qd_full[st], (it / NST) & 1, abort_flag, p.status, 4)) return false;
         tc_fence_after();
         // The buffer's previous contents (P^T, dS^T of sub-block it-2) were consumed by MMAs issued earlier, which
         // the tensor core executes in order before these.
 #pragma unroll
         for (int ks = 0; ks < 4 * NH; ++ks)
-          umma_ss(tS + buf * BQ, desc_kmajor(k_base, ks), sub_desc_kmajor(q_base + st * Q_TILE, ks), idesc_s, ks > 0 ? 1u : 0u);
+          umma_ss(tS + buf * BQ, desc_kmajor(k_base, ks), sub_desc_kmajor(q_base + st * Q_TILE, ks), idesc_s, ks > 0 ? 1u : 0u, e);
 #pragma unroll
         for (int ks = 0; ks < 4 * NH; ++ks)
-          umma_ss(tDP + buf * BQ, desc_kmajor(v_base, ks), sub_desc_kmajor(do_base + st * Q_TILE, ks), idesc_s, ks > 0 ? 1u : 0u);
-        umma_commit(&bars->s_full[buf]);
+          umma_ss(tDP + buf * BQ, desc_kmajor(v_base, ks), sub_desc_kmajor(do_base + st * Q_TILE, ks), idesc_s, ks > 0 ? 1u : 0u, e);
+        umma_commit(&bars->s_full[buf], e);
         return true;
       };
       if (ok) ok = issue_sp(0);
       for (int it = 0; ok && it < iters; ++it) {
         if (it + 1 < iters) { ok = issue_sp(it + 1); if (!ok) break; }
         const int st = it % NST, buf = it & 1;
-        if (!mbar_wait(&bars->p_ready[buf], (it >> 1) & 1, abort_flag, p.status, 4)) break;
+        if (!mbar_wait_warp(&bars->p_ready[buf], (it >> 1) & 1, abort_flag, p.status, 4)) break;
         tc_fence_after();
 #pragma unroll
         for (int ks = 0; ks < BQ / 16; ++ks)
-          umma_ts(tDV, tS + buf * BQ + ks * 8, sub_desc_mnmajor(do_base + st * Q_TILE, ks), idesc_acc, (it > 0 || ks > 0) ? 1u : 0u);
+          umma_ts(tDV, tS + buf * BQ + ks * 8, sub_desc_mnmajor(do_base + st * Q_TILE, ks), idesc_acc, (it > 0 || ks > 0) ? 1u : 0u, e);
 #pragma unroll
         for (int ks = 0; ks < BQ / 16; ++ks)
-          umma_ts(tDK, tDP + buf * BQ + ks * 8, sub_desc_mnmajor(q_base + st * Q_TILE, ks), idesc_acc, (it > 0 || ks > 0) ? 1u : 0u);
-        umma_commit(&bars->qd_empty[st]);
+          umma_ts(tDK, tDP + buf * BQ + ks * 8, sub_desc_mnmajor(q_base + st * Q_TILE, ks), idesc_acc, (it > 0 || ks > 0) ? 1u : 0u, e);
+        umma_commit(&bars->qd_empty[st], e);
       }
-      if (ok) umma_commit(&bars->acc_done);
+      if (ok) umma_commit(&bars->acc_done, e);
     }
   } else {
     // ------------------------------------------------------------ softmax / epilogue: one thread per key row
@@ -274,7 +276,7 @@ flash_bwd_dq_t_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   DqBars* bars = reinterpret_cast<DqBars*>(sV + NST * Q_TILE);
   volatile int* abort_flag = &bars->abort_flag;
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_id(), lane = threadIdx.x & 31;
   int sblk, h, b;
   attn_block_coords(sblk, h, b);
   const int qb = gridDim.x - 1 - sblk;                 // heavy (late) query blocks first
@@ -295,55 +297,57 @@ flash_bwd_dq_t_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = bars->tmem_slot;
+  const uint32_t tmem = __shfl_sync(0xffffffffu, bars->tmem_slot, 0);
   const uint32_t tS = tmem, tDP = tmem + 128, tDQ = tmem + 256;
 
   if (warp == 0) {
-    if (lane == 0) {
-      mbar_expect_tx(&bars->qd_full, 2 * TILE_BYTES);
-      load_head_tile<NH>(sQ, HALF_BYTES, &tmQ, &bars->qd_full, h, qb * AT, b);
-      load_head_tile<NH>(sDO, HALF_BYTES, &tmDO, &bars->qd_full, h, qb * AT, b);
+    {
+      const uint32_t e = elect_one();
+      mbar_expect_tx(&bars->qd_full, 2 * TILE_BYTES, e);
+      load_head_tile<NH>(sQ, HALF_BYTES, &tmQ, &bars->qd_full, h, qb * AT, b, e);
+      load_head_tile<NH>(sDO, HALF_BYTES, &tmDO, &bars->qd_full, h, qb * AT, b, e);
       for (int j = 0; j < nkv; ++j) {
         const int st = j % NST;
-        if (!mbar_wait(&bars->kv_empty[st], ((j / NST) & 1) ^ 1, abort_flag, p.status, 4)) break;
-        mbar_expect_tx(&bars->kv_full[st], 2 * Q_TILE);
+        if (!mbar_wait_warp(&bars->kv_empty[st], ((j / NST) & 1) ^ 1, abort_flag, p.status, 4)) break;
+        mbar_expect_tx(&bars->kv_full[st], 2 * Q_TILE, e);
         uint8_t* k_dst = sK + st * Q_TILE;
         uint8_t* v_dst = sV + st * Q_TILE;
-        load_head_tile<NH>(k_dst, Q_HALF, &tmK, &bars->kv_full[st], hk, j * BQ, b);
-        load_head_tile<NH>(v_dst, Q_HALF, &tmV, &bars->kv_full[st], hk, j * BQ, b);
+        load_head_tile<NH>(k_dst, Q_HALF, &tmK, &bars->kv_full[st], hk, j * BQ, b, e);
+        load_head_tile<NH>(v_dst, Q_HALF, &tmV, &bars->kv_full[st], hk, j * BQ, b, e);
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    {
+      const uint32_t e = elect_one();
       constexpr uint32_t idesc_s = umma_idesc_bf16(128, BQ, false, false);
       constexpr uint32_t idesc_acc = umma_idesc_bf16(128, 64 * NH, false, true);
       const uint32_t q_base = smem_u32(sQ), do_base = smem_u32(sDO), k_base = smem_u32(sK), v_base = smem_u32(sV);
-      bool ok = mbar_wait(&bars->qd_full, 0, abort_flag, p.status, 4);
+      bool ok = mbar_wait_warp(&bars->qd_full, 0, abort_flag, p.status, 4);
       auto issue_sp = [&](int j) -> bool {
         const int st = j % NST, buf = j & 1;
-        if (!mbar_wait(&bars->kv_full[st], (j / NST) & 1, abort_flag, p.status, 4)) return false;
+        if (!mbar_wait_warp(&bars->kv_full[st], (j / NST) & 1, abort_flag, p.status, 4)) return false;
         tc_fence_after();
 #pragma unroll
         for (int ks = 0; ks < 4 * NH; ++ks)
-          umma_ss(tS + buf * BQ, desc_kmajor(q_base, ks), sub_desc_kmajor(k_base + st * Q_TILE, ks), idesc_s, ks > 0 ? 1u : 0u);
+          umma_ss(tS + buf * BQ, desc_kmajor(q_base, ks), sub_desc_kmajor(k_base + st * Q_TILE, ks), idesc_s, ks > 0 ? 1u : 0u, e);
 #pragma unroll
         for (int ks = 0; ks < 4 * NH; ++ks)
-          umma_ss(tDP + buf * BQ, desc_kmajor(do_base, ks), sub_desc_kmajor(v_base + st * Q_TILE, ks), idesc_s, ks > 0 ? 1u : 0u);
-        umma_commit(&bars->s_full[buf]);
+          umma_ss(tDP + buf * BQ, desc_kmajor(do_base, ks), sub_desc_kmajor(v_base + st * Q_TILE, ks), idesc_s, ks > 0 ? 1u : 0u, e);
+        umma_commit(&bars->s_full[buf], e);
         return true;
       };
       if (ok) ok = issue_sp(0);
       for (int j = 0; ok && j < nkv; ++j) {
         if (j + 1 < nkv) { ok = issue_sp(j + 1); if (!ok) break; }
         const int st = j % NST, buf = j & 1;
-        if (!mbar_wait(&bars->p_ready[buf], (j >> 1) & 1, abort_flag, p.status, 4)) break;
+        if (!mbar_wait_warp(&bars->p_ready[buf], (j >> 1) & 1, abort_flag, p.status, 4)) break;
         tc_fence_after();
 #pragma unroll
         for (int ks = 0; ks < BQ / 16; ++ks)
-          umma_ts(tDQ, tDP + buf * BQ + ks * 8, sub_desc_mnmajor(k_base + st * Q_TILE, ks), idesc_acc, (j > 0 || ks > 0) ? 1u : 0u);
-        umma_commit(&bars->kv_empty[st]);
+          umma_ts(tDQ, tDP + buf * BQ + ks * 8, sub_desc_mnmajor(k_base + st * Q_TILE, ks), idesc_acc, (j > 0 || ks > 0) ? 1u : 0u, e);
+        umma_commit(&bars->kv_empty[st], e);
       }
-      if (ok) umma_commit(&bars->acc_done);
+      if (ok) umma_commit(&bars->acc_done, e);
     }
   } else {
     const int wg = (warp - 2) >> 2;                       // 0: even KV sub-blocks (buffer 0), 1: odd (buffer 1)

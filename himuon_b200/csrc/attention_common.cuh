@@ -57,12 +57,12 @@ __device__ __forceinline__ void attn_block_coords(int& sblk, int& head, int& bat
   head = r - batch * gridDim.y;
 }
 
-// Loads `rows` positions (NH halves of `half_bytes` each) of one head into a swizzled tile.
+// Loads `rows` positions (NH halves of `half_bytes` each) of one head into a swizzled tile (a converged warp's elected lane).
 template <int NH>
 __device__ __forceinline__ void load_head_tile(uint8_t* dst, uint32_t half_bytes, const CUtensorMap* tm, uint64_t* bar,
-                                               int head, int s0, int b) {
+                                               int head, int s0, int b, uint32_t e) {
 #pragma unroll
-  for (int j = 0; j < NH; ++j) tma_load_4d(dst + j * half_bytes, tm, bar, j * 64, head, s0, b);
+  for (int j = 0; j < NH; ++j) tma_load_4d(dst + j * half_bytes, tm, bar, j * 64, head, s0, b, e);
 }
 // delta = sum over the head of o * d_o for one row (hd is a multiple of 8).
 __device__ __forceinline__ float row_delta(const __nv_bfloat16* op, const __nv_bfloat16* gp, int hd) {

@@ -48,7 +48,7 @@ flash_fwd64_t_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   Fwd64TBars* bars = reinterpret_cast<Fwd64TBars*>(sV + 2 * KV_TILE);
   volatile int* abort_flag = &bars->abort_flag;
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_id(), lane = threadIdx.x & 31;
   int sblk, h, b;
   attn_block_coords(sblk, h, b);
   const int qb = gridDim.x - 1 - sblk;         // heavy (late) query blocks first
@@ -73,58 +73,60 @@ flash_fwd64_t_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = bars->tmem_slot;
+  const uint32_t tmem = __shfl_sync(0xffffffffu, bars->tmem_slot, 0);
   const uint32_t tS0 = tmem, tO = tmem + 128;   // S / P buffers at columns 0 and 64, O at 128
 
   if (warp == 0) {
-    if (lane == 0) {
-      mbar_expect_tx(&bars->q_full, TILE_BYTES);
-      load_head_tile<NH>(sQ, HALF_BYTES, &tmQ, &bars->q_full, h, qb * AT, b);
+    {
+      const uint32_t e = elect_one();
+      mbar_expect_tx(&bars->q_full, TILE_BYTES, e);
+      load_head_tile<NH>(sQ, HALF_BYTES, &tmQ, &bars->q_full, h, qb * AT, b, e);
       for (int j = 0; j < nkv; ++j) {
         const int st = j & 1;
         const uint32_t par = ((j >> 1) & 1) ^ 1;
-        if (!mbar_wait(&bars->k_empty[st], par, abort_flag, p.status, 4)) break;
-        mbar_expect_tx(&bars->k_full[st], KV_TILE);
-        load_head_tile<NH>(sK + st * KV_TILE, KV_HALF, &tmK, &bars->k_full[st], hk, j * BKV, b);
-        if (!mbar_wait(&bars->v_empty[st], par, abort_flag, p.status, 4)) break;
-        mbar_expect_tx(&bars->v_full[st], KV_TILE);
-        load_head_tile<NH>(sV + st * KV_TILE, KV_HALF, &tmV, &bars->v_full[st], hk, j * BKV, b);
+        if (!mbar_wait_warp(&bars->k_empty[st], par, abort_flag, p.status, 4)) break;
+        mbar_expect_tx(&bars->k_full[st], KV_TILE, e);
+        load_head_tile<NH>(sK + st * KV_TILE, KV_HALF, &tmK, &bars->k_full[st], hk, j * BKV, b, e);
+        if (!mbar_wait_warp(&bars->v_empty[st], par, abort_flag, p.status, 4)) break;
+        mbar_expect_tx(&bars->v_full[st], KV_TILE, e);
+        load_head_tile<NH>(sV + st * KV_TILE, KV_HALF, &tmV, &bars->v_full[st], hk, j * BKV, b, e);
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    {
+      const uint32_t e = elect_one();
       constexpr uint32_t idesc_s = umma_idesc_bf16(128, BKV, false, false);
       constexpr uint32_t idesc_pv = umma_idesc_bf16(128, 64 * NH, false, true);
       const uint32_t q_base = smem_u32(sQ), v_base = smem_u32(sV);
-      bool ok = mbar_wait(&bars->q_full, 0, abort_flag, p.status, 4);
+      bool ok = mbar_wait_warp(&bars->q_full, 0, abort_flag, p.status, 4);
       auto issue_s = [&](int j) -> bool {
         const int st = j & 1;
-        if (!mbar_wait(&bars->k_full[st], (j >> 1) & 1, abort_flag, p.status, 4)) return false;
+        if (!mbar_wait_warp(&bars->k_full[st], (j >> 1) & 1, abort_flag, p.status, 4)) return false;
         tc_fence_after();
         // buffer st held S(j-2) / P(j-2): the softmax threads are done with it (p_ready(j-2) was waited for) and the
         // P(j-2)·V MMAs were issued earlier, which the tensor core executes in order before these
         const uint32_t k_base = smem_u32(sK + st * KV_TILE);
 #pragma unroll
         for (int ks = 0; ks < 4 * NH; ++ks)
-          umma_ss(tS0 + st * BKV, desc_kmajor(q_base, ks), kv_desc_kmajor(k_base, ks), idesc_s, ks > 0 ? 1u : 0u);
-        umma_commit(&bars->k_empty[st]);
-        umma_commit(&bars->s_full[st]);
+          umma_ss(tS0 + st * BKV, desc_kmajor(q_base, ks), kv_desc_kmajor(k_base, ks), idesc_s, ks > 0 ? 1u : 0u, e);
+        umma_commit(&bars->k_empty[st], e);
+        umma_commit(&bars->s_full[st], e);
         return true;
       };
       if (ok) ok = issue_s(0);
       for (int j = 0; ok && j < nkv; ++j) {
         if (j + 1 < nkv) { ok = issue_s(j + 1); if (!ok) break; }
         const int st = j & 1;
-        if (!mbar_wait(&bars->p_ready[st], (j >> 1) & 1, abort_flag, p.status, 4)) break;
-        if (!mbar_wait(&bars->v_full[st], (j >> 1) & 1, abort_flag, p.status, 4)) break;
+        if (!mbar_wait_warp(&bars->p_ready[st], (j >> 1) & 1, abort_flag, p.status, 4)) break;
+        if (!mbar_wait_warp(&bars->v_full[st], (j >> 1) & 1, abort_flag, p.status, 4)) break;
         tc_fence_after();
 #pragma unroll
         for (int ks = 0; ks < BKV / 16; ++ks)
-          umma_ts(tO, tS0 + st * BKV + ks * 8, kv_desc_mnmajor(v_base + st * KV_TILE, ks), idesc_pv, (j > 0 || ks > 0) ? 1u : 0u);
-        umma_commit(&bars->v_empty[st]);
-        umma_commit(&bars->o_done[st]);
+          umma_ts(tO, tS0 + st * BKV + ks * 8, kv_desc_mnmajor(v_base + st * KV_TILE, ks), idesc_pv, (j > 0 || ks > 0) ? 1u : 0u, e);
+        umma_commit(&bars->v_empty[st], e);
+        umma_commit(&bars->o_done[st], e);
       }
-      if (ok) umma_commit(&bars->acc_done);
+      if (ok) umma_commit(&bars->acc_done, e);
     }
   } else {
     // ------------------------------------------------------------ softmax / epilogue: one thread per query row

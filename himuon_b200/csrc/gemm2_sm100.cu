@@ -72,10 +72,10 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer (both CTAs)
-    const uint32_t e = elect_one();
-    tma_prefetch_desc(&tmA);
-    tma_prefetch_desc(&tmB);
     {
+      const uint32_t e = elect_one();
+      tma_prefetch_desc(&tmA);
+      tma_prefetch_desc(&tmB);
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;

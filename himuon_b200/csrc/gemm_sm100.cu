@@ -80,10 +80,10 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
-    const uint32_t e = elect_one();
-    tma_prefetch_desc(&tmA);
-    tma_prefetch_desc(&tmB);
     {
+      const uint32_t e = elect_one();
+      tma_prefetch_desc(&tmA);
+      tma_prefetch_desc(&tmB);
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -116,8 +116,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
-    const uint32_t e = elect_one();
     {
+      const uint32_t e = elect_one();
       constexpr uint32_t idesc = umma_idesc_bf16(BM, BN, A_MN, B_MN);
       int stage = 0;
       uint32_t phase = 0;

@@ -22,8 +22,9 @@ namespace himuon {
 constexpr int BN2 = 256;     // tile width
 constexpr int BNH = 128;     // rows of B staged by each CTA
 
+constexpr int GEMM2_THREADS = 384;   // warps 0-3: TMA, MMA, TMEM allocation, none; 4-11: epilogue, two groups of four
 template <int STAGES, bool A_MN, bool B_MN>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(256, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM2_THREADS, 1)
 gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                   const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CUtensorMap tmW, GemmDev p) {
   constexpr uint32_t A_BYTES = BM * BK * 2;
@@ -54,7 +55,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(&tfull[a], 1);
-      mbar_init(&tempty[a], 8);      // four epilogue warps in each CTA of the pair
+      mbar_init(&tempty[a], 16);     // eight epilogue warps in each CTA of the pair
     }
     *abort_flag = 0;
     mbar_fence_init();
@@ -154,11 +155,12 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     }
   } else if (warp >= 4) {
     // ------------------------------------------------------------ epilogue (both CTAs, own 128 accumulator rows)
-    const int ew = warp & 3;
+    const int ew = warp & 3, group = (warp - 4) >> 2;
     int acc = 0;
     uint32_t acc_phase = 0;
-    uint32_t slab_seq = 0;
-    const bool issuer = (threadIdx.x == 128);
+    uint8_t* slab = sC + group * SLAB_BYTES;
+    const bool issuer = ew == 0 && lane == 0;
+    const uint32_t tempty_lead = map_to_cta(smem_u32(tempty), 0);   // the leader owns the accumulator hand-off
     if (issuer) tma_prefetch_desc(&tmC);
     WorkCursor cur(p, pair, n_pairs);
     WorkItem w;
@@ -169,7 +171,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
       const int mt = r % p.tiles_m;
       const int nt = r / p.tiles_m;
       // the 128 threads meet on named barriers below, so they also leave together when the wait runs out
-      if (!named_barrier_and(1, 128, mbar_wait(&tfull[acc], acc_phase, abort_flag, p.status, 3))) break;
+      if (!named_barrier_and(1 + 2 * group, 128, mbar_wait(&tfull[acc], acc_phase, abort_flag, p.status, 3))) break;
       tc_fence_after();
       const int row_in_tile = ew * 32 + lane;
       const int m0 = mt * 2 * BM + static_cast<int>(rank) * BM;
@@ -178,25 +180,25 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
       if (w.split) {
         // K-slice of a last-wave tile: add the fp32 partial into the scratch tile (rows tail*256 + rank*128 ..);
         // a follow-up kernel applies the epilogue to the complete sums
-        epilogue_tile_tma<BN2, true>(&tmW, sC, t_acc, row_in_tile, w.tail * 2 * BM + static_cast<int>(rank) * BM, 0, 0, nullptr, 0,
-                                     1 << 30, BN2, 1.f, 0.f, 0, slab_seq, issuer, true);
+        epilogue_tile_tma<BN2, true>(&tmW, slab, group, t_acc, row_in_tile, w.tail * 2 * BM + static_cast<int>(rank) * BM, 0, 0, nullptr, 0,
+                                     1 << 30, BN2, 1.f, 0.f, 0, issuer, true);
       } else if (m0 < p.M) {              // uniform: the second CTA of a ragged last row block has nothing to store
         if (p.reduce_out && p.out_fp32)   // C += alpha*acc without reading C: the L2 adds the staged slabs
-          epilogue_tile_tma<BN2, true>(&tmC, sC, t_acc, row_in_tile, m0, nt * BN2, b, nullptr, 0, p.M, p.N, p.alpha,
-                                       0.f, 0, slab_seq, issuer, true);
+          epilogue_tile_tma<BN2, true>(&tmC, slab, group, t_acc, row_in_tile, m0, nt * BN2, b, nullptr, 0, p.M, p.N, p.alpha,
+                                       0.f, 0, issuer, true);
         else if (p.reduce_out)            // same for a bf16 C: the partial is rounded to bf16, then added in bf16
-          epilogue_tile_tma<BN2, false>(&tmC, sC, t_acc, row_in_tile, m0, nt * BN2, b, nullptr, 0, p.M, p.N, p.alpha,
-                                        0.f, 0, slab_seq, issuer, true);
+          epilogue_tile_tma<BN2, false>(&tmC, slab, group, t_acc, row_in_tile, m0, nt * BN2, b, nullptr, 0, p.M, p.N, p.alpha,
+                                        0.f, 0, issuer, true);
         else if (p.out_fp32)
-          epilogue_tile_tma<BN2, true>(&tmC, sC, t_acc, row_in_tile, m0, nt * BN2, b, p.aux, aux_row, p.M, p.N, p.alpha,
-                                       p.beta, p.round_acc, slab_seq, issuer);
+          epilogue_tile_tma<BN2, true>(&tmC, slab, group, t_acc, row_in_tile, m0, nt * BN2, b, p.aux, aux_row, p.M, p.N, p.alpha,
+                                       p.beta, p.round_acc, issuer);
         else
-          epilogue_tile_tma<BN2, false>(&tmC, sC, t_acc, row_in_tile, m0, nt * BN2, b, p.aux, aux_row, p.M, p.N, p.alpha,
-                                        p.beta, p.round_acc, slab_seq, issuer);
+          epilogue_tile_tma<BN2, false>(&tmC, slab, group, t_acc, row_in_tile, m0, nt * BN2, b, p.aux, aux_row, p.M, p.N, p.alpha,
+                                        p.beta, p.round_acc, issuer);
       }
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive_cluster(map_to_cta(smem_u32(&tempty[acc]), 0));   // the leader owns the accumulator hand-off
+      if (lane == 0) mbar_arrive_remote(tempty_lead + acc * 8);
       acc ^= 1;
       if (acc == 0) acc_phase ^= 1;
     }
@@ -271,6 +273,14 @@ static float* pair_scratch() {
   return per_device[dev];
 }
 
+static CUtensorMap operand_tmap(const void* ptr, bool mn, int extent, int K, long long ld, int batch, long long stride) {
+  const uint64_t row = static_cast<uint64_t>(ld) * 2, rows = static_cast<uint64_t>(mn ? K : extent);
+  const uint64_t dims[3] = {static_cast<uint64_t>(mn ? extent : K), rows, static_cast<uint64_t>(batch)};
+  const uint64_t strides[2] = {row, batch > 1 ? static_cast<uint64_t>(stride) * 2 : row * rows};
+  const uint32_t box[3] = {64, static_cast<uint32_t>(mn ? BK : BM), 1};
+  return make_tmap(ptr, 3, dims, strides, box, 2, true);
+}
+
 template <int STAGES, bool A_MN, bool B_MN>
 static void launch_gemm2(const GemmArgs& a, cudaStream_t stream) {
   constexpr uint32_t STAGE_BYTES = (BM + BNH) * BK * 2;
@@ -282,20 +292,8 @@ static void launch_gemm2(const GemmArgs& a, cudaStream_t stream) {
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(SMEM));
     attr_done = true;
   }
-  uint64_t dimsA[3], strA[2], dimsB[3], strB[2];
-  uint32_t boxA[3], boxB[3];
-  if (!A_MN) { dimsA[0] = a.K; dimsA[1] = a.M; boxA[0] = BK; boxA[1] = BM; }
-  else       { dimsA[0] = a.M; dimsA[1] = a.K; boxA[0] = 64; boxA[1] = BK; }
-  dimsA[2] = a.batch; boxA[2] = 1;
-  strA[0] = static_cast<uint64_t>(a.lda) * 2;
-  strA[1] = a.batch > 1 ? static_cast<uint64_t>(a.strideA) * 2 : strA[0] * dimsA[1];
-  if (!B_MN) { dimsB[0] = a.K; dimsB[1] = a.N; boxB[0] = BK; boxB[1] = BNH; }
-  else       { dimsB[0] = a.N; dimsB[1] = a.K; boxB[0] = 64; boxB[1] = BK; }
-  dimsB[2] = a.batch; boxB[2] = 1;
-  strB[0] = static_cast<uint64_t>(a.ldb) * 2;
-  strB[1] = a.batch > 1 ? static_cast<uint64_t>(a.strideB) * 2 : strB[0] * dimsB[1];
-  const CUtensorMap tmA = make_tmap(a.A, 3, dimsA, strA, boxA, 2, true);
-  const CUtensorMap tmB = make_tmap(a.B, 3, dimsB, strB, boxB, 2, true);
+  const CUtensorMap tmA = operand_tmap(a.A, A_MN, a.M, a.K, a.lda, a.batch, a.strideA);
+  const CUtensorMap tmB = operand_tmap(a.B, B_MN, a.N, a.K, a.ldb, a.batch, a.strideB);
   const int esz = a.out_fp32 ? 4 : 2;
   const uint64_t dimsC[3] = {static_cast<uint64_t>(a.N), static_cast<uint64_t>(a.M), static_cast<uint64_t>(a.batch)};
   const uint64_t strC[2] = {static_cast<uint64_t>(a.ldc) * esz,
@@ -313,7 +311,8 @@ static void launch_gemm2(const GemmArgs& a, cudaStream_t stream) {
   p.kblocks = (a.K + BK - 1) / BK;
   p.tma_store = 1;
   p.nslices = 1;
-  p.reduce_out = (a.aux == a.C && a.beta == 1.f && !a.round_acc &&
+  // (a bf16 C takes one rounding more that way, of the partial: long reductions only, as ever)
+  p.reduce_out = (a.K >= 2048 && a.aux == a.C && a.beta == 1.f && !a.round_acc &&
                   a.ldaux == a.ldc && a.strideAux == a.strideC) ? 1 : 0;
   p.status = status_word_ptr();
   const long long total = static_cast<long long>(p.tiles_m) * p.tiles_n * a.batch;
@@ -323,7 +322,7 @@ static void launch_gemm2(const GemmArgs& a, cudaStream_t stream) {
   if (max_pairs == 0) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(num_sms());
-    cfg.blockDim = dim3(256);
+    cfg.blockDim = dim3(GEMM2_THREADS);
     cfg.dynamicSmemBytes = SMEM;
     cudaLaunchAttribute attr;
     attr.id = cudaLaunchAttributeClusterDimension;
@@ -365,7 +364,7 @@ static void launch_gemm2(const GemmArgs& a, cudaStream_t stream) {
     p.stream_k = 1;
     pairs = cap;
   }
-  kern<<<static_cast<int>(2 * pairs), 256, SMEM, stream>>>(tmA, tmB, tmC, tmW, p);
+  kern<<<static_cast<int>(2 * pairs), GEMM2_THREADS, SMEM, stream>>>(tmA, tmB, tmC, tmW, p);
   if (p.nslices > 1) {
     const long long groups = 256LL * 256 / 4 * rem;
     const int blocks = static_cast<int>((groups + 255) / 256 < num_sms() * 4 ? (groups + 255) / 256 : num_sms() * 4);
@@ -375,13 +374,18 @@ static void launch_gemm2(const GemmArgs& a, cudaStream_t stream) {
 }
 
 // True when the pair kernel can run this problem and is expected to win: TMA-storable output (whole 16-byte groups of
-// columns: a TMA store writes those whole, past the output's last column if need be), more than one CTA
-// tile of rows, and a reduction long enough (K >= 2048) to amortise the 256-column epilogue; short-K batched
-// products (the Newton-Schulz GEMMs) are faster on the one-CTA kernel.
+// columns: a TMA store writes those whole, past the output's last column if need be), more than one CTA tile of rows, and
+//   * a reduction of 2048 or more, or
+//   * one of 512 or more and enough 256 x 256 tiles to occupy half of the pairs.  Below that the one-CTA kernel's smaller tiles
+//     spread over more SMs (32 tiles, 512 x 4096 x 512: 13.3 us there, 15.4 here; 48 tiles, 4096 x 640 x 1728: 23.6 / 21.5; 80,
+//     4096 x 1280 x 640: 19.5 / 18.4; 384, 8192 x 3072 x 1024: 52.5 / 44.1; 4096 x 64128 x 640: 290 / 224).
+// Symmetric products of short reductions stay with the one-CTA kernel, which computes one triangle of them.
 bool gemm2_supported(const GemmArgs& a) {
   const int esz = a.out_fp32 ? 4 : 2;
   const int row_align = 16 / esz;
-  return a.M > BM && a.N > 192 && a.N % row_align == 0 && a.K >= 2048 && (a.ldc % row_align == 0) && (a.batch == 1 || a.strideC % row_align == 0) &&
+  const long long tiles = static_cast<long long>((a.M + 255) / 256) * ((a.N + 255) / 256) * a.batch;
+  const bool long_enough = a.K >= 2048 || (a.K >= 512 && !a.symmetric && tiles >= 40);
+  return a.M > BM && a.N > 192 && a.N % row_align == 0 && long_enough && (a.ldc % row_align == 0) && (a.batch == 1 || a.strideC % row_align == 0) &&
          (reinterpret_cast<uintptr_t>(a.C) % 16 == 0);
 }
 

@@ -229,26 +229,26 @@ __device__ __noinline__ void store_tail(T* c, long long ldc, int rows, int n, co
   }
 }
 
-// Pair kernel: epilogue of one accumulator tile through swizzled shared-memory slabs and TMA stores.  Called by the 128
-// epilogue threads together.  `slab_seq` numbers the slabs this CTA has stored so far (selects the staging buffer).
+// Pair kernel: epilogue of one accumulator tile through a swizzled shared-memory slab and TMA stores, by the 128 threads of
+// group 0 or 1, which takes the slabs of its parity and has a slab of its own.  Two groups, because one needed 6.6 us for a
+// tile: as long as the products of a reduction of 1600, and the tile's columns are all that a second accumulator hides.
+// A slab's values are computed before its memory is waited for, so that the previous store's read is hidden.
 template <int BN, bool OUT_FP32>
-__device__ __forceinline__ void epilogue_tile_tma(const CUtensorMap* tmC, uint8_t* sC, uint32_t t_row, int row_in_tile,
+__device__ __forceinline__ void epilogue_tile_tma(const CUtensorMap* tmC, uint8_t* slab, int group, uint32_t t_row, int row_in_tile,
                                                   int m0, int n0, int b, const void* aux, long long aux_row_off,
-                                                  int M, int N, float alpha, float beta, int round_acc,
-                                                  uint32_t& slab_seq, bool issuer, bool reduce_add = false) {
+                                                  int M, int N, float alpha, float beta, int round_acc, bool issuer,
+                                                  bool reduce_add = false) {
   constexpr int SW = OUT_FP32 ? 32 : 64;
   constexpr int SLABS = BN / SW;
   const bool row_ok = (m0 + row_in_tile) < M;
-  uint4 xa[8], xn[8];
-  load_aux_slab<OUT_FP32>(aux, aux_row_off + n0, row_ok, N - n0, xa);
+  uint8_t* my_row = slab + row_in_tile * 128;
+  uint4 xa[8];
+  load_aux_slab<OUT_FP32>(aux, aux_row_off + n0 + group * SW, row_ok, N - n0 - group * SW, xa);
 #pragma unroll 1
-  for (int sl = 0; sl < SLABS; ++sl) {
+  for (int sl = group; sl < SLABS; sl += 2) {
     const int col = n0 + sl * SW;
-    if (col >= N) break;                                   // uniform over the 128 threads
-    if (sl + 1 < SLABS) load_aux_slab<OUT_FP32>(aux, aux_row_off + col + SW, row_ok, N - col - SW, xn);
-    named_barrier(1, 128);                                 // the staging buffer is free (issuer waited on its reads)
-    uint8_t* buf = sC + (slab_seq & 1) * SLAB_BYTES;
-    uint8_t* my_row = buf + row_in_tile * 128;
+    if (col >= N) break;                                   // uniform over the group
+    uint4 o[8];
 #pragma unroll
     for (int ch = 0; ch < SW / 32; ++ch) {
       uint32_t v[32];
@@ -256,43 +256,40 @@ __device__ __forceinline__ void epilogue_tile_tma(const CUtensorMap* tmC, uint8_
       tmem_ld_wait();
       if (OUT_FP32) {
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          float4 o;
-          o.x = alpha * __uint_as_float(v[4 * j + 0]) + beta * __uint_as_float(xa[j].x);
-          o.y = alpha * __uint_as_float(v[4 * j + 1]) + beta * __uint_as_float(xa[j].y);
-          o.z = alpha * __uint_as_float(v[4 * j + 2]) + beta * __uint_as_float(xa[j].z);
-          o.w = alpha * __uint_as_float(v[4 * j + 3]) + beta * __uint_as_float(xa[j].w);
-          *reinterpret_cast<float4*>(my_row + ((j ^ (row_in_tile & 7)) << 4)) = o;
-        }
+        for (int j = 0; j < 8; ++j)
+          o[j] = make_uint4(__float_as_uint(alpha * __uint_as_float(v[4 * j + 0]) + beta * __uint_as_float(xa[j].x)),
+                            __float_as_uint(alpha * __uint_as_float(v[4 * j + 1]) + beta * __uint_as_float(xa[j].y)),
+                            __float_as_uint(alpha * __uint_as_float(v[4 * j + 2]) + beta * __uint_as_float(xa[j].z)),
+                            __float_as_uint(alpha * __uint_as_float(v[4 * j + 3]) + beta * __uint_as_float(xa[j].w)));
       } else {
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
           const uint4 e = xa[ch * 4 + q];
           const uint32_t ew[4] = {e.x, e.y, e.z, e.w};
-          uint32_t o[4];
+          uint32_t r[4];
 #pragma unroll
           for (int t = 0; t < 4; ++t) {
             float f0 = alpha * __uint_as_float(v[8 * q + 2 * t]);
             float f1 = alpha * __uint_as_float(v[8 * q + 2 * t + 1]);
-            if (round_acc) { f0 = round_bf16(f0); f1 = round_bf16(f1); }
-            o[t] = pack_bf16x2(f0 + beta * bf16_lo(ew[t]), f1 + beta * bf16_hi(ew[t]));
+            if (round_acc) { const uint32_t h = pack_bf16x2(f0, f1); f0 = bf16_lo(h); f1 = bf16_hi(h); }
+            r[t] = pack_bf16x2(f0 + beta * bf16_lo(ew[t]), f1 + beta * bf16_hi(ew[t]));
           }
-          const int j = ch * 4 + q;
-          *reinterpret_cast<uint4*>(my_row + ((j ^ (row_in_tile & 7)) << 4)) = make_uint4(o[0], o[1], o[2], o[3]);
+          o[ch * 4 + q] = make_uint4(r[0], r[1], r[2], r[3]);
         }
       }
     }
-    fence_proxy_async_smem();
-    named_barrier(2, 128);                                 // the slab is complete
-    if (issuer) {
-      if (reduce_add) tma_reduce_add_3d(tmC, buf, col, m0, b);     // split-K: accumulate into the fp32 scratch tile
-      else tma_store_3d(tmC, buf, col, m0, b);
-      tma_store_commit();
-      tma_store_wait_read<1>();                            // the other buffer's previous store has drained
-    }
-    ++slab_seq;
+    if (sl + 2 < SLABS) load_aux_slab<OUT_FP32>(aux, aux_row_off + col + 2 * SW, row_ok, N - col - 2 * SW, xa);
+    if (issuer) tma_store_wait_read<0>();
+    named_barrier(1 + 2 * group, 128);                     // the slab is free
 #pragma unroll
-    for (int j = 0; j < 8; ++j) xa[j] = xn[j];
+    for (int j = 0; j < 8; ++j) *reinterpret_cast<uint4*>(my_row + ((j ^ (row_in_tile & 7)) << 4)) = o[j];
+    fence_proxy_async_smem();
+    named_barrier(2 + 2 * group, 128);                     // the slab is complete
+    if (issuer) {
+      if (reduce_add) tma_reduce_add_3d(tmC, slab, col, m0, b);    // split-K: accumulate into the fp32 scratch tile
+      else tma_store_3d(tmC, slab, col, m0, b);
+      tma_store_commit();
+    }
   }
 }
 

@@ -126,11 +126,7 @@ __device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity
   }
   return __all_sync(0xffffffffu, ok);
 }
-// Arrives on a barrier of a CTA of the cluster: behind tensor-memory reads and their fence ...
-__device__ __forceinline__ void mbar_arrive_remote(uint32_t cluster_addr) {
-  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
-}
-// ... or behind a fence of the cluster.
+// Arrives on a barrier of a CTA of the cluster behind a fence of the cluster.
 __device__ __forceinline__ void mbar_arrive_relaxed(uint32_t cluster_addr) {
   asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }

@@ -1064,3 +1064,39 @@ def test_ns_pair_kernel_keeps_a_bad_matrix_to_itself():
     x[4] = 0
     assert (ns.newton_schulz(x)[4] == 0).all()
     _assert_status_clean()
+
+
+# Reductions of 512 to 2047 on the pair kernel: the first and a ragged last length, 40 tiles (the fewest) and some rounds of
+# them, ragged rows and columns, every operand-major combination, and each epilogue form.
+@pytest.mark.parametrize("M,N,K,batch", [(1281, 2048, 512, 1), (2056, 1288, 1096, 1), (328, 520, 2040, 8), (2560, 2560, 640, 1)])
+@pytest.mark.parametrize("trans_a,trans_b", [(False, True), (False, False), (True, True), (True, False)])
+@pytest.mark.parametrize("mode", ["plain", "aux", "add", "fp32"])
+def test_pair_gemm_on_short_reductions(M, N, K, batch, trans_a, trans_b, mode):
+    from himuon_b200 import ops
+
+    if trans_a and M % 8:
+        M += 8 - M % 8                                     # the rows of a transposed operand are 16-byte aligned
+    g = torch.Generator("cuda").manual_seed(M + N + K)
+    a = torch.randn(batch, *((K, M) if trans_a else (M, K)), device="cuda", dtype=torch.bfloat16, generator=g)
+    b = torch.randn(batch, *((N, K) if trans_b else (K, N)), device="cuda", dtype=torch.bfloat16, generator=g)
+    ref = (a.float().mT if trans_a else a.float()) @ (b.float().mT if trans_b else b.float())
+    out = torch.randn(batch, M, N, device="cuda", generator=g).to(torch.float32 if mode == "fp32" else torch.bfloat16)
+    x = torch.randn(batch, M, N, device="cuda", generator=g).to(out.dtype)
+    kw = dict(trans_a=trans_a, trans_b=trans_b, out=out)
+    atol = 4e-4 if mode == "fp32" else 1e-2
+    if mode == "plain":
+        ops.gemm(a, b, **kw)
+    elif mode == "add":
+        ref = ref + out.float()
+        ops.gemm(a, b, aux=out, beta=1.0, **kw)
+    else:
+        ops.gemm(a, b, aux=x, alpha=0.5, beta=-2.0, round_acc=mode == "aux", **kw)
+        ref = 0.5 * ref
+        if mode == "aux":                                  # the rounded accumulator: half an ulp of it, which the sum may cancel
+            atol += 2 ** -9 * ref.abs().max().item()
+        ref = ref - 2.0 * x.float()
+    torch.cuda.synchronize()
+    _assert_status_clean()
+    # fp32 sums of K products of unit normals differ by some 2^-24 of sqrt(K) per term in any order; a bf16 result adds half
+    # an ulp, 2^-9 of the value
+    _close(out, ref, atol=atol, rtol=1e-5 if mode == "fp32" else 2 ** -8)

@@ -9,12 +9,19 @@
 // Nothing but Q/dO/K/V touches shared memory, which leaves room for four streamed stages, and the two S^T/dP^T
 // buffers let the tensor core work on sub-block i+1 while the softmax threads work on sub-block i.
 //
-// TMEM (512 columns): S^T buffers at 0 and 64 (P^T over the first 32 columns of each), dP^T buffers at 128 and 192
+// TMEM (512 columns): S^T buffers at 0 and 64 (P^T over columns 0-15 and 32-47 of each), dP^T buffers at 128 and 192
 // (dS^T likewise), dV at 256, dK at 384.
 // Any sequence length: rows past S arrive as zeros (TMA) with a log-sum-exp of +inf, so their probabilities are 0, and
 // are not stored.  The per-row statistics (log-sum-exp, delta) arrive by bulk copies with the Q/dO stage when S is a
-// multiple of 64 (every sub-block is then whole and starts on 16 bytes); otherwise (RAGGED) each softmax group fetches
-// its sub-block's values itself, ahead of the wait for the scores.
+// multiple of 64 (every sub-block is then whole and starts on 16 bytes); otherwise (RAGGED) the softmax groups fetch
+// their sub-block's values themselves, ahead of the wait for the scores.
+//
+// What bounds both kernels (clock readings in one block, heads of 128): a sub-block takes 1480 cycles here and 1210 in the dQ
+// pass, against 1280 and 1020 that the tensor core needs (a 128 x 64 x 16 product from shared memory is bound by the 6 KB of
+// its operands, 48 cycles).  The rest is some 10000 cycles a block: set-up and first loads 5000-7000, the last products 2000,
+// the epilogue 1400-2900.  Descriptors that are one addition each, 16 softmax warps, the first loads ahead of the set-up, the
+// staged epilogue and delta by rows of lanes took, dK/dV and dQ: 4 x 2048 tokens, 16 heads over 8, 167 and 156 -> 145 and
+// 133 us; 2 x 1024, 32 over 8, 61 and 58 -> 53 and 47; 8 x 512, 10 heads of 64, 24.5 and 22.5 -> 22 and 19.
 // Measured, whole backward pass on ragged lengths against the unpipelined kernels that served them before: 5 x 777 tokens
 // with 16 heads over 8 191 -> 139 us, 4 x 1000 with 32 over 8 373 -> 270 us, 2 x 1984 with 16 over 8 304 -> 205 us;
 // 4 x 1024 (whole sub-blocks) 149 us before and after.
@@ -30,9 +37,12 @@ constexpr int BQ = 64;                               // query positions per stre
 constexpr uint32_t Q_HALF = BQ * 128;                // one 64-column half of a sub-block: 8 KB
 constexpr int NST = 4;                               // streamed stages of (Q, dO, lse, delta)
 constexpr uint32_t STAT_BYTES = 2 * BQ * 4;          // lse[64] then delta[64]
-// warp 0: TMA producer, warp 1: MMA issue, warps 2-5 and 6-9: two softmax groups of 128 threads (one per TMEM
-// lane) that take alternate sub-blocks, so two warps per scheduler hide each other's MUFU and TMEM latencies
-constexpr int BWD_THREADS = 320;
+// warp 0: TMA producer, warp 1: MMA issue, warps 2-17: four softmax groups of 128 threads (one per TMEM lane).  Groups 0 and
+// 2 share the even sub-blocks, 32 of the 64 columns each, 1 and 3 the odd ones.  A sub-block's chain of TMEM load, exponential
+// and TMEM store has to stay shorter than the products of the sub-block before, which are issued ahead of it.
+constexpr int BWD_THREADS = 576;
+// A packed bf16 tile lies over the fp32 columns that its writers have read themselves: columns 0-15 and 32-47 of its buffer.
+__device__ __forceinline__ uint32_t packed_col(int ks) { return static_cast<uint32_t>((ks >> 1) * 32 + (ks & 1) * 8); }
 
 struct DkvBars {
   uint64_t kv_full, qd_full[NST], qd_empty[NST], s_full[2], p_ready[2], stat_ready[2], acc_done;
@@ -40,12 +50,6 @@ struct DkvBars {
   int abort_flag;
 };
 
-__device__ __forceinline__ uint64_t sub_desc_kmajor(uint32_t base, int ks) {   // [64 q][128 hd] as the K-major B operand
-  return umma_smem_desc(base + (ks >> 2) * Q_HALF + (ks & 3) * 32, 16, 1024);
-}
-__device__ __forceinline__ uint64_t sub_desc_mnmajor(uint32_t base, int ks) {  // the same bytes read along the head dim
-  return umma_smem_desc(base + ks * 2048, Q_HALF, 1024);
-}
 __device__ __forceinline__ void bulk_load_1d(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                ::"r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar))
@@ -80,13 +84,35 @@ flash_bwd_dkv_t_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
   const int nsub = (p.S - kb * AT + BQ - 1) / BQ;      // query sub-blocks from the diagonal to the end
   const int iters = G * nsub;
 
-  if (threadIdx.x == 0) {
-    mbar_init(&bars->kv_full, 1);
-    for (int i = 0; i < NST; ++i) { mbar_init(&bars->qd_full[i], 1); mbar_init(&bars->qd_empty[i], 1); }
-    for (int i = 0; i < 2; ++i) { mbar_init(&bars->s_full[i], 1); mbar_init(&bars->p_ready[i], 128); mbar_init(&bars->stat_ready[i], 128); }
-    mbar_init(&bars->acc_done, 1);
-    bars->abort_flag = 0;
-    mbar_fence_init();
+  auto load_stage = [&](int it, uint32_t e) {
+    const int g = it / nsub;
+    const int h = h_first + g;
+    const int q0 = kb * AT + (it - g * nsub) * BQ;
+    const int st = it % NST;
+    mbar_expect_tx(&bars->qd_full[st], 2 * Q_TILE + (RAGGED ? 0 : STAT_BYTES), e);
+    load_head_tile<NH>(sQ + st * Q_TILE, Q_HALF, &tmQ, &bars->qd_full[st], h, q0, b, e);
+    load_head_tile<NH>(sDO + st * Q_TILE, Q_HALF, &tmDO, &bars->qd_full[st], h, q0, b, e);
+    if (!RAGGED) {
+      const long long stat_idx = (static_cast<long long>(b) * p.Hq + h) * p.S + q0;
+      if (e) bulk_load_1d(sStat + st * 2 * BQ, p.lse + stat_idx, BQ * 4, &bars->qd_full[st]);
+      if (e) bulk_load_1d(sStat + st * 2 * BQ + BQ, p.delta + stat_idx, BQ * 4, &bars->qd_full[st]);
+    }
+  };
+  if (warp == 0) {                     // the first loads are on their way while the block sets itself up
+    if (lane == 0) {
+      mbar_init(&bars->kv_full, 1);
+      for (int i = 0; i < NST; ++i) { mbar_init(&bars->qd_full[i], 1); mbar_init(&bars->qd_empty[i], 1); }
+      for (int i = 0; i < 2; ++i) { mbar_init(&bars->s_full[i], 1); mbar_init(&bars->p_ready[i], 256); mbar_init(&bars->stat_ready[i], 256); }
+      mbar_init(&bars->acc_done, 1);
+      bars->abort_flag = 0;
+      mbar_fence_init();
+    }
+    __syncwarp();
+    const uint32_t e = elect_one();
+    mbar_expect_tx(&bars->kv_full, 2 * TILE_BYTES, e);
+    load_head_tile<NH>(sK, HALF_BYTES, &tmK, &bars->kv_full, hk, kb * AT, b, e);
+    load_head_tile<NH>(sV, HALF_BYTES, &tmV, &bars->kv_full, hk, kb * AT, b, e);
+    for (int it = 0; it < NST && it < iters; ++it) load_stage(it, e);
   }
   if (warp == 1) tmem_alloc(&bars->tmem_slot, 512);
   tc_fence_before();
@@ -97,28 +123,10 @@ flash_bwd_dkv_t_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
 
   if (warp == 0) {
     // ------------------------------------------------------------ producer
-    {
-      const uint32_t e = elect_one();
-      mbar_expect_tx(&bars->kv_full, 2 * TILE_BYTES, e);
-      load_head_tile<NH>(sK, HALF_BYTES, &tmK, &bars->kv_full, hk, kb * AT, b, e);
-      load_head_tile<NH>(sV, HALF_BYTES, &tmV, &bars->kv_full, hk, kb * AT, b, e);
-      for (int it = 0; it < iters; ++it) {
-        const int g = it / nsub;
-        const int h = h_first + g;
-        const int q0 = kb * AT + (it - g * nsub) * BQ;
-        const int st = it % NST;
-        if (!mbar_wait_warp(&bars->qd_empty[st], ((it / NST) & 1) ^ 1, abort_flag, p.status, 4)) break;
-        mbar_expect_tx(&bars->qd_full[st], 2 * Q_TILE + (RAGGED ? 0 : STAT_BYTES), e);
-        uint8_t* q_dst = sQ + st * Q_TILE;
-        uint8_t* do_dst = sDO + st * Q_TILE;
-        load_head_tile<NH>(q_dst, Q_HALF, &tmQ, &bars->qd_full[st], h, q0, b, e);
-        load_head_tile<NH>(do_dst, Q_HALF, &tmDO, &bars->qd_full[st], h, q0, b, e);
-        if (!RAGGED) {
-          const long long stat_idx = (static_cast<long long>(b) * p.Hq + h) * p.S + q0;
-          if (e) bulk_load_1d(sStat + st * 2 * BQ, p.lse + stat_idx, BQ * 4, &bars->qd_full[st]);
-          if (e) bulk_load_1d(sStat + st * 2 * BQ + BQ, p.delta + stat_idx, BQ * 4, &bars->qd_full[st]);
-        }
-      }
+    const uint32_t e = elect_one();
+    for (int it = NST; it < iters; ++it) {
+      if (!mbar_wait_warp(&bars->qd_empty[it % NST], ((it / NST) & 1) ^ 1, abort_flag, p.status, 4)) break;
+      load_stage(it, e);
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issue
@@ -126,7 +134,8 @@ flash_bwd_dkv_t_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
       const uint32_t e = elect_one();
       constexpr uint32_t idesc_s = umma_idesc_bf16(128, BQ, false, false);
       constexpr uint32_t idesc_acc = umma_idesc_bf16(128, 64 * NH, false, true);
-      const uint32_t k_base = smem_u32(sK), v_base = smem_u32(sV), q_base = smem_u32(sQ), do_base = smem_u32(sDO);
+      const uint64_t k_desc = kmajor_desc(sK), v_desc = kmajor_desc(sV), q_desc = kmajor_desc(sQ), do_desc = kmajor_desc(sDO);
+      const uint64_t q_mn = mnmajor_desc(sQ, Q_HALF), do_mn = mnmajor_desc(sDO, Q_HALF);
       bool ok = mbar_wait_warp(&bars->kv_full, 0, abort_flag, p.status, 4);
       auto issue_sp = [&](int it) -> bool {
         const int st = it % NST, buf = it & 1;
@@ -136,10 +145,10 @@ flash_bwd_dkv_t_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
         // the tensor core executes in order before these.
 #pragma unroll
         for (int ks = 0; ks < 4 * NH; ++ks)
-          umma_ss(tS + buf * BQ, desc_kmajor(k_base, ks), sub_desc_kmajor(q_base + st * Q_TILE, ks), idesc_s, ks > 0 ? 1u : 0u, e);
+          umma_ss(tS + buf * BQ, desc_at(k_desc, kmajor_off(HALF_BYTES, ks)), desc_at(q_desc, st * Q_TILE + kmajor_off(Q_HALF, ks)), idesc_s, ks > 0 ? 1u : 0u, e);
 #pragma unroll
         for (int ks = 0; ks < 4 * NH; ++ks)
-          umma_ss(tDP + buf * BQ, desc_kmajor(v_base, ks), sub_desc_kmajor(do_base + st * Q_TILE, ks), idesc_s, ks > 0 ? 1u : 0u, e);
+          umma_ss(tDP + buf * BQ, desc_at(v_desc, kmajor_off(HALF_BYTES, ks)), desc_at(do_desc, st * Q_TILE + kmajor_off(Q_HALF, ks)), idesc_s, ks > 0 ? 1u : 0u, e);
         umma_commit(&bars->s_full[buf], e);
         return true;
       };
@@ -151,39 +160,41 @@ flash_bwd_dkv_t_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
         tc_fence_after();
 #pragma unroll
         for (int ks = 0; ks < BQ / 16; ++ks)
-          umma_ts(tDV, tS + buf * BQ + ks * 8, sub_desc_mnmajor(do_base + st * Q_TILE, ks), idesc_acc, (it > 0 || ks > 0) ? 1u : 0u, e);
+          umma_ts(tDV, tS + buf * BQ + packed_col(ks), desc_at(do_mn, st * Q_TILE + mnmajor_off(ks)), idesc_acc, (it > 0 || ks > 0) ? 1u : 0u, e);
 #pragma unroll
         for (int ks = 0; ks < BQ / 16; ++ks)
-          umma_ts(tDK, tDP + buf * BQ + ks * 8, sub_desc_mnmajor(q_base + st * Q_TILE, ks), idesc_acc, (it > 0 || ks > 0) ? 1u : 0u, e);
+          umma_ts(tDK, tDP + buf * BQ + packed_col(ks), desc_at(q_mn, st * Q_TILE + mnmajor_off(ks)), idesc_acc, (it > 0 || ks > 0) ? 1u : 0u, e);
         umma_commit(&bars->qd_empty[st], e);
       }
       if (ok) umma_commit(&bars->acc_done, e);
     }
   } else {
     // ------------------------------------------------------------ softmax / epilogue: one thread per key row
-    const int wg = (warp - 2) >> 2;                       // 0: even sub-blocks (buffer 0), 1: odd sub-blocks (buffer 1)
+    const int wg = (warp - 2) >> 2, buf = wg & 1, part = wg >> 1;
     const int row = (warp & 3) * 32 + lane;
     const uint32_t lane_off = static_cast<uint32_t>((warp & 3) * 32) << 16;
     const int kv_idx = kb * AT + row;
-    const int buf = wg;
+    const f32x2 nscale = pack2(-p.scale_log2, -p.scale_log2), minus = pack2(-1.f, -1.f);
     bool ok = true;
-    for (int it = wg; it < iters; it += 2) {
+    for (int it = buf; it < iters; it += 2) {
       const int g = it / nsub;
       const int q0 = kb * AT + (it - g * nsub) * BQ;
       const int st = it % NST;
-      // RAGGED: sub-block `it` has statistics slot it % NST, so a group alternates between two slots of its own.  A
-      // thread rewrites a slot two of its sub-blocks later, past the group's barrier of the one between, at which every
-      // thread of the group arrives only after it has read this one.  The group meets on an mbarrier, because a thread
-      // may leave the loop on its own when a bounded wait runs out: the others then give up here as well.
+      // RAGGED: sub-block `it` has statistics slot it % NST, so the two groups of a buffer alternate between two slots of
+      // their own, which the first of them fills.  It rewrites a slot two of its sub-blocks later, past the groups' barrier of
+      // the one between, at which every thread of both arrives only after it has read this one.  They meet on an mbarrier,
+      // because a thread may leave the loop on its own when a bounded wait runs out: the others then give up here as well.
       if (RAGGED) {
-        const int qi = q0 + (row & (BQ - 1));
-        const long long stat_idx = (static_cast<long long>(b) * p.Hq + h_first + g) * p.S + qi;
-        const bool want_lse = row < BQ;
-        float v = want_lse ? INFINITY : 0.f;
-        if (qi < p.S) v = want_lse ? p.lse[stat_idx] : p.delta[stat_idx];
-        sStat[st * 2 * BQ + row] = v;
-        mbar_arrive(&bars->stat_ready[wg]);
-        if (!mbar_wait(&bars->stat_ready[wg], (it >> 1) & 1, abort_flag, p.status, 4)) { ok = false; break; }
+        if (part == 0) {
+          const int qi = q0 + (row & (BQ - 1));
+          const long long stat_idx = (static_cast<long long>(b) * p.Hq + h_first + g) * p.S + qi;
+          const bool want_lse = row < BQ;
+          float v = want_lse ? INFINITY : 0.f;
+          if (qi < p.S) v = want_lse ? p.lse[stat_idx] : p.delta[stat_idx];
+          sStat[st * 2 * BQ + row] = v;
+        }
+        mbar_arrive(&bars->stat_ready[buf]);
+        if (!mbar_wait(&bars->stat_ready[buf], (it >> 1) & 1, abort_flag, p.status, 4)) { ok = false; break; }
       }
       if (!mbar_wait(&bars->qd_full[st], (it / NST) & 1, abort_flag, p.status, 4)) { ok = false; break; }
       if (!mbar_wait(&bars->s_full[buf], (it >> 1) & 1, abort_flag, p.status, 4)) { ok = false; break; }
@@ -191,35 +202,34 @@ flash_bwd_dkv_t_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
       const float* lse_s = sStat + st * 2 * BQ;
       const float* delta_s = lse_s + BQ;
       const bool diag = q0 < kb * AT + AT;               // some keys of this block lie after some of these queries
+      const uint32_t col = buf * BQ + part * 32 + lane_off;
 #pragma unroll
-      for (int c = 0; c < BQ / 32; ++c) {
-        uint32_t sv[32], dv[32];
-        tmem_ld32(tS + buf * BQ + lane_off + c * 32, sv);
-        tmem_ld32(tDP + buf * BQ + lane_off + c * 32, dv);
+      for (int c = 0; c < 32; c += 16) {                    // 32 at once would take more than the 96 registers there are
+        uint32_t sv[16], dv[16], pk[8], dk[8];
+        tmem_ld16(tS + col + c, sv);
+        tmem_ld16(tDP + col + c, dv);
         tmem_ld_wait();
-        uint32_t pk[16], dk[16];
 #pragma unroll
-        for (int t = 0; t < 32; t += 4) {
-          const float4 l4 = *reinterpret_cast<const float4*>(lse_s + c * 32 + t);
-          const float4 d4 = *reinterpret_cast<const float4*>(delta_s + c * 32 + t);
-          const float lv[4] = {l4.x, l4.y, l4.z, l4.w}, dl[4] = {d4.x, d4.y, d4.z, d4.w};
-          float pr[4], ds[4];
+        for (int t = 0; t < 16; t += 4) {
+          const float4 l4 = *reinterpret_cast<const float4*>(lse_s + part * 32 + c + t);
+          const float4 d4 = *reinterpret_cast<const float4*>(delta_s + part * 32 + c + t);
+          const f32x2 lv[2] = {pack2(l4.x, l4.y), pack2(l4.z, l4.w)}, dl[2] = {pack2(d4.x, d4.y), pack2(d4.z, d4.w)};
 #pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            float pv = exp2f(fmaf(__uint_as_float(sv[t + u]), p.scale_log2, -lv[u]));
-            if (diag && (q0 + c * 32 + t + u < kv_idx)) pv = 0.f;
-            pr[u] = pv;
-            ds[u] = pv * (__uint_as_float(dv[t + u]) - dl[u]);      // the softmax scale is applied to dK once, at the end
+          for (int u = 0; u < 2; ++u) {
+            const int j = t + 2 * u, q = q0 + part * 32 + c + j;
+            float x0, x1, s0, s1;
+            unpack2(fma2(pack2(sv[j], sv[j + 1]), nscale, lv[u]), x0, x1);         // log-sum-exp minus score
+            float p0 = exp2f(-x0), p1 = exp2f(-x1);
+            if (diag && (q < kv_idx)) p0 = 0.f;
+            if (diag && (q + 1 < kv_idx)) p1 = 0.f;
+            // the softmax scale is applied to dK once, at the end
+            unpack2(mul2(pack2(p0, p1), fma2(dl[u], minus, pack2(dv[j], dv[j + 1]))), s0, s1);
+            pk[j >> 1] = pack_bf16x2(p0, p1);
+            dk[j >> 1] = pack_bf16x2(s0, s1);
           }
-          pk[t >> 1] = pack_bf16x2(pr[0], pr[1]);
-          pk[(t >> 1) + 1] = pack_bf16x2(pr[2], pr[3]);
-          dk[t >> 1] = pack_bf16x2(ds[0], ds[1]);
-          dk[(t >> 1) + 1] = pack_bf16x2(ds[2], ds[3]);
         }
-        // The bf16 tiles occupy the first 32 columns of their buffers, i.e. only columns of the first fp32 chunk,
-        // which this thread has already read: 16 packed columns per chunk.
-        tmem_st16(tS + buf * BQ + lane_off + c * 16, pk);
-        tmem_st16(tDP + buf * BQ + lane_off + c * 16, dk);
+        tmem_st8(tS + col + c / 2, pk);                     // over columns that this thread has read (packed_col)
+        tmem_st8(tDP + col + c / 2, dk);
       }
       tmem_st_wait();
       tc_fence_before();
@@ -227,18 +237,22 @@ flash_bwd_dkv_t_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     }
     if (ok && mbar_wait(&bars->acc_done, 0, abort_flag, p.status, 4)) {
       tc_fence_after();
-      // group 0 stores dV, group 1 stores dK
-      __nv_bfloat16* dst0 = reinterpret_cast<__nv_bfloat16*>(wg == 0 ? p.dv : p.dk) +
-                            (static_cast<long long>(b) * p.S + kv_idx) * (wg == 0 ? p.ld_dv : p.ld_dk) + out_head * p.hd;
-      const uint32_t t_src = (wg == 0 ? tDV : tDK) + lane_off;
-      const float out_scale = wg == 0 ? 1.f : p.scale;
+      // groups 0 and 2 store dV, 1 and 3 dK, half of the columns each
+      const long long ld = buf == 0 ? p.ld_dv : p.ld_dk;
+      const int row0 = kb * AT + (warp & 3) * 32;
+      __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(buf == 0 ? p.dv : p.dk) + (static_cast<long long>(b) * p.S + row0) * ld +
+                           out_head * p.hd + part * NH * 32;
+      const uint32_t t_src = (buf == 0 ? tDV : tDK) + lane_off;
+      const float out_scale = buf == 0 ? 1.f : p.scale;
+      uint8_t* stage = smem + (warp - 2) * (NH * 2048);     // over K and V: every product has been computed
 #pragma unroll 1
-      for (int c = 0; c < 2 * NH; ++c) {
+      for (int c = 0; c < NH; ++c) {
         uint32_t v[32];
-        tmem_ld32(t_src + c * 32, v);
+        tmem_ld32(t_src + (part * NH + c) * 32, v);
         tmem_ld_wait();
-        if (kv_idx < p.S) store_head32(dst0, c * 32, p.hd, v, out_scale);
+        stage_head32<4 * NH>(stage, lane, c, v, out_scale);
       }
+      store_staged<4 * NH>(dst, ld, stage, lane, p.S - row0, p.hd - part * NH * 32);
     }
   }
   tc_fence_before();
@@ -252,7 +266,7 @@ flash_bwd_dkv_t_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
 // ================================================================================================ backward: dQ
 // CTA = (query block of 128 positions, head, batch).  Q_i and dO_i stay in shared memory; K and V stream through in
 // sub-blocks of 64 positions.  S = Q K^T and dP = dO V^T land in one of two TMEM buffer pairs; the softmax threads
-// (one per query row) write dS as bf16 over the first 32 columns of the dP buffer, which is then the tensor-memory
+// (two per query row) write dS as bf16 over half of the dP buffer's columns, which are then the tensor-memory
 // A operand of dQ += dS K.  Also produces delta = rowsum(O * dO) for the dK/dV pass.
 // TMEM: S buffers at 0 and 64, dP buffers at 128 and 192, dQ at 256.
 struct DqBars {
@@ -285,13 +299,40 @@ flash_bwd_dq_t_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   const int nkv_all = (p.S + BQ - 1) / BQ;
   if (nkv > nkv_all) nkv = nkv_all;
 
-  if (threadIdx.x == 0) {
-    mbar_init(&bars->qd_full, 1);
-    for (int i = 0; i < NST; ++i) { mbar_init(&bars->kv_full[i], 1); mbar_init(&bars->kv_empty[i], 1); }
-    for (int i = 0; i < 2; ++i) { mbar_init(&bars->s_full[i], 1); mbar_init(&bars->p_ready[i], 128); }
-    mbar_init(&bars->acc_done, 1);
-    bars->abort_flag = 0;
-    mbar_fence_init();
+  auto load_stage = [&](int j, uint32_t e) {
+    const int st = j % NST;
+    mbar_expect_tx(&bars->kv_full[st], 2 * Q_TILE, e);
+    load_head_tile<NH>(sK + st * Q_TILE, Q_HALF, &tmK, &bars->kv_full[st], hk, j * BQ, b, e);
+    load_head_tile<NH>(sV + st * Q_TILE, Q_HALF, &tmV, &bars->kv_full[st], hk, j * BQ, b, e);
+  };
+  if (warp == 0) {                     // the first loads are on their way while the block sets itself up
+    if (lane == 0) {
+      mbar_init(&bars->qd_full, 1);
+      for (int i = 0; i < NST; ++i) { mbar_init(&bars->kv_full[i], 1); mbar_init(&bars->kv_empty[i], 1); }
+      for (int i = 0; i < 2; ++i) { mbar_init(&bars->s_full[i], 1); mbar_init(&bars->p_ready[i], 256); }
+      mbar_init(&bars->acc_done, 1);
+      bars->abort_flag = 0;
+      mbar_fence_init();
+    }
+    __syncwarp();
+    const uint32_t e = elect_one();
+    mbar_expect_tx(&bars->qd_full, 2 * TILE_BYTES, e);
+    load_head_tile<NH>(sQ, HALF_BYTES, &tmQ, &bars->qd_full, h, qb * AT, b, e);
+    load_head_tile<NH>(sDO, HALF_BYTES, &tmDO, &bars->qd_full, h, qb * AT, b, e);
+    for (int j = 0; j < NST && j < nkv; ++j) load_stage(j, e);
+  }
+  // delta = sum over the head of o * dO.  The 16 warps take 8 rows of o each, LPR lanes to a row, and find dO in shared memory
+  // later.  One thread to a row, reading both rows 16 bytes at a time, took 9000 of the 50000 cycles of the longest block.
+  constexpr int LPR = 8 * NH, PASSES = LPR / 4;
+  uint4 o4[PASSES];
+  if (warp >= 2) {
+#pragma unroll
+    for (int i = 0; i < PASSES; ++i) {
+      const int r = qb * AT + (warp - 2) * 8 + (i * 32 + lane) / LPR, c = (lane % LPR) * 8;
+      o4[i] = make_uint4(0, 0, 0, 0);
+      if (r < p.S && c < p.hd)
+        o4[i] = *reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(p.o_in) + (static_cast<long long>(b) * p.S + r) * p.ld_o + h * p.hd + c);
+    }
   }
   if (warp == 1) tmem_alloc(&bars->tmem_slot, 512);
   tc_fence_before();
@@ -301,27 +342,18 @@ flash_bwd_dq_t_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   const uint32_t tS = tmem, tDP = tmem + 128, tDQ = tmem + 256;
 
   if (warp == 0) {
-    {
-      const uint32_t e = elect_one();
-      mbar_expect_tx(&bars->qd_full, 2 * TILE_BYTES, e);
-      load_head_tile<NH>(sQ, HALF_BYTES, &tmQ, &bars->qd_full, h, qb * AT, b, e);
-      load_head_tile<NH>(sDO, HALF_BYTES, &tmDO, &bars->qd_full, h, qb * AT, b, e);
-      for (int j = 0; j < nkv; ++j) {
-        const int st = j % NST;
-        if (!mbar_wait_warp(&bars->kv_empty[st], ((j / NST) & 1) ^ 1, abort_flag, p.status, 4)) break;
-        mbar_expect_tx(&bars->kv_full[st], 2 * Q_TILE, e);
-        uint8_t* k_dst = sK + st * Q_TILE;
-        uint8_t* v_dst = sV + st * Q_TILE;
-        load_head_tile<NH>(k_dst, Q_HALF, &tmK, &bars->kv_full[st], hk, j * BQ, b, e);
-        load_head_tile<NH>(v_dst, Q_HALF, &tmV, &bars->kv_full[st], hk, j * BQ, b, e);
-      }
+    const uint32_t e = elect_one();
+    for (int j = NST; j < nkv; ++j) {
+      if (!mbar_wait_warp(&bars->kv_empty[j % NST], ((j / NST) & 1) ^ 1, abort_flag, p.status, 4)) break;
+      load_stage(j, e);
     }
   } else if (warp == 1) {
     {
       const uint32_t e = elect_one();
       constexpr uint32_t idesc_s = umma_idesc_bf16(128, BQ, false, false);
       constexpr uint32_t idesc_acc = umma_idesc_bf16(128, 64 * NH, false, true);
-      const uint32_t q_base = smem_u32(sQ), do_base = smem_u32(sDO), k_base = smem_u32(sK), v_base = smem_u32(sV);
+      const uint64_t q_desc = kmajor_desc(sQ), do_desc = kmajor_desc(sDO), k_desc = kmajor_desc(sK), v_desc = kmajor_desc(sV);
+      const uint64_t k_mn = mnmajor_desc(sK, Q_HALF);
       bool ok = mbar_wait_warp(&bars->qd_full, 0, abort_flag, p.status, 4);
       auto issue_sp = [&](int j) -> bool {
         const int st = j % NST, buf = j & 1;
@@ -329,10 +361,10 @@ flash_bwd_dq_t_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         tc_fence_after();
 #pragma unroll
         for (int ks = 0; ks < 4 * NH; ++ks)
-          umma_ss(tS + buf * BQ, desc_kmajor(q_base, ks), sub_desc_kmajor(k_base + st * Q_TILE, ks), idesc_s, ks > 0 ? 1u : 0u, e);
+          umma_ss(tS + buf * BQ, desc_at(q_desc, kmajor_off(HALF_BYTES, ks)), desc_at(k_desc, st * Q_TILE + kmajor_off(Q_HALF, ks)), idesc_s, ks > 0 ? 1u : 0u, e);
 #pragma unroll
         for (int ks = 0; ks < 4 * NH; ++ks)
-          umma_ss(tDP + buf * BQ, desc_kmajor(do_base, ks), sub_desc_kmajor(v_base + st * Q_TILE, ks), idesc_s, ks > 0 ? 1u : 0u, e);
+          umma_ss(tDP + buf * BQ, desc_at(do_desc, kmajor_off(HALF_BYTES, ks)), desc_at(v_desc, st * Q_TILE + kmajor_off(Q_HALF, ks)), idesc_s, ks > 0 ? 1u : 0u, e);
         umma_commit(&bars->s_full[buf], e);
         return true;
       };
@@ -344,69 +376,77 @@ flash_bwd_dq_t_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         tc_fence_after();
 #pragma unroll
         for (int ks = 0; ks < BQ / 16; ++ks)
-          umma_ts(tDQ, tDP + buf * BQ + ks * 8, sub_desc_mnmajor(k_base + st * Q_TILE, ks), idesc_acc, (j > 0 || ks > 0) ? 1u : 0u, e);
+          umma_ts(tDQ, tDP + buf * BQ + packed_col(ks), desc_at(k_mn, st * Q_TILE + mnmajor_off(ks)), idesc_acc, (j > 0 || ks > 0) ? 1u : 0u, e);
         umma_commit(&bars->kv_empty[st], e);
       }
       if (ok) umma_commit(&bars->acc_done, e);
     }
   } else {
-    const int wg = (warp - 2) >> 2;                       // 0: even KV sub-blocks (buffer 0), 1: odd (buffer 1)
+    const int wg = (warp - 2) >> 2, buf = wg & 1, part = wg >> 1;
     const int row = (warp & 3) * 32 + lane;
     const uint32_t lane_off = static_cast<uint32_t>((warp & 3) * 32) << 16;
     const int q_idx = qb * AT + row;
     const long long stat_idx = (static_cast<long long>(b) * p.Hq + h) * p.S + q_idx;
     const bool row_ok = q_idx < p.S;
     const float lse2 = row_ok ? p.lse[stat_idx] : INFINITY;
-    if (wg == 0) {
+    bool ok = mbar_wait(&bars->qd_full, 0, abort_flag, p.status, 4);
+#pragma unroll
+    for (int i = 0; i < PASSES; ++i) {
+      const int r = (warp - 2) * 8 + (i * 32 + lane) / LPR, c = lane % LPR;
+      const uint4 g4 = *reinterpret_cast<const uint4*>(sDO + (c >> 3) * HALF_BYTES + r * 128 + (((c & 7) ^ (r & 7)) << 4));
+      const uint32_t ow[4] = {o4[i].x, o4[i].y, o4[i].z, o4[i].w}, gw[4] = {g4.x, g4.y, g4.z, g4.w};
       float d = 0.f;
-      const __nv_bfloat16* op = reinterpret_cast<const __nv_bfloat16*>(p.o_in) + (static_cast<long long>(b) * p.S + q_idx) * p.ld_o + h * p.hd;
-      const __nv_bfloat16* gp = reinterpret_cast<const __nv_bfloat16*>(p.d_o) + (static_cast<long long>(b) * p.S + q_idx) * p.ld_do + h * p.hd;
-      if (row_ok) {
-        d = row_delta(op, gp, p.hd);
-        p.delta[stat_idx] = d;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) d += bf16_lo(ow[q]) * bf16_lo(gw[q]) + bf16_hi(ow[q]) * bf16_hi(gw[q]);
+#pragma unroll
+      for (int m = LPR / 2; m > 0; m >>= 1) d += __shfl_xor_sync(0xffffffffu, d, m);
+      if (lane % LPR == 0) {
+        bars->delta[r] = d;
+        if (qb * AT + r < p.S) p.delta[(static_cast<long long>(b) * p.Hq + h) * p.S + qb * AT + r] = d;
       }
-      bars->delta[row] = d;
     }
-    named_barrier(1, 256);                                // both groups: the block's delta values are in shared memory
+    named_barrier(1, 512);                                // all groups: the block's delta values are in shared memory
     const float delta = bars->delta[row];
-    const int buf = wg;
-    bool ok = true;
-    for (int j = wg; j < nkv; j += 2) {
+    const f32x2 nscale = pack2(-p.scale_log2, -p.scale_log2), lse_2 = pack2(lse2, lse2), ndelta = pack2(-delta, -delta);
+    for (int j = buf; ok && j < nkv; j += 2) {
       if (!mbar_wait(&bars->s_full[buf], (j >> 1) & 1, abort_flag, p.status, 4)) { ok = false; break; }
       tc_fence_after();
       const int kv0 = j * BQ;
       const bool diag = (kv0 + BQ - 1 > qb * AT);
+      const uint32_t col = buf * BQ + part * 32 + lane_off;
+      uint32_t sv[32], dv[32];
+      tmem_ld32(tS + col, sv);
+      tmem_ld32(tDP + col, dv);
+      tmem_ld_wait();
+      uint32_t dk[16];
 #pragma unroll
-      for (int c = 0; c < BQ / 32; ++c) {
-        uint32_t sv[32], dv[32];
-        tmem_ld32(tS + buf * BQ + lane_off + c * 32, sv);
-        tmem_ld32(tDP + buf * BQ + lane_off + c * 32, dv);
-        tmem_ld_wait();
-        uint32_t dk[16];
-#pragma unroll
-        for (int t = 0; t < 32; t += 2) {
-          float p0 = exp2f(fmaf(__uint_as_float(sv[t]), p.scale_log2, -lse2));
-          float p1 = exp2f(fmaf(__uint_as_float(sv[t + 1]), p.scale_log2, -lse2));
-          if (diag && (kv0 + c * 32 + t > q_idx)) p0 = 0.f;
-          if (diag && (kv0 + c * 32 + t + 1 > q_idx)) p1 = 0.f;
-          dk[t >> 1] = pack_bf16x2(p0 * (__uint_as_float(dv[t]) - delta), p1 * (__uint_as_float(dv[t + 1]) - delta));
-        }
-        tmem_st16(tDP + buf * BQ + lane_off + c * 16, dk);  // dS over columns of the first dP chunk (already read)
+      for (int t = 0; t < 32; t += 2) {
+        float x0, x1, s0, s1;
+        unpack2(fma2(pack2(sv[t], sv[t + 1]), nscale, lse_2), x0, x1);             // log-sum-exp minus score
+        float p0 = exp2f(-x0), p1 = exp2f(-x1);
+        if (diag && (kv0 + part * 32 + t > q_idx)) p0 = 0.f;
+        if (diag && (kv0 + part * 32 + t + 1 > q_idx)) p1 = 0.f;
+        unpack2(mul2(pack2(p0, p1), add2(pack2(dv[t], dv[t + 1]), ndelta)), s0, s1);
+        dk[t >> 1] = pack_bf16x2(s0, s1);
       }
+      tmem_st16(tDP + col, dk);                             // over columns that this thread has read (packed_col)
       tmem_st_wait();
       tc_fence_before();
       mbar_arrive(&bars->p_ready[buf]);
     }
     if (ok && mbar_wait(&bars->acc_done, 0, abort_flag, p.status, 4)) {
       tc_fence_after();
-      // each group stores one half of the dQ columns; dS was left unscaled, so the softmax scale lands here
-      __nv_bfloat16* dqp = reinterpret_cast<__nv_bfloat16*>(p.dq) + (static_cast<long long>(b) * p.S + q_idx) * p.ld_dq + h * p.hd;
-#pragma unroll 1
-      for (int c = wg * NH; c < (wg + 1) * NH; ++c) {
+      // the groups store 32 dQ columns each (two of them where the head is one half wide); dS was left unscaled, so the
+      // softmax scale lands here
+      if (wg < 2 * NH) {
+        const int row0 = qb * AT + (warp & 3) * 32;
+        uint8_t* stage = smem + (warp - 2) * 2048;          // over Q and dO: every product has been computed
         uint32_t v[32];
-        tmem_ld32(tDQ + lane_off + c * 32, v);
+        tmem_ld32(tDQ + lane_off + wg * 32, v);
         tmem_ld_wait();
-        if (row_ok) store_head32(dqp, c * 32, p.hd, v, p.scale);
+        stage_head32<4>(stage, lane, 0, v, p.scale);
+        store_staged<4>(reinterpret_cast<__nv_bfloat16*>(p.dq) + (static_cast<long long>(b) * p.S + row0) * p.ld_dq + h * p.hd + wg * 32,
+                        p.ld_dq, stage, lane, p.S - row0, p.hd - wg * 32);
       }
     }
   }

@@ -18,10 +18,12 @@ constexpr uint32_t HALF_BYTES = 16384;  // [128 rows][64 columns] bf16
 inline int head_halves(int hd) { return hd <= 64 ? 1 : 2; }
 constexpr float kLog2e = 1.4426950408889634f;
 
-// K-major operand descriptor for k-step ks (16 columns each) of a [128 rows][64 * NH columns] tile in swizzled halves.
-__device__ __forceinline__ uint64_t desc_kmajor(uint32_t base, int ks) {
-  return umma_smem_desc(base + (ks >> 2) * HALF_BYTES + (ks & 3) * 32, 16, 1024);
-}
+// Byte offsets of k-step ks (16 deep) in a tile of swizzled halves of 64 columns: read K-major (along the columns, halves
+// `half` bytes apart) and MN-major (along the rows).
+__device__ __forceinline__ constexpr uint32_t kmajor_off(uint32_t half, int ks) { return (ks >> 2) * half + (ks & 3) * 32; }
+__device__ __forceinline__ constexpr uint32_t mnmajor_off(int ks) { return ks * 2048; }
+__device__ __forceinline__ uint64_t kmajor_desc(const void* tile) { return umma_smem_desc(smem_u32(tile), 16, 1024); }
+__device__ __forceinline__ uint64_t mnmajor_desc(const void* tile, uint32_t half) { return umma_smem_desc(smem_u32(tile), half, 1024); }
 
 struct AttnDev {
   void* o; float* lse; float* delta;
@@ -64,20 +66,17 @@ __device__ __forceinline__ void load_head_tile(uint8_t* dst, uint32_t half_bytes
 #pragma unroll
   for (int j = 0; j < NH; ++j) tma_load_4d(dst + j * half_bytes, tm, bar, j * 64, head, s0, b, e);
 }
-// delta = sum over the head of o * d_o for one row (hd is a multiple of 8).
-__device__ __forceinline__ float row_delta(const __nv_bfloat16* op, const __nv_bfloat16* gp, int hd) {
-  float d = 0.f;
-#pragma unroll 4
-  for (int c = 0; c < (hd >> 3); ++c) {
-    const uint4 a = reinterpret_cast<const uint4*>(op)[c], g = reinterpret_cast<const uint4*>(gp)[c];
-    const uint32_t aw[4] = {a.x, a.y, a.z, a.w}, gw[4] = {g.x, g.y, g.z, g.w};
-#pragma unroll
-    for (int q = 0; q < 4; ++q) d += bf16_lo(aw[q]) * bf16_lo(gw[q]) + bf16_hi(aw[q]) * bf16_hi(gw[q]);
-  }
-  return d;
+// The epilogues go through shared memory: a thread has one row of the accumulator, and a warp that stores 32 rows of 16 bytes
+// touches 32 lines with every instruction (3000-4000 cycles for the dK and dV of a block).  Each warp turns its own 32 rows
+// around in a buffer of its own, 16-byte chunks exchanged within a row so that neither side meets a bank conflict, and stores
+// whole row pieces.  CHUNKS = 16-byte chunks per row: 4, 8 or 16.
+template <int CHUNKS>
+__device__ __forceinline__ uint32_t staged_at(int row, int c) {
+  return (row * CHUNKS + (c ^ (CHUNKS == 4 ? (row >> 1) & 3 : row & 7))) * 16;
 }
-// Stores 32 accumulator columns (first one: column `col` of the head) as bf16, scaled, cut off at the head's width.
-__device__ __forceinline__ void store_head32(__nv_bfloat16* row, int col, int hd, const uint32_t (&v)[32], float f) {
+// 32 accumulator columns of this lane's row, scaled, as bf16: chunks 4 * part .. 4 * part + 3.
+template <int CHUNKS>
+__device__ __forceinline__ void stage_head32(uint8_t* buf, int lane, int part, const uint32_t (&v)[32], float f) {
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
     uint4 o4;
@@ -85,7 +84,18 @@ __device__ __forceinline__ void store_head32(__nv_bfloat16* row, int col, int hd
     o4.y = pack_bf16x2(__uint_as_float(v[8 * q + 2]) * f, __uint_as_float(v[8 * q + 3]) * f);
     o4.z = pack_bf16x2(__uint_as_float(v[8 * q + 4]) * f, __uint_as_float(v[8 * q + 5]) * f);
     o4.w = pack_bf16x2(__uint_as_float(v[8 * q + 6]) * f, __uint_as_float(v[8 * q + 7]) * f);
-    if (col + q * 8 < hd) *reinterpret_cast<uint4*>(row + col + q * 8) = o4;
+    *reinterpret_cast<uint4*>(buf + staged_at<CHUNKS>(lane, part * 4 + q)) = o4;
+  }
+}
+// The warp's 32 rows from `first` (the row and column that buf starts with), cut off at `rows` rows and `cols` columns.
+template <int CHUNKS>
+__device__ __forceinline__ void store_staged(__nv_bfloat16* first, long long ld, const uint8_t* buf, int lane, int rows, int cols) {
+  __syncwarp();
+#pragma unroll
+  for (int i = 0; i < CHUNKS; ++i) {
+    const int row = (i * 32 + lane) / CHUNKS, c = (i * 32 + lane) % CHUNKS;
+    if (row < rows && c * 8 < cols)
+      *reinterpret_cast<uint4*>(first + row * ld + c * 8) = *reinterpret_cast<const uint4*>(buf + staged_at<CHUNKS>(row, c));
   }
 }
 

@@ -11,13 +11,6 @@ namespace himuon {
 constexpr int BKV = 64;                              // KV positions per block
 constexpr uint32_t KV_HALF = BKV * 128;              // one 64-column half of a K or V block: 8 KB
 
-__device__ __forceinline__ uint64_t kv_desc_kmajor(uint32_t base, int ks) {   // K block as the K-major B operand of Q K^T
-  return umma_smem_desc(base + (ks >> 2) * KV_HALF + (ks & 3) * 32, 16, 1024);
-}
-__device__ __forceinline__ uint64_t kv_desc_mnmajor(uint32_t base, int ks) {  // K or V block read along the head dim
-  return umma_smem_desc(base + ks * 2048, KV_HALF, 1024);
-}
-
 // ================================================================================================ forward, P in TMEM
 // CTA = (128 query rows, head, batch); loops over 64-wide KV blocks up to the diagonal; S(j+1) = Q K^T is issued
 // before P(j) V so the tensor core overlaps the softmax; O stays in TMEM and is rescaled lazily (only when a row max
@@ -57,17 +50,34 @@ flash_fwd64_t_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   const int nkv_all = (p.S + BKV - 1) / BKV;
   if (nkv > nkv_all) nkv = nkv_all;
 
-  if (threadIdx.x == 0) {
-    mbar_init(&bars->q_full, 1);
-    for (int i = 0; i < 2; ++i) {
-      mbar_init(&bars->k_full[i], 1); mbar_init(&bars->k_empty[i], 1);
-      mbar_init(&bars->v_full[i], 1); mbar_init(&bars->v_empty[i], 1);
-      mbar_init(&bars->s_full[i], 1); mbar_init(&bars->p_ready[i], 128);
+  auto load_k = [&](int j, uint32_t e) {
+    const int st = j & 1;
+    mbar_expect_tx(&bars->k_full[st], KV_TILE, e);
+    load_head_tile<NH>(sK + st * KV_TILE, KV_HALF, &tmK, &bars->k_full[st], hk, j * BKV, b, e);
+  };
+  auto load_v = [&](int j, uint32_t e) {
+    const int st = j & 1;
+    mbar_expect_tx(&bars->v_full[st], KV_TILE, e);
+    load_head_tile<NH>(sV + st * KV_TILE, KV_HALF, &tmV, &bars->v_full[st], hk, j * BKV, b, e);
+  };
+  if (warp == 0) {                             // the first loads are on their way while the block sets itself up
+    if (lane == 0) {
+      mbar_init(&bars->q_full, 1);
+      for (int i = 0; i < 2; ++i) {
+        mbar_init(&bars->k_full[i], 1); mbar_init(&bars->k_empty[i], 1);
+        mbar_init(&bars->v_full[i], 1); mbar_init(&bars->v_empty[i], 1);
+        mbar_init(&bars->s_full[i], 1); mbar_init(&bars->p_ready[i], 128);
+      }
+      for (int i = 0; i < 2; ++i) mbar_init(&bars->o_done[i], 1);
+      mbar_init(&bars->acc_done, 1);
+      bars->abort_flag = 0;
+      mbar_fence_init();
     }
-    for (int i = 0; i < 2; ++i) mbar_init(&bars->o_done[i], 1);
-    mbar_init(&bars->acc_done, 1);
-    bars->abort_flag = 0;
-    mbar_fence_init();
+    __syncwarp();
+    const uint32_t e = elect_one();
+    mbar_expect_tx(&bars->q_full, TILE_BYTES, e);
+    load_head_tile<NH>(sQ, HALF_BYTES, &tmQ, &bars->q_full, h, qb * AT, b, e);
+    for (int j = 0; j < 2 && j < nkv; ++j) { load_k(j, e); load_v(j, e); }
   }
   if (warp == 1) tmem_alloc(&bars->tmem_slot, 256);
   tc_fence_before();
@@ -77,27 +87,20 @@ flash_fwd64_t_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   const uint32_t tS0 = tmem, tO = tmem + 128;   // S / P buffers at columns 0 and 64, O at 128
 
   if (warp == 0) {
-    {
-      const uint32_t e = elect_one();
-      mbar_expect_tx(&bars->q_full, TILE_BYTES, e);
-      load_head_tile<NH>(sQ, HALF_BYTES, &tmQ, &bars->q_full, h, qb * AT, b, e);
-      for (int j = 0; j < nkv; ++j) {
-        const int st = j & 1;
-        const uint32_t par = ((j >> 1) & 1) ^ 1;
-        if (!mbar_wait_warp(&bars->k_empty[st], par, abort_flag, p.status, 4)) break;
-        mbar_expect_tx(&bars->k_full[st], KV_TILE, e);
-        load_head_tile<NH>(sK + st * KV_TILE, KV_HALF, &tmK, &bars->k_full[st], hk, j * BKV, b, e);
-        if (!mbar_wait_warp(&bars->v_empty[st], par, abort_flag, p.status, 4)) break;
-        mbar_expect_tx(&bars->v_full[st], KV_TILE, e);
-        load_head_tile<NH>(sV + st * KV_TILE, KV_HALF, &tmV, &bars->v_full[st], hk, j * BKV, b, e);
-      }
+    const uint32_t e = elect_one();
+    for (int j = 2; j < nkv; ++j) {
+      const uint32_t par = ((j >> 1) & 1) ^ 1;
+      if (!mbar_wait_warp(&bars->k_empty[j & 1], par, abort_flag, p.status, 4)) break;
+      load_k(j, e);
+      if (!mbar_wait_warp(&bars->v_empty[j & 1], par, abort_flag, p.status, 4)) break;
+      load_v(j, e);
     }
   } else if (warp == 1) {
     {
       const uint32_t e = elect_one();
       constexpr uint32_t idesc_s = umma_idesc_bf16(128, BKV, false, false);
       constexpr uint32_t idesc_pv = umma_idesc_bf16(128, 64 * NH, false, true);
-      const uint32_t q_base = smem_u32(sQ), v_base = smem_u32(sV);
+      const uint64_t q_desc = kmajor_desc(sQ), k_desc = kmajor_desc(sK), v_mn = mnmajor_desc(sV, KV_HALF);
       bool ok = mbar_wait_warp(&bars->q_full, 0, abort_flag, p.status, 4);
       auto issue_s = [&](int j) -> bool {
         const int st = j & 1;
@@ -105,10 +108,9 @@ flash_fwd64_t_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         tc_fence_after();
         // buffer st held S(j-2) / P(j-2): the softmax threads are done with it (p_ready(j-2) was waited for) and the
         // P(j-2)·V MMAs were issued earlier, which the tensor core executes in order before these
-        const uint32_t k_base = smem_u32(sK + st * KV_TILE);
 #pragma unroll
         for (int ks = 0; ks < 4 * NH; ++ks)
-          umma_ss(tS0 + st * BKV, desc_kmajor(q_base, ks), kv_desc_kmajor(k_base, ks), idesc_s, ks > 0 ? 1u : 0u, e);
+          umma_ss(tS0 + st * BKV, desc_at(q_desc, kmajor_off(HALF_BYTES, ks)), desc_at(k_desc, st * KV_TILE + kmajor_off(KV_HALF, ks)), idesc_s, ks > 0 ? 1u : 0u, e);
         umma_commit(&bars->k_empty[st], e);
         umma_commit(&bars->s_full[st], e);
         return true;
@@ -122,7 +124,7 @@ flash_fwd64_t_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         tc_fence_after();
 #pragma unroll
         for (int ks = 0; ks < BKV / 16; ++ks)
-          umma_ts(tO, tS0 + st * BKV + ks * 8, kv_desc_mnmajor(v_base + st * KV_TILE, ks), idesc_pv, (j > 0 || ks > 0) ? 1u : 0u, e);
+          umma_ts(tO, tS0 + st * BKV + ks * 8, desc_at(v_mn, st * KV_TILE + mnmajor_off(ks)), idesc_pv, (j > 0 || ks > 0) ? 1u : 0u, e);
         umma_commit(&bars->v_empty[st], e);
         umma_commit(&bars->o_done[st], e);
       }
@@ -196,16 +198,18 @@ flash_fwd64_t_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     if (ok && mbar_wait(&bars->acc_done, 0, abort_flag, p.status, 4)) {
       tc_fence_after();
       const float inv = 1.f / l;
-      const bool row_ok = q_idx < p.S;
-      __nv_bfloat16* op = reinterpret_cast<__nv_bfloat16*>(p.o) + (static_cast<long long>(b) * p.S + q_idx) * p.ld_o + h * p.hd;
+      const int row0 = qb * AT + (warp & 3) * 32;
+      uint8_t* stage = smem + (warp & 3) * (NH * 4096);    // over Q: every product has been computed
 #pragma unroll 1
       for (int c = 0; c < 2 * NH; ++c) {
         uint32_t v[32];
         tmem_ld32(tO + lane_off + c * 32, v);
         tmem_ld_wait();
-        if (row_ok) store_head32(op, c * 32, p.hd, v, inv);
+        stage_head32<8 * NH>(stage, lane, c, v, inv);
       }
-      if (row_ok) p.lse[(static_cast<long long>(b) * p.Hq + h) * p.S + q_idx] = m_used + log2f(l);   // base-2 log-sum-exp of the scaled scores
+      store_staged<8 * NH>(reinterpret_cast<__nv_bfloat16*>(p.o) + (static_cast<long long>(b) * p.S + row0) * p.ld_o + h * p.hd,
+                           p.ld_o, stage, lane, p.S - row0, p.hd);
+      if (q_idx < p.S) p.lse[(static_cast<long long>(b) * p.Hq + h) * p.S + q_idx] = m_used + log2f(l);   // base-2 log-sum-exp of the scaled scores
     }
   }
   tc_fence_before();

@@ -184,7 +184,7 @@ __device__ __forceinline__ void slab_bf16(uint32_t t_slab, uint8_t* my_row, int 
       for (int t = 0; t < 4; ++t) {
         float f0 = alpha * __uint_as_float(v[8 * q + 2 * t]);
         float f1 = alpha * __uint_as_float(v[8 * q + 2 * t + 1]);
-        if (round_acc) { f0 = round_bf16(f0); f1 = round_bf16(f1); }
+        if (round_acc) round_bf16x2(f0, f1);
         o[t] = pack_bf16x2(f0 + beta * bf16_lo(ew[t]), f1 + beta * bf16_hi(ew[t]));
       }
       *cell = make_uint4(o[0], o[1], o[2], o[3]);

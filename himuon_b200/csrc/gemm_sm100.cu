@@ -317,7 +317,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                 const uint32_t ew4[4] = {e.x, e.y, e.z, e.w};
                 if (p.round_acc) {
 #pragma unroll
-                  for (int t = 0; t < 8; ++t) f[t] = round_bf16(f[t]);
+                  for (int t = 0; t < 8; t += 2) round_bf16x2(f[t], f[t + 1]);
                 }
 #pragma unroll
                 for (int t = 0; t < 4; ++t) {

@@ -93,8 +93,11 @@ rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __r
       const uint32_t k[4] = {ww.x, ww.y, ww.z, ww.w};
       uint32_t o[4];
 #pragma unroll
-      for (int q = 0; q < 4; ++q)
-        o[q] = pack_bf16x2(round_bf16(bf16_lo(u[q]) * rs) * bf16_lo(k[q]), round_bf16(bf16_hi(u[q]) * rs) * bf16_hi(k[q]));
+      for (int q = 0; q < 4; ++q) {
+        float f0 = bf16_lo(u[q]) * rs, f1 = bf16_hi(u[q]) * rs;
+        round_bf16x2(f0, f1);
+        o[q] = pack_bf16x2(f0 * bf16_lo(k[q]), f1 * bf16_hi(k[q]));
+      }
       yr[i] = make_uint4(o[0], o[1], o[2], o[3]);
     }
   }
@@ -558,7 +561,8 @@ swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gate, const __nv_bfloat16* _
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
       const float g0 = bf16_lo(gw[q]), g1 = bf16_hi(gw[q]);
-      const float s0 = round_bf16(g0 / (1.f + __expf(-g0))), s1 = round_bf16(g1 / (1.f + __expf(-g1)));
+      float s0 = g0 / (1.f + __expf(-g0)), s1 = g1 / (1.f + __expf(-g1));
+      round_bf16x2(s0, s1);
       o[q] = pack_bf16x2(s0 * bf16_lo(uw[q]), s1 * bf16_hi(uw[q]));
     }
     *reinterpret_cast<uint4*>(out + r * ld_o + c) = make_uint4(o[0], o[1], o[2], o[3]);

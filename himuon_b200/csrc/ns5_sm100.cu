@@ -208,9 +208,11 @@ ns5_fused_kernel(const __grid_constant__ CUtensorMap tmX, __nv_bfloat16* __restr
           const uint32_t xw[4] = {xv.x, xv.y, xv.z, xv.w};
           uint32_t o[4];
 #pragma unroll
-          for (int t = 0; t < 4; ++t)
-            o[t] = pack_bf16x2(round_bf16(__uint_as_float(v[8 * q + 2 * t])) + ca * bf16_lo(xw[t]),
-                               round_bf16(__uint_as_float(v[8 * q + 2 * t + 1])) + ca * bf16_hi(xw[t]));
+          for (int t = 0; t < 4; ++t) {
+            float f0 = __uint_as_float(v[8 * q + 2 * t]), f1 = __uint_as_float(v[8 * q + 2 * t + 1]);
+            round_bf16x2(f0, f1);
+            o[t] = pack_bf16x2(f0 + ca * bf16_lo(xw[t]), f1 + ca * bf16_hi(xw[t]));
+          }
           *ptr = make_uint4(o[0], o[1], o[2], o[3]);
         }
       }

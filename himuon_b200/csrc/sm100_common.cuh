@@ -364,5 +364,12 @@ __device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
 __device__ __forceinline__ float bf16_lo(uint32_t v) { return __uint_as_float(v << 16); }
 __device__ __forceinline__ float bf16_hi(uint32_t v) { return __uint_as_float(v & 0xFFFF0000u); }
 __device__ __forceinline__ float round_bf16(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
+// Two at a time, for what a kernel does to every element: a conversion of one value runs at an eighth of the rate.
+// (32 Newton-Schulz chains of fifteen 128 x 128 products, ns5_sm100.cu: 22.5 -> 19.0 us.)
+__device__ __forceinline__ void round_bf16x2(float& a, float& b) {
+  const uint32_t r = pack_bf16x2(a, b);
+  a = bf16_lo(r);
+  b = bf16_hi(r);
+}
 
 }  // namespace himuon

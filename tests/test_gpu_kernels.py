@@ -467,6 +467,35 @@ def test_attention_narrow_heads(D, B, S, Hq, Hkv):
             _close(t.grad, r.grad.reshape(t.shape), atol=3e-2, rtol=3e-2)
 
 
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("tokens,H", [(1, 2), (37, 3), (74, 4), (37, 6), (1998, 8), (999, 10)])
+def test_head_norm_rope_heads_taken_together_match_one_by_one(tokens, H, D):
+    """The kernels take up to four heads of a token per pass; a head's values have the same bits as when it is the only one."""
+    from himuon_b200.ops import reference as ref
+
+    e = _ext()
+    torch.manual_seed(5)
+    S = 37 if tokens % 37 == 0 else 1
+    x, dy = (torch.randn(tokens, H, D, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+    w = (1 + 0.1 * torch.randn(D, device="cuda")).bfloat16()
+    cs = ref.rope_tables(S, D, 1e4, device="cuda")
+
+    def run(x, dy, heads):
+        y, dx, rstd, dw = torch.empty_like(x), torch.empty_like(x), torch.empty(tokens, heads, device="cuda"), torch.zeros(D, device="cuda")
+        e.headnorm_rope_fwd(x, w, y, rstd, cs, heads, S, 1e-6)
+        e.headnorm_rope_bwd(dy, x, w, rstd, dx, dw, cs, heads, S)
+        return y, dx, rstd, dw
+
+    y, dx, rstd, dw = run(x.view(tokens, H * D), dy.view(tokens, H * D), H)
+    alone = [run(x[:, h].contiguous(), dy[:, h].contiguous(), 1) for h in range(H)]
+    assert torch.equal(y.view(tokens, H, D), torch.stack([a[0] for a in alone], 1))
+    assert torch.equal(dx.view(tokens, H, D), torch.stack([a[1] for a in alone], 1))
+    assert torch.equal(rstd, torch.cat([a[2] for a in alone], 1))
+    # fp32 sums of tokens * H terms in another order: 2^-24 times the number of additions times the sum of magnitudes bounds it;
+    # terms here are below 32, and the order of the atomics varies from run to run
+    torch.testing.assert_close(dw, torch.stack([a[3] for a in alone]).sum(0), atol=32 * tokens * H * 2.0 ** -24 * 64, rtol=1e-4)
+
+
 @pytest.mark.parametrize("use_norm", [True, False])
 @pytest.mark.parametrize("aligned", [True, False])
 def test_head_norm_rope_64(use_norm, aligned):

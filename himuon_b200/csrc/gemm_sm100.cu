@@ -10,7 +10,8 @@
 // Why two groups: a 128 x 256 x 512 tile (Newton-Schulz on 512 tiles) is 3 us of MMA, and one group of four warps
 // needed 6.6 us to drain it - the epilogue, not the main loop, bound every short-K product.
 // Measured with two: optimizer step on 2300 tiles of 512 15.1 -> 12.8 ms, on 28 of them 346 -> 287 us, 128 tiles through
-// newton_schulz 853 -> 756 us.
+// newton_schulz 853 -> 756 us, when tiles of 512 ran here; ns_pair_sm100.cu takes them now (475 us), and the products of larger
+// tiles and of layers keep this epilogue.
 //
 // Either operand may be K-major (reduction dim contiguous) or MN-major (M/N contiguous),
 // so forward (x W^T), dgrad (dy W) and wgrad (dy^T x) all run without a transpose pass.
@@ -475,6 +476,7 @@ static long long tile_count(const GemmArgs& a, int bn) {
 // and the step that holds them took 4.5 % longer.  Narrow tiles win where the wide ones do not fill the chip (6 matrices of
 // 333 x 500: 211 -> 179 us for the whole newton_schulz call) or just overflow it (symmetric products of 28 tiles of 512: 168 wide
 // tiles are two rounds, 280 narrow ones two rounds of half the length; the optimizer step went from 277 to 250 us).
+// Tiles up to 512 have since gone to ns_pair_sm100.cu; the figures are of the GEMM launches, which shapes it declines still take.
 constexpr double kNarrowRound = 0.7;
 static long long rounds(long long tiles, long long slots) { return (tiles + slots - 1) / slots; }
 static int tile_width(const GemmArgs& a) {

@@ -287,7 +287,8 @@ flash_bwd_dq_t_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   uint8_t* sDO = smem + TILE_BYTES;
   uint8_t* sK = smem + 2 * TILE_BYTES;                 // NST x 16 KB
   uint8_t* sV = sK + NST * Q_TILE;                     // NST x 16 KB
-  DqBars* bars = reinterpret_cast<DqBars*>(sV + NST * Q_TILE);
+  uint8_t* sTerm = sV + NST * Q_TILE;                  // what delta is summed from, 16 bytes for each 8 columns of a row
+  DqBars* bars = reinterpret_cast<DqBars*>(sTerm + TILE_BYTES);
   volatile int* abort_flag = &bars->abort_flag;
 
   const int warp = warp_id(), lane = threadIdx.x & 31;
@@ -323,6 +324,9 @@ flash_bwd_dq_t_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   }
   // delta = sum over the head of o * dO.  The 16 warps take 8 rows of o each, LPR lanes to a row, and find dO in shared memory
   // later.  One thread to a row, reading both rows 16 bytes at a time, took 9000 of the 50000 cycles of the longest block.
+  // What one thread to a row still does is the sum, from shared memory: pairs of columns, first to last, so that delta is the
+  // same for every split of the loads.  (Summed over the lanes instead, its last bit moved one dS in some thousand across a
+  // bf16 boundary.)
   constexpr int LPR = 8 * NH, PASSES = LPR / 4;
   uint4 o4[PASSES];
   if (warp >= 2) {
@@ -395,17 +399,23 @@ flash_bwd_dq_t_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       const int r = (warp - 2) * 8 + (i * 32 + lane) / LPR, c = lane % LPR;
       const uint4 g4 = *reinterpret_cast<const uint4*>(sDO + (c >> 3) * HALF_BYTES + r * 128 + (((c & 7) ^ (r & 7)) << 4));
       const uint32_t ow[4] = {o4[i].x, o4[i].y, o4[i].z, o4[i].w}, gw[4] = {g4.x, g4.y, g4.z, g4.w};
+      float t[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) t[q] = bf16_lo(ow[q]) * bf16_lo(gw[q]) + bf16_hi(ow[q]) * bf16_hi(gw[q]);
+      *reinterpret_cast<float4*>(sTerm + staged_at<LPR>(r, c)) = make_float4(t[0], t[1], t[2], t[3]);
+    }
+    named_barrier(1, 512);                                // all groups: the terms are in shared memory
+    if (wg == 0) {
       float d = 0.f;
 #pragma unroll
-      for (int q = 0; q < 4; ++q) d += bf16_lo(ow[q]) * bf16_lo(gw[q]) + bf16_hi(ow[q]) * bf16_hi(gw[q]);
-#pragma unroll
-      for (int m = LPR / 2; m > 0; m >>= 1) d += __shfl_xor_sync(0xffffffffu, d, m);
-      if (lane % LPR == 0) {
-        bars->delta[r] = d;
-        if (qb * AT + r < p.S) p.delta[(static_cast<long long>(b) * p.Hq + h) * p.S + qb * AT + r] = d;
+      for (int c = 0; c < LPR; ++c) {
+        const float4 t = *reinterpret_cast<const float4*>(sTerm + staged_at<LPR>(row, c));
+        d += t.x; d += t.y; d += t.z; d += t.w;
       }
+      bars->delta[row] = d;
+      if (row_ok) p.delta[stat_idx] = d;
     }
-    named_barrier(1, 512);                                // all groups: the block's delta values are in shared memory
+    named_barrier(1, 512);                                // and the block's delta values
     const float delta = bars->delta[row];
     const f32x2 nscale = pack2(-p.scale_log2, -p.scale_log2), lse_2 = pack2(lse2, lse2), ndelta = pack2(-delta, -delta);
     for (int j = buf; ok && j < nkv; j += 2) {
@@ -482,7 +492,8 @@ void flash_bwd_dkv_t(const AttnArgs& a, const AttnDev& p, int heads_y, cudaStrea
 
 template <int NH>
 static void launch_dq_t(const AttnArgs& a, const AttnDev& p, cudaStream_t s) {
-  constexpr size_t SMEM = 1024 + 2 * NH * HALF_BYTES + 2 * NST * NH * Q_HALF + sizeof(DqBars) + 64;
+  constexpr size_t SMEM = 1024 + 3 * NH * HALF_BYTES + 2 * NST * NH * Q_HALF + sizeof(DqBars) + 64;
+  static_assert(SMEM <= 232448, "shared memory budget of one CTA exceeded");
   static bool attr = false;
   if (!attr) { cudaFuncSetAttribute(flash_bwd_dq_t_kernel<NH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM); attr = true; }
   const CUtensorMap tq = head_tmap(a.q, a.B, a.S, a.Hq, a.hd, a.ld_q), tk = head_tmap(a.k, a.B, a.S, a.Hkv, a.hd, a.ld_k, BQ),

@@ -467,6 +467,28 @@ def test_attention_narrow_heads(D, B, S, Hq, Hkv):
             _close(t.grad, r.grad.reshape(t.shape), atol=3e-2, rtol=3e-2)
 
 
+@pytest.mark.parametrize("D", [8, 40, 64, 72, 128])
+@pytest.mark.parametrize("B,S,Hq,Hkv", [(1, 1, 1, 1), (2, 64, 2, 2), (1, 129, 4, 2), (2, 333, 2, 1)])
+def test_attention_backward_sums_delta_in_column_order(D, B, S, Hq, Hkv):
+    """delta = sum of o * dO over a head: pairs of columns, each rounded once, added first to last in fp32.  The score gradients
+    are rounded to bf16 after it is subtracted, so its last bit shows in dQ and dK: the order is part of the result."""
+    e = _ext()
+    torch.manual_seed(3)
+    bf = dict(device="cuda", dtype=torch.bfloat16)
+    q, k, v, do = (torch.randn(B * S, h * D, **bf) for h in (Hq, Hkv, Hkv, Hq))
+    o, dq, dk, dv = torch.empty_like(q), torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
+    lse, delta = torch.empty(B * Hq * S, device="cuda"), torch.full((B * Hq * S,), float("nan"), device="cuda")
+    part = torch.empty(2, B * S, Hq * D, **bf) if Hq != Hkv else None
+    e.flash_attn_fwd(q, k, v, o, lse, B, S, Hq, Hkv, D ** -0.5)
+    e.flash_attn_bwd(do, q, k, v, o, lse, dq, dk, dv, delta, part, B, S, Hq, Hkv, D ** -0.5)
+    _assert_status_clean()
+    term = (o.float() * do.float()).view(B, S, Hq, D // 2, 2).sum(-1)      # products of two bf16 values are exact in fp32
+    want = torch.zeros(B, S, Hq, device="cuda")
+    for c in range(D // 2):
+        want = want + term[..., c]
+    assert torch.equal(delta.view(B, Hq, S), want.transpose(1, 2))
+
+
 @pytest.mark.parametrize("D", [64, 128])
 @pytest.mark.parametrize("tokens,H", [(1, 2), (37, 3), (74, 4), (37, 6), (1998, 8), (999, 10)])
 def test_head_norm_rope_heads_taken_together_match_one_by_one(tokens, H, D):

@@ -337,6 +337,9 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         py::arg("dw_accum"), py::arg("dres") = py::none());
   m.def("headnorm_rope_fwd", &headnorm_rope_fwd);
   m.def("headnorm_rope_bwd", &headnorm_rope_bwd);
+  m.def("headnorm_heads_per_pass", [](int64_t tokens, int64_t heads, int64_t head_dim, bool backward) {
+    return himuon::headnorm_heads_per_pass(tokens * heads, (int)heads, (int)head_dim, backward);
+  });
   m.def("swiglu_fwd", &swiglu_fwd);
   m.def("swiglu_bwd", &swiglu_bwd);
   m.def("embedding_fwd", &embedding_fwd);

@@ -124,6 +124,8 @@ void headnorm_rope_fwd(const void* x, const void* w, void* y, float* rstd, const
 void headnorm_rope_bwd(const void* dy, const void* x, const void* w, const float* rstd, void* dx, float* dw_accum,
                        const float* cos_sin, int tokens, int heads, int hd, int seq_len, long long ld_dy, long long ld_x,
                        long long ld_dx, int use_norm, cudaStream_t s);
+// Heads of one token that a group of lanes takes per pass (n_vec = tokens * heads).
+int headnorm_heads_per_pass(long long n_vec, int heads, int hd, bool backward);
 void swiglu_fwd(const void* gate, const void* up, void* out, long long rows, int cols, long long ld_g, long long ld_u,
                 long long ld_o, cudaStream_t s);
 void swiglu_bwd(const void* dout, const void* gate, const void* up, void* dgate, void* dup, long long rows, int cols,

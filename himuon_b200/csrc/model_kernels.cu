@@ -363,8 +363,8 @@ void rmsnorm_bwd(const void* dy, const void* x, const void* w, const float* rstd
 //   y[i+h]    = xn[i+h]*cos[i] + xn[i]*sin[i]
 // Layout of the two kernels below: LN = D/8 lanes per head vector, lane l owning elements [8l, 8l+8) (one 16-byte
 // access); the lower LN/2 lanes hold the first half, the others the second half, so the rotation partner of every
-// element sits at the same register index in lane l^(LN/2).  LN lanes take HU heads of one token per pass, the most of 4, 2
-// and 1 that the head count is a multiple of: their loads are in flight together, and the token's angles, 64 bytes a lane
+// element sits at the same register index in lane l^(LN/2).  LN lanes take HU heads of one token per pass (4, 2 or 1, see
+// headnorm_heads_per_pass): their loads are in flight together, and the token's angles, 64 bytes a lane
 // against 16 of a head, are fetched once for all of them.  With one vector per pass the kernels waited for memory: 8192 tokens,
 // 16 and 8 heads of 128, mean of both, forward 21.3 -> 15.7 us (14.0 with paired conversions), backward 25.1 -> 19.5; 2048 tokens,
 // 32 and 8 heads, 12.6 -> 9.0 (7.8) and 14.9 -> 11.8; 4096 tokens, 10 heads of 64, forward 6.4 -> 4.3.
@@ -545,14 +545,24 @@ headnorm_rope_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat
   }
 }
 
-static int heads_per_pass(int heads) { return heads % 4 == 0 ? 4 : heads % 2 == 0 ? 2 : 1; }
+// Several heads per pass pay once the launch keeps most SMs busy all the same; below that a pass of four only lengthens the
+// kernel's one round.  Heads of 128, one / several per pass, us: 4 heads, 256 tokens forward 2.5 / 2.9, backward 2.8 / 3.4; 1024
+// tokens 2.9 / 3.0 and 3.5 / 3.4; 2048 tokens 3.7 / 3.0 and 5.3 / 3.7; two at a time 2 heads, 1024 tokens 2.5 / 2.5 and
+// 3.0 / 2.9; 10 heads, 256 tokens 2.8 / 2.5 and 3.2 / 3.0; 2 heads, 2048 tokens 2.8 / 2.6 and 3.7 / 3.2.  The backward kernel
+// takes one 64-wide head per pass: the registers of several would cost blocks in flight (4096 tokens, 10 heads: 5.0 us, 6.4
+// with two).
+int headnorm_heads_per_pass(long long n_vec, int heads, int hd, bool backward) {
+  const long long blocks = n_vec * hd / (8 * 256);         // of one vector per pass
+  if (backward && hd == 64) return 1;
+  return heads % 4 == 0 && blocks >= 512 ? 4 : heads % 2 == 0 && blocks >= 160 ? 2 : 1;
+}
 void headnorm_rope_fwd(const void* x, const void* w, void* y, float* rstd, const float* cos_sin, int tokens, int heads,
                        int hd, int seq_len, long long ld_in, long long ld_out, float eps, int use_norm, cudaStream_t s) {
   const long long n_vec = static_cast<long long>(tokens) * heads;
   if (n_vec <= 0) return;
   if (n_vec >= (1LL << 31)) throw std::runtime_error("himuon headnorm_rope: too many head vectors for one launch");
   if (hd != 128 && hd != 64) throw std::runtime_error("himuon headnorm_rope: head_dim must be 64 or 128");
-  const int per_block = hd == 64 ? 32 : 16, hu = heads_per_pass(heads);
+  const int per_block = hd == 64 ? 32 : 16, hu = headnorm_heads_per_pass(n_vec, heads, hd, false);
   const long long n_task = n_vec / hu, blocks = (n_task + per_block - 1) / per_block;
   const int grid = static_cast<int>(blocks < num_sms() * 8 ? blocks : num_sms() * 8);
   auto kern = hd == 64 ? (hu == 4 ? headnorm_rope_fwd_kernel<8, 4> : hu == 2 ? headnorm_rope_fwd_kernel<8, 2> : headnorm_rope_fwd_kernel<8, 1>)
@@ -568,8 +578,7 @@ void headnorm_rope_bwd(const void* dy, const void* x, const void* w, const float
   if (n_vec <= 0) return;
   if (n_vec >= (1LL << 31)) throw std::runtime_error("himuon headnorm_rope: too many head vectors for one launch");
   if (hd != 128 && hd != 64) throw std::runtime_error("himuon headnorm_rope: head_dim must be 64 or 128");
-  // One 64-wide head per pass: the registers of several would cost blocks in flight (4096 tokens, 10 heads: 5.0 us, 6.4 with two).
-  const int per_block = hd == 64 ? 32 : 16, hu = hd == 64 ? 1 : heads_per_pass(heads);
+  const int per_block = hd == 64 ? 32 : 16, hu = headnorm_heads_per_pass(n_vec, heads, hd, true);
   const long long n_task = n_vec / hu, blocks = (n_task + per_block - 1) / per_block;
   const int grid = static_cast<int>(blocks < num_sms() * 4 ? blocks : num_sms() * 4);
   auto kern = hd == 64 ? headnorm_rope_bwd_kernel<8, 1>

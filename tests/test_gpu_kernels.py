@@ -490,7 +490,8 @@ def test_attention_backward_sums_delta_in_column_order(D, B, S, Hq, Hkv):
 
 
 @pytest.mark.parametrize("D", [64, 128])
-@pytest.mark.parametrize("tokens,H", [(1, 2), (37, 3), (74, 4), (37, 6), (1998, 8), (999, 10)])
+@pytest.mark.parametrize("tokens,H", [(1, 2), (37, 3), (74, 4), (37, 6), (1998, 8), (999, 10), (2047, 4), (2048, 4), (4096, 4),
+                                      (1279, 2), (1280, 2), (2560, 2)])
 def test_head_norm_rope_heads_taken_together_match_one_by_one(tokens, H, D):
     """The kernels take up to four heads of a token per pass; a head's values have the same bits as when it is the only one."""
     from himuon_b200.ops import reference as ref
@@ -516,6 +517,18 @@ def test_head_norm_rope_heads_taken_together_match_one_by_one(tokens, H, D):
     # fp32 sums of tokens * H terms in another order: 2^-24 times the number of additions times the sum of magnitudes bounds it;
     # terms here are below 32, and the order of the atomics varies from run to run
     torch.testing.assert_close(dw, torch.stack([a[3] for a in alone]).sum(0), atol=32 * tokens * H * 2.0 ** -24 * 64, rtol=1e-4)
+
+
+def test_head_norm_rope_takes_heads_together_only_where_the_chip_stays_busy():
+    """Few vectors go one by one: a pass of four heads would only make their one round of blocks longer."""
+    rule = _ext().headnorm_heads_per_pass
+    for D, lanes in ((64, 8), (128, 16)):
+        four, two = 512 * 256 // lanes, 160 * 256 // lanes          # vectors
+        assert [rule(t // 4, 4, D, False) for t in (4, 1024, two - 4, two, four - 4, four, 1 << 20)] == [1, 1, 1, 2, 2, 4, 4]
+        assert [rule(t // 2, 2, D, False) for t in (2, two - 2, two, 1 << 20)] == [1, 1, 2, 2]
+        assert rule(1 << 20, 3, D, False) == 1
+    assert [rule(t, 4, 128, True) for t in (16, 1024, 2048, 1 << 18)] == [1, 2, 4, 4]
+    assert rule(1 << 18, 4, 64, True) == 1
 
 
 @pytest.mark.parametrize("use_norm", [True, False])

@@ -17,14 +17,13 @@ static bool is_bf16(const at::Tensor& t) { return t.scalar_type() == at::kBFloat
 static bool is_f32(const at::Tensor& t) { return t.scalar_type() == at::kFloat; }
 
 // out = alpha * op(a) @ op(b) + beta * aux.   a: (.., M, K) or (.., K, M) when trans_a; b: (.., K, N) or (.., N, K) when trans_b.
-static void gemm(const at::Tensor& a, const at::Tensor& b, at::Tensor& out, const c10::optional<at::Tensor>& aux,
-                 bool trans_a, bool trans_b, double alpha, double beta, bool round_acc, int64_t max_ctas,
-                 bool symmetric) {
+static GemmArgs gemm_args(const at::Tensor& a, const at::Tensor& b, const at::Tensor& out, const c10::optional<at::Tensor>& aux,
+                          bool trans_a, bool trans_b, double alpha, double beta, bool round_acc, int64_t max_ctas,
+                          bool symmetric) {
   HM_CHECK(a.is_cuda() && b.is_cuda() && out.is_cuda(), "gemm operands must be CUDA tensors");
   HM_CHECK(is_bf16(a) && is_bf16(b), "gemm operands must be bf16");
   HM_CHECK(is_bf16(out) || is_f32(out), "gemm output must be bf16 or fp32");
   HM_CHECK(a.dim() == b.dim() && a.dim() == out.dim() && (a.dim() == 2 || a.dim() == 3), "gemm takes 2-D or 3-D operands");
-  const c10::cuda::CUDAGuard guard(a.device());
   const int nd = a.dim();
   GemmArgs g;
   g.batch = nd == 3 ? static_cast<int>(a.size(0)) : 1;
@@ -58,7 +57,22 @@ static void gemm(const at::Tensor& a, const at::Tensor& b, at::Tensor& out, cons
     HM_CHECK(x.size(nd - 2) == g.M && x.size(nd - 1) == g.N && (nd == 2 || x.size(0) >= g.batch), "gemm aux has the wrong shape");
     g.aux = x.data_ptr(); g.ldaux = x.stride(nd - 2); g.strideAux = nd == 3 ? x.stride(0) : 0;
   }
+  return g;
+}
+static void gemm(const at::Tensor& a, const at::Tensor& b, at::Tensor& out, const c10::optional<at::Tensor>& aux,
+                 bool trans_a, bool trans_b, double alpha, double beta, bool round_acc, int64_t max_ctas,
+                 bool symmetric) {
+  const GemmArgs g = gemm_args(a, b, out, aux, trans_a, trans_b, alpha, beta, round_acc, max_ctas, symmetric);
+  const c10::cuda::CUDAGuard guard(a.device());
   himuon::gemm_bf16(g, cur_stream());
+}
+// Whether gemm() with these arguments runs on CTA pairs.
+static bool gemm_on_pairs(const at::Tensor& a, const at::Tensor& b, const at::Tensor& out, const c10::optional<at::Tensor>& aux,
+                          bool trans_a, bool trans_b, double alpha, double beta, bool round_acc, int64_t max_ctas,
+                          bool symmetric) {
+  const GemmArgs g = gemm_args(a, b, out, aux, trans_a, trans_b, alpha, beta, round_acc, max_ctas, symmetric);
+  const c10::cuda::CUDAGuard guard(a.device());
+  return himuon::gemm2_supported(g);
 }
 
 static void momentum_tile(const at::Tensor& entries, int64_t n_entries, int64_t total_units, int64_t Th, int64_t Tw,
@@ -322,6 +336,9 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("soap_moments", &soap_moments);
   m.def("soap_ratio", &soap_ratio);
   m.def("gemm", &gemm, py::arg("a"), py::arg("b"), py::arg("out"), py::arg("aux") = py::none(), py::arg("trans_a") = false,
+        py::arg("trans_b") = false, py::arg("alpha") = 1.0, py::arg("beta") = 0.0, py::arg("round_acc") = false,
+        py::arg("max_ctas") = 0, py::arg("symmetric") = false);
+  m.def("gemm_on_pairs", &gemm_on_pairs, py::arg("a"), py::arg("b"), py::arg("out"), py::arg("aux") = py::none(), py::arg("trans_a") = false,
         py::arg("trans_b") = false, py::arg("alpha") = 1.0, py::arg("beta") = 0.0, py::arg("round_acc") = false,
         py::arg("max_ctas") = 0, py::arg("symmetric") = false);
   m.def("momentum_tile", &momentum_tile);

@@ -373,20 +373,46 @@ static void launch_gemm2(const GemmArgs& a, cudaStream_t stream) {
   }
 }
 
+// Whether the pair kernel is the faster one.  Reductions of 2048 or more always are its own.  Symmetric products of shorter
+// ones stay with the one-CTA kernel, which computes one triangle of them.  For the others the rounds of tiles decide that the
+// two kernels need, 128 x 256 over the SMs and 256 x 256 over the pairs (`nt` products unless said, one-CTA / pair, us):
+//   * Where 128-wide tiles fit in one round, the one-CTA kernel spreads over more SMs: 320 x 5120 x 512 8.6 / 9.1, 12 of
+//     384 x 384 x 512 8.6 / 9.3.
+//   * Padding can cost the pairs a round: 384 x 12288 (one round of 144 tiles, two of 96) x 640 11.3 / 12.9, x 1728 17.5 / 23.0;
+//     777 x 5120 x 1024 13.4 / 16.2; 40 of 320 x 320 x 1024 (two rounds, three) 18.8 / 21.1.  Without aux values and with rows of
+//     A along K a fourth more rounds are made up for: 100 of 264 x 264 (five, six) 0.87-0.93 of the one-CTA time.
+//   * The longer a round, the less the pair kernel's epilogue matters.  It reads aux values by threads where the other has them
+//     loaded by TMA ahead of time, and an fp32 tile leaves in twice as many slabs.  Plain bf16 products gain from K = 512 on
+//     (one round 0.92-0.97, several 0.78-0.90 of the one-CTA time).  Two rounds / four rounds, ratio: bf16 with aux K 768
+//     1.06 / 1.03, 1024 0.98 / 0.93, 1280 0.92 / 0.86; fp32 512 1.09 / 1.03, 768 1.02 / 0.90, 1024 0.95 / 0.83; fp32 added to C 1024
+//     1.09 / 1.09, 1280 1.08 / 1.02, 1536 1.04 / 0.95.  In one round all of these are slower until 1984 (1.02-1.45).  `slack`
+//     below draws these lines: the reduction that pays for the epilogue is the longer the fewer rounds there are.
+//   * Operand rows that start off the 32-byte grid of memory sectors cost the loads more, and the pair loads B once for two CTAs.
+//     1024 x 3072 in one round, ratio: plain K 520 0.86, 1544 0.79; with aux 520 1.03, 648 0.99, 1032 0.94; added to fp32 C 520 0.99,
+//     1032 0.94 (1728 x 2560 1.05, 1.01).  With only A's rows off it (`nn`) the lines move half as far: 1000 x 6144 (two rounds) with
+//     aux 776 0.98, fp32 648 0.96.
+static bool pairs_win(const GemmArgs& a) {
+  if (a.K >= 2048) return true;
+  if (a.K < 512 || a.symmetric) return false;
+  const long long sms = a.max_ctas > 0 ? a.max_ctas : num_sms();
+  auto rounds = [&](int bm, int bn, long long slots) {
+    return (static_cast<long long>((a.M + bm - 1) / bm) * ((a.N + bn - 1) / bn) * a.batch + slots - 1) / slots;
+  };
+  const long long wide = rounds(128, 256, sms), pairs = rounds(256, 256, sms > 1 ? sms / 2 : 1);
+  if (rounds(128, 128, sms) == 1 || pairs > (a.aux || a.a_mn ? wide : wide * 5 / 4)) return false;
+  const bool a_off = !a.a_mn && a.lda % 16 != 0, b_off = !a.b_mn && a.ldb % 16 != 0;
+  if (a_off && b_off) return a.K >= (!a.aux ? 512 : a.out_fp32 ? 1024 : 640);
+  if ((wide == 1 && (a.aux || a.out_fp32)) || (a.aux && a.K < 768)) return false;
+  const int slack = (a.out_fp32 ? (a.aux ? -1024 : -256) : (a.aux ? -512 : 1024)) + (a_off ? 512 : 0);
+  return (a.K + slack) * wide >= 1536;
+}
 // True when the pair kernel can run this problem and is expected to win: TMA-storable output (whole 16-byte groups of
-// columns: a TMA store writes those whole, past the output's last column if need be), more than one CTA tile of rows, and
-//   * a reduction of 2048 or more, or
-//   * one of 512 or more and enough 256 x 256 tiles to occupy half of the pairs.  Below that the one-CTA kernel's smaller tiles
-//     spread over more SMs (32 tiles, 512 x 4096 x 512: 13.3 us there, 15.4 here; 48 tiles, 4096 x 640 x 1728: 23.6 / 21.5; 80,
-//     4096 x 1280 x 640: 19.5 / 18.4; 384, 8192 x 3072 x 1024: 52.5 / 44.1; 4096 x 64128 x 640: 290 / 224).
-// Symmetric products of short reductions stay with the one-CTA kernel, which computes one triangle of them.
+// columns: a TMA store writes those whole, past the output's last column if need be) and more than one CTA tile of rows.
 bool gemm2_supported(const GemmArgs& a) {
   const int esz = a.out_fp32 ? 4 : 2;
   const int row_align = 16 / esz;
-  const long long tiles = static_cast<long long>((a.M + 255) / 256) * ((a.N + 255) / 256) * a.batch;
-  const bool long_enough = a.K >= 2048 || (a.K >= 512 && !a.symmetric && tiles >= 40);
-  return a.M > BM && a.N > 192 && a.N % row_align == 0 && long_enough && (a.ldc % row_align == 0) && (a.batch == 1 || a.strideC % row_align == 0) &&
-         (reinterpret_cast<uintptr_t>(a.C) % 16 == 0);
+  return a.M > BM && a.N > 192 && a.N % row_align == 0 && (a.ldc % row_align == 0) && (a.batch == 1 || a.strideC % row_align == 0) &&
+         (reinterpret_cast<uintptr_t>(a.C) % 16 == 0) && pairs_win(a);
 }
 
 void gemm2_bf16(const GemmArgs& a, cudaStream_t stream) {

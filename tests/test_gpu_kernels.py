@@ -1130,8 +1130,8 @@ def test_ns_pair_kernel_keeps_a_bad_matrix_to_itself():
     _assert_status_clean()
 
 
-# Reductions of 512 to 2047 on the pair kernel: the first and a ragged last length, 40 tiles (the fewest) and some rounds of
-# them, ragged rows and columns, every operand-major combination, and each epilogue form.
+# Reductions of 512 to 2047, plain and with every epilogue form, ragged rows and columns, every operand-major combination: the plain
+# products run on CTA pairs, the others on either kernel (test_pair_gemm_rule has the line between them).
 @pytest.mark.parametrize("M,N,K,batch", [(1281, 2048, 512, 1), (2056, 1288, 1096, 1), (328, 520, 2040, 8), (2560, 2560, 640, 1)])
 @pytest.mark.parametrize("trans_a,trans_b", [(False, True), (False, False), (True, True), (True, False)])
 @pytest.mark.parametrize("mode", ["plain", "aux", "add", "fp32"])
@@ -1164,3 +1164,56 @@ def test_pair_gemm_on_short_reductions(M, N, K, batch, trans_a, trans_b, mode):
     # fp32 sums of K products of unit normals differ by some 2^-24 of sqrt(K) per term in any order; a bf16 result adds half
     # an ulp, 2^-9 of the value
     _close(out, ref, atol=atol, rtol=1e-5 if mode == "fp32" else 2 ** -8)
+
+
+# mode, batch, M, N and the shortest reduction that goes to CTA pairs; 16 less does not.  One round of 128 x 256 tiles and
+# several, matrices that barely overflow one row of tiles, ragged rows and columns.
+_PAIR_LINES = [("plain", 1, 1281, 2048, 512), ("plain", 20, 136, 520, 512), ("plain", 100, 264, 264, 512),
+               ("aux", 1, 1281, 4104, 1280), ("aux", 8, 1000, 1032, 1024), ("add", 1, 1281, 4104, 1280), ("add", 8, 1000, 1032, 1024),
+               ("fp32", 1, 1281, 4104, 1024), ("fp32", 8, 1000, 1032, 768), ("fp32 add", 8, 1000, 1032, 1536),
+               ("add", 1, 1024, 3072, 648), ("fp32 add", 1, 1024, 3072, 1032)]
+
+
+def _pair_case(mode, batch, M, N, K, trans_a=False, trans_b=True):
+    g = torch.Generator("cuda").manual_seed(M + N + K)
+    a = torch.randn(batch, *((K, M) if trans_a else (M, K)), device="cuda", dtype=torch.bfloat16, generator=g)
+    b = torch.randn(batch, *((N, K) if trans_b else (K, N)), device="cuda", dtype=torch.bfloat16, generator=g)
+    out = torch.randn(batch, M, N, device="cuda", generator=g).to(torch.float32 if "fp32" in mode else torch.bfloat16)
+    aux = {"aux": lambda: torch.randn_like(out), "add": lambda: out, "fp32 add": lambda: out}.get(mode, lambda: None)()
+    beta = 0.0 if aux is None else 1.0 if aux is out else -2.0
+    return a, b, out, aux, trans_a, trans_b, 1.0 if beta == 1.0 else 0.5, beta, mode == "aux"
+
+
+@pytest.mark.parametrize("mode,batch,M,N,K", _PAIR_LINES)
+def test_pair_gemm_rule(mode, batch, M, N, K):
+    from himuon_b200 import ops
+
+    on_pairs = _ext().gemm_on_pairs
+    assert on_pairs(*_pair_case(mode, batch, M, N, K)) and not on_pairs(*_pair_case(mode, batch, M, N, K - 16))
+    assert on_pairs(*_pair_case(mode, batch, M, N, 2048))
+    for trans_a, trans_b in ((False, True), (False, False), (True, True), (True, False)):
+        if trans_a and M % 8:
+            continue                                       # the rows of a transposed operand are 16-byte aligned
+        a, b, out, aux, ta, tb, alpha, beta, round_acc = _pair_case(mode, batch, M, N, K, trans_a, trans_b)
+        parts = []
+        for r in range(0, M, 128):                         # rows of one tile at a time run on the one-CTA kernel
+            rows = a[:, :, r:r + 128].contiguous() if ta else a[:, r:r + 128]
+            part = out[:, r:r + 128].clone()
+            x = None if aux is None else part if aux is out else aux[:, r:r + 128]
+            assert not on_pairs(rows, b, part, x, ta, tb, alpha, beta, round_acc)
+            parts.append(ops.gemm(rows, b, trans_a=ta, trans_b=tb, alpha=alpha, beta=beta, aux=x, out=part, round_acc=round_acc))
+        ops.gemm(a, b, trans_a=ta, trans_b=tb, alpha=alpha, beta=beta, aux=aux, out=out, round_acc=round_acc)
+        _assert_status_clean()
+        assert torch.equal(out, torch.cat(parts, 1))       # the same products and sums, in the same order
+
+
+def test_pair_gemm_declines_where_padding_or_few_tiles_cost_a_round():
+    on_pairs = _ext().gemm_on_pairs
+    for batch, M, N, K in ((1, 320, 12288, 1728), (1, 257, 12288, 640), (1, 777, 5120, 1024), (40, 320, 320, 1024), (12, 384, 384, 512),
+                           (1, 320, 5120, 512), (10, 264, 264, 1536)):
+        assert not on_pairs(*_pair_case("plain", batch, M, N, K))
+    for mode in ("aux", "add", "fp32", "fp32 add"):          # one round of tiles, unless the operands' rows are off the sectors' grid
+        assert not on_pairs(*_pair_case(mode, 1, 1024, 3072, 1536)) and on_pairs(*_pair_case(mode, 1, 1024, 3072, 1544))
+        assert not on_pairs(*_pair_case(mode, 1, 1024, 3072, 1544, True, False))
+    assert on_pairs(*_pair_case("plain", 1, 1024, 3072, 512))
+    assert on_pairs(*_pair_case("plain", 100, 264, 264, 1024)) and not on_pairs(*_pair_case("plain", 100, 264, 264, 1024, True))

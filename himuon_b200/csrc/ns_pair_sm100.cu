@@ -548,18 +548,41 @@ static int nsp_max_clusters(int P) {
 }
 
 // Pairs per matrix and matrices interleaved per cluster, or false where the GEMM launches are the better path.
-//   * Short sides above 512 stay with the GEMMs: their reductions are long enough (1024 x 1024: 28 matrices 779 us there, 608
-//     here, but 4 of them 248 / 389).  So do more than 1024 columns in two blocks (one matrix of 512 x 2048 191 / 207), 2048
-//     in one.  Short sides up to 128 use half of a block's rows, so the GEMMs catch up with many matrices (16 x 512: 296
-//     matrices 216 / 208, 600 334 / 426; 64 x 2000: 74 224 / 194, 100 257 / 348).
+//   * Short sides above 512 stay with the GEMMs: 4 matrices of 1024 x 1024 took 248 us there, 389 here (28 of them 779 / 608, but no
+//     rule is drawn from one figure).  So do more than 1024 columns in two blocks (one matrix of 512 x 2048 191 / 207), 2048
+//     in one.  Short sides up to 128 use half of a block's rows, so the GEMMs catch up with many matrices.
 //   * As many pairs per matrix as all matrices at once leave, while they have work: 4 of 336 x 504 with 1, 2, 4 pairs 145,
 //     112, 107 us, of 256 x 1024 120, 101, 101, of 256 x 512 91, 85, 89, of 256 x 256 77, 80, 84.
 //   * One block per phase leaves nothing to hide the hand-on behind but other matrices: 396 of 256 x 256 interleaved by
 //     1, 2, 3, 4: 480, 381, 345, 309 us; with several blocks two are enough (296 of 256 x 512: 266 with two, 311 with four).
+//   * More matrices than pairs take whole rounds, where the GEMMs' time goes with the number: ns_rounds_pay.
+//   * One to four matrices that half-fill eight blocks: 384 x 1024 135 us there, 139 here (264 x 1024 139 / 135).
+// Below, time here / there, from one round of matrices (74) to four.
+static bool ns_rounds_pay(long long n_mats, int s, int l, bool tall, long long slots) {
+  const int nb = (s + 255) / 256, nc = (l + 255) / 256;
+  const long long rounds = (n_mats + slots - 1) / slots;
+  auto filled = [&](int percent) { return n_mats * 100 >= percent * rounds * slots; };
+  if (rounds == 1) return true;
+  if (s <= 128) {
+    if (n_mats > 4 * slots) return false;             // 64 x 2000: 100 matrices 257 / 348
+    // wide: 16 x 512 75-148 matrices 0.79-0.82, 150-296 1.04-1.10; 128 x 768 92 1.04, 100 0.95, 150-296 1.03-1.15; 16 x 1024
+    // 75-148 1.03-1.15.  The GEMMs are slower on tall ones: 512 x 128 150-296 0.92-0.99, 264 x 16 0.88-0.93, but 264 x 128 1.01-1.08;
+    // 768 x 128 185-296 0.92-0.97, 640 x 128 1.01-1.09, 1024 x 16 75-148 0.83-0.95, 150-260 0.99-1.08.
+    if (nc == 1) return true;
+    if (!tall) return rounds == 2 && (nc == 2 || (nc == 3 && filled(66)));
+    return rounds == 2 || (nc < 4 && (l * 10 >= nc * 2304 || (nc == 2 && s <= 64)));
+  }
+  if (nb == 1 || nc < 3) return true;                 // 256 x 2048 75 matrices 0.94; 384 x 512 75 1.00, 150 0.94
+  // Two block rows, the second up to half full: 264 x 768 75 matrices 1.11, 100 0.90, 150 1.01, 185 0.87, 223 0.91; 384 x 1024 75
+  // 1.20, 100 0.99, 150 1.17; 264 x 1024 165 1.06, 185 0.95; tall 768 x 264 75 0.94, 150 0.83, but 1024 x 384 92 1.11.  More than
+  // half: 512 x 1024 75 1.01, 84 0.97; 448 x 768 0.69-0.89.
+  if (s > 384) return nc == 3 || filled(54);
+  return (tall && s <= 288) || filled(rounds == 2 ? 66 : nc == 3 ? 72 : 80);
+}
 bool ns_pair_plan(long long n_mats, int m, int n, int* P, int* W) {
   const int s = m < n ? m : n, l = m < n ? n : m, nb = (s + 255) / 256, nc = (l + 255) / 256;
   if (n_mats <= 0 || m <= 0 || n <= 0 || m % 8 || n % 8 || nb > 2 || nc > (nb == 2 || s <= 128 ? 4 : 8)) return false;
-  if (s <= 128 && n_mats > 4LL * nsp_max_clusters(1)) return false;
+  if (!ns_rounds_pay(n_mats, s, l, m > n, nsp_max_clusters(1)) || (nc == 4 && nb == 2 && s > 288 && n_mats < 5)) return false;
   *P = n_mats <= nsp_max_clusters(4) && nb * nc >= 4 ? 4 : n_mats <= nsp_max_clusters(2) && nb * nc >= 2 ? 2 : 1;
   const long long each = (n_mats + nsp_max_clusters(1) - 1) / nsp_max_clusters(1), most = nc == 1 ? 4 : 2;
   *W = nb == 2 || *P > 1 ? 1 : static_cast<int>(each < most ? each : most);

@@ -1114,6 +1114,23 @@ def test_ns_pair_kernel_matches_the_gemms_bit_for_bit(shape, steps):
     assert (out[-1].float().cpu() - ref).norm() <= 0.03 * ref.norm()
 
 
+def test_ns_pair_plan_declines_rounds_that_do_not_pay():
+    """Matrices beyond the pairs take whole rounds; the lines lie between shapes measured slower and faster than the GEMMs."""
+    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("the shapes are those of 74 CTA pairs")
+
+    def taken(b, m, n):
+        return _ext().ns_pair_plan(torch.empty(b, m, n, device="cuda", dtype=torch.bfloat16)) is not None
+
+    for shape in [(160, 16, 512), (230, 128, 264), (80, 128, 768), (160, 128, 768), (80, 16, 1024), (300, 16, 264), (200, 264, 128),
+                  (150, 640, 128), (80, 264, 768), (80, 384, 1024), (150, 264, 1024), (1, 512, 1024), (4, 384, 1024), (75, 512, 1024)]:
+        assert not taken(*shape), shape
+    for shape in [(74, 16, 1024), (148, 16, 512), (100, 128, 768), (148, 1024, 16), (296, 512, 16), (296, 264, 64), (296, 256, 128), (296, 128, 200),
+                  (80, 264, 512), (100, 384, 1024), (185, 264, 768), (92, 768, 264), (1, 264, 1024), (5, 512, 1024), (84, 512, 1024),
+                  (75, 448, 768), (592, 256, 256), (80, 192, 2048)]:
+        assert taken(*shape), shape
+
+
 def test_ns_pair_kernel_keeps_a_bad_matrix_to_itself():
     from himuon_b200.ops import ns
 

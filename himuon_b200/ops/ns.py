@@ -31,11 +31,13 @@ EPS = 1e-7
 
 
 class NSWorkspace:
-    """Reusable scratch of the Newton-Schulz paths (keeps addresses stable for CUDA graphs)."""
+    """Reusable scratch of the Newton-Schulz paths (keeps addresses stable for CUDA graphs).  Matrices of one shape share a
+    scratch: calls that may overlap, on two streams, need a workspace each unless their shapes differ."""
 
     def __init__(self):
         self.bufs: dict[tuple, tuple[torch.Tensor, torch.Tensor, torch.Tensor]] = {}
-        self.flat: dict[str, list[torch.Tensor]] = {}      # last: the one in use; a captured graph may hold the others
+        self.flat: dict[tuple, torch.Tensor] = {}          # scratch of ns_pair
+        self.captured: dict[int, torch.Tensor] = {}        # by address: those of `flat` that a CUDA graph may replay on
 
     def get(self, B: int, m: int, n: int, device) -> tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
         k = min(m, n)
@@ -50,15 +52,20 @@ class NSWorkspace:
             self.bufs[key] = cur
         return cur[0][:B], cur[1][:B], cur[2][:B]
 
-    def scratch(self, nbytes: int, device) -> torch.Tensor:
-        have = self.flat.setdefault(str(device), [])
-        if not have or have[-1].numel() < nbytes:
-            have.append(torch.empty(nbytes, device=device, dtype=torch.uint8))
-        return have[-1]
+    def scratch(self, nbytes: int, m: int, n: int, device) -> torch.Tensor:
+        """At least `nbytes` for matrices of m x n.  A buffer that has become too small is given back, unless a graph holds it."""
+        key = (m, n, str(device))
+        cur = self.flat.get(key)
+        if cur is None or cur.numel() < nbytes:
+            cur = self.flat[key] = torch.empty(nbytes, device=device, dtype=torch.uint8)
+        if torch.cuda.is_current_stream_capturing():
+            self.captured[cur.data_ptr()] = cur
+        return cur
 
     def clear(self):
         self.bufs.clear()
         self.flat.clear()
+        self.captured.clear()
 
 
 def fused_supported(m: int, n: int) -> bool:
@@ -91,7 +98,7 @@ def ns_inplace_cuda(X: torch.Tensor, steps: int = 5, eps: float = EPS, workspace
         if normalize:
             e.ns_normalize(src, Bt, m * n, float(eps), X)
             _count()
-        e.ns_pair(X, X, ws.scratch(nbytes, X.device), int(steps), pairs, interleaved)
+        e.ns_pair(X, X, ws.scratch(nbytes, m, n, X.device), int(steps), pairs, interleaved)
         _count()
         return X
     A, Bm, Y = ws.get(Bt, m, n, X.device)

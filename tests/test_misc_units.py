@@ -113,6 +113,31 @@ def test_symmetric_heap_guard_zones_catch_an_overrun():
     assert plain.check_canaries() == []
 
 
+def test_newton_schulz_scratch_is_per_shape_and_given_back(monkeypatch):
+    """Matrices of different shapes never share scratch; an outgrown buffer is freed unless a CUDA graph may still use it."""
+    import weakref
+
+    from himuon_b200.ops.ns import NSWorkspace
+
+    capturing = False
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: capturing)
+    ws, cpu = NSWorkspace(), torch.device("cpu")
+    a, b = ws.scratch(256, 512, 512, cpu), ws.scratch(256, 512, 256, cpu)
+    assert a.data_ptr() != b.data_ptr() and ws.scratch(128, 512, 512, cpu) is a
+    gone = weakref.ref(a)
+    del a
+    held = ws.scratch(512, 512, 512, cpu)
+    assert gone() is None and held.numel() == 512
+    capturing = True
+    ws.scratch(512, 512, 512, cpu)
+    capturing = False
+    ref = weakref.ref(held)
+    del held
+    assert ws.scratch(1024, 512, 512, cpu).numel() == 1024 and ref() is not None
+    ws.clear()
+    assert ref() is None and not ws.flat
+
+
 def test_phase_timer_is_inert_without_cuda_and_ranges_nest():
     from himuon_b200.utils import PhaseTimer, nvtx_range
 

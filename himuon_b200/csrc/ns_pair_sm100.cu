@@ -16,7 +16,8 @@
 //
 // Tasks of different pairs, and of the two CTAs of a pair, hand on through `done` barriers: behind its outputs' completion
 // (cp.async.bulk.wait_group, then a fence of the cluster) a CTA arrives on the barrier of that task in every CTA of the cluster,
-// and whoever loads the block waits there.  Between a block and its first reader lies at least one other task and a half, in
+// and whoever loads the block waits there, with a proxy fence between the wait and the TMA loads (aux values are a CTA's
+// own stores, which one proxy orders).  Between a block and its first reader lies at least one other task and a half, in
 // which its drain, store and hand-on (4000-7000 cycles) are hidden but for 1000-2000; with one matrix block per phase
 // (short and long side up to 256) a pair interleaves up to four matrices instead.
 // What is overwritten: a buffer's readers are loads of earlier tasks, whose products a pair issues in order, and with
@@ -297,7 +298,6 @@ ns_pair_kernel(const __grid_constant__ NsPairMaps maps, const __grid_constant__ 
         return o;
       };
       for (int kc = 0; kc * 4 < nk; ++kc) {
-        waited = false;
         const int kb0 = kc * 4, kb1 = min(nk, kb0 + 4);
         NsOperand oa, ob;
         if (t.phase == 0) {
@@ -317,6 +317,8 @@ ns_pair_kernel(const __grid_constant__ NsPairMaps maps, const __grid_constant__ 
           if (!TALL) { oa = a_op(bb, kc > t.i, ri, kb0); ob = x_op(true, rj, kb0); }
           else { oa = x_op(false, rj, kb0); ob = a_op(bb, kc > t.i, ri, kb0); }
         }
+        if (waited) fence_proxy_async_global();       // what the waits have shown, for the loads that follow
+        waited = false;
         for (int kb = kb0; kb < kb1; ++kb) {
           if (!ok || !mbar_wait_warp(&empty[stage], phase ^ 1, abort_flag, p.status, 5)) return ok = false;
           uint8_t* sA = smem + stage * NSP_STAGE;

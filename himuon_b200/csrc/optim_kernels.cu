@@ -624,7 +624,9 @@ adamw_multi_kernel(const AdamEntry* __restrict__ entries, int n_entries, long lo
         for (int q = 0; q < VN; ++q) {
           mf[q] = mf[q] + (gf[q] - mf[q]) * (1.f - b1);
           vf[q] = vf[q] + (gf[q] * gf[q] - vf[q]) * (1.f - b2);
-          if (sizeof(S) == 2) round_bf16x2(mf[q], vf[q]);
+          // (one at a time here: pairs gain 1-3 % on an embedding alone, 866 -> 843 us for 389 M elements, and lose 2 % on 60 matrices
+          // of 1024 x 1024, 156 -> 160)
+          if (sizeof(S) == 2) { mf[q] = round_bf16(mf[q]); vf[q] = round_bf16(vf[q]); }
           pf[q] = adam_apply(mode, pf[q], mf[q], vf[q], lr, wd, eps, bc1, bc2);
         }
         *reinterpret_cast<uint4*>(m + i) = Vec16<S>::pack(mf);

@@ -467,6 +467,25 @@ def test_attention_narrow_heads(D, B, S, Hq, Hkv):
             _close(t.grad, r.grad.reshape(t.shape), atol=3e-2, rtol=3e-2)
 
 
+@pytest.mark.parametrize("D", [40, 64, 96, 128])
+@pytest.mark.parametrize("S", [1, 33, 64, 65, 128, 129, 192, 193])
+def test_attention_of_a_prefix_has_the_same_bits(S, D):
+    """A causal row does not see what follows it: the first S rows of 256 are those of the prefix alone, whatever rows the
+    prefix's last tile holds (its epilogue depends on them)."""
+    e = _ext()
+    torch.manual_seed(S + D)
+    H, whole = 3, 256
+    q, k, v = (torch.randn(whole, H * D, device="cuda", dtype=torch.bfloat16) for _ in range(3))
+    outs = []
+    for n in (whole, S):
+        o, lse = torch.full((n + 1, H * D), 7.0, device="cuda", dtype=torch.bfloat16), torch.empty(H, n, device="cuda")
+        e.flash_attn_fwd(q[:n], k[:n], v[:n], o, lse, 1, n, H, H, D ** -0.5)
+        assert (o[n] == 7.0).all()                         # nothing past the last row
+        outs.append((o[:S], lse[:, :S]))
+    _assert_status_clean()
+    assert torch.equal(outs[0][0], outs[1][0]) and torch.equal(outs[0][1], outs[1][1])
+
+
 @pytest.mark.parametrize("D", [8, 40, 64, 72, 128])
 @pytest.mark.parametrize("B,S,Hq,Hkv", [(1, 1, 1, 1), (2, 64, 2, 2), (1, 129, 4, 2), (2, 333, 2, 1)])
 def test_attention_backward_sums_delta_in_column_order(D, B, S, Hq, Hkv):

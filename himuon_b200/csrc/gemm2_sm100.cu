@@ -380,7 +380,9 @@ static void launch_gemm2(const GemmArgs& a, cudaStream_t stream) {
 //     384 x 384 x 512 8.6 / 9.3.
 //   * Padding can cost the pairs a round: 384 x 12288 (one round of 144 tiles, two of 96) x 640 11.3 / 12.9, x 1728 17.5 / 23.0;
 //     777 x 5120 x 1024 13.4 / 16.2; 40 of 320 x 320 x 1024 (two rounds, three) 18.8 / 21.1.  Without aux values and with rows of
-//     A along K a fourth more rounds are made up for: 100 of 264 x 264 (five, six) 0.87-0.93 of the one-CTA time.
+//     A along K a fourth more rounds are made up for: 100 of 264 x 264 (five, six) 0.87-0.93 of the one-CTA time.  A third more are
+//     not, on the whole: 150 of 264 x 1024 x 1024 (13, 17) 108 / 115, 60 of 320 x 2048 x 1536 (10, 13) 124 / 132, though 320 x 150000 x 640
+//     (12, 16) 82 / 75.
 //   * The longer a round, the less the pair kernel's epilogue matters.  It reads aux values by threads where the other has them
 //     loaded by TMA ahead of time, and an fp32 tile leaves in twice as many slabs.  Plain bf16 products gain from K = 512 on
 //     (one round 0.92-0.97, several 0.78-0.90 of the one-CTA time).  Two rounds / four rounds, ratio: bf16 with aux K 768

@@ -485,16 +485,21 @@ static int tile_width(const GemmArgs& a) {
 }
 
 // 256-wide tiles without an aux operand that need the longer operand ring: many rounds of tiles with a reduction so long
-// that the main loop, not the epilogue, sets the pace (an fp32 slab takes half the columns, so that line lies lower and the
-// slabs are less of a help), and outputs that leave by plain stores and use no slabs at all.  Measured, three stages and
-// four slabs against four and two: 4096 x 8192 x 512 35.6 / 45.9 us, x 896 56.1 / 56.1, x 1024 62.5 / 57.3, x 1984
-// 110.9 / 98.7; 2048 x 32000 x 1024 118 / 111; fp32 4096 x 8192 x 256 30.5 / 34.4, x 384 38.5 / 37.1, x 1024 70.9 / 67.0.  With
-// few rounds the slabs win at any length: 1895 x 2560 x 1984 (two rounds) 30.7 / 33.4, symmetric 128 x 512 x 512 x 1280 (six)
+// that the main loop, not the epilogue, sets the pace, and outputs that leave by plain stores and use no slabs at all.  The
+// shapes that arrive here are those that pairs_win() declines; measured, four stages and two slabs against three and four:
+//   * batches of at most 128 rows, and matrices that the pairs' tiles would pad: 150 of 264 x 1024 x 1024 107 / 115 us, x 768
+//     88.3 / 88.4, x 504 82 / 83; 320 x 150000 x 1536 146 / 157, x 384 56 / 55; 300 of 100 x 1024 x 2040 237 / 244;
+//   * symmetric products, whose epilogue also writes the mirrored tile: 120 of 1024 x 1024 x 1024 162 / 153, x 1280 183 / 184, x 1536
+//     205 / 211 and 215; 400 of 512 x 512 x 1792 241 / 257;
+//   * fp32, short ones only where M > 128 (an fp32 slab takes half the columns: more stages help earlier, and the pairs have the
+//     longer ones): 4096 x 8192 x 384 39.4 / 42.3, x 504 60.1 / 64.9; 64 of 128 x 4096 x 384 66 / 60, x 504 69 / 66, x 768 86 / 86, x 2040
+//     204 / 209.
+// With few rounds the slabs win at any length: 1895 x 2560 x 1984 (two rounds) 30.7 / 33.4, symmetric 128 x 512 x 512 x 1280 (six)
 // 71.3 / 73.3.
 static bool long_plain(const GemmArgs& a) {
   if (!c_rows_aligned(a)) return true;
   const long long sms = a.max_ctas > 0 ? a.max_ctas : num_sms();
-  return a.K >= (a.out_fp32 ? 384 : 1024) && rounds(tile_count(a, 256), sms) > 6;
+  return a.K >= (a.out_fp32 ? (a.M > BM ? 384 : 768) : (a.symmetric ? 1280 : 1024)) && rounds(tile_count(a, 256), sms) > 6;
 }
 
 void gemm_bf16(const GemmArgs& a, cudaStream_t stream) {

@@ -5,11 +5,12 @@
 //     A = X X^T,   B = c A A + b A,   X' = bf16(B X) + a X          (X with its sides exchanged where it is tall)
 // in tasks of one 256 x 256 block each (tcgen05.mma.cta_group::2, K = 64 a stage).  Of the symmetric products only the blocks
 // on and below the diagonal are computed; the others are read as their transposes, through the operand's major mode, so
-// nothing is mirrored.  Intermediates stay in a scratch of three or four buffers per resident matrix (116 MB for 512 x 512
-// matrices on every pair), which the L2 mostly serves: 148 matrices of 512 x 512 read 244 MB from HBM, 78 of them the input,
-// and write 821 MB, as lines are written back before they are overwritten (of 5.7 GB that pass the L2 in 409 us; the tensor
-// pipe is busy for 69 % of it).  As fifteen GEMM launches the same products stream every intermediate through HBM both ways, and
-// each launch pays its ramp and tail.
+// nothing is mirrored.  Intermediates stay in a scratch of three or four buffers per resident matrix, each of X's padded size
+// (116 MB for 512 x 512 matrices on every pair).  The L2 mostly serves that much: 148 matrices of 512 x 512 read 244 MB from HBM,
+// 78 of them the input, and write 821 MB, as lines are written back before they are overwritten (of 5.7 GB that pass the L2 in
+// 409 us; the tensor pipe is busy for 69 % of it).  Long matrices overflow it, as two of them are resident on a pair: 148 of
+// 256 x 2048 have 465 MB of scratch, tall ones 620 (the GEMM launches 194).  As fifteen GEMM launches the same products stream
+// every intermediate through HBM both ways, and each launch pays its ramp and tail.
 //
 // Scratch layout: chunks of 64 columns, each [rows][64] with its rows one after the other.  A TMA box of it is one run of
 // memory, and the same 128-byte-swizzled shared-memory image serves as K-major and as MN-major operand.

@@ -6,9 +6,9 @@
 // in tasks of one 256 x 256 block each (tcgen05.mma.cta_group::2, K = 64 a stage).  Of the symmetric products only the blocks
 // on and below the diagonal are computed; the others are read as their transposes, through the operand's major mode, so
 // nothing is mirrored.  Intermediates stay in a scratch of three or four buffers per resident matrix, each of X's padded size
-// (116 MB for 512 x 512 matrices on every pair).  The L2 mostly serves that much: 148 matrices of 512 x 512 read 244 MB from HBM,
-// 78 of them the input, and write 821 MB, as lines are written back before they are overwritten (of 5.7 GB that pass the L2 in
-// 409 us; the tensor pipe is busy for 69 % of it).  Long matrices overflow it, as two of them are resident on a pair: 148 of
+// (116 MB for 512 x 512 matrices on every pair).  The L2 mostly serves that much: 512 matrices of 512 x 512 read 850 MB from HBM,
+// 268 of them the input, and write 2.9 GB, as lines are written back before they are overwritten (of 19.5 GB that pass the L2 in
+// 1447 us; the tensor pipe is busy for 70 % of it).  Long matrices overflow it, as two of them are resident on a pair: 148 of
 // 256 x 2048 have 465 MB of scratch, tall ones 620 (the GEMM launches 194).  As fifteen GEMM launches the same products stream
 // every intermediate through HBM both ways, and each launch pays its ramp and tail.
 //

@@ -1204,7 +1204,8 @@ def test_pair_gemm_on_short_reductions(M, N, K, batch, trans_a, trans_b, mode):
 
 # mode, batch, M, N and the shortest reduction that goes to CTA pairs; 16 less does not.  One round of 128 x 256 tiles and
 # several, matrices that barely overflow one row of tiles, ragged rows and columns.
-_PAIR_LINES = [("plain", 1, 1281, 2048, 512), ("plain", 20, 136, 520, 512), ("plain", 100, 264, 264, 512),
+_PAIR_LINES = [("plain", 1, 1281, 2048, 512), ("plain", 20, 136, 520, 512), ("plain", 80, 136, 200, 512),
+               ("plain", 100, 264, 264, 512),
                ("aux", 1, 1281, 4104, 1280), ("aux", 8, 1000, 1032, 1024), ("add", 1, 1281, 4104, 1280), ("add", 8, 1000, 1032, 1024),
                ("fp32", 1, 1281, 4104, 1024), ("fp32", 8, 1000, 1032, 768), ("fp32 add", 8, 1000, 1032, 1536),
                ("add", 1, 1024, 3072, 648), ("fp32 add", 1, 1024, 3072, 1032)]
